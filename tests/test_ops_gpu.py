@@ -12,6 +12,30 @@ def relerr(x, ref):
     return ((x - ref).abs().max() / (ref.abs().max() + 1e-6)).item()
 
 
+# rows of more than 1024 elements take a CTA each: the smallest and largest, a width that fills no whole warp, more rows than CTAs
+@pytest.mark.parametrize("rows,D", [(1, 1032), (5, 8192), (700, 1608), (1300, 2048)])
+@pytest.mark.parametrize("rms", [False, True])
+def test_wide_norm_against_64_bits(rows, D, rms):
+    from cogito_b200.ops import norm as N
+    torch.manual_seed(rows)
+    x, r, dy = (torch.randn(rows, D, device=DEV, dtype=torch.bfloat16) for _ in range(3))
+    g = (torch.randn(D, device=DEV) * 0.1 + 1).bfloat16()
+    b = None if rms else torch.randn(D, device=DEV).bfloat16()
+    y, s, mean, rstd = N.norm_forward_raw(x, g, b, 1e-5, rms, r, True)
+    assert torch.equal(s, (x.float() + r.float()).bfloat16())
+    dx, dg, db = N.norm_backward_raw(dy, s, g, mean, rstd, rms, r)
+    sd, gd = s.double(), g.double()
+    m = 0.0 if rms else sd.mean(-1, keepdim=True)
+    rs = ((sd - m).pow(2).mean(-1, keepdim=True) + 1e-5).rsqrt()
+    h, t = (sd - m) * rs, dy.double() * gd
+    s1 = 0.0 if rms else t.mean(-1, keepdim=True)
+    rel = lambda u, v: ((u.double() - v).norm() / v.norm()).item()
+    # bf16 results of fp32 arithmetic: 2^-9 at most, half that on average; fp32 column sums of `rows` terms
+    assert rel(y, h * gd + (0.0 if rms else b.double())) < 2 ** -9 * 1.1
+    assert rel(dx, rs * (t - s1 - h * (t * h).mean(-1, keepdim=True)) + r.double()) < 2 ** -9 * 1.1
+    assert rel(dg, (dy.double() * h).sum(0)) < 2e-6 and (rms or rel(db, dy.double().sum(0)) < 2e-6)
+
+
 @pytest.mark.parametrize("rows,D", [(64, 768), (33, 128), (1000, 4096), (7, 8)])
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("with_res", [False, True])
