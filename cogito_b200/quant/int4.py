@@ -73,7 +73,10 @@ class Int4Linear(torch.nn.Module):
     # Which tcgen05 kernel multiplies: "wb" keeps the weights as the B operand (converted tile in shared
     # memory, 128 token rows per instruction), "wa" makes them the A operand fed from tensor memory (cost
     # follows the token count; needs group % 128 == 0).  "auto": "wa" up to 32 token rows, where it measured
-    # faster, "wb" above.  Each kernel has its own tile-major copy of the weights, made on first use.
+    # faster, "wb" up to two row tiles, and beyond that (prompts) the weights are dequantised to bf16 once per call for the
+    # dense GEMM: "wb" converts every weight tile again for each row tile (4096 x 22016: 111 us against 116 us at 256 rows,
+    # 180 against 136 us at 512).  Each of the two kernels has its own tile-major copy of the weights, made on first use.
+    DENSE_ROWS = 256
     kernel = os.environ.get("COGITO_INT4_KERNEL", "auto")
 
     def __init__(self, weight: torch.Tensor, bias: torch.Tensor | None = None, group: int = 128):
@@ -115,6 +118,20 @@ class Int4Linear(torch.nn.Module):
         return dequantize_int4(self.packed, self.scales, self.in_features * self.out_features, self.group, dtype) \
             .view(self.in_features, self.out_features)
 
+    def _takes_dense(self, rows: int, splits: int = 0) -> bool:
+        return self.kernel == "auto" and splits == 0 and rows > self.DENSE_ROWS
+
+    def _dense(self, x2, **kw):
+        from ..ops.gemm import gemm
+        return gemm(x2.to(torch.bfloat16).contiguous(), self.dequantized(torch.bfloat16), b_mn=True, bias=self.bias, **kw)
+
+    def forward_f32(self, x: torch.Tensor) -> torch.Tensor:
+        """fp32 result (logits); many rows leave the GEMM in fp32 without a bf16 copy in between."""
+        rows = x.numel() // self.in_features
+        if not x.is_cuda or not self._takes_dense(rows):
+            return self.forward(x).float()
+        return self._dense(x.reshape(rows, self.in_features), out_dtype=torch.float32).view(*x.shape[:-1], self.out_features)
+
     def forward(self, x: torch.Tensor, splits: int = 0, out: torch.Tensor | None = None) -> torch.Tensor:
         """``out``: an optional contiguous [rows, out_features] buffer for the result (bf16 on CUDA),
         e.g. a slot of symmetric memory that a collective kernel reads next."""
@@ -136,9 +153,13 @@ class Int4Linear(torch.nn.Module):
         N, K = self.out_features, self.in_features
         if N % 128 or K % 64 or self.group % 64:
             # shapes the streaming kernel does not cover: dequantise once, then the bf16 GEMM
-            from ..ops.gemm import gemm
-            w = self.dequantized(torch.bfloat16)
-            return done(gemm(x2.to(torch.bfloat16).contiguous(), w, b_mn=True, bias=self.bias))
+            return done(self._dense(x2))
+        if self._takes_dense(M, splits):
+            if out is None:
+                return self._dense(x2).view(*lead, N)
+            if out.dtype != torch.bfloat16 or not out.is_contiguous() or out.numel() != M * N:
+                raise ValueError("out must be a contiguous bf16 [rows, out_features] tensor")
+            return self._dense(x2, out=out.view(M, N)).view(*lead, N)
         x2 = x2.to(torch.bfloat16).contiguous()
         L = _lib.lib()
         # "wa": weights on the M side of the tensor core (needs one scale per k for a 128-feature tile)

@@ -64,6 +64,36 @@ __global__ void int4_dequantize_kernel(const uint8_t* __restrict__ packed, const
   }
 }
 
+// bf16 output, whole groups of a multiple of 8, aligned buffers: eight values (one word, one scale) per thread and step, so
+// that a warp reads 128 and writes 512 consecutive bytes; four steps' loads go out together.  The kernel above stores two
+// bytes at a time.
+__global__ void __launch_bounds__(256)
+int4_dequantize_words_kernel(const uint32_t* __restrict__ packed, const float* __restrict__ scales, long long words, int group, uint4* __restrict__ out) {
+  constexpr int U = 4;
+  for (long long w0 = (long long)blockIdx.x * 256 * U + threadIdx.x; w0 < words; w0 += (long long)gridDim.x * 256 * U) {
+    uint32_t v[U];
+    float sc[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long w = w0 + u * 256;
+      v[u] = w < words ? __ldg(packed + w) : 0u;
+      sc[u] = w < words ? __ldg(scales + w * 8 / group) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long w = w0 + u * 256;
+      if (w >= words) break;
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int q0 = (int)(v[u] << (28 - 8 * j)) >> 28, q1 = (int)(v[u] << (24 - 8 * j)) >> 28;      // sign-extended nibbles 2j, 2j + 1
+        o[j] = pack_bf16x2((float)q0 * sc[u], (float)q1 * sc[u]);
+      }
+      out[w] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+  }
+}
+
 // ------------------------------------------------------------ KV cache (A3)
 // The pool layout and the KvDev view are in kv_dev.cuh.
 // k_new / v_new: bf16 [batch, T, heads, D]; token t of sequence b lands at position lengths[b] + t.
@@ -522,6 +552,12 @@ CGK_API int cgk_int4_quantize(const float* x, long long n, int group, void* pack
 }
 CGK_API int cgk_int4_dequantize(const void* packed, const float* scales, long long n, int group, float* out_f32, void* out_bf16, void* stream) {
   CGK_REQUIRE(packed && scales && n > 0 && group > 0 && (out_f32 || out_bf16), "cgk_int4_dequantize: bad argument");
+  if (!out_f32 && n % 8 == 0 && group % 8 == 0 && (((uintptr_t)packed) & 3) == 0 && (((uintptr_t)out_bf16) & 15) == 0) {
+    const long long words = n / 8, need = (words + 1023) / 1024;
+    int4_dequantize_words_kernel<<<(unsigned)(need < 148 * 8 ? need : 148 * 8), 256, 0, (cudaStream_t)stream>>>((const uint32_t*)packed, scales, words, group, (uint4*)out_bf16);
+    CGK_LAUNCH_CHECK();
+    return 0;
+  }
   const long long bytes = (n + 1) / 2;
   const int blocks = (int)((bytes + 255) / 256 < 2368 ? (bytes + 255) / 256 : 2368);
   int4_dequantize_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const uint8_t*)packed, scales, n, group, out_f32, (__nv_bfloat16*)out_bf16);

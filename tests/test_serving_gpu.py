@@ -45,6 +45,25 @@ def test_int4_gemm_matches_dequantised_product(M, K, N, group, splits, kernel):
     _lib.assert_device_ok()
 
 
+@pytest.mark.parametrize("n,group", [(8, 8), (1024, 32), (8 * 1031, 8), (128 * 999, 128), (24 * 100, 24)])
+def test_int4_dequantize_by_words(n, group):
+    p, s = quantize_int4(torch.randn(n), group)
+    got = dequantize_int4(p.to(DEV), s.to(DEV), n, group, torch.bfloat16).cpu()
+    assert torch.equal(got, dequantize_int4(p, s, n, group).bfloat16())
+
+
+@pytest.mark.parametrize("rows", [258, 513])
+def test_int4_linear_many_rows_goes_through_the_dense_product(rows):
+    torch.manual_seed(rows)
+    lin = Int4Linear(torch.randn(384, 256) * 0.05, torch.randn(384) * 0.1, 128).to(DEV)
+    x = torch.randn(3, rows // 3, 256, device=DEV, dtype=torch.bfloat16)
+    ref = (x.double() @ lin.dequantized(torch.bfloat16).double() + lin.bias.double())
+    assert ((lin(x).double() - ref).abs() <= ref.abs() * 2 ** -8 + 1e-4).all()          # bf16 result of fp32 sums
+    assert ((lin.forward_f32(x).double() - ref).abs() <= 256 * 2 ** -24 * 8 + 1e-5).all()   # fp32 sums of 256 products
+    out = torch.empty(x.shape[0] * x.shape[1], 384, device=DEV, dtype=torch.bfloat16)
+    assert lin(x, out=out).data_ptr() == out.data_ptr() and torch.equal(out.view_as(lin(x)), lin(x))
+
+
 @pytest.mark.parametrize("D,group,Hk,Hq,Tq", [(128, 32, 2, 8, 5), (64, 16, 1, 4, 1), (128, 128, 2, 2, 3),
                                                  (128, 64, 2, 16, 5), (128, 32, 1, 4, 40), (128, 16, 1, 2, 2)])
 def test_kv_append_and_attention_match_host(D, group, Hk, Hq, Tq):
