@@ -100,6 +100,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "cgk_int4_wa_gemm": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
         "cgk_int4_wa_tile_weights": [vp, vp, i, i, i, vp, vp],
         "cgk_kv_int4_append": [vp, vp, vp, i, vp],
+        "cgk_kv_int4_append_rows": [vp, vp, vp, ll, ll, ll, i, vp, vp, vp],
         "cgk_kv_int4_attention": [vp, vp, vp, i, i, f, i, vp, vp],
         "cgk_sample": [vp, i, ll, i, i, f, i, f, c_ulonglong, vp, vp, vp, vp],
         "cgk_spec_accept": [vp, vp, vp, i, i, i, c_ulonglong, vp, vp, vp, vp, vp, vp],

@@ -201,11 +201,14 @@ class LlamaInt4Engine:
         for i, l in enumerate(self.layers):
             qkv = l["qkv"](h).view(B, Tq, Hq + 2 * Hk, D)
             M.rope_apply_(qkv[:, :, :Hq + Hk], self.rope[0], self.rope[1], positions=positions)
-            self.cache.append(i, qkv[:, :, Hq:Hq + Hk], qkv[:, :, Hq + Hk:])
+            k, v = qkv[:, :, Hq:Hq + Hk], qkv[:, :, Hq + Hk:]
+            kept = self.cache.append_rows(i, k, v, want=fresh)
+            if kept is None:
+                self.cache.append(i, k, v)
             if fresh:
                 # prompt over an empty cache: causal flash attention over the values the cache now
                 # holds (K and V pass through the same quantise / dequantise), no history to stream
-                kq, vq = (self._fake_quant(qkv[:, :, a:a + Hk]) for a in (Hq, Hq + Hk))
+                kq, vq = kept if kept is not None else (self._fake_quant(t) for t in (k, v))
                 o = flash_forward(qkv[:, :, :Hq], kq, vq, causal=True)[0]
             else:
                 o = self.cache.attention(i, qkv[:, :, :Hq].contiguous())

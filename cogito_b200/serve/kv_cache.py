@@ -157,6 +157,22 @@ class PagedKVCacheInt4(PagedCache):
                     pages[page, pos % self.page_size] = packed[b, t]
                     scales[page, pos % self.page_size] = s[b, t]
 
+    def append_rows(self, layer: int, k_new: torch.Tensor, v_new: torch.Tensor, want: bool = False):
+        """``append`` of slices of one packed projection, read where they lie; with ``want`` returns (k, v) as the cache now holds
+        them ([batch, T, heads, D] bf16).  None: not these rows (the caller appends them the general way)."""
+        B, T, H, D = k_new.shape
+        lanes = self.group // 8
+        if not (k_new.is_cuda and k_new.dtype == v_new.dtype == torch.bfloat16 and k_new.stride() == v_new.stride() and k_new.stride(3) == 1
+                and (B, H, D) == (self.batch, self.heads, self.D) and v_new.shape == k_new.shape and lanes & (lanes - 1) == 0
+                and all(s % 8 == 0 for s in k_new.stride()[:3]) and k_new.data_ptr() % 16 == 0 and v_new.data_ptr() % 16 == 0):
+            return None
+        out = [torch.empty(B, T, H, D, dtype=torch.bfloat16, device=k_new.device) if want else None for _ in range(2)]
+        a = self._args(layer)
+        _lib.check(_lib.lib().cgk_kv_int4_append_rows(ctypes.byref(a), k_new.data_ptr(), v_new.data_ptr(), k_new.stride(0), k_new.stride(1), k_new.stride(2),
+                                                      T, _lib.ptr(out[0]), _lib.ptr(out[1]), _lib.stream_ptr()), "cgk_kv_int4_append_rows")
+        _lib.count_launch()
+        return out
+
     # -------------------------------------------------------------------- read
     def gather(self, layer: int, b: int, length: int):
         """Dequantised (k, v) [length, heads, D] of one sequence (fp32)."""

@@ -126,6 +126,53 @@ __global__ void kv_append_kernel(KvDev c, const __nv_bfloat16* __restrict__ k_ne
   }
 }
 
+// The same for strided rows (slices of the packed projection), eight elements per thread: a group's lanes meet in shuffles, and
+// a group of 32 is read, reduced, quantised and written in one go instead of by one warp in four rounds of two-byte loads.
+// k_out / v_out (optional, [batch, T, heads, D]): the values the cache now holds, which a prompt's attention reads.
+struct KvRows { const __nv_bfloat16* src[2]; __nv_bfloat16* out[2]; long long bs, ts, hs; };
+__global__ void __launch_bounds__(256)
+kv_append_rows_kernel(KvDev c, const KvRows r, int T, int group_lanes, int* status) {
+  const int which = blockIdx.y, upr = c.D >> 3;                       // units of eight elements per row
+  const long long units = (long long)c.batch * T * c.heads * upr;
+  const long long u = (long long)blockIdx.x * 256 + threadIdx.x;
+  const bool in = u < units;
+  const int d = (int)(u % upr) * 8;
+  const long long row = u / upr;
+  const int h = (int)(row % c.heads), bt = (int)(row / c.heads), t = bt % T, b = in ? bt / T : 0;
+  float x[8];
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if (in) v = *reinterpret_cast<const uint4*>(r.src[which] + b * r.bs + t * r.ts + h * r.hs + d);
+  float2 f;
+  f = unpack_bf16x2(v.x); x[0] = f.x; x[1] = f.y;
+  f = unpack_bf16x2(v.y); x[2] = f.x; x[3] = f.y;
+  f = unpack_bf16x2(v.z); x[4] = f.x; x[5] = f.y;
+  f = unpack_bf16x2(v.w); x[6] = f.x; x[7] = f.y;
+  float m = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) m = fmaxf(m, fabsf(x[j]));
+  for (int o = group_lanes >> 1; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (!in) return;
+  const float s = m < 1e-10f ? 1.0f : m / 7.0f;
+  uint32_t packed = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int q = max(-8, min(7, (int)roundf(x[j] / s)));
+    packed |= (uint32_t)(q & 0xF) << (4 * j);
+    x[j] = q * s;
+  }
+  if (r.out[which]) {
+    uint4 o;
+    o.x = pack_bf16x2(x[0], x[1]); o.y = pack_bf16x2(x[2], x[3]); o.z = pack_bf16x2(x[4], x[5]); o.w = pack_bf16x2(x[6], x[7]);
+    *reinterpret_cast<uint4*>(r.out[which] + row * c.D + d) = o;
+  }
+  const int pos = c.lengths[b] + t, lp = pos / c.page_size;
+  if (lp >= c.max_pages) { report_status(status, KST_BAD_ARG, 400, pos); return; }
+  const int page = c.page_table[CGK_IDX(b * c.max_pages + lp, c.batch * c.max_pages)];
+  const long long tok = ((long long)page * c.page_size + pos % c.page_size) * c.heads + h;
+  *reinterpret_cast<uint32_t*>((which ? c.v_pages : c.k_pages) + tok * (c.D / 2) + d / 2) = packed;
+  if (d % c.group == 0) (which ? c.v_scales : c.k_scales)[tok * (c.D / c.group) + d / c.group] = s;
+}
+
 // Attention of R = Tq * (Hq / Hk) query rows per (sequence, kv head) over the quantised
 // history, split along the keys.  Each lane scores one key (its bytes are read once and
 // dequantised in registers), the warp keeps an online softmax per row, then the lanes switch
@@ -580,6 +627,24 @@ CGK_API int cgk_kv_int4_append(const cgk_kv_args* a, const void* k_new, const vo
   CGK_CUDA_CHECK(cudaGetDevice(&dev));
   const int warps = a->batch * T * a->heads;
   kv_append_kernel<<<(warps + 7) / 8, 256, 0, (cudaStream_t)stream>>>(kv_dev(a), (const __nv_bfloat16*)k_new, (const __nv_bfloat16*)v_new, T, device_status(dev));
+  CGK_LAUNCH_CHECK();
+  return 0;
+}
+// k_new / v_new: rows of D contiguous elements at b * bs + t * ts + h * hs (elements, multiples of 8, 16-byte aligned bases);
+// k_out / v_out: both or neither.  The quantisation group is 8 times a power of two.
+CGK_API int cgk_kv_int4_append_rows(const cgk_kv_args* a, const void* k_new, const void* v_new, long long bs, long long ts, long long hs, int T,
+                                    void* k_out, void* v_out, void* stream) {
+  if (int rc = check_kv(a, "cgk_kv_int4_append_rows")) return rc;
+  CGK_REQUIRE(k_new && v_new && T > 0 && !k_out == !v_out, "cgk_kv_int4_append_rows: bad argument");
+  const int gl = a->group / 8;
+  CGK_REQUIRE((gl & (gl - 1)) == 0, "cgk_kv_int4_append_rows: group %d must be 8 times a power of two", a->group);
+  CGK_REQUIRE(((bs | ts | hs) & 7) == 0 && (((uintptr_t)k_new | (uintptr_t)v_new | (uintptr_t)k_out | (uintptr_t)v_out) & 15) == 0 &&
+              (((uintptr_t)a->k_pages | (uintptr_t)a->v_pages) & 3) == 0, "cgk_kv_int4_append_rows: misaligned rows");
+  int dev = 0;
+  CGK_CUDA_CHECK(cudaGetDevice(&dev));
+  const long long units = (long long)a->batch * T * a->heads * (a->D / 8);
+  const KvRows r{{(const __nv_bfloat16*)k_new, (const __nv_bfloat16*)v_new}, {(__nv_bfloat16*)k_out, (__nv_bfloat16*)v_out}, bs, ts, hs};
+  kv_append_rows_kernel<<<dim3((unsigned)((units + 255) / 256), 2), 256, 0, (cudaStream_t)stream>>>(kv_dev(a), r, T, gl, device_status(dev));
   CGK_LAUNCH_CHECK();
   return 0;
 }

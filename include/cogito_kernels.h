@@ -242,6 +242,9 @@ typedef struct {
 /* k_new, v_new: bf16 [batch, T, heads, D]; written at positions lengths[b] .. lengths[b]+T-1
  * (lengths is not changed: cgk_spec_accept or the caller commits). */
 int cgk_kv_int4_append(const cgk_kv_args* a, const void* k_new, const void* v_new, int T, void* stream);
+// strided rows; k_out / v_out (optional): the values the cache now holds
+int cgk_kv_int4_append_rows(const cgk_kv_args* a, const void* k_new, const void* v_new, long long bs, long long ts, long long hs, int T,
+                            void* k_out, void* v_out, void* stream);
 long long cgk_kv_int4_attention_scratch_floats(int batch, int Hq, int Tq, int D, int splits);
 /* q, out: bf16 [batch, Tq, Hq, D]; the Tq newest tokens are already in the cache; query t sees
  * keys 0 .. lengths[b] + t.  Hq a multiple of heads (grouped-query attention). */

@@ -88,6 +88,29 @@ def test_kv_append_and_attention_match_host(D, group, Hk, Hq, Tq):
     _lib.assert_device_ok()
 
 
+@pytest.mark.parametrize("D,group,Hk,T", [(128, 32, 2, 5), (64, 8, 3, 1), (128, 128, 1, 7), (64, 16, 1, 3), (64, 64, 5, 9)])
+def test_kv_append_of_strided_rows(D, group, Hk, T):
+    torch.manual_seed(D + T)
+    B = 3
+    one, two = (PagedKVCacheInt4(1, B, 64, Hk, D, group, page_size=16, device=DEV) for _ in range(2))
+    lengths = torch.tensor([0, 11, 30], dtype=torch.int32, device=DEV)
+    for c in (one, two):
+        c.commit(lengths)
+    qkv = torch.randn(B, T, 2 * Hk + 4, D, device=DEV).bfloat16()
+    qkv[0, 0, 4] = 0.0                                         # a group of zeros has scale 1
+    k, v = qkv[:, :, 4:4 + Hk], qkv[:, :, 4 + Hk:]
+    one.append(0, k, v)
+    kept = two.append_rows(0, k, v, want=True)
+    for x, y in zip((one.k_pages, one.v_pages, one.k_scales, one.v_scales), (two.k_pages, two.v_pages, two.k_scales, two.v_scales)):
+        assert torch.equal(x[0], y[0])
+    for b in range(B):
+        held = two.gather(0, b, int(lengths[b]) + T)
+        for h, kt in zip(held, kept):
+            assert torch.equal(h[int(lengths[b]):].bfloat16(), kt[b])
+    assert two.append_rows(0, k[..., ::2], v[..., ::2]) is None
+    _lib.assert_device_ok()
+
+
 def test_kv_attention_long_history_many_key_blocks():
     torch.manual_seed(3)
     B, hist, Hk, Hq, D, Tq = 2, 700, 2, 8, 128, 5
