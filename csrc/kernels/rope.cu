@@ -61,6 +61,37 @@ __global__ void rope_apply_kernel(T* x, const float* __restrict__ cos_t, const f
   }
 }
 
+// bf16 rows whose halves are multiples of 8 elements on 16-byte boundaries: eight pairs per thread, two 16-byte loads and stores, and
+// the row's index worked out once (three 64-bit divisions per pair of elements bound the kernel above).
+__global__ void __launch_bounds__(256)
+rope_apply_vec_kernel(__nv_bfloat16* x, const float* __restrict__ cos_t, const float* __restrict__ sin_t, const int* __restrict__ positions,
+                      int units, int Tn, int H, int half, long long bs, long long ts, long long hs, int pos_offset, int max_seq, float sign) {
+  const int u = blockIdx.x * 256 + threadIdx.x;
+  if (u >= units) return;
+  const int upr = half >> 3, row = u / upr, j = (u - row * upr) * 8, bt = row / H, h = row - bt * H, b = bt / Tn, t = bt - b * Tn;
+  int pos = positions ? positions[bt] : pos_offset + t;
+  if (pos < 0) pos = 0;
+  if (pos >= max_seq) pos = max_seq - 1;
+  const float4* cp = reinterpret_cast<const float4*>(cos_t + (long long)pos * half + j);
+  const float4* sp = reinterpret_cast<const float4*>(sin_t + (long long)pos * half + j);
+  const float4 c0 = __ldg(cp), c1 = __ldg(cp + 1), s0 = __ldg(sp), s1 = __ldg(sp + 1);
+  __nv_bfloat16* p = x + b * bs + t * ts + h * hs + j;
+  const uint4 lo = *reinterpret_cast<const uint4*>(p), hi = *reinterpret_cast<const uint4*>(p + half);
+  const uint32_t lw[4] = {lo.x, lo.y, lo.z, lo.w}, hw[4] = {hi.x, hi.y, hi.z, hi.w};
+  const float cs[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+  const float sn[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+  uint32_t lr[4], hr[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float2 a = unpack_bf16x2(lw[e]), bb = unpack_bf16x2(hw[e]);
+    const float ca = cs[2 * e], cb = cs[2 * e + 1], sa = sign * sn[2 * e], sb = sign * sn[2 * e + 1];
+    lr[e] = pack_bf16x2(a.x * ca - bb.x * sa, a.y * cb - bb.y * sb);
+    hr[e] = pack_bf16x2(bb.x * ca + a.x * sa, bb.y * cb + a.y * sb);
+  }
+  *reinterpret_cast<uint4*>(p) = make_uint4(lr[0], lr[1], lr[2], lr[3]);
+  *reinterpret_cast<uint4*>(p + half) = make_uint4(hr[0], hr[1], hr[2], hr[3]);
+}
+
 }  // namespace cgk
 
 using namespace cgk;
@@ -88,6 +119,13 @@ CGK_API int cgk_rope_apply(int dtype, void* x, const float* cos_t, const float* 
   long long blocks = (n + 255) / 256, cap = (long long)sm_count(dev) * 16;
   if (blocks > cap) blocks = cap;
   const float sign = backward ? -1.0f : 1.0f;
+  if (dtype != 0 && D % 16 == 0 && ((bs | ts | hs) & 7) == 0 && n / 8 <= 0x7fffff00LL &&
+      (((uintptr_t)x | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15) == 0) {
+    rope_apply_vec_kernel<<<(unsigned)((n / 8 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        (__nv_bfloat16*)x, cos_t, sin_t, positions, (int)(n / 8), T, H, D / 2, bs, ts, hs, pos_offset, max_seq, sign);
+    CGK_LAUNCH_CHECK();
+    return 0;
+  }
   if (dtype == 0)
     rope_apply_kernel<float><<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(
         (float*)x, cos_t, sin_t, positions, B, T, H, D, bs, ts, hs, pos_offset, max_seq, sign);

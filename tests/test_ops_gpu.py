@@ -12,6 +12,22 @@ def relerr(x, ref):
     return ((x - ref).abs().max() / (ref.abs().max() + 1e-6)).item()
 
 
+@pytest.mark.parametrize("B,T,H,D", [(1, 1, 1, 16), (3, 7, 5, 64), (2, 33, 3, 128), (1, 5, 2, 48)])
+@pytest.mark.parametrize("backward", [False, True])
+def test_rope_by_eight_pairs(B, T, H, D, backward):
+    from cogito_b200.ops import misc as M
+    torch.manual_seed(T)
+    cos, sin = M.rope_tables(40, D, 10000.0, DEV)
+    packed = torch.randn(B, T, H + 2, D, device=DEV, dtype=torch.bfloat16)
+    pos = torch.randint(-2, 45, (B, T), dtype=torch.int32, device=DEV)                   # clamped to the table
+    for how in ({"pos_offset": 4}, {"positions": pos}):
+        got, ref = packed.clone(), packed.cpu()
+        M.rope_apply_(got[:, :, 1:1 + H], cos, sin, backward=backward, **how)
+        how = {k: v.cpu() if isinstance(v, torch.Tensor) else v for k, v in how.items()}
+        M.rope_apply_(ref[:, :, 1:1 + H], cos.cpu(), sin.cpu(), backward=backward, **how)
+        assert relerr(got, ref) < 2 ** -8 and torch.equal(got[:, :, 0].cpu(), packed[:, :, 0].cpu()) and torch.equal(got[:, :, -1].cpu(), packed[:, :, -1].cpu())
+
+
 # rows of more than 1024 elements take a CTA each: the smallest and largest, a width that fills no whole warp, more rows than CTAs
 @pytest.mark.parametrize("rows,D", [(1, 1032), (5, 8192), (700, 1608), (1300, 2048)])
 @pytest.mark.parametrize("rms", [False, True])
