@@ -72,7 +72,7 @@ class Int4Linear(torch.nn.Module):
 
     # Which tcgen05 kernel multiplies: "wb" keeps the weights as the B operand (converted tile in shared
     # memory, 128 token rows per instruction), "wa" makes them the A operand fed from tensor memory (cost
-    # follows the token count; needs group % 128 == 0).  "auto": "wa" up to 32 token rows, where it measured
+    # follows the token count; needs group % 128 == 0).  "auto": "wa" up to 16 token rows, where it measured
     # faster, "wb" up to two row tiles, and beyond that (prompts) the weights are dequantised to bf16 once per call for the
     # dense GEMM: "wb" converts every weight tile again for each row tile (4096 x 22016: 111 us against 116 us at 256 rows,
     # 180 against 136 us at 512).  Each of the two kernels has its own tile-major copy of the weights, made on first use.
@@ -163,7 +163,7 @@ class Int4Linear(torch.nn.Module):
         x2 = x2.to(torch.bfloat16).contiguous()
         L = _lib.lib()
         # "wa": weights on the M side of the tensor core (needs one scale per k for a 128-feature tile)
-        wa = (self.kernel == "wa" or (self.kernel == "auto" and M <= 32)) and self.group % 128 == 0 and K % 128 == 0
+        wa = (self.kernel == "wa" or (self.kernel == "auto" and M <= 16)) and self.group % 128 == 0 and K % 128 == 0
         tiles = self._tiles.get(wa)
         if tiles is None or tiles.device != x2.device:
             # one-time tile-major reordering of the same quantised values

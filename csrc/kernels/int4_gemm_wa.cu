@@ -31,9 +31,16 @@
 //
 // One step = 128 k.  Thread (warp w, lane l): feature 32 (w % 4) + l, 64-k block w / 4 of the step:
 // two 16-byte units of nibbles -> 32 TMEM columns; and the X chunks (token row, 8 k) number
-// tid, tid + 256, ... of the step.  Split-K: partial sums go to an fp32 buffer with red.add; the CTA
-// that arrives last at the tile's counter adds the bias, writes bf16 and leaves buffer and counter
-// zeroed.
+// tid, tid + 256, ... of the step.
+//
+// Work is dealt out by steps, not by tiles: the steps of all feature tiles are one line (which is also how the stream lies in
+// memory) and every resident CTA takes an equal piece of it, so that no SM has two tiles while its neighbour has one, and a
+// K of 11 008 (86 steps, whose only power-of-two divisor is 2) fills the machine like any other.  A piece covers the end of
+// one tile and the start of the next; a tile covered by one CTA is written at once, the parts of the others go to an fp32
+// buffer with red.add, and the CTA that arrives last at the tile's counter adds the bias, writes bf16 and leaves buffer and
+// counter zeroed.  The MMA warp runs its loop converged (see umma_f16_lane): eight MMAs of 16 columns a step are few tensor
+// cycles, and issuing them from a one-lane branch took longer than the step's conversion.  16 rows, device time: 11008 x 4096
+// 47.8 -> about 25 us, 4096 x 22016 44.5 -> 38 us.
 #include <cuda_bf16.h>
 
 #include "host_common.h"
@@ -59,7 +66,6 @@ struct WaDev {
   __nv_bfloat16* out; long long ldo;
   const __nv_bfloat16* bias;
   int M, N, K;
-  int splits, ksteps;              // 128-k steps per CTA
   int x_rows;                      // token columns of the MMA: round_up(min(M, 128), 16)
   int* status;
 };
@@ -69,6 +75,56 @@ __device__ __forceinline__ uint4 ldg_stream_16(const void* p) {     // read once
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
+}
+
+// A part's accumulator (warps 0-3): lane = output feature, column = token.  whole: the part is the tile.
+__device__ __noinline__ void wa_store_part(const WaDev& g, uint32_t tmem, int x_rows, int m0, int nt, const float* xsum_s, bool whole,
+                                           uint32_t acc_full, uint32_t parity, volatile int* dead, bool ok) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp >= 4 || !__all_sync(0xffffffffu, ok && mbar_wait(acc_full, parity, dead, g.status, 331))) return;
+  tc_fence_after();
+  const int fo = nt * WF + warp * 32 + lane;
+  const float bias = (g.bias && whole) ? __bfloat162float(g.bias[fo]) : 0.0f;
+#pragma unroll 1
+  for (int c = 0; c < x_rows; c += 16) {
+    uint32_t rr[16];
+    __syncwarp();
+    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c, rr);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int t = m0 + c + j;
+      if (t < g.M) {
+        const float v = __uint_as_float(rr[j]) - 136.0f * xsum_s[c + j];
+        if (whole) g.out[(long long)t * g.ldo + fo] = __float2bfloat16(v + bias);
+        else atomicAdd(g.acc + (long long)t * g.N + fo, v);
+      }
+    }
+  }
+  if (!whole) __threadfence();
+}
+
+// Counts a finished part of a tile that `others` + 1 CTAs share; the last one writes the output.  All conversion threads.
+__device__ __noinline__ void wa_finish_tile(const WaDev& g, int m0, int mt, int nt, int others, volatile int* is_last, volatile int* dead) {
+  const int tid = threadIdx.x, n0 = nt * WF;
+  int* counter = g.counters + mt * (g.N / WF) + nt;
+  if (tid == 0) *is_last = (atomicAdd(counter, 1) == others) && !*dead;
+  asm volatile("bar.sync 1, 256;" ::: "memory");
+  if (!*is_last) return;
+  __threadfence();
+  const int rows = min(128, g.M - m0);
+  for (int i = tid; i < rows * (WF / 4); i += W_CONV_THREADS) {
+    const int t = i / (WF / 4), c4 = (i % (WF / 4)) * 4;
+    float4* src = reinterpret_cast<float4*>(g.acc + (long long)(m0 + t) * g.N + n0 + c4);
+    float4 v = __ldcg(src);
+    *src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (g.bias) {
+      v.x += __bfloat162float(g.bias[n0 + c4]); v.y += __bfloat162float(g.bias[n0 + c4 + 1]);
+      v.z += __bfloat162float(g.bias[n0 + c4 + 2]); v.w += __bfloat162float(g.bias[n0 + c4 + 3]);
+    }
+    *reinterpret_cast<uint2*>(g.out + (long long)(m0 + t) * g.ldo + n0 + c4) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+  }
+  if (tid == 0) *counter = 0;
 }
 
 template <int NCH>                   // X chunks per thread and step (x_rows * 16 / 256, rounded up)
@@ -91,11 +147,11 @@ int4_wa_kernel(const WaDev g) {
   auto a_empty = [&](int s) { return sBar + 8u * (W_STAGES + s); };
   const uint32_t acc_full = sBar + 8u * 2 * W_STAGES;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_tiles = g.N / WF, k_tiles = g.K / (WSUB * WK);
-  const int nt = blockIdx.x % n_tiles, split = blockIdx.x / n_tiles, mt = blockIdx.y;
-  const int n0 = nt * WF, ks0 = split * g.ksteps, m0 = mt * 128, ksteps = g.ksteps;
-  const uint8_t* stream = g.tiles + ((long long)nt * k_tiles + ks0) * W_STEP;        // this CTA's slab, W_STEP bytes a step
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int n_tiles = g.N / WF, k_tiles = g.K / (WSUB * WK), mt = blockIdx.y, m0 = mt * 128;
+  const long long total = (long long)n_tiles * k_tiles, ctas = gridDim.x;
+  const long long u0 = total * blockIdx.x / ctas;                    // this CTA's steps: [u0, u0 + steps)
+  const int steps = (int)(total * (blockIdx.x + 1) / ctas - u0);
   const uint32_t acc_cols = x_rows <= 32 ? 32u : x_rows <= 64 ? 64u : 128u;
   const uint32_t tmem_cols = acc_cols + W_STAGES * W_ACOLS <= 256 ? 256u : 512u;     // accumulator, then the operand stages
 
@@ -106,55 +162,71 @@ int4_wa_kernel(const WaDev g) {
     *is_last = 0;
     mbar_fence_init();
   }
+  for (int i = tid; i < 128; i += W_THREADS) xsum_s[i] = 0.0f;
   if (warp == 0) { tmem_alloc(smem_u32(tmem_slot), tmem_cols); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot, tmem_a = tmem + acc_cols;
-  // X chunk c = tid + 256 j: block (c / 8) / x_rows, token row (c / 8) % x_rows, piece c % 8 (k = 8 (c % 8) ..)
-  const int ch = tid & 7;
-  const int chunks = WSUB * x_rows * 8;                              // per step
-  float xs[NCH];
-#pragma unroll
-  for (int j = 0; j < NCH; ++j) xs[j] = 0.0f;
-  bool ok = true;
+  // A part of a tile ends at two barriers of all threads: its row sums are complete and its MMAs issued; its accumulator has
+  // been read.  Both roles pass them for every part, also after a wait that gave up (later waits then return at once).
+  auto part_steps = [&](int i) -> int { return (int)min((long long)(steps - i), k_tiles - (u0 + i) % k_tiles); };
 
   if (warp == W_CONV_THREADS / 32) {
-    // ---- MMA warp: one thread issues; a stage is free again when its MMAs have completed
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc_bf16(WF, x_rows, 0, 0);
-      for (int i = 0; i < ksteps; ++i) {
-        const int s = i % W_STAGES;
-        if (!mbar_wait(a_full(s), (i / W_STAGES) & 1, dead, g.status, 332)) break;
+    // ---- MMA warp: one lane issues; a stage is free again when its MMAs have completed
+    const uint32_t mine = lane == 0, idesc = make_idesc_bf16(WF, x_rows, 0, 0);
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), tm_a = tm + acc_cols;
+    const uint64_t x_desc = make_smem_desc_sw128(sX, 16u, 1024u);
+    bool ok = true;
+    uint32_t s = 0, par = 0;
+    int left = 0;
+    bool first = true;
+    for (int i = 0; i < steps; ++i) {
+      if (left == 0) { left = part_steps(i); first = true; }
+      ok = __all_sync(0xffffffffu, mbar_wait(a_full(s), par, dead, g.status, 332)) && ok;
+      if (ok) {
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < WSUB * WK / 16; ++kk) {
           // 16 k per instruction: 8 TMEM columns of A, 32 bytes along a row of the X' block
-          const uint32_t x_addr = sX + (s * WSUB + kk / (WK / 16)) * x_bytes + (kk % (WK / 16)) * 32;
-          umma_f16_ts(tmem, tmem_a + s * W_ACOLS + kk * 8, make_smem_desc_sw128(x_addr, 16u, 1024u), idesc, (i | kk) != 0 ? 1u : 0u);
+          const uint32_t x_off = (s * WSUB + kk / (WK / 16)) * x_bytes + (kk % (WK / 16)) * 32;
+          umma_f16_ts_lane(mine, tm, tm_a + s * W_ACOLS + kk * 8, x_desc + (x_off >> 4), idesc, (first && kk == 0) ? 0u : 1u);
         }
-        umma_commit(a_empty(s));
-        if (i + 1 == ksteps) umma_commit(acc_full);
+        umma_commit_lane(mine, a_empty(s));
+      }
+      first = false;
+      if (++s == W_STAGES) { s = 0; par ^= 1; }
+      if (--left == 0) {
+        if (ok) umma_commit_lane(mine, acc_full);
+        asm volatile("bar.sync 2, 288;" ::: "memory");
+        asm volatile("bar.sync 2, 288;" ::: "memory");
+        tc_fence_after();
       }
     }
   } else {
     // ---- conversion warps: this thread's share of a step
     const int quad = warp & 3, sub = warp >> 2, f = quad * 32 + lane;
-    const uint8_t* wsrc = stream + sub * W_RAW + f * 16;             // k half 0; half 1 is W_NIB / 2 further
+    // X chunk c = tid + 256 j: block (c / 8) / x_rows, token row (c / 8) % x_rows, piece c % 8 (k = 8 (c % 8) ..)
+    const int ch = tid & 7;
+    const int chunks = WSUB * x_rows * 8;                              // per step
+    const uint8_t* wsrc = g.tiles + u0 * W_STEP + sub * W_RAW + f * 16;   // k half 0; half 1 is W_NIB / 2 further
     constexpr int NB = NCH == 1 ? 1 : WSUB;                          // scale blocks a thread needs (one chunk: one block)
     // Everything that does not change from step to step is worked out once: where each of this thread's
-    // X chunks comes from (advances by 128 elements a step) and where it goes inside a stage's X' tile.
+    // X chunks comes from (128 elements a step, from the start again with the next tile) and where it goes inside a stage's X' tile.
     const __nv_bfloat16* xsrc[NCH];                                   // null: padding row or no chunk
     uint32_t xdst[NCH];
-    int xblk[NCH];
+    int xblk[NCH], xrow[NCH];
+    float xs[NCH];
 #pragma unroll
     for (int j = 0; j < NCH; ++j) {
       const int c = tid + j * W_CONV_THREADS, rowb = c >> 3, blk = rowb / x_rows, t = rowb - blk * x_rows;
       xblk[j] = c < chunks ? blk : -1;
+      xrow[j] = t;
+      xs[j] = 0.0f;
       xdst[j] = (uint32_t)blk * x_bytes + sw128_offset((uint32_t)t, (uint32_t)ch);
-      xsrc[j] = (c < chunks && m0 + t < g.M) ? g.x + (long long)(m0 + t) * g.ldx + ((long long)ks0 * WSUB + blk) * WK + ch * 8 : nullptr;
+      xsrc[j] = (c < chunks && m0 + t < g.M) ? g.x + (long long)(m0 + t) * g.ldx + blk * WK + ch * 8 : nullptr;
     }
-    const uint8_t* ssrc = stream + (NCH == 1 ? (tid >> 3) / x_rows : 0) * W_RAW + W_NIB + ch * 32;
+    const uint8_t* ssrc = g.tiles + u0 * W_STEP + (NCH == 1 ? min((tid >> 3) / x_rows, WSUB - 1) : 0) * W_RAW + W_NIB + ch * 32;
     uint4 raw[W_PREFETCH][2];
     uint4 xr[2][NCH];                                                // X chunks and scales of the next two steps, by step parity
     float4 sc[2][NB][2];
@@ -163,10 +235,12 @@ int4_wa_kernel(const WaDev g) {
       raw[d][0] = ldg_stream_16(p);
       raw[d][1] = ldg_stream_16(p + W_NIB / 2);
     };
+    int kx = (int)(u0 % k_tiles);                                    // step of its tile that load_x fetches next
     auto load_x = [&](int p, int step) {
 #pragma unroll
       for (int j = 0; j < NCH; ++j)
-        xr[p][j] = xsrc[j] ? __ldg(reinterpret_cast<const uint4*>(xsrc[j] + step * (WSUB * WK))) : make_uint4(0, 0, 0, 0);
+        xr[p][j] = xsrc[j] ? __ldg(reinterpret_cast<const uint4*>(xsrc[j] + kx * (WSUB * WK))) : make_uint4(0, 0, 0, 0);
+      if (++kx == k_tiles) kx = 0;
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         const float4* sp = reinterpret_cast<const float4*>(ssrc + (long long)step * W_STEP + b * W_RAW);
@@ -174,22 +248,24 @@ int4_wa_kernel(const WaDev g) {
       }
     };
 #pragma unroll
-    for (int d = 0; d < W_PREFETCH; ++d) { raw[d][0] = raw[d][1] = make_uint4(0, 0, 0, 0); if (d < ksteps) load_w(d, d); }
-    load_x(0, 0);
-    if (ksteps > 1) load_x(1, 1);
+    for (int d = 0; d < W_PREFETCH; ++d) { raw[d][0] = raw[d][1] = make_uint4(0, 0, 0, 0); if (d < steps) load_w(d, d); }
+    if (steps > 0) load_x(0, 0);
+    if (steps > 1) load_x(1, 1);
     const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32) << 16) + sub * 32;      // + stage * W_ACOLS + half * 16
     int s = 0;                                                       // stage of the step, and the parity its a_empty wait needs
-    uint32_t par = 1;
-    for (int i0 = 0; i0 < ksteps && ok; i0 += W_PREFETCH) {
+    uint32_t par = 1, part = 0;
+    bool ok = true;
+    int left = steps > 0 ? part_steps(0) : 0;
+    for (int i0 = 0; i0 < steps; i0 += W_PREFETCH) {
 #pragma unroll
       for (int d = 0; d < W_PREFETCH; ++d) {
         const int i = i0 + d;
-        if (i >= ksteps || !ok) break;
+        if (i >= steps) break;
         // stage s (TMEM operand columns and the X' tile) was last read by the MMAs of step i - W_STAGES;
         // one thread polls, a hardware barrier releases the rest
         if (tid == 0) go_s[d & 1] = (int)mbar_wait(a_empty(s), par, dead, g.status, 330);
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (!go_s[d & 1]) { ok = false; break; }
+        if (!go_s[d & 1]) ok = false;
         tc_fence_after();
         // nibbles -> bf16 pairs -> 32 TMEM columns of this feature's lane
 #pragma unroll
@@ -206,7 +282,7 @@ int4_wa_kernel(const WaDev g) {
           }
           tmem_st16(t_st + s * W_ACOLS + hh * 16, t);
         }
-        if (i + W_PREFETCH < ksteps) load_w(d, i + W_PREFETCH);
+        if (i + W_PREFETCH < steps) load_w(d, i + W_PREFETCH);
         // X chunks: times the scale of their k, rounded to bf16, summed for the offset correction, stored swizzled
         uint8_t* xstage = gen + s * (WSUB * x_bytes);
 #pragma unroll
@@ -223,80 +299,41 @@ int4_wa_kernel(const WaDev g) {
             *reinterpret_cast<uint4*>(xstage + xdst[j]) = o;
           }
         }
-        if (i + 2 < ksteps) load_x(d & 1, i + 2);
+        if (i + 2 < steps) load_x(d & 1, i + 2);
         tmem_st_wait();
         fence_proxy_async_smem();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(a_full(s));
         if (++s == W_STAGES) { s = 0; par ^= 1; }
-      }
-    }
-  }
-  // ---- row sums of x': a chunk's row is fixed per (thread, j); sum the 8 pieces of a row, then over the blocks
+        if (--left == 0) {
+          // row sums of x' over this part: a chunk's row is fixed per (thread, j); the 8 pieces of a row, then the blocks
 #pragma unroll
-  for (int j = 0; j < NCH; ++j) {
-    float v = xs[j];
-    v += __shfl_xor_sync(0xffffffffu, v, 1); v += __shfl_xor_sync(0xffffffffu, v, 2); v += __shfl_xor_sync(0xffffffffu, v, 4);
-    xs[j] = v;
-  }
-  for (int i = tid; i < 128; i += W_THREADS) xsum_s[i] = 0.0f;
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < NCH; ++j) {
-    const int c = tid + j * W_CONV_THREADS, rowb = c >> 3, blk = rowb / x_rows, t = rowb - blk * x_rows;
-    if (ch == 0 && c < chunks && tid < W_CONV_THREADS) atomicAdd(xsum_s + t, xs[j]);         // two blocks per row: two adds per row
-  }
-  __syncthreads();
-  // ---- epilogue (warps 0-3): lane = output feature, column = token
-  if (warp < 4 && ok) {
-    if (tid == 0) go_s[0] = (int)mbar_wait(acc_full, 0, dead, g.status, 331);
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (go_s[0]) {
-      tc_fence_after();
-      const int fo = n0 + warp * 32 + lane;
-      const float bias = (g.bias && g.splits == 1) ? __bfloat162float(g.bias[fo]) : 0.0f;
-#pragma unroll 1
-      for (int c = 0; c < x_rows; c += 16) {
-        uint32_t rr[16];
-        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c, rr);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int t = m0 + c + j;
-          if (t < g.M) {
-            const float v = __uint_as_float(rr[j]) - 136.0f * xsum_s[c + j];
-            if (g.splits == 1) g.out[(long long)t * g.ldo + fo] = __float2bfloat16(v + bias);
-            else atomicAdd(g.acc + (long long)t * g.N + fo, v);
+          for (int j = 0; j < NCH; ++j) {
+            float v = xs[j];
+            v += __shfl_xor_sync(0xffffffffu, v, 1); v += __shfl_xor_sync(0xffffffffu, v, 2); v += __shfl_xor_sync(0xffffffffu, v, 4);
+            if (ch == 0 && xblk[j] >= 0) atomicAdd(xsum_s + xrow[j], v);         // two blocks per row: two adds per row
+            xs[j] = 0.0f;
           }
+          asm volatile("bar.sync 2, 288;" ::: "memory");
+          const int nt = (int)((u0 + i) / k_tiles);
+          // CTA of step x: the largest c with total c / ctas <= x
+          const long long lo = (((long long)nt * k_tiles + 1) * ctas - 1) / total, hi = ((long long)(nt + 1) * k_tiles * ctas - 1) / total;
+          wa_store_part(g, tmem, x_rows, m0, nt, xsum_s, lo == hi, acc_full, part & 1, dead, ok);
+          ++part;
+          tc_fence_before();
+          asm volatile("bar.sync 2, 288;" ::: "memory");
+          if (tid < 128) xsum_s[tid] = 0.0f;                         // used again behind the next step's barrier
+          if (lo != hi) wa_finish_tile(g, m0, mt, nt, (int)(hi - lo), is_last, dead);
+          left = i + 1 < steps ? part_steps(i + 1) : 0;
         }
       }
-      if (g.splits > 1) __threadfence();
     }
   }
+  if (*dead) __nanosleep(100000);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) { tc_fence_after(); tmem_dealloc(tmem, tmem_cols); }
-  if (g.splits > 1) {
-    if (tid == 0) *is_last = (atomicAdd(g.counters + mt * n_tiles + nt, 1) == g.splits - 1) && !*dead;
-    __syncthreads();
-    if (*is_last) {
-      __threadfence();
-      const int rows = min(128, g.M - m0);
-      for (int i = tid; i < rows * (WF / 4); i += W_THREADS) {
-        const int t = i / (WF / 4), c4 = (i % (WF / 4)) * 4;
-        float4* src = reinterpret_cast<float4*>(g.acc + (long long)(m0 + t) * g.N + n0 + c4);
-        float4 v = __ldcg(src);
-        *src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (g.bias) {
-          v.x += __bfloat162float(g.bias[n0 + c4]); v.y += __bfloat162float(g.bias[n0 + c4 + 1]);
-          v.z += __bfloat162float(g.bias[n0 + c4 + 2]); v.w += __bfloat162float(g.bias[n0 + c4 + 3]);
-        }
-        *reinterpret_cast<uint2*>(g.out + (long long)(m0 + t) * g.ldo + n0 + c4) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
-      }
-      if (tid == 0) g.counters[mt * n_tiles + nt] = 0;
-    }
-  }
 }
 
 // packed [K][N/2] bytes + scales (flat groups along N) -> tiles [N/128][K/64][4352]
@@ -362,17 +399,21 @@ CGK_API int cgk_int4_wa_gemm(const void* x, long long ldx, const void* tiles, fl
   const int x_rows = m_tiles > 1 ? 128 : (M + 15) / 16 * 16;
   const int nch = (WSUB * x_rows * 8 + W_CONV_THREADS - 1) / W_CONV_THREADS;
   const int per_sm = nch <= 2 ? 2 : 1;                     // resident CTAs per SM (registers, TMEM columns)
-  if (splits <= 0) {
-    splits = 1;
-    const int max_s = (acc && counters) ? 16 : 1;
-    for (int s = 2; s <= max_s && ksteps % s == 0 && ksteps / s >= 4 && n_tiles * m_tiles * s <= sms * per_sm; s *= 2) splits = s;
+  CGK_REQUIRE(splits <= 0 || ksteps % splits == 0, "cgk_int4_wa_gemm: K/128 = %d is not divisible by splits = %d", ksteps, splits);
+  CGK_REQUIRE(splits <= 1 || (acc && counters), "cgk_int4_wa_gemm: split-K needs the acc and counters buffers");
+  // CTAs: all that are resident at once, with at least three steps each; given splits, or no scratch to meet in: whole
+  // tiles or equal parts of them
+  const long long total = (long long)n_tiles * ksteps;
+  long long ctas = (long long)n_tiles * (splits > 0 ? splits : 1);
+  if (splits <= 0 && acc && counters) {
+    ctas = (long long)sms * per_sm / m_tiles;
+    if (ctas > total / 3) ctas = total / 3;
+    if (ctas < 1) ctas = 1;
   }
-  CGK_REQUIRE(ksteps % splits == 0, "cgk_int4_wa_gemm: K/128 = %d is not divisible by splits = %d", ksteps, splits);
-  CGK_REQUIRE(splits == 1 || (acc && counters), "cgk_int4_wa_gemm: split-K needs the acc and counters buffers");
   const int smem = 1024 + W_STAGES * WSUB * x_rows * 128 + 128 + 512 + 1024;
   WaDev g{(const uint8_t*)tiles, (const __nv_bfloat16*)x, ldx, acc, counters, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)bias, M, N, K,
-          splits, ksteps / splits, x_rows, device_status(dev)};
-  const dim3 grid(n_tiles * splits, m_tiles);
+          x_rows, device_status(dev)};
+  const dim3 grid((unsigned)ctas, m_tiles);
   cudaStream_t st = (cudaStream_t)stream;
   switch (nch) {
     case 1: return launch_wa<1>(g, grid, smem, st);

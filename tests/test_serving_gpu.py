@@ -45,6 +45,25 @@ def test_int4_gemm_matches_dequantised_product(M, K, N, group, splits, kernel):
     _lib.assert_device_ok()
 
 
+# the line of steps is cut into equal pieces: fewer steps than CTAs (one tile), pieces inside a tile, over several tiles, an odd
+# number of steps per tile, every number of X chunks per thread, two row tiles
+@pytest.mark.parametrize("M,K,N", [(1, 128, 128), (16, 384, 128), (16, 11008, 640), (17, 128 * 29, 1280), (48, 256, 12800), (80, 4096, 6144),
+                                   (96, 640, 8192), (128, 1408, 4096), (150, 512, 1024)])
+@pytest.mark.parametrize("kernel", ["wa", "wb"])
+def test_int4_gemm_pieces_of_the_weight_stream(M, K, N, kernel):
+    torch.manual_seed(M + K)
+    lin = Int4Linear(torch.randn(N, K) * 0.05, torch.randn(N) * 0.1, 128).to(DEV)
+    lin.kernel = kernel
+    x = (torch.randn(M, K) + 0.5).bfloat16().to(DEV)
+    ref = x.double() @ lin.dequantized().double() + lin.bias.double()
+    for _ in range(2):                                        # the scratch is left zero for the next call
+        # one operand is scaled and rounded to bf16 once per element (wb: its scale before that), the sums are fp32: 2^-8 of the
+        # terms' norm at most, and the result's rounding
+        err = (lin(x).double() - ref).norm() / ref.norm()
+        assert err < 2 ** -7, err
+    _lib.assert_device_ok()
+
+
 @pytest.mark.parametrize("n,group", [(8, 8), (1024, 32), (8 * 1031, 8), (128 * 999, 128), (24 * 100, 24)])
 def test_int4_dequantize_by_words(n, group):
     p, s = quantize_int4(torch.randn(n), group)
