@@ -108,7 +108,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::NUM_BARS * 8);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int kt = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   const int k0 = kt * C::BN;
   const int off = p.Tk - p.Tq;
@@ -156,7 +156,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (warp < 4) {
     if (warp == 0) {
       // ------------------------------ TMA producer ------------------------------
-      if (lane == 0 && total_steps > 0) {
+      if (total_steps > 0 && elect_one()) {
         tma_prefetch_desc(&tmQ);
         tma_prefetch_desc(&tmDO);
         mbar_expect_tx(kv_full, 2 * C::TILE_BYTES);
@@ -188,7 +188,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // issuing all 32 to 40 MMAs of a step was the kernel's critical path (some seventy cycles
       // per MMA, hundreds per barrier wait), and the P / dS tiles cannot be rewritten before the
       // last of the three products has read them.
-      if (lane == 0 && total_steps > 0) {
+      if (total_steps > 0 && elect_one()) {
         const uint32_t idesc_s = make_idesc_bf16(128, 128, 0, 0);   // S, dP: both K-major
         const uint32_t idesc_kv = make_idesc_bf16(128, D, 1, 1);    // dV, dK: A and B MN-major
         const uint32_t idesc_q = make_idesc_bf16(128, D, 0, 1);     // dQ: A K-major, B MN-major

@@ -118,7 +118,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem + C::OFF_BAR + C::NUM_BARS * 8);
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int qblk = gridDim.x - 1 - blockIdx.x;  // heavy (late) causal blocks first
   const int h = blockIdx.y, b = blockIdx.z;
   const int hk = (int)(((long long)h * p.Hk) / p.Hq);
@@ -179,7 +179,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
    if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0 && hi > lo) {
+    if (hi > lo && elect_one()) {
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
@@ -217,7 +217,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // cycles and every barrier wait a few hundred, against 32 to 64 tensor cycles per MMA.
     // Both walk the K/V ring in the producer's order; a slot is free again when both have
     // released it (after their MMAs on it, or at once when their tile does not use it).
-    if (lane == 0 && hi > lo) {
+    if (hi > lo && elect_one()) {
       const int t = warp == 1 ? 0 : 1;
       const uint32_t idesc_s = make_idesc_bf16(C::BM, C::BN, 0, 0);
       const uint32_t idesc_o = make_idesc_bf16(C::BM, D, 0, 1);

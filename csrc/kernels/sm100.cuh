@@ -90,6 +90,22 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
+// One lane of a converged warp.  Roles that one thread plays (issuing loads and MMAs) branch on this and not on lane == 0:
+// the compiler then knows that the branch is taken by a single lane and keeps descriptors and addresses in uniform
+// registers; otherwise every operand is moved there before each instruction.  GEMM of 32768 x 768 x 50304 with B stored
+// [k][n] (five loads per stage): 2225 -> 1953 us; weight gradient 50304 x 768 over 32768 rows: 1994 -> 1778 us.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t mine;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(mine));
+  return mine != 0;
+}
+// Warp index, uniform for the compiler too.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
+
 // ---------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------
