@@ -136,10 +136,10 @@ constexpr int GROUP_M = 8;
 constexpr int GEMM_THREADS = 384;       // TMA warp, MMA warp, TMEM warp, one spare, eight epilogue warps
 constexpr int RS_SIGNAL_BATCH = 4;      // reduce-scatter tiles published per system-scope fence
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool PAIR = false>
 struct GemmSmem {
   static constexpr int A_BYTES = BM * BK * 2;
-  static constexpr int B_BYTES = BN * BK * 2;
+  static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   // per-warp staging tiles of the epilogue (8 warps x 4 KiB = 32 rows x 128 bytes each, 128-byte
   // swizzle, 1024-byte aligned): outputs are transposed through them so that they leave as whole
@@ -177,15 +177,21 @@ __device__ __forceinline__ void tile_coords(const GemmDev& g, int tiles_m, int t
   if (g.m_rot) tm = (tm + g.m_rot) % g.tiles_m;
 }
 
-// cta / nctas: index and count of the CTAs that run this body (the fused kernels
+// cta / nctas: index and count of the CTAs (PAIR: of the pairs) that run this body (the fused kernels
 // give some CTAs of the grid other roles).  GEMM_THREADS threads.
-template <int BN, int STAGES, bool GROUPED = false>
+// PAIR: a cluster of two CTAs computes a 256 x BN tile.  Each CTA loads its 128 rows of A and half of B's rows and
+// drains its 128 rows of the accumulator; the MMAs read both halves of B, so a stage is 32 KiB instead of 48 at
+// BN = 256 (six stages instead of four) and the operand bytes per MMA fall by a third.
+template <int BN, int STAGES, bool GROUPED = false, bool PAIR = false>
 __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB,
                                              const CUtensorMap* tmC, const CUtensorMap* tmAux,
                                              const CUtensorMap* tmIn,
                                              const GemmDev& g, int cta, int nctas,
                                              uint8_t* smem_raw) {
-  using L = GemmSmem<BN, STAGES>;
+  using L = GemmSmem<BN, STAGES, PAIR>;
+  constexpr int TM = PAIR ? 2 * BM : BM;               // rows of a tile: g.tiles_m counts these
+  constexpr int BROWS = PAIR ? BN / 2 : BN;            // rows of B that this CTA loads
+  const uint32_t crank = PAIR ? cluster_rank() : 0u;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   const uint32_t smem_base = smem_u32(smem);
@@ -212,7 +218,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmA, const CUten
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 8);     // one arrival per epilogue warp
+      mbar_init(tempty_bar(a), PAIR ? 16 : 8);     // one arrival per epilogue warp (a pair: of both CTAs, at the leader's)
       mbar_init(epi_bar(a), 8);
     }
     for (int w = 0; w < 8; ++w) mbar_init(in_bar(w), 1);
@@ -220,11 +226,16 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmA, const CUten
     mbar_fence_init();
   }
   if (warp == 2) {
-    tmem_alloc(smem_u32(tmem_holder), TMEM_COLS);
-    tmem_relinquish();
+    if (PAIR) {
+      tmem_alloc_pair(smem_u32(tmem_holder), TMEM_COLS);
+    } else {
+      tmem_alloc(smem_u32(tmem_holder), TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();        // the other CTA's barriers are set up before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
 
@@ -253,7 +264,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmA, const CUten
         int b, tm, tn, kb0, kb1;
         tile_coords(g, tiles_m, t % out_tiles, b, tm, tn);
         k_range(t, kb0, kb1);
-        const int m0 = tm * BM, n0 = tn * BN;
+        const int m0 = tm * TM + (int)crank * BM, n0 = tn * BN + (int)crank * BROWS;
         const int bb = GROUPED ? g.m_group[tm] : b;
         if (g.a_ready) {
           // rows of this tile may span two chunks when a_ready_rows < 128: wait for the last one
@@ -273,27 +284,33 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmA, const CUten
           if (!mbar_wait(empty_bar(s), ph ^ 1u, dead, g.status, 100)) { ok = false; break; }
           const uint32_t sA = smem_base + s * L::STAGE_BYTES;
           const uint32_t sB = sA + L::A_BYTES;
-          mbar_expect_tx(full_bar(s), L::STAGE_BYTES);
+          // a pair's loads all complete on the leader's barrier, which expects the bytes of both CTAs
+          const uint32_t fb = PAIR ? cluster_map(full_bar(s), 0) : full_bar(s);
+          if (crank == 0) mbar_expect_tx(full_bar(s), (PAIR ? 2 : 1) * L::STAGE_BYTES);
+          auto load = [&](uint32_t dst, const CUtensorMap& m, int x, int y, int z) {
+            if constexpr (PAIR) tma_load_3d_pair(dst, &m, fb, x, y, z);
+            else tma_load_3d(dst, &m, fb, x, y, z);
+          };
           if (!g.a_mn) {
-            tma_load_3d(sA, &tmA, full_bar(s), kb * BK, m0, b);
+            load(sA, tmA, kb * BK, m0, b);
           } else {
 #pragma unroll
             for (int blk = 0; blk < BM / 64; ++blk)
-              tma_load_3d(sA + blk * 8192, &tmA, full_bar(s), m0 + blk * 64, kb * BK, b);
+              load(sA + blk * 8192, tmA, m0 + blk * 64, kb * BK, b);
           }
           if (!g.b_mn) {
-            tma_load_3d(sB, &tmB, full_bar(s), kb * BK, n0, bb);
+            load(sB, tmB, kb * BK, n0, bb);
           } else {
 #pragma unroll
-            for (int blk = 0; blk < BN / 64; ++blk)
-              tma_load_3d(sB + blk * 8192, &tmB, full_bar(s), n0 + blk * 64, kb * BK, bb);
+            for (int blk = 0; blk < BROWS / 64; ++blk)
+              load(sB + blk * 8192, tmB, n0 + blk * 64, kb * BK, bb);
           }
         }
       }
     }
   } else if (warp == 1) {
-    if (elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(BM, BN, g.a_mn, g.b_mn);
+    if (crank == 0 && elect_one()) {
+      const uint32_t idesc = make_idesc_bf16(TM, BN, g.a_mn, g.b_mn);
       const uint32_t a_lbo = g.a_mn ? 8192u : 16u;
       const uint32_t b_lbo = g.b_mn ? 8192u : 16u;
       // Shared-memory descriptors: the high word (1024-byte stride between 8-row groups, 128-byte
@@ -324,12 +341,19 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmA, const CUten
           const uint32_t a_lo = a_lo0 + (uint32_t)s * (L::STAGE_BYTES >> 4);
           const uint32_t b_lo = b_lo0 + (uint32_t)s * (L::STAGE_BYTES >> 4);
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk)
-            umma_f16(d_tmem, desc_hi | (uint64_t)(a_lo + kk * a_k16), desc_hi | (uint64_t)(b_lo + kk * b_k16), idesc,
-                     (kb != kb0 || kk != 0) ? 1u : 0u);
-          umma_commit(empty_bar(s));  // frees the stage once these MMAs have read it
+          for (int kk = 0; kk < BK / 16; ++kk) {
+            const uint64_t da = desc_hi | (uint64_t)(a_lo + kk * a_k16), db = desc_hi | (uint64_t)(b_lo + kk * b_k16);
+            if (PAIR) umma_f16_pair(d_tmem, da, db, idesc, (kb != kb0 || kk != 0) ? 1u : 0u);
+            else umma_f16(d_tmem, da, db, idesc, (kb != kb0 || kk != 0) ? 1u : 0u);
+          }
+          // frees the stage (of both CTAs) once these MMAs have read it
+          if (PAIR) umma_commit_pair(empty_bar(s));
+          else umma_commit(empty_bar(s));
         }
-        if (ok) umma_commit(tfull_bar(acc));
+        if (ok) {
+          if (PAIR) umma_commit_pair(tfull_bar(acc));
+          else umma_commit(tfull_bar(acc));
+        }
       }
     }
   } else if (warp >= 4) {
@@ -341,9 +365,11 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmA, const CUten
   if (*dead) __nanosleep(100000);
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();        // neither CTA leaves while the other may still read its memory or arrive on its barriers
   if (warp == 2) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    if (PAIR) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 

@@ -27,6 +27,16 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   gemm_tc_body<BN, STAGES>(tmA, tmB, &tmC, &tmAux, &tmIn, g, (int)blockIdx.x, (int)gridDim.x, smem_raw);
 }
 
+// The same by CTA pairs: 256 x BN tiles, one cluster of two CTAs per tile.
+template <int BN, int STAGES>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                      const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAux,
+                      const __grid_constant__ CUtensorMap tmIn, const GemmDev g) {
+  extern __shared__ uint8_t smem_raw[];
+  gemm_tc_body<BN, STAGES, false, true>(tmA, tmB, &tmC, &tmAux, &tmIn, g, (int)blockIdx.x >> 1, (int)gridDim.x >> 1, smem_raw);
+}
+
 // Grouped product: the rows of A lie in expert order, every expert's segment starts on a row tile, and the
 // number of row tiles is known on the device only.
 template <int BN, int STAGES>
@@ -203,6 +213,35 @@ int pick_bn(const cgk_gemm_args& a, int ctas) {
   return 64;
 }
 
+constexpr int PAIR_BN = 256, PAIR_STAGES = 6;
+
+static int launch_pair(const cgk_gemm_args& a, const GemmDev& g0, int ctas, cudaStream_t stream) {
+  using L = GemmSmem<PAIR_BN, PAIR_STAGES, true>;
+  GemmDev g = g0;
+  g.tiles_m = (a.M + 2 * BM - 1) / (2 * BM);
+  g.tiles_n = (a.N + PAIR_BN - 1) / PAIR_BN;
+  CUtensorMap tmA, tmB, tmC, tmAux, tmIn;
+  int rc = make_gemm_tmaps(a, PAIR_BN / 2, &tmA, &tmB);        // a CTA loads half of B's rows
+  if (rc) return rc;
+  int out_ok = 0, in_kind = 0;
+  if ((rc = make_gemm_out_tmaps(a, &tmC, &tmAux, &tmIn, &out_ok, &in_kind))) return rc;
+  g.tma_store = (out_ok && g.split_k == 1) ? 1 : 0;
+  g.tma_in = g.tma_store ? in_kind : 0;
+  CGK_CUDA_CHECK(cudaFuncSetAttribute(gemm_bf16_pair_kernel<PAIR_BN, PAIR_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+  const int total = g.batch * g.tiles_m * g.tiles_n * g.split_k, pairs = ctas / 2;
+  gemm_bf16_pair_kernel<PAIR_BN, PAIR_STAGES><<<2 * (total < pairs ? total : pairs), GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, tmC, tmAux, tmIn, g);
+  CGK_LAUNCH_CHECK();
+  return 0;
+}
+
+// Pairs or single CTAs for a 256-wide tile.  Pairs wherever the main loop is what a tile waits for (22016 x 4096, 8176 rows:
+// 1035 -> 935 us; weight gradient 50304 x 768 over 32768 rows 1778 -> 1771) and where many tiles stream wide outputs
+// (32768 x 50304 x 768: 2606 -> 2469 us); with K below 1024 and fewer columns the epilogue bounds the tile, and two CTAs
+// waiting for each other's cost a little (32768 x 2304 x 768: 125 / 133 us).
+static bool by_pairs(const cgk_gemm_args& a, int ctas) {
+  return ctas >= 2 && a.M > BM && (a.K >= 1024 || a.N >= 8192);
+}
+
 template <int BN, int STAGES>
 static int launch_tc(const cgk_gemm_args& a, const GemmDev& g0, int sms, cudaStream_t stream) {
   using L = GemmSmem<BN, STAGES>;
@@ -323,14 +362,14 @@ CGK_API int cgk_gemm_bf16(const cgk_gemm_args* pa, void* stream_) {
       g.kb_per_split = (kblocks + S - 1) / S;
       g.split_k = (kblocks + g.kb_per_split - 1) / g.kb_per_split;     // no empty slice
       switch (bn) {
-        case 256: return launch_tc<256, 4>(a, g, sms, stream);
+        case 256: return by_pairs(a, ctas) ? launch_pair(a, g, ctas, stream) : launch_tc<256, 4>(a, g, sms, stream);
         case 128: return launch_tc<128, 6>(a, g, sms, stream);
         default: return launch_tc<64, 8>(a, g, sms, stream);
       }
     }
   }
   switch (pick_bn(a, a.max_ctas > 0 ? a.max_ctas : sms)) {
-    case 256: return launch_tc<256, 4>(a, g, sms, stream);
+    case 256: return by_pairs(a, ctas) ? launch_pair(a, g, ctas, stream) : launch_tc<256, 4>(a, g, sms, stream);
     case 128: return launch_tc<128, 6>(a, g, sms, stream);
     default: return launch_tc<64, 8>(a, g, sms, stream);
   }

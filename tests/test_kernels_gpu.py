@@ -39,6 +39,30 @@ def test_gemm_layouts(M, N, K, a_mn, b_mn):
     assert relerr(out, ref) < 1e-2
 
 
+# pairs of CTAs (256 x 256 tiles): the second CTA's rows missing in part and in whole, ragged columns, all operand orders, and
+# every epilogue that leaves through staging tiles
+@pytest.mark.parametrize("M,N,K", [(5120, 2048, 1024), (5000, 2056, 1032), (4225, 8200, 96), (4097, 2304, 4096)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+def test_gemm_by_cta_pairs(M, N, K, a_mn, b_mn):
+    from cogito_b200.ops.gemm import gemm, gemm_reference
+    if a_mn:
+        M = M // 8 * 8
+    torch.manual_seed(K)
+    a = torch.randn((K, M) if a_mn else (M, K), device=DEV, dtype=torch.bfloat16)
+    b = torch.randn((K, N) if b_mn else (N, K), device=DEV, dtype=torch.bfloat16)
+    bias, other = torch.randn(N, device=DEV, dtype=torch.bfloat16), torch.randn(M, N, device=DEV, dtype=torch.bfloat16)
+    aux = torch.empty_like(other)
+    for kw in ({}, {"bias": bias, "act": "gelu"}, {"bias": bias, "residual": other}, {"aux_in": other, "dact": "gelu"}):
+        ref = gemm_reference(a, b, a_mn=a_mn, b_mn=b_mn, out_dtype=torch.float32, **kw)
+        if "act" in kw:
+            assert relerr(gemm(a, b, a_mn=a_mn, b_mn=b_mn, aux_out=aux, **kw), ref) < 1e-2
+            assert relerr(aux, gemm_reference(a, b, a_mn=a_mn, b_mn=b_mn, bias=bias, out_dtype=torch.float32)) < 1e-2
+        else:
+            assert relerr(gemm(a, b, a_mn=a_mn, b_mn=b_mn, **kw), ref) < 1e-2
+    f32 = gemm(a, b, a_mn=a_mn, b_mn=b_mn, out_dtype=torch.float32)
+    assert relerr(f32, gemm_reference(a, b, a_mn=a_mn, b_mn=b_mn, out_dtype=torch.float32)) < 2e-3
+
+
 @pytest.mark.parametrize("Mw,Nw,K,split", [(384, 768, 16384, 0), (768, 768, 8192, 4), (288, 768, 4096 + 64, 3),
                                            (3072, 768, 2048, 0)])
 def test_gemm_split_k_weight_gradient(Mw, Nw, K, split):
