@@ -21,7 +21,7 @@ if not _DEBUG and not _LIB_PATH.exists() and (_LIB_DIR / "libcogito_kernels_serv
     _LIB_PATH = _LIB_DIR / "libcogito_kernels_serve.so"           # a checkout that only serves: part of the kernels
 _lib = None
 # source files that carry index checks in the debug build (one recorded violation each)
-_BOUNDS_FILES = ("gemm_tcgen05", "softmax_ce", "serving", "elementwise", "flash_fwd", "flash_bwd", "residual_stream", "latent_kv",
+_BOUNDS_FILES = ("gemm_tcgen05", "gemm_few", "softmax_ce", "serving", "elementwise", "flash_fwd", "flash_bwd", "residual_stream", "latent_kv",
                  "latent_attn_tc", "moe", "kv_rows", "linear_state", "linear_state_tc")
 
 

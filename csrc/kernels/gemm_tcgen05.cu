@@ -81,14 +81,14 @@ __global__ void gemm_bf16_simt_kernel(const __nv_bfloat16* __restrict__ A,
   if (m < g.M && n < g.N) epilogue_scalar(g, b, m, n, acc);
 }
 
-int make_gemm_tmaps(const cgk_gemm_args& a, int BN, CUtensorMap* tmA, CUtensorMap* tmB) {
+int make_gemm_tmaps(const cgk_gemm_args& a, int BN, CUtensorMap* tmA, CUtensorMap* tmB, int a_rows) {
   int rc;
   {
     uint64_t dims[3], strides[2];
     uint32_t box[3];
     if (!a.a_mn) {
       dims[0] = (uint64_t)a.K; dims[1] = (uint64_t)a.M;
-      box[0] = BK; box[1] = BM;
+      box[0] = BK; box[1] = (uint32_t)a_rows;
     } else {
       dims[0] = (uint64_t)a.M; dims[1] = (uint64_t)a.K;
       box[0] = 64; box[1] = BK;
@@ -347,6 +347,8 @@ CGK_API int cgk_gemm_bf16(const cgk_gemm_args* pa, void* stream_) {
   }
   const int sms = sm_count(dev);
   const int ctas = a.max_ctas > 0 && a.max_ctas < sms ? a.max_ctas : sms;
+  FewPlan few;
+  if (gemm_few_plan(a, ctas, &few)) return launch_gemm_few(a, g, few, stream);
   // Split-K for accumulating fp32 outputs (weight gradients) whose tiles would leave SMs idle:
   // the widest tile the output allows, and as many K slices as fill the machine.
   const bool can_split = a.out_fp32 && a.accumulate && a.batch == 1 && !a.bias && a.act == 0 && !a.residual &&

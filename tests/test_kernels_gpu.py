@@ -39,6 +39,32 @@ def test_gemm_layouts(M, N, K, a_mn, b_mn):
     assert relerr(out, ref) < 1e-2
 
 
+# few output tiles: a cluster per tile (gemm_few.cu).  One row tile with 64 and with 128 columns, each number of CTAs per tile
+# (K = 64 .. 2048), ragged rows, columns and K; several row tiles with a long K; ragged columns with a short one
+@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (8, 200, 128), (31, 512, 256), (32, 768, 2048), (33, 1000, 1000), (128, 2048, 520), (128, 72, 4096),
+                                   (40, 11264, 512), (16, 32000, 256), (129, 64, 2048), (300, 136, 1536), (256, 784, 256), (500, 52, 256)])
+@pytest.mark.parametrize("form", ["plain", "mn", "epilogue", "accumulate"])
+def test_gemm_with_few_tiles(M, N, K, form):
+    from cogito_b200.ops.gemm import gemm, gemm_reference
+    torch.manual_seed(M + N + K)
+    mn = form in ("mn", "accumulate")
+    if mn and (M % 8 or N % 8):
+        pytest.skip("MN-major operands need leading dimensions that are multiples of 8")
+    a = torch.randn((K, M) if mn else (M, K), device=DEV, dtype=torch.bfloat16)
+    b = torch.randn((K, N) if mn else (N, K), device=DEV, dtype=torch.bfloat16)
+    kw = {}
+    if form == "epilogue":
+        kw = {"bias": torch.randn(N, device=DEV), "act": "gelu", "residual": torch.randn(M, N, device=DEV, dtype=torch.bfloat16), "alpha": 0.5}
+    if form == "accumulate":
+        base = torch.randn(M, N, device=DEV)
+        got = gemm(a, b, a_mn=True, b_mn=True, out=base.clone(), accumulate=True)
+        # fp32 sums of K products of two N(0, 1) values: K 2^-24 of a result of about sqrt(K), with a margin of 16
+        assert relerr(got, base.double() + a.double().T @ b.double()) < 16 * K * 2 ** -24 + 1e-6
+        return
+    got = gemm(a, b, a_mn=mn, b_mn=mn, **kw)
+    assert relerr(got, gemm_reference(a, b, a_mn=mn, b_mn=mn, out_dtype=torch.float32, **kw)) < 1e-2
+
+
 # pairs of CTAs (256 x 256 tiles): the second CTA's rows missing in part and in whole, ragged columns, all operand orders, and
 # every epilogue that leaves through staging tiles
 @pytest.mark.parametrize("M,N,K", [(5120, 2048, 1024), (5000, 2056, 1032), (4225, 8200, 96), (4097, 2304, 4096)])
