@@ -48,6 +48,19 @@ def norm_forward_raw(x2, gamma, beta, eps, rms, residual2=None, want_sum=False):
     return y, s, mean, rstd
 
 
+def add_rms_norm_(x, y, gamma, eps: float):
+    """x += y in place (bf16), and the RMSNorm of the sum, by one kernel on CUDA; x contiguous, not under autograd."""
+    if not (x.is_cuda and x.dtype == y.dtype == gamma.dtype == _BF16 and x.is_contiguous() and y.is_contiguous()):
+        x += y.view_as(x)
+        return rms_norm(x, gamma, eps)
+    D = x.shape[-1]
+    out = torch.empty_like(x)
+    _lib.check(_lib.lib().cgk_norm_forward(x.data_ptr(), y.data_ptr(), gamma.data_ptr(), None, out.data_ptr(), x.data_ptr(), None, None,
+                                           x.numel() // D, D, float(eps), 1, _lib.stream_ptr()), "cgk_norm_forward")
+    _lib.count_launch()
+    return out
+
+
 def norm_backward_raw(dy2, s2, gamma, mean, rstd, rms, dres2=None, dgamma_out=None, dbeta_out=None):
     """Returns (dx, dgamma fp32, dbeta fp32 or None).  When *_out are given the
     parameter gradients are accumulated into them."""

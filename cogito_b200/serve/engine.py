@@ -24,7 +24,7 @@ from ..models.llama import Llama, LlamaConfig
 from ..ops import _lib
 from ..ops import misc as M
 from ..ops.attention import flash_forward
-from ..ops.norm import rms_norm
+from ..ops.norm import add_rms_norm_, rms_norm
 from ..quant.int4 import Int4Linear, dequantize_int4, quantize_int4
 from .kv_cache import PagedKVCacheInt4
 from .sampling import sample, spec_accept
@@ -177,8 +177,7 @@ class LlamaInt4Engine:
         y = lin(inp)
         if self.tp > 1:
             dist.all_reduce(y, group=self.tp_group)
-        x += y.view_as(x)
-        return rms_norm(x, norm_w, self.cfg.norm_eps)
+        return add_rms_norm_(x, y, norm_w, self.cfg.norm_eps)
 
     def _fake_quant(self, t: torch.Tensor) -> torch.Tensor:
         """bf16 [B, T, H, D] -> the values an INT4 cache entry of it dequantises to."""

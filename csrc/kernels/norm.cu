@@ -38,9 +38,9 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 // ceil(D / 256) of them.  The row stays in registers as packed bf16.
 template <int MAXV, bool RMS>
 __global__ void __launch_bounds__(NORM_WARPS * 32)
-norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
+norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ residual,
                 const __nv_bfloat16* __restrict__ gamma, const __nv_bfloat16* __restrict__ beta,
-                __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ sum_out,
+                __nv_bfloat16* __restrict__ y, __nv_bfloat16* sum_out,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int D,
                 float eps) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -563,7 +563,7 @@ static int norm_bwd_cap(int dev, int D) {
 }
 
 // rms = 0: LayerNorm (beta may be null), rms = 1: RMSNorm (beta ignored, mean unused).
-// residual / sum_out / mean / rstd may be null.  D must be a multiple of 8, D <= 8192.
+// residual / sum_out / mean / rstd may be null; sum_out may be x.  D must be a multiple of 8, D <= 8192.
 CGK_API int cgk_norm_forward(const void* x, const void* residual, const void* gamma,
                              const void* beta, void* y, void* sum_out, float* mean, float* rstd,
                              int rows, int D, float eps, int rms, void* stream_) {

@@ -50,6 +50,9 @@ def test_wide_norm_against_64_bits(rows, D, rms):
     assert rel(y, h * gd + (0.0 if rms else b.double())) < 2 ** -9 * 1.1
     assert rel(dx, rs * (t - s1 - h * (t * h).mean(-1, keepdim=True)) + r.double()) < 2 ** -9 * 1.1
     assert rel(dg, (dy.double() * h).sum(0)) < 2e-6 and (rms or rel(db, dy.double().sum(0)) < 2e-6)
+    if rms:
+        u = x.clone()
+        assert torch.equal(N.add_rms_norm_(u, r, g, 1e-5), y) and torch.equal(u, s)
 
 
 @pytest.mark.parametrize("rows,D", [(64, 768), (33, 128), (1000, 4096), (7, 8)])
