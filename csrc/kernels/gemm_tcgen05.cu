@@ -347,8 +347,6 @@ CGK_API int cgk_gemm_bf16(const cgk_gemm_args* pa, void* stream_) {
   }
   const int sms = sm_count(dev);
   const int ctas = a.max_ctas > 0 && a.max_ctas < sms ? a.max_ctas : sms;
-  FewPlan few;
-  if (gemm_few_plan(a, ctas, &few)) return launch_gemm_few(a, g, few, stream);
   // Split-K for accumulating fp32 outputs (weight gradients) whose tiles would leave SMs idle:
   // the widest tile the output allows, and as many K slices as fill the machine.
   const bool can_split = a.out_fp32 && a.accumulate && a.batch == 1 && !a.bias && a.act == 0 && !a.residual &&
@@ -370,6 +368,8 @@ CGK_API int cgk_gemm_bf16(const cgk_gemm_args* pa, void* stream_) {
       }
     }
   }
+  FewPlan few;
+  if (gemm_few_plan(a, ctas, &few)) return launch_gemm_few(a, g, few, stream);
   switch (pick_bn(a, a.max_ctas > 0 ? a.max_ctas : sms)) {
     case 256: return by_pairs(a, ctas) ? launch_pair(a, g, ctas, stream) : launch_tc<256, 4>(a, g, sms, stream);
     case 128: return launch_tc<128, 6>(a, g, sms, stream);
