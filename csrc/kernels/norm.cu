@@ -133,10 +133,11 @@ __device__ __forceinline__ float2 block_sum2(float a, float b, float* sh) {
   return make_float2(warp_sum(a), warp_sum(b));
 }
 
-// Rows of more than 1024 elements: one CTA per row, 16 bytes per thread.  A warp alone with a row of 4096 has sixteen
+// Few rows of more than 1024 elements: one CTA per row, 16 bytes per thread.  A warp alone with a row of 4096 has sixteen
 // dependent steps per pass and, in decoding, an SM to itself: RMSNorm of 16 x 4096 took 6.2 us, of 80 x 4096 9.3 us; 2.0 us
-// each like this.
-constexpr int NORM_WIDE = 1024;
+// each like this.  With rows for four warps on every SM the warps cover each other's steps (4096 x 4096: 20.1 us by
+// warps, 21.5 us by CTAs).
+constexpr int NORM_WIDE = 1024, NORM_WIDE_ROWS_PER_SM = 4;
 template <bool RMS>
 __global__ void __launch_bounds__(1024)
 norm_fwd_wide_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ residual,
@@ -573,7 +574,7 @@ CGK_API int cgk_norm_forward(const void* x, const void* residual, const void* ga
   cudaStream_t st = (cudaStream_t)stream_;
   int dev = 0;
   CGK_CUDA_CHECK(cudaGetDevice(&dev));
-  if (D > NORM_WIDE) {
+  if (D > NORM_WIDE && rows <= sm_count(dev) * NORM_WIDE_ROWS_PER_SM) {
     const auto kernel = rms ? norm_fwd_wide_kernel<true> : norm_fwd_wide_kernel<false>;
     kernel<<<rows, wide_threads(D), 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)gamma,
                                              rms ? nullptr : (const __nv_bfloat16*)beta, (__nv_bfloat16*)y, (__nv_bfloat16*)sum_out, mean, rstd, D, eps);
@@ -596,7 +597,10 @@ CGK_API int cgk_norm_forward(const void* x, const void* residual, const void* ga
         rows, D, eps);
   if (need <= 1) { LAUNCH(1) }
   else if (need <= 2) { LAUNCH(2) }
-  else { LAUNCH(4) }
+  else if (need <= 4) { LAUNCH(4) }
+  else if (need <= 8) { LAUNCH(8) }
+  else if (need <= 16) { LAUNCH(16) }
+  else { LAUNCH(32) }
 #undef LAUNCH
   CGK_LAUNCH_CHECK();
   return 0;
