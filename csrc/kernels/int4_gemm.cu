@@ -13,14 +13,18 @@
 //   warp 3    TMA: X tiles [rows, 64 k] into their own ring of up to 12 stages; only
 //             round_up(M, 8) rows are fetched — the tensor core still multiplies 128 rows, the
 //             others hold whatever shared memory held and only feed output rows nobody stores
-//   warps 4-11 nibbles -> bf16: exact integer (magic-number trick), one multiply by the scale,
+//   warps 4-19 nibbles -> bf16: exact integer (magic-number trick), one multiply by the scale,
 //             stored in the 128-byte-swizzled MN-major operand layout tcgen05 reads.  Columns
 //             stay in the pair order the extraction yields (0,4,1,5,2,6,3,7 within each group
 //             of 8); the epilogue undoes the permutation when it addresses the output.
-//   warp 1    tcgen05.mma, accumulator in TMEM (128 lanes x 128 columns)
-//   warps 4-7 epilogue.  One split: TMEM -> bias -> bf16 -> global.  Split-K: vector red.add
+//   warp 1    tcgen05.mma, two accumulators in TMEM (128 lanes x 128 columns)
+//   warps 20-23 epilogue.  Whole tile: TMEM -> bias -> bf16 -> global.  Part of a tile: vector red.add
 //             into a zeroed fp32 buffer; the CTA that arrives last at the tile's counter adds
 //             the bias, writes bf16 and leaves buffer and counter zeroed for the next call.
+// One CTA per SM.  Each takes as many whole tiles as there are for all of them, then an equal piece of the line of the left-over
+// tiles' steps of 128 k (see int4_gemm_wa.cu).  Whole tiles only left 172 of them (22 016 columns) in two waves on 148 SMs, and a
+// K of 11 008 on 64 CTAs.  80 rows, event times with cold caches: 4096 x 22016 72.6 -> 57.3 us, 11008 x 4096 62.4 -> 38.9, 4096 x 32000 74.7 -> 77.9
+// (two thirds of a wave left over: its tiles meet in the fp32 buffer).
 #include <cuda_bf16.h>
 #include <stdlib.h>
 
@@ -34,10 +38,10 @@ using namespace cgk;
 constexpr int BM = 128, BN = 128, BK = 64;
 constexpr int ISSUE_LANES = 8;                                // threads of a producer warp that issue copies
 constexpr int SUB = 2;                                        // 64-row sub-tiles per pipeline step (a step covers 128 k)
-constexpr int B_STAGES = 3, MAX_RAW_STAGES = 16, MAX_A_STAGES = 8, CONVERT_WARPS = 16;
+constexpr int B_STAGES = 2, MAX_RAW_STAGES = 16, MAX_A_STAGES = 8, CONVERT_WARPS = 16;
 constexpr int B_BYTES = BK * BN * 2;
 constexpr int NIB_BYTES = BK * BN / 2, SCALE_BYTES = BK * 2 * 4, RAW_BYTES = NIB_BYTES + SCALE_BYTES;   // 4096 + 512
-constexpr int THREADS = 128 + 32 * CONVERT_WARPS;
+constexpr int EPI_WARP0 = 4 + CONVERT_WARPS, THREADS = 32 * (EPI_WARP0 + 4);
 constexpr int SMEM_BYTES = 226 * 1024;                       // alignment slack | X ring | B ring | W ring | barriers
 constexpr int RING_BUDGET = SMEM_BYTES - 1024 - B_STAGES * SUB * B_BYTES - 2048;   // shared by the X and W rings
 
@@ -48,10 +52,8 @@ struct Int4Dev {
   __nv_bfloat16* out; long long ldo;
   const __nv_bfloat16* bias;
   int M, N, K;
-  int splits, ksteps;              // k-steps per CTA
   int a_rows, a_stages;            // rows fetched per X tile (multiple of 8), depth of the X ring
   int raw_stages;                  // depth of the W ring
-  int skip_convert;                // profiling aid: leave the operand tile unwritten (results are then meaningless)
   int* status;
 };
 
@@ -76,25 +78,31 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
   auto b_empty = [&](int s) { return sBar + 8u * (2 * MAX_A_STAGES + B_STAGES + s); };
   auto raw_full = [&](int s) { return sBar + 8u * (2 * MAX_A_STAGES + 2 * B_STAGES + s); };
   auto raw_empty = [&](int s) { return sBar + 8u * (2 * MAX_A_STAGES + 2 * B_STAGES + MAX_RAW_STAGES + s); };
-  const uint32_t acc_full = sBar + 8u * (2 * MAX_A_STAGES + 2 * B_STAGES + 2 * MAX_RAW_STAGES);
+  auto acc_full = [&](int a) { return sBar + 8u * (2 * MAX_A_STAGES + 2 * B_STAGES + 2 * MAX_RAW_STAGES + a); };
+  auto acc_empty = [&](int a) { return sBar + 8u * (2 * MAX_A_STAGES + 2 * B_STAGES + 2 * MAX_RAW_STAGES + 2 + a); };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_tiles = g.N / BN, k_tiles = g.K / (SUB * BK);
-  const int nt = blockIdx.x % n_tiles, split = blockIdx.x / n_tiles, mt = blockIdx.y;
-  const int n0 = nt * BN, ks0 = split * g.ksteps, m0 = mt * BM;     // ks0, ksteps count 128-row steps
-  const int ksteps = g.ksteps, a_stages = g.a_stages, RAW_STAGES = g.raw_stages;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const int n_tiles = g.N / BN, k_tiles = g.K / (SUB * BK), mt = blockIdx.y, m0 = mt * BM;
+  // This CTA's steps of 128 k: its `own` steps of whole tiles, then its piece of the line of the tiles that are left over.
+  const long long ctas = gridDim.x, whole = n_tiles / ctas * ctas, rest = (n_tiles - whole) * (long long)k_tiles;
+  const long long sharers = min(ctas, max(1LL, rest / 2));          // of the left-over tiles: at least two steps each
+  const int own = (int)(n_tiles / ctas) * k_tiles;
+  const long long r0 = rest * min((long long)blockIdx.x, sharers) / sharers;
+  const int ksteps = own + (int)(rest * min(blockIdx.x + 1LL, sharers) / sharers - r0), a_stages = g.a_stages, RAW_STAGES = g.raw_stages;
+  auto line = [&](int i) -> long long { return i < own ? (long long)blockIdx.x * own + i : whole * k_tiles + r0 + (i - own); };
+  auto part_steps = [&](int i) -> int { return (int)min((long long)(ksteps - i), k_tiles - line(i) % k_tiles); };
   const uint32_t a_bytes = (uint32_t)g.a_rows * 128u;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < MAX_A_STAGES; ++s) { mbar_init(a_full(s), 1); mbar_init(a_empty(s), 1); }
     for (int s = 0; s < B_STAGES; ++s) { mbar_init(b_full(s), CONVERT_WARPS); mbar_init(b_empty(s), 1); }
     for (int s = 0; s < MAX_RAW_STAGES; ++s) { mbar_init(raw_full(s), 1); mbar_init(raw_empty(s), CONVERT_WARPS); }
-    mbar_init(acc_full, 1);
+    for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), 4); }
     *dead = 0;
     *is_last = 0;
     mbar_fence_init();
   }
-  if (warp == 2) { tmem_alloc(smem_u32(tmem_slot), BN); tmem_relinquish(); }
+  if (warp == 2) { tmem_alloc(smem_u32(tmem_slot), 2 * BN); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -106,13 +114,12 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
     // belongs to the same lane: its uses are then waited for in order, which the one-bit phase
     // parity of an mbarrier requires.
     if (lane < ISSUE_LANES) {
-      const uint8_t* src = g.w_tiles + ((long long)nt * k_tiles + ks0) * (SUB * RAW_BYTES);
       for (int i = 0; i < ksteps; ++i) {
         const int r = i % RAW_STAGES;
         if (r % ISSUE_LANES != lane) continue;
         if (!mbar_wait(raw_empty(r), ((i / RAW_STAGES) & 1) ^ 1, dead, g.status, 300)) break;
         mbar_expect_tx(raw_full(r), SUB * RAW_BYTES);
-        bulk_load_1d(sRaw + r * (SUB * RAW_BYTES), src + (long long)i * (SUB * RAW_BYTES), SUB * RAW_BYTES, raw_full(r));
+        bulk_load_1d(sRaw + r * (SUB * RAW_BYTES), g.w_tiles + line(i) * (SUB * RAW_BYTES), SUB * RAW_BYTES, raw_full(r));
       }
     }
   } else if (warp == 3) {
@@ -121,36 +128,47 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
       for (int i = 0; i < ksteps; ++i) {
         const int s = i % a_stages;
         if (s % ISSUE_LANES != lane) continue;
+        const int ks = (int)(line(i) % k_tiles);                      // step within its tile
         if (!mbar_wait(a_empty(s), ((i / a_stages) & 1) ^ 1, dead, g.status, 301)) break;
         mbar_expect_tx(a_full(s), SUB * a_bytes);
 #pragma unroll
         for (int sub = 0; sub < SUB; ++sub)
-          tma_load_2d(sA + (s * SUB + sub) * a_bytes, &tmX, a_full(s), ((ks0 + i) * SUB + sub) * BK, m0);
+          tma_load_2d(sA + (s * SUB + sub) * a_bytes, &tmX, a_full(s), (ks * SUB + sub) * BK, m0);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_bf16(BM, BN, 0, 1);
       bool ok = true;
+      int left = 0, part = -1;
+      bool first = true;
       for (int i = 0; i < ksteps && ok; ++i) {
         const int sa = i % a_stages, sb = i % B_STAGES;
+        if (left == 0) {
+          left = part_steps(i);
+          first = true;
+          ++part;
+          if (!mbar_wait(acc_empty(part & 1), ((part >> 1) & 1) ^ 1, dead, g.status, 307)) { ok = false; break; }
+        }
         if (!mbar_wait(a_full(sa), (i / a_stages) & 1, dead, g.status, 302) ||
             !mbar_wait(b_full(sb), (i / B_STAGES) & 1, dead, g.status, 303)) { ok = false; break; }
         tc_fence_after();
+        const uint32_t d = tmem + (uint32_t)(part & 1) * BN;
 #pragma unroll
         for (int sub = 0; sub < SUB; ++sub) {
           const uint32_t a_addr = sA + (sa * SUB + sub) * a_bytes, b_addr = sB + (sb * SUB + sub) * B_BYTES;
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk)
-            if (!(g.skip_convert & 2)) umma_f16(tmem, make_smem_desc_sw128(a_addr + kk * 32, 16u, 1024u), make_smem_desc_sw128(b_addr + kk * 2048, 8192u, 1024u), idesc,
-                     (i | sub | kk) != 0 ? 1u : 0u);
+            umma_f16(d, make_smem_desc_sw128(a_addr + kk * 32, 16u, 1024u), make_smem_desc_sw128(b_addr + kk * 2048, 8192u, 1024u), idesc,
+                     (!first || (sub | kk) != 0) ? 1u : 0u);
         }
+        first = false;
         umma_commit(a_empty(sa));
         umma_commit(b_empty(sb));
+        if (--left == 0) umma_commit(acc_full(part & 1));
       }
-      if (ok) umma_commit(acc_full);
     }
-  } else if (warp >= 4) {
+  } else if (warp >= 4 && warp < EPI_WARP0) {
     const int tid = threadIdx.x - 128;                 // 0 .. 32*CONVERT_WARPS-1
     constexpr int WORDS_PER_THREAD = (SUB * BK * BN / 8) / (32 * CONVERT_WARPS);
     bool ok = true;
@@ -162,93 +180,110 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
                            mbar_wait(b_empty(s), ((i / B_STAGES) & 1) ^ 1, dead, g.status, 305);
       got = __shfl_sync(0xffffffffu, got, 0);
       if (!got) { ok = false; break; }
-      if (!(g.skip_convert & 1)) {
 #pragma unroll
-        for (int it = 0; it < WORDS_PER_THREAD; ++it) {
-          // word of the step: sub-tile, then row k = w / 16 (16 words = 128 columns), 8 columns per word
-          const int wi = it * (32 * CONVERT_WARPS) + tid, sub = wi >> 10, w = wi & 1023, k = w >> 4, jw = w & 15;
-          const uint8_t* tile = raw_s + (r * SUB + sub) * RAW_BYTES;
-          const uint32_t* raw = reinterpret_cast<const uint32_t*>(tile);
-          const float* scale = reinterpret_cast<const float*>(tile + NIB_BYTES);
-          const uint32_t b_addr = sB + (s * SUB + sub) * B_BYTES;
-          const uint32_t v = raw[w] ^ 0x88888888u;         // two's complement -> q + 8
-          const __nv_bfloat162 off = __float2bfloat162_rn(136.0f), sc = __float2bfloat162_rn(scale[2 * k + (jw >> 3)]);
-          uint32_t t[4];
+      for (int it = 0; it < WORDS_PER_THREAD; ++it) {
+        // word of the step: sub-tile, then row k = w / 16 (16 words = 128 columns), 8 columns per word
+        const int wi = it * (32 * CONVERT_WARPS) + tid, sub = wi >> 10, w = wi & 1023, k = w >> 4, jw = w & 15;
+        const uint8_t* tile = raw_s + (r * SUB + sub) * RAW_BYTES;
+        const uint32_t* raw = reinterpret_cast<const uint32_t*>(tile);
+        const float* scale = reinterpret_cast<const float*>(tile + NIB_BYTES);
+        const uint32_t b_addr = sB + (s * SUB + sub) * B_BYTES;
+        const uint32_t v = raw[w] ^ 0x88888888u;         // two's complement -> q + 8
+        const __nv_bfloat162 off = __float2bfloat162_rn(136.0f), sc = __float2bfloat162_rn(scale[2 * k + (jw >> 3)]);
+        uint32_t t[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t u = ((v >> (4 * j)) & 0x000F000Fu) | 0x43004300u;      // bf16 (128 + q + 8) for columns j and j + 4
-            __nv_bfloat162 h = __hmul2(__hsub2(*reinterpret_cast<__nv_bfloat162*>(&u), off), sc);
-            t[j] = *reinterpret_cast<uint32_t*>(&h);
-          }
-          // positions 0..7 of the chunk hold columns 0,4,1,5,2,6,3,7
-          const uint32_t dst = b_addr + (jw >> 3) * 8192u + sw128_offset((uint32_t)k, (uint32_t)(jw & 7));
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");
+        for (int j = 0; j < 4; ++j) {
+          uint32_t u = ((v >> (4 * j)) & 0x000F000Fu) | 0x43004300u;      // bf16 (128 + q + 8) for columns j and j + 4
+          __nv_bfloat162 h = __hmul2(__hsub2(*reinterpret_cast<__nv_bfloat162*>(&u), off), sc);
+          t[j] = *reinterpret_cast<uint32_t*>(&h);
         }
+        // positions 0..7 of the chunk hold columns 0,4,1,5,2,6,3,7
+        const uint32_t dst = b_addr + (jw >> 3) * 8192u + sw128_offset((uint32_t)k, (uint32_t)(jw & 7));
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");
       }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) { mbar_arrive(b_full(s)); mbar_arrive(raw_empty(r)); }
     }
-    // ---- epilogue (first four conversion warps): lane = output row inside the 128-row tile.
+  } else if (warp >= EPI_WARP0) {
+    // ---- epilogue: lane = output row inside the 128-row tile.
     // Accumulator positions j..j+7 of a group of 8 are columns j + {0,4,1,5,2,6,3,7}.
-    if (warp < 8 && ok && mbar_wait(acc_full, 0, dead, g.status, 306)) {
+    // Every thread goes through every part and its barriers, also after a wait that gave up (later waits return at once).
+    const int q = warp & 3, et = threadIdx.x - 32 * EPI_WARP0, row = m0 + q * 32 + lane;
+    bool ok = true;
+    int part = 0;
+    for (int i = 0; i < ksteps; ++part) {
+      const int nt = (int)(line(i) / k_tiles), n0 = nt * BN, a = part & 1;
+      // CTAs that share a left-over tile: that of its step x is the largest c with rest c / sharers <= x
+      const long long lo = nt < whole ? 0 : ((nt - whole) * k_tiles * sharers + sharers - 1) / rest;
+      const long long hi = nt < whole ? 0 : ((nt + 1 - whole) * k_tiles * sharers - 1) / rest;
+      i += part_steps(i);
+      ok = __all_sync(0xffffffffu, mbar_wait(acc_full(a), (part >> 1) & 1, dead, g.status, 306)) && ok;
       tc_fence_after();
-      const int row = m0 + (warp & 3) * 32 + lane;
+      if (ok) {
 #pragma unroll 1
-      for (int c = 0; c < BN; c += 32) {
-        uint32_t rr[32];
-        tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c, rr);
-        tmem_ld_wait();
-        if (row >= g.M) continue;
-        if (g.splits == 1) {
-          __nv_bfloat16* dstp = g.out + (long long)row * g.ldo + n0 + c;
+        for (int c = 0; c < BN; c += 32) {
+          uint32_t rr[32];
+          __syncwarp();
+          tmem_ld32(tmem + a * BN + ((uint32_t)(q * 32) << 16) + c, rr);
+          tmem_ld_wait();
+          if (row >= g.M) continue;
+          if (lo == hi) {
+            __nv_bfloat16* dstp = g.out + (long long)row * g.ldo + n0 + c;
 #pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            float v[8] = {__uint_as_float(rr[j]), __uint_as_float(rr[j + 2]), __uint_as_float(rr[j + 4]), __uint_as_float(rr[j + 6]),
-                          __uint_as_float(rr[j + 1]), __uint_as_float(rr[j + 3]), __uint_as_float(rr[j + 5]), __uint_as_float(rr[j + 7])};
-            if (g.bias) {
+            for (int j = 0; j < 32; j += 8) {
+              float v[8] = {__uint_as_float(rr[j]), __uint_as_float(rr[j + 2]), __uint_as_float(rr[j + 4]), __uint_as_float(rr[j + 6]),
+                            __uint_as_float(rr[j + 1]), __uint_as_float(rr[j + 3]), __uint_as_float(rr[j + 5]), __uint_as_float(rr[j + 7])};
+              if (g.bias) {
 #pragma unroll
-              for (int e = 0; e < 8; ++e) v[e] += __bfloat162float(g.bias[n0 + c + j + e]);
+                for (int e = 0; e < 8; ++e) v[e] += __bfloat162float(g.bias[n0 + c + j + e]);
+              }
+              uint4 pk = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+              *reinterpret_cast<uint4*>(dstp + j) = pk;
             }
-            uint4 pk = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
-            *reinterpret_cast<uint4*>(dstp + j) = pk;
-          }
-        } else {
-          float* dstp = g.acc + (long long)row * g.N + n0 + c;
+          } else {
+            float* dstp = g.acc + (long long)row * g.N + n0 + c;
 #pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            red_add_f32x4(dstp + j, __uint_as_float(rr[j]), __uint_as_float(rr[j + 2]), __uint_as_float(rr[j + 4]), __uint_as_float(rr[j + 6]));
-            red_add_f32x4(dstp + j + 4, __uint_as_float(rr[j + 1]), __uint_as_float(rr[j + 3]), __uint_as_float(rr[j + 5]), __uint_as_float(rr[j + 7]));
+            for (int j = 0; j < 32; j += 8) {
+              red_add_f32x4(dstp + j, __uint_as_float(rr[j]), __uint_as_float(rr[j + 2]), __uint_as_float(rr[j + 4]), __uint_as_float(rr[j + 6]));
+              red_add_f32x4(dstp + j + 4, __uint_as_float(rr[j + 1]), __uint_as_float(rr[j + 3]), __uint_as_float(rr[j + 5]), __uint_as_float(rr[j + 7]));
+            }
           }
         }
       }
-      if (g.splits > 1) __threadfence();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty(a));
+      if (lo == hi) continue;
+      // the CTA that arrives last at the tile's counter turns the fp32 sums into the output
+      __threadfence();
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      int* counter = g.counters + mt * n_tiles + nt;
+      if (et == 0) *is_last = (atomicAdd(counter, 1) == (int)(hi - lo)) && !*dead;
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (*is_last) {
+        __threadfence();
+        const int rows = min(BM, g.M - m0);
+        for (int e = et; e < rows * (BN / 4); e += 128) {
+          const int r = e / (BN / 4), c4 = (e % (BN / 4)) * 4;
+          float4* src = reinterpret_cast<float4*>(g.acc + (long long)(m0 + r) * g.N + n0 + c4);
+          float4 v = __ldcg(src);
+          *src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (g.bias) {
+            v.x += __bfloat162float(g.bias[n0 + c4]); v.y += __bfloat162float(g.bias[n0 + c4 + 1]);
+            v.z += __bfloat162float(g.bias[n0 + c4 + 2]); v.w += __bfloat162float(g.bias[n0 + c4 + 3]);
+          }
+          *reinterpret_cast<uint2*>(g.out + (long long)(m0 + r) * g.ldo + n0 + c4) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+        }
+        if (et == 0) *counter = 0;
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");        // is_last has been read
     }
   }
+  if (*dead) __nanosleep(100000);
   tc_fence_before();
   __syncthreads();
-  if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, BN); }
-  if (g.splits > 1) {
-    // the split that arrives last at the tile's counter turns the fp32 sums into the output
-    if (threadIdx.x == 0) *is_last = (atomicAdd(g.counters + mt * n_tiles + nt, 1) == g.splits - 1) && !*dead;
-    __syncthreads();
-    if (*is_last) {
-      __threadfence();
-      const int rows = min(BM, g.M - m0);
-      for (int i = threadIdx.x; i < rows * (BN / 4); i += THREADS) {
-        const int r = i / (BN / 4), c4 = (i % (BN / 4)) * 4;
-        float4* src = reinterpret_cast<float4*>(g.acc + (long long)(m0 + r) * g.N + n0 + c4);
-        float4 v = __ldcg(src);
-        *src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (g.bias) {
-          v.x += __bfloat162float(g.bias[n0 + c4]); v.y += __bfloat162float(g.bias[n0 + c4 + 1]);
-          v.z += __bfloat162float(g.bias[n0 + c4 + 2]); v.w += __bfloat162float(g.bias[n0 + c4 + 3]);
-        }
-        *reinterpret_cast<uint2*>(g.out + (long long)(m0 + r) * g.ldo + n0 + c4) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
-      }
-      if (threadIdx.x == 0) g.counters[mt * n_tiles + nt] = 0;
-    }
-  }
+  if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, 2 * BN); }
 }
 
 // packed [K][N/2] bytes + scales (flat groups) -> tiles [N/128][K/64][4608]
@@ -299,19 +334,22 @@ CGK_API int cgk_int4_gemm(const void* x, long long ldx, const void* w_tiles, flo
   int dev = 0;
   CGK_CUDA_CHECK(cudaGetDevice(&dev));
   const int sms = sm_count(dev), n_tiles = N / BN, m_tiles = (M + BM - 1) / BM, ksteps = K / (SUB * BK);
-  if (splits <= 0) {
-    // one wave: the largest power-of-two split whose CTAs all fit on the SMs at once (a second,
-    // partly filled wave measured slower than fewer, longer CTAs), at least 2 steps per CTA
-    splits = 1;
-    const int max_s = (acc && counters) ? 16 : 1;
-    for (int s = 2; s <= max_s && ksteps % s == 0 && ksteps / s >= 2 && n_tiles * m_tiles * s <= sms; s *= 2) splits = s;
+  CGK_REQUIRE(splits <= 0 || ksteps % splits == 0, "cgk_int4_gemm: K/128 = %d is not divisible by splits = %d", ksteps, splits);
+  CGK_REQUIRE(splits <= 1 || (acc && counters), "cgk_int4_gemm: split-K needs the acc and counters buffers");
+  // one CTA per SM, with at least two steps each; given splits, or no scratch to meet in: whole tiles or equal parts of them
+  const long long total = (long long)n_tiles * ksteps;
+  long long ctas = (long long)n_tiles * (splits > 0 ? splits : 1);
+  if (splits <= 0 && acc && counters) {
+    ctas = sms / m_tiles;
+    if (ctas > total / 2) ctas = total / 2;
+    if (ctas < 1) ctas = 1;
   }
-  CGK_REQUIRE(ksteps % splits == 0, "cgk_int4_gemm: K/128 = %d is not divisible by splits = %d", ksteps, splits);
-  CGK_REQUIRE(splits == 1 || (acc && counters), "cgk_int4_gemm: split-K needs the acc and counters buffers");
   const int a_rows = m_tiles > 1 ? BM : (M + 7) / 8 * 8;
-  // the X ring gets up to a quarter of the ring budget (at least 2 stages), the W ring the rest
+  // X comes from L2 a microsecond after it is asked for: four stages of it, as long as five of W fit beside them (at least 2),
+  // and up to a quarter of the ring budget where rows are few
   int a_stages = (RING_BUDGET / 4) / (SUB * a_rows * 128);
-  if (a_stages < 2) a_stages = 2;
+  if (a_stages < 4) a_stages = 4;
+  while (a_stages > 2 && RING_BUDGET - a_stages * SUB * a_rows * 128 < 5 * SUB * RAW_BYTES) --a_stages;
   if (a_stages > MAX_A_STAGES) a_stages = MAX_A_STAGES;
   int raw_stages = (RING_BUDGET - a_stages * SUB * a_rows * 128) / (SUB * RAW_BYTES);
   if (raw_stages > MAX_RAW_STAGES) raw_stages = MAX_RAW_STAGES;
@@ -325,10 +363,9 @@ CGK_API int cgk_int4_gemm(const void* x, long long ldx, const void* w_tiles, flo
     CGK_CUDA_CHECK(cudaFuncSetAttribute(int4_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     attr_set[dev] = true;
   }
-  static const int skip_convert = getenv("CGK_INT4_SKIP_CONVERT") ? atoi(getenv("CGK_INT4_SKIP_CONVERT")) : 0;
   Int4Dev g{(const uint8_t*)w_tiles, acc, counters, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)bias, M, N, K,
-            splits, ksteps / splits, a_rows, a_stages, raw_stages, skip_convert, device_status(dev)};
-  int4_gemm_kernel<<<dim3(n_tiles * splits, m_tiles), THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(tmX, g);
+            a_rows, a_stages, raw_stages, device_status(dev)};
+  int4_gemm_kernel<<<dim3((unsigned)ctas, m_tiles), THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(tmX, g);
   CGK_LAUNCH_CHECK();
   return 0;
 }
