@@ -14,8 +14,8 @@
 //     written straight into tensor memory (tcgen05.st); the MMA reads A from TMEM and only the
 //     small X tile from shared memory;
 //   * a warp-specialised pipeline of five roles chained by mbarriers spent ~1000 cycles per
-//     128-k step on the hand-offs alone.  Here every thread does the same work per step and two
-//     block barriers order it; two CTAs per SM overlap one CTA's barriers with the other's loads;
+//     128-k step on the hand-offs alone.  Here every conversion warp does the same work per step and
+//     meets the others only in the MMA warp's barriers; two CTAs per SM overlap their waits;
 //   * the tensor core multiplies 128 features by round_up(M, 16) token columns per instruction,
 //     so its time shrinks with the batch;
 //   * the scale of a weight depends on (k, n / group).  With group % 128 == 0 a CTA's 128 features
@@ -142,7 +142,6 @@ int4_wa_kernel(const WaDev g) {
   volatile int* dead = reinterpret_cast<volatile int*>(misc + 64);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc + 68);
   volatile int* is_last = reinterpret_cast<volatile int*>(misc + 72);
-  volatile int* go_s = reinterpret_cast<volatile int*>(misc + 76);   // [2], by step parity
   auto a_full = [&](int s) { return sBar + 8u * s; };
   auto a_empty = [&](int s) { return sBar + 8u * (W_STAGES + s); };
   const uint32_t acc_full = sBar + 8u * 2 * W_STAGES;
@@ -261,11 +260,11 @@ int4_wa_kernel(const WaDev g) {
       for (int d = 0; d < W_PREFETCH; ++d) {
         const int i = i0 + d;
         if (i >= steps) break;
-        // stage s (TMEM operand columns and the X' tile) was last read by the MMAs of step i - W_STAGES;
-        // one thread polls, a hardware barrier releases the rest
-        if (tid == 0) go_s[d & 1] = (int)mbar_wait(a_empty(s), par, dead, g.status, 330);
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (!go_s[d & 1]) ok = false;
+        // stage s (TMEM operand columns and the X' tile) was last read by the MMAs of step i - W_STAGES; one lane polls for its
+        // warp, and the warps keep their own pace: a barrier of all of them in every step held each to the slowest
+        int got = 1;
+        if (lane == 0) got = (int)mbar_wait(a_empty(s), par, dead, g.status, 330);
+        if (!__shfl_sync(0xffffffffu, got, 0)) ok = false;
         tc_fence_after();
         // nibbles -> bf16 pairs -> 32 TMEM columns of this feature's lane
 #pragma unroll
@@ -323,8 +322,9 @@ int4_wa_kernel(const WaDev g) {
           ++part;
           tc_fence_before();
           asm volatile("bar.sync 2, 288;" ::: "memory");
-          if (tid < 128) xsum_s[tid] = 0.0f;                         // used again behind the next step's barrier
+          if (tid < 128) xsum_s[tid] = 0.0f;
           if (lo != hi) wa_finish_tile(g, m0, mt, nt, (int)(hi - lo), is_last, dead);
+          asm volatile("bar.sync 1, 256;" ::: "memory");             // row sums and is_last can be used again
           left = i + 1 < steps ? part_steps(i + 1) : 0;
         }
       }

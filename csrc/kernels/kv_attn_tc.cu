@@ -61,11 +61,13 @@ __device__ __forceinline__ uint4 kvt_convert(uint32_t w, __nv_bfloat162 s2) {
 
 template <int N>
 __device__ __forceinline__ void kvt_tmem_ld(uint32_t taddr, uint32_t (&r)[N]) {
-  if constexpr (N == 16) tmem_ld16(taddr, r); else tmem_ld32(taddr, r);
+  if constexpr (N == 8) tmem_ld8(taddr, r);
+  else if constexpr (N == 16) tmem_ld16(taddr, r);
+  else tmem_ld32(taddr, r);
 }
 
 template <int NP>
-__global__ void __launch_bounds__(KVT_THREADS, NP == 32 ? 2 : 1)
+__global__ void __launch_bounds__(KVT_THREADS, NP <= 32 ? 2 : 1)
 kv_attention_tc_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, int Tq, int Hq, float scale_log2, int splits,
                        float* __restrict__ part_acc, float* __restrict__ part_ml, int* status) {
   using S = KvtSmem<NP>;
@@ -83,7 +85,7 @@ kv_attention_tc_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, int Tq, int
   volatile int* go = reinterpret_cast<volatile int*>(sm + S::OFF_MISC + 8);      // [2] "the wait succeeded"
   const uint32_t bar_s = sb + S::OFF_BAR, bar_o = bar_s + 8;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, half = warp >> 2;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31, quad = warp & 3, half = warp >> 2;
   const int split = blockIdx.x % splits, pass = blockIdx.x / splits, hk = blockIdx.y, b = blockIdx.z;
   const int rep = Hq / c.heads, R = Tq * rep, r0 = pass * NP, rows = min(NP, R - r0);
   const int len = c.lengths[b] + Tq;                        // the Tq new tokens were appended before the call
@@ -158,7 +160,7 @@ kv_attention_tc_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, int Tq, int
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after();
 #pragma unroll
       for (int kk = 0; kk < D / 16; ++kk)
@@ -220,7 +222,7 @@ kv_attention_tc_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, int Tq, int
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after();
 #pragma unroll
       for (int kk = 0; kk < KVT_KB / 16; ++kk)
@@ -280,6 +282,7 @@ cudaError_t launch_np(const KvDev& c, const __nv_bfloat16* q, int Tq, int Hq, fl
 cudaError_t launch_kv_attention_tc(const KvDev& c, const __nv_bfloat16* q, int Tq, int Hq, float scale, int splits,
                                    float* part_acc, float* part_ml, int* status, cudaStream_t stream) {
   const int R = Tq * (Hq / c.heads);
+  if (R <= 16) return launch_np<16>(c, q, Tq, Hq, scale, splits, 1, part_acc, part_ml, status, stream);
   if (R <= 32) return launch_np<32>(c, q, Tq, Hq, scale, splits, 1, part_acc, part_ml, status, stream);
   return launch_np<64>(c, q, Tq, Hq, scale, splits, (R + 63) / 64, part_acc, part_ml, status, stream);
 }
