@@ -154,6 +154,12 @@ struct GemmSmem {
   static_assert(TOTAL <= 227 * 1024, "GEMM: shared memory budget of one CTA exceeded");
 };
 
+// What the epilogue of a kernel does: EPI_ANY reads it from the arguments; the other forms are fixed at compile time (a sum of
+// terms, applied in this order) for a bf16 output with alpha 1 whose rows take bulk stores and whose columns are a multiple of
+// 32, a bf16 bias, and inputs that come by bulk loads.  With the code of every form in one loop a chunk of 32 columns took
+// 2000 cycles, 1000 of them for a hundred instructions of arithmetic: the warps waited for instructions.
+enum EpiForm : int { EPI_ANY = -1, EPI_PLAIN = 0, EPI_BIAS = 1, EPI_AUX_OUT = 2, EPI_GELU = 4, EPI_DGELU = 8, EPI_RESIDUAL = 16 };
+
 // tiles_m: g.tiles_m, or the number of row tiles in use (grouped product)
 __device__ __forceinline__ void tile_coords(const GemmDev& g, int tiles_m, int t, int& b, int& tm, int& tn) {
   const int per_batch = tiles_m * g.tiles_n;
@@ -182,7 +188,7 @@ __device__ __forceinline__ void tile_coords(const GemmDev& g, int tiles_m, int t
 // PAIR: a cluster of two CTAs computes a 256 x BN tile.  Each CTA loads its 128 rows of A and half of B's rows and
 // drains its 128 rows of the accumulator; the MMAs read both halves of B, so a stage is 32 KiB instead of 48 at
 // BN = 256 (six stages instead of four) and the operand bytes per MMA fall by a third.
-template <int BN, int STAGES, bool GROUPED = false, bool PAIR = false>
+template <int BN, int STAGES, bool GROUPED = false, bool PAIR = false, int EPI = EPI_ANY>
 __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& tmA, const CUtensorMap& tmB,
                                              const CUtensorMap* tmC, const CUtensorMap* tmAux,
                                              const CUtensorMap* tmIn,

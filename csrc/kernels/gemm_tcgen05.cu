@@ -18,33 +18,33 @@
 
 namespace cgk {
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, int EPI = EPI_ANY>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAux,
                     const __grid_constant__ CUtensorMap tmIn, const GemmDev g) {
   extern __shared__ uint8_t smem_raw[];
-  gemm_tc_body<BN, STAGES>(tmA, tmB, &tmC, &tmAux, &tmIn, g, (int)blockIdx.x, (int)gridDim.x, smem_raw);
+  gemm_tc_body<BN, STAGES, false, false, EPI>(tmA, tmB, &tmC, &tmAux, &tmIn, g, (int)blockIdx.x, (int)gridDim.x, smem_raw);
 }
 
 // The same by CTA pairs: 256 x BN tiles, one cluster of two CTAs per tile.
-template <int BN, int STAGES>
+template <int BN, int STAGES, int EPI = EPI_ANY>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAux,
                       const __grid_constant__ CUtensorMap tmIn, const GemmDev g) {
   extern __shared__ uint8_t smem_raw[];
-  gemm_tc_body<BN, STAGES, false, true>(tmA, tmB, &tmC, &tmAux, &tmIn, g, (int)blockIdx.x >> 1, (int)gridDim.x >> 1, smem_raw);
+  gemm_tc_body<BN, STAGES, false, true, EPI>(tmA, tmB, &tmC, &tmAux, &tmIn, g, (int)blockIdx.x >> 1, (int)gridDim.x >> 1, smem_raw);
 }
 
 // Grouped product: the rows of A lie in expert order, every expert's segment starts on a row tile, and the
 // number of row tiles is known on the device only.
-template <int BN, int STAGES>
+template <int BN, int STAGES, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const __grid_constant__ CUtensorMap tmC, const GemmDev g) {
   extern __shared__ uint8_t smem_raw[];
-  gemm_tc_body<BN, STAGES, true>(tmA, tmB, &tmC, &tmC, &tmC, g, (int)blockIdx.x, (int)gridDim.x, smem_raw);
+  gemm_tc_body<BN, STAGES, true, false, EPI>(tmA, tmB, &tmC, &tmC, &tmC, g, (int)blockIdx.x, (int)gridDim.x, smem_raw);
 }
 
 // CUDA-core fallback for operands that TMA cannot address (leading dimension not a
@@ -215,31 +215,68 @@ int pick_bn(const cgk_gemm_args& a, int ctas) {
 
 constexpr int PAIR_BN = 256, PAIR_STAGES = 6;
 
-static int launch_pair(const cgk_gemm_args& a, const GemmDev& g0, int ctas, cudaStream_t stream) {
-  using L = GemmSmem<PAIR_BN, PAIR_STAGES, true>;
+// The fixed form of the epilogue that these arguments ask for (a sum of EpiForm terms), or EPI_ANY.
+static int epi_form(const cgk_gemm_args& a, const GemmDev& g) {
+  if (!g.tma_store || a.alpha != 1.0f || a.N % 32 != 0 || (a.bias && a.bias_fp32) || (a.act != CGK_ACT_NONE && a.act != CGK_ACT_GELU)) return EPI_ANY;
+  if (a.residual && (a.ldr % 8 != 0 || g.tma_in != 2)) return EPI_ANY;
+  if (a.aux_in && (a.dact != CGK_ACT_GELU || g.tma_in != 1)) return EPI_ANY;
+  return (a.bias ? EPI_BIAS : 0) | (a.aux_out ? EPI_AUX_OUT : 0) | (a.act ? EPI_GELU : 0) | (a.aux_in ? EPI_DGELU : 0) | (a.residual ? EPI_RESIDUAL : 0);
+}
+
+using GemmKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GemmDev);
+// The kernel for a 256-wide tile: the forms that training steps and prompts use are compiled for themselves.
+template <bool PAIR, int EPI>
+static GemmKernel wide_kernel() {
+  if constexpr (PAIR) return gemm_bf16_pair_kernel<PAIR_BN, PAIR_STAGES, EPI>;
+  else return gemm_bf16_tc_kernel<256, 4, EPI>;
+}
+template <bool PAIR>
+static GemmKernel pick_wide_kernel(int form) {
+  switch (form) {
+    case EPI_PLAIN: return wide_kernel<PAIR, EPI_PLAIN>();
+    case EPI_BIAS: return wide_kernel<PAIR, EPI_BIAS>();
+    case EPI_BIAS | EPI_AUX_OUT | EPI_GELU: return wide_kernel<PAIR, EPI_BIAS | EPI_AUX_OUT | EPI_GELU>();
+    case EPI_DGELU: return wide_kernel<PAIR, EPI_DGELU>();
+    case EPI_RESIDUAL: return wide_kernel<PAIR, EPI_RESIDUAL>();
+    case EPI_BIAS | EPI_RESIDUAL: return wide_kernel<PAIR, EPI_BIAS | EPI_RESIDUAL>();
+    default: return wide_kernel<PAIR, EPI_ANY>();
+  }
+}
+
+// 256-wide tiles, by single CTAs (128 rows) or by pairs (256 rows); ctas: SMs to use
+template <bool PAIR>
+static int launch_wide(const cgk_gemm_args& a, const GemmDev& g0, int ctas, cudaStream_t stream) {
+  constexpr int SMEM = PAIR ? GemmSmem<PAIR_BN, PAIR_STAGES, true>::TOTAL : GemmSmem<256, 4>::TOTAL;
+  constexpr int CL = PAIR ? 2 : 1;
   GemmDev g = g0;
-  g.tiles_m = (a.M + 2 * BM - 1) / (2 * BM);
+  g.tiles_m = (a.M + CL * BM - 1) / (CL * BM);
   g.tiles_n = (a.N + PAIR_BN - 1) / PAIR_BN;
   CUtensorMap tmA, tmB, tmC, tmAux, tmIn;
-  int rc = make_gemm_tmaps(a, PAIR_BN / 2, &tmA, &tmB);        // a CTA loads half of B's rows
+  int rc = make_gemm_tmaps(a, PAIR_BN / CL, &tmA, &tmB);        // a CTA of a pair loads half of B's rows
   if (rc) return rc;
   int out_ok = 0, in_kind = 0;
   if ((rc = make_gemm_out_tmaps(a, &tmC, &tmAux, &tmIn, &out_ok, &in_kind))) return rc;
   g.tma_store = (out_ok && g.split_k == 1) ? 1 : 0;
   g.tma_in = g.tma_store ? in_kind : 0;
-  CGK_CUDA_CHECK(cudaFuncSetAttribute(gemm_bf16_pair_kernel<PAIR_BN, PAIR_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
-  const int total = g.batch * g.tiles_m * g.tiles_n * g.split_k, pairs = ctas / 2;
-  gemm_bf16_pair_kernel<PAIR_BN, PAIR_STAGES><<<2 * (total < pairs ? total : pairs), GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, tmC, tmAux, tmIn, g);
+  const GemmKernel kernel = pick_wide_kernel<PAIR>(epi_form(a, g));
+  CGK_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+  const int total = g.batch * g.tiles_m * g.tiles_n * g.split_k, units = ctas / CL;
+  kernel<<<CL * (total < units ? total : units), GEMM_THREADS, SMEM, stream>>>(tmA, tmB, tmC, tmAux, tmIn, g);
   CGK_LAUNCH_CHECK();
   return 0;
 }
 
-// Pairs or single CTAs for a 256-wide tile.  Pairs wherever the main loop is what a tile waits for (22016 x 4096, 8176 rows:
-// 1035 -> 935 us; weight gradient 50304 x 768 over 32768 rows 1778 -> 1771) and where many tiles stream wide outputs
-// (32768 x 50304 x 768: 2606 -> 2469 us); with K below 1024 and fewer columns the epilogue bounds the tile, and two CTAs
-// waiting for each other's cost a little (32768 x 2304 x 768: 125 / 133 us).
+// Pairs or single CTAs for a 256-wide tile (single / pair, us, timed in turn).  Pairs where the main loop is what a tile waits
+// for: 8176 x 22016 x 4096 1029 / 929, weight gradient 3072 x 768 over 131 072 rows 450 / 421; with K below 1024 where the
+// epilogue is light and there are tiles for two rounds: 131072 x 2304 x 768 409 / 372, 32768 x 50304 x 768 2154 / 1911, but
+// with GELU' 613 / 650 and 5555 x 768 x 768 19.4 / 21.2.  A single round of tiles pays for a pair's longer start unless K is long
+// (5555 x 768 x 2304 24.6 / 26.7, x 3072 31.7 / 31.8, 1000 x 4096 x 11008 87 / 77), and few rows for its taller tile
+// (300 x 22016 x 4096 70.5 / 79.9, 520 rows 95 / 101, 1000 rows 151 / 132).
 static bool by_pairs(const cgk_gemm_args& a, int ctas) {
-  return ctas >= 2 && a.M > BM && (a.K >= 1024 || a.N >= 8192);
+  if (ctas < 2 || a.M <= 6 * BM) return false;
+  const long long tiles = (long long)a.batch * ((a.M + 2 * BM - 1) / (2 * BM)) * ((a.N + PAIR_BN - 1) / PAIR_BN), pairs = ctas / 2;
+  if (a.K < 1024) return !a.act && !a.aux_in && !a.aux_out && tiles >= 2 * pairs;
+  return tiles > pairs || a.K >= 3072;
 }
 
 template <int BN, int STAGES>
@@ -281,9 +318,10 @@ static int launch_grouped(const cgk_gemm_args& a, const GemmDev& g0, int sms, cu
   int out_ok = 0, in_kind = 0;
   if ((rc = make_gemm_out_tmaps(one, &tmC, &tmAux, &tmIn, &out_ok, &in_kind))) return rc;
   g.tma_store = out_ok ? 1 : 0;
-  CGK_CUDA_CHECK(cudaFuncSetAttribute(gemm_bf16_grouped_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
+  const auto kernel = epi_form(one, g) == EPI_PLAIN ? gemm_bf16_grouped_kernel<BN, STAGES, EPI_PLAIN> : gemm_bf16_grouped_kernel<BN, STAGES, EPI_ANY>;
+  CGK_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL));
   const int total = g.tiles_m * g.tiles_n;
-  gemm_bf16_grouped_kernel<BN, STAGES><<<total < sms ? total : sms, GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, tmC, g);
+  kernel<<<total < sms ? total : sms, GEMM_THREADS, L::TOTAL, stream>>>(tmA, tmB, tmC, g);
   CGK_LAUNCH_CHECK();
   return 0;
 }
@@ -362,7 +400,7 @@ CGK_API int cgk_gemm_bf16(const cgk_gemm_args* pa, void* stream_) {
       g.kb_per_split = (kblocks + S - 1) / S;
       g.split_k = (kblocks + g.kb_per_split - 1) / g.kb_per_split;     // no empty slice
       switch (bn) {
-        case 256: return by_pairs(a, ctas) ? launch_pair(a, g, ctas, stream) : launch_tc<256, 4>(a, g, sms, stream);
+        case 256: return by_pairs(a, ctas) ? launch_wide<true>(a, g, ctas, stream) : launch_wide<false>(a, g, ctas, stream);
         case 128: return launch_tc<128, 6>(a, g, sms, stream);
         default: return launch_tc<64, 8>(a, g, sms, stream);
       }
@@ -371,7 +409,7 @@ CGK_API int cgk_gemm_bf16(const cgk_gemm_args* pa, void* stream_) {
   FewPlan few;
   if (gemm_few_plan(a, ctas, &few)) return launch_gemm_few(a, g, few, stream);
   switch (pick_bn(a, a.max_ctas > 0 ? a.max_ctas : sms)) {
-    case 256: return by_pairs(a, ctas) ? launch_pair(a, g, ctas, stream) : launch_tc<256, 4>(a, g, sms, stream);
+    case 256: return by_pairs(a, ctas) ? launch_wide<true>(a, g, ctas, stream) : launch_wide<false>(a, g, ctas, stream);
     case 128: return launch_tc<128, 6>(a, g, sms, stream);
     default: return launch_tc<64, 8>(a, g, sms, stream);
   }
