@@ -95,36 +95,72 @@ struct AdamHyper {
   float max_grad_norm;  // <= 0: no clipping
 };
 
+struct AdamStep { float inv_scale, bc1, bc2, decay; };
+__device__ __forceinline__ float adam_update(float pv, float& m, float& v, float g, const AdamHyper& h, const AdamStep& a) {
+  const float gr = g * a.inv_scale;
+  if (h.weight_decay > 0.0f) pv *= a.decay;
+  m = h.beta1 * m + (1.0f - h.beta1) * gr;
+  v = h.beta2 * v + (1.0f - h.beta2) * gr * gr;
+  return pv - h.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + h.eps);
+}
+
+// 30 bytes per parameter and nothing read twice.  vec: all pointers take four elements per access (16 bytes; 8 of p16); two
+// such groups per thread are in flight before the arithmetic, whose three divisions and square root are long.
+// 661 M parameters: 3.90 ms by single elements, 3.53 like this (5.6 TB/s).
 __global__ void __launch_bounds__(256)
 adam_step_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
-                 const float* __restrict__ g, __nv_bfloat16* __restrict__ p16, long long n,
+                 const float* __restrict__ g, __nv_bfloat16* __restrict__ p16, long long n, int vec,
                  AdamHyper h, const ScalerState* __restrict__ st) {
-  float inv_scale = 1.0f;
+  AdamStep a;
+  a.inv_scale = 1.0f;
   int t = 1;
   if (st) {
     if (st->found_inf) return;
-    inv_scale = 1.0f / st->scale;
+    a.inv_scale = 1.0f / st->scale;
     t = st->step + 1;
     if (h.max_grad_norm > 0.0f) {
-      float norm = sqrtf(st->norm_sq) * inv_scale;
-      if (norm > h.max_grad_norm) inv_scale *= h.max_grad_norm / (norm + 1e-6f);
+      float norm = sqrtf(st->norm_sq) * a.inv_scale;
+      if (norm > h.max_grad_norm) a.inv_scale *= h.max_grad_norm / (norm + 1e-6f);
     }
   }
-  const float bc1 = 1.0f - powf(h.beta1, (float)t);
-  const float bc2 = 1.0f - powf(h.beta2, (float)t);
-  const float decay = 1.0f - h.lr * h.weight_decay;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const float gr = g[i] * inv_scale;
-    float pv = p[i];
-    if (h.weight_decay > 0.0f) pv *= decay;
-    const float mi = h.beta1 * m[i] + (1.0f - h.beta1) * gr;
-    const float vi = h.beta2 * v[i] + (1.0f - h.beta2) * gr * gr;
+  a.bc1 = 1.0f - powf(h.beta1, (float)t);
+  a.bc2 = 1.0f - powf(h.beta2, (float)t);
+  a.decay = 1.0f - h.lr * h.weight_decay;
+  const long long start = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+  const long long n4 = vec ? n >> 2 : 0;
+  constexpr int U = 2;
+  for (long long i = start; i < n4; i += stride * U) {
+    float4 gv[U], pv[U], mv[U], vv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long at = i + u * stride;
+      if (at >= n4) break;
+      gv[u] = reinterpret_cast<const float4*>(g)[at];
+      pv[u] = reinterpret_cast<const float4*>(p)[at];
+      mv[u] = reinterpret_cast<const float4*>(m)[at];
+      vv[u] = reinterpret_cast<const float4*>(v)[at];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long at = i + u * stride;
+      if (at >= n4) break;
+      pv[u].x = adam_update(pv[u].x, mv[u].x, vv[u].x, gv[u].x, h, a);
+      pv[u].y = adam_update(pv[u].y, mv[u].y, vv[u].y, gv[u].y, h, a);
+      pv[u].z = adam_update(pv[u].z, mv[u].z, vv[u].z, gv[u].z, h, a);
+      pv[u].w = adam_update(pv[u].w, mv[u].w, vv[u].w, gv[u].w, h, a);
+      reinterpret_cast<float4*>(m)[at] = mv[u];
+      reinterpret_cast<float4*>(v)[at] = vv[u];
+      reinterpret_cast<float4*>(p)[at] = pv[u];
+      if (p16) reinterpret_cast<uint2*>(p16)[at] = make_uint2(pack_bf16x2(pv[u].x, pv[u].y), pack_bf16x2(pv[u].z, pv[u].w));
+    }
+  }
+  for (long long i = (n4 << 2) + start; i < n; i += stride) {
+    float mi = m[i], vi = v[i];
+    const float pn = adam_update(p[i], mi, vi, g[i], h, a);
     m[i] = mi;
     v[i] = vi;
-    pv -= h.lr * (mi / bc1) / (sqrtf(vi / bc2) + h.eps);
-    p[i] = pv;
-    if (p16) p16[i] = __float2bfloat16(pv);
+    p[i] = pn;
+    if (p16) p16[i] = __float2bfloat16(pn);
   }
 }
 
@@ -241,8 +277,9 @@ CGK_API int cgk_adam_step(float* p, float* m, float* v, const float* g, void* p1
   CGK_REQUIRE(p && m && v && g, "cgk_adam_step: null pointer");
   if (n == 0) return 0;
   AdamHyper h{lr, beta1, beta2, eps, weight_decay, max_grad_norm};
-  adam_step_kernel<<<flat_grid(n, 256), 256, 0, (cudaStream_t)stream>>>(
-      p, m, v, g, (__nv_bfloat16*)p16, n, h, (const ScalerState*)state);
+  const int vec = (((uintptr_t)p | (uintptr_t)m | (uintptr_t)v | (uintptr_t)g) & 15) == 0 && ((uintptr_t)p16 & 7) == 0;
+  adam_step_kernel<<<flat_grid(vec ? (n + 3) / 4 : n, 256), 256, 0, (cudaStream_t)stream>>>(
+      p, m, v, g, (__nv_bfloat16*)p16, n, vec, h, (const ScalerState*)state);
   CGK_LAUNCH_CHECK();
   return 0;
 }
