@@ -37,27 +37,28 @@ flash_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __r
                    long long do_ts, long long do_hs) {
   constexpr int LPR = D / 8;                 // lanes per row
   constexpr int U = 4;
-  const long long rows = (long long)B * T * H;            // row r = (b * T + t) * H + h
-  const long long groups = (long long)gridDim.x * blockDim.x / LPR;
-  const long long g0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LPR;
+  // 32-bit indexes (the host checks): with 64-bit divisions by H and T the index took longer than the loads
+  const uint32_t rows = (uint32_t)B * T * H;              // row r = (b * T + t) * H + h
+  const uint32_t groups = gridDim.x * blockDim.x / LPR;
+  const uint32_t g0 = (blockIdx.x * blockDim.x + threadIdx.x) / LPR;
   const int c = ((int)threadIdx.x % LPR) * 8;
-  for (long long r0 = g0; r0 < rows; r0 += groups * U) {
+  for (uint32_t r0 = g0; r0 < rows; r0 += groups * U) {
     uint4 a[U], g[U];
+    uint32_t at[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const long long r = r0 + u * groups;
+      const uint32_t r = r0 + u * groups;
+      at[u] = 0;
       if (r < rows) {
-        const int h = (int)(r % H);
-        const long long bt = r / H;
-        const int t = (int)(bt % T);
-        const long long b = bt / T;
+        const uint32_t bt = r / H, h = r - bt * H, b = bt / T, t = bt - b * T;
         a[u] = __ldg(reinterpret_cast<const uint4*>(O + b * o_bs + t * o_ts + h * o_hs + c));
         g[u] = __ldg(reinterpret_cast<const uint4*>(dO + b * do_bs + t * do_ts + h * do_hs + c));
+        at[u] = (b * H + h) * T + t;
       }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const long long r = r0 + u * groups;
+      const uint32_t r = r0 + u * groups;
       float s = 0.0f;
       if (r < rows) {
         float2 x, y;
@@ -68,31 +69,45 @@ flash_delta_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bfloat16* __r
       }
 #pragma unroll
       for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (r < rows && (threadIdx.x % LPR) == 0) {
-        const int h = (int)(r % H);
-        const long long bt = r / H;
-        delta[CGK_IDX(((bt / T) * H + h) * T + (bt % T), rows)] = s;
-      }
+      if (r < rows && (threadIdx.x % LPR) == 0) delta[CGK_IDX(at[u], rows)] = s;
     }
   }
 }
 
-// dq[b, t, h, :] = bf16(accum[b, t, h, :])
-__global__ void flash_dq_cast_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int B,
-                                     int T, int H, int D, long long bs, long long ts, long long hs) {
-  const long long total = (long long)B * T * H * (D / 4);
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(i % (D / 4)) * 4;
-    long long r = i / (D / 4);
-    const int h = (int)(r % H); r /= H;
-    const int t = (int)(r % T);
-    const int b = (int)(r / T);
-    const float4 v = *reinterpret_cast<const float4*>(acc + (((long long)b * T + t) * H + h) * D + c);
-    uint2 o;
-    o.x = pack_bf16x2(v.x, v.y);
-    o.y = pack_bf16x2(v.z, v.w);
-    *reinterpret_cast<uint2*>(dq + b * bs + t * ts + h * hs + c) = o;
+// dq[b, t, h, :] = bf16(accum[b, t, h, :]), rows shared by D / 8 lanes as above: 32 bytes in, 16 out, four rows at a time.
+// 64 x 2048 x 12 x 64: 177 -> 103 us, the kernel above 155 -> 87 us.
+template <int D>
+__global__ void __launch_bounds__(256)
+flash_dq_cast_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int B, int T, int H, long long bs, long long ts, long long hs, int vec16) {
+  constexpr int LPR = D / 8, U = 4;
+  const uint32_t rows = (uint32_t)B * T * H, groups = gridDim.x * blockDim.x / LPR, g0 = (blockIdx.x * blockDim.x + threadIdx.x) / LPR;
+  const int c = ((int)threadIdx.x % LPR) * 8;
+  for (uint32_t r0 = g0; r0 < rows; r0 += groups * U) {
+    float4 v[U][2];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t r = r0 + u * groups;
+      if (r >= rows) break;
+      const float4* p = reinterpret_cast<const float4*>(acc + (long long)r * D + c);
+      v[u][0] = __ldg(p);
+      v[u][1] = __ldg(p + 1);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t r = r0 + u * groups;
+      if (r >= rows) break;
+      const uint32_t bt = r / H, h = r - bt * H, b = bt / T, t = bt - b * T;
+      uint4 o;
+      o.x = pack_bf16x2(v[u][0].x, v[u][0].y); o.y = pack_bf16x2(v[u][0].z, v[u][0].w);
+      o.z = pack_bf16x2(v[u][1].x, v[u][1].y); o.w = pack_bf16x2(v[u][1].z, v[u][1].w);
+      __nv_bfloat16* dst = dq + b * bs + t * ts + h * hs + c;
+      if (vec16) {
+        *reinterpret_cast<uint4*>(dst) = o;
+      } else {                                            // dq itself on an 8-byte boundary only
+        reinterpret_cast<uint2*>(dst)[0] = make_uint2(o.x, o.y);
+        reinterpret_cast<uint2*>(dst)[1] = make_uint2(o.z, o.w);
+      }
+    }
   }
 }
 
@@ -153,6 +168,7 @@ CGK_API int cgk_flash_backward(const cgk_flash_args* pa, void* stream) {
   int dev = 0;
   CGK_CUDA_CHECK(cudaGetDevice(&dev));
   const long long rows = (long long)a.B * a.Hq * a.Tq;
+  CGK_REQUIRE(rows < (1LL << 31), "cgk_flash_backward: too many rows");
   {
     long long blocks = (rows * (a.D / 8) + 256 * 4 - 1) / (256 * 4);
     long long cap = (long long)sm_count(dev) * 8;
@@ -180,12 +196,10 @@ CGK_API int cgk_flash_backward(const cgk_flash_args* pa, void* stream) {
   int rc = (a.D == 64) ? launch_bwd<64>(a, p, st) : launch_bwd<128>(a, p, st);
   if (rc) return rc;
   {
-    long long n = rows * (a.D / 4);
-    long long blocks = (n + 255) / 256;
-    long long cap = (long long)sm_count(dev) * 16;
-    if (blocks > cap) blocks = cap;
-    flash_dq_cast_kernel<<<(int)blocks, 256, 0, st>>>(a.dq_accum, (__nv_bfloat16*)a.dq, a.B, a.Tq, a.Hq,
-                                                      a.D, a.dq_bs, a.dq_ts, a.dq_hs);
+    const long long blocks = (rows * (a.D / 8) + 256 * 4 - 1) / (256 * 4), cap = (long long)sm_count(dev) * 8;
+    const auto cast = a.D == 64 ? flash_dq_cast_kernel<64> : flash_dq_cast_kernel<128>;
+    cast<<<(int)(blocks < cap ? blocks : cap), 256, 0, st>>>(a.dq_accum, (__nv_bfloat16*)a.dq, a.B, a.Tq, a.Hq, a.dq_bs, a.dq_ts, a.dq_hs,
+                                                                     ((uintptr_t)a.dq & 15) == 0);
     CGK_LAUNCH_CHECK();
   }
   return 0;
