@@ -651,6 +651,7 @@ __device__ __forceinline__ float dsilu_f(float x) {
   return s * (1.0f + x * (1.0f - s));
 }
 
+
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -695,32 +696,40 @@ __device__ __forceinline__ void fmul2(float& d0, float& d1, float a0, float a1, 
       : "=f"(d0), "=f"(d1)
       : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
-// gelu_tanh and v * dgelu_tanh(x) for two elements: 5 packed instructions and 2 MUFU, and 11 and 2.
+// gelu_tanh and v * dgelu_tanh(x) for two elements, in the operations (and roundings) of the scalar forms: 7 packed instructions
+// and 2 MUFU, and 15 and 2.
 __device__ __forceinline__ void gelu_tanh2(float& x0, float& x1) {
-  const float c = 0.7978845608028654f, c1 = c * 0.044715f;
-  float s0, s1, w0, w1, h0, h1;
-  fmul2(s0, s1, x0, x1, x0, x1);
-  ffma2(w0, w1, s0, s1, c1, c1, c, c);
-  fmul2(w0, w1, w0, w1, x0, x1);
+  const float c = 0.7978845608028654f, k = 0.044715f;
+  float p0, p1, h0, h1;
+  fmul2(p0, p1, x0, x1, k, k);
+  fmul2(p0, p1, p0, p1, x0, x1);
+  ffma2(p0, p1, p0, p1, x0, x1, x0, x1);
+  fmul2(p0, p1, p0, p1, c, c);
+  float t0 = tanh_fast(p0), t1 = tanh_fast(p1);
+  fadd2(t0, t1, 1.0f, 1.0f);
   fmul2(h0, h1, x0, x1, 0.5f, 0.5f);
-  ffma2(x0, x1, h0, h1, tanh_fast(w0), tanh_fast(w1), h0, h1);
+  fmul2(x0, x1, h0, h1, t0, t1);
 }
 __device__ __forceinline__ void mul_dgelu_tanh2(float& v0, float& v1, float x0, float x1) {
-  const float c = 0.7978845608028654f, c1 = c * 0.044715f;
-  float s0, s1, w0, w1, q0, q1, b0, b1, h0, h1;
+  const float c = 0.7978845608028654f, k = 0.044715f;
+  float s0, s1, p0, p1, q0, q1, h0, h1;
   fmul2(s0, s1, x0, x1, x0, x1);
-  ffma2(w0, w1, s0, s1, c1, c1, c, c);
-  fmul2(w0, w1, w0, w1, x0, x1);
-  ffma2(q0, q1, s0, s1, 3.0f * c1, 3.0f * c1, c, c);
-  const float t0 = tanh_fast(w0), t1 = tanh_fast(w1);
-  fmul2(s0, s1, t0, t1, t0, t1);
-  ffma2(s0, s1, s0, s1, -1.0f, -1.0f, 1.0f, 1.0f);        // 1 - t^2
-  fmul2(s0, s1, s0, s1, q0, q1);
+  fmul2(p0, p1, x0, x1, k, k);
+  ffma2(p0, p1, p0, p1, s0, s1, x0, x1);
+  fmul2(p0, p1, p0, p1, c, c);
+  float t0 = tanh_fast(p0), t1 = tanh_fast(p1);
+  ffma2(q0, q1, s0, s1, 3.0f * k, 3.0f * k, 1.0f, 1.0f);
+  fmul2(q0, q1, q0, q1, c, c);
+  fmul2(p0, p1, t0, t1, -1.0f, -1.0f);
+  ffma2(p0, p1, p0, p1, t0, t1, 1.0f, 1.0f);              // 1 - t^2
   fmul2(h0, h1, x0, x1, 0.5f, 0.5f);
-  ffma2(b0, b1, t0, t1, 0.5f, 0.5f, 0.5f, 0.5f);
-  ffma2(b0, b1, h0, h1, s0, s1, b0, b1);
-  fmul2(v0, v1, v0, v1, b0, b1);
+  fmul2(h0, h1, h0, h1, p0, p1);
+  fmul2(h0, h1, h0, h1, q0, q1);
+  fadd2(t0, t1, 1.0f, 1.0f);
+  ffma2(t0, t1, t0, t1, 0.5f, 0.5f, h0, h1);
+  fmul2(v0, v1, v0, v1, t0, t1);
 }
+
 // Counter-based random bits: a hash of (seed, element index).  The dropout kernels draw their
 // keep / drop decision from it, forward and backward alike, so no mask is ever stored.
 __device__ __forceinline__ uint32_t mix32(uint64_t z) {
