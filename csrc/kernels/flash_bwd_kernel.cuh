@@ -19,6 +19,7 @@ struct FlashBwdDev {
   __nv_bfloat16* dV;
   long long dv_bs, dv_ts, dv_hs;
   int* status;
+  int tiles, chunk;       // order of the key tiles over the grid (attention_tile)
 };
 
 template <int D>
@@ -109,7 +110,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  const int kt = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+  int kt, hk;
+  attention_tile(blockIdx.x, p.tiles, p.B * p.Hk, p.chunk, kt, hk);       // under a causal mask the first keys are seen most
+  const int b = hk / p.Hk;
+  hk -= b * p.Hk;
   const int k0 = kt * C::BN;
   const int off = p.Tk - p.Tq;
   const int group = p.Hq / p.Hk;

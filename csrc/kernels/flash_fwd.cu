@@ -50,6 +50,7 @@ struct FlashFwdDev {
   const float2* turn;      // [B * Tq][o_cols / 2] or null
   int o_cols, o_vec;       // columns stored; 1: rows take 16-byte stores
   int* status;
+  int tiles, chunk;       // order of the tiles over the grid (attention_tile)
 };
 
 template <int D>
@@ -119,8 +120,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   volatile int* dead = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  const int qblk = gridDim.x - 1 - blockIdx.x;  // heavy (late) causal blocks first
-  const int h = blockIdx.y, b = blockIdx.z;
+  int qblk, h;
+  attention_tile(blockIdx.x, p.tiles, p.B * p.Hq, p.chunk, qblk, h);
+  qblk = p.tiles - 1 - qblk;                    // heavy (late) causal blocks first
+  const int b = h / p.Hq;
+  h -= b * p.Hq;
   const int hk = (int)(((long long)h * p.Hk) / p.Hq);
   const int q0 = qblk * 2 * C::BM;
   const int off = p.Tk - p.Tq;  // causal alignment: key k visible to query q iff k <= q + off
@@ -556,8 +560,9 @@ static int launch_fwd(const cgk_flash_args& a, const FlashFwdDev& p, cudaStream_
   if ((rc = make_qkv_tmap(&tv, a.v, a.B, a.Tk, a.Hk, D, a.v_bs, a.v_ts, a.v_hs, C::BN))) return rc;
   CGK_CUDA_CHECK(cudaFuncSetAttribute(flash_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       C::TOTAL));
-  dim3 grid((a.Tq + 2 * C::BM - 1) / (2 * C::BM), a.Hq, a.B);
-  flash_fwd_kernel<D><<<grid, 384, C::TOTAL, st>>>(tq, tk, tv, p);
+  const long long ctas = (long long)p.tiles * a.Hq * a.B;
+  CGK_REQUIRE(ctas <= 0x7fffffffLL, "cgk_flash_forward: too many tiles");
+  flash_fwd_kernel<D><<<(unsigned)ctas, 384, C::TOTAL, st>>>(tq, tk, tv, p);
   CGK_LAUNCH_CHECK();
   return 0;
 }
@@ -593,6 +598,8 @@ CGK_API int cgk_flash_forward(const cgk_flash_args* pa, void* stream) {
   p.o_cols = a.o_cols > 0 ? a.o_cols : a.D;
   p.o_vec = o_vec;
   p.status = device_status(dev);
+  p.tiles = (a.Tq + 255) / 256;                 // pairs of 128-row query tiles
+  p.chunk = attention_chunk(p.tiles, a.B * a.Hq, sm_count(dev));
   if (a.D == 64) return launch_fwd<64>(a, p, (cudaStream_t)stream);
   return launch_fwd<128>(a, p, (cudaStream_t)stream);
 }

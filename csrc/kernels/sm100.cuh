@@ -729,6 +729,21 @@ __device__ __forceinline__ void mul_dgelu_tanh2(float& v0, float& v1, float x0, 
   ffma2(t0, t1, t0, t1, 0.5f, 0.5f, h0, h1);
   fmul2(v0, v1, v0, v1, t0, t1);
 }
+// Order of attention tiles over a one-dimensional grid: `tiles` of each head with the longest first, `heads` heads in groups
+// of `chunk`; inside a group all heads' first tiles, then their second ones, so that the last CTAs to start are short ones.
+// (With a head's tiles one after the other the longest tile of the last head started when the others were nearly done:
+// backward of 32 query on 8 key heads, 4096 tokens, head_dim 128: 1122 us, 773 in this order; forward
+// 227, 190.)  A group is a few waves of CTAs: its heads'
+// operands are still in L2 when their next tiles come.
+__device__ __forceinline__ void attention_tile(int id, int tiles, int heads, int chunk, int& tile, int& head) {
+  const int group = id / (chunk * tiles), rem = id - group * chunk * tiles, in = min(chunk, heads - group * chunk);
+  tile = rem / in;
+  head = group * chunk + rem - tile * in;
+}
+__host__ __forceinline__ int attention_chunk(int tiles, int heads, int sms) {
+  const int n = (4 * sms + tiles - 1) / tiles;
+  return n < heads ? n : heads;
+}
 
 // Counter-based random bits: a hash of (seed, element index).  The dropout kernels draw their
 // keep / drop decision from it, forward and backward alike, so no mask is ever stored.
