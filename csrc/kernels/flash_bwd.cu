@@ -137,11 +137,11 @@ static int launch_bwd(const cgk_flash_args& a, const FlashBwdDev& p, cudaStream_
   if ((rc = make_tmap4(&tk, a.k, a.B, a.Tk, a.Hk, D, a.k_bs, a.k_ts, a.k_hs))) return rc;
   if ((rc = make_tmap4(&tv, a.v, a.B, a.Tk, a.Hk, D, a.v_bs, a.v_ts, a.v_hs))) return rc;
   if ((rc = make_tmap4(&tdo, a.d_o, a.B, a.Tq, a.Hq, D, a.o_bs, a.o_ts, a.o_hs))) return rc;
-  CGK_CUDA_CHECK(cudaFuncSetAttribute(flash_bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      C::TOTAL));
+  const auto kernel = a.alibi_slopes ? flash_bwd_kernel<D, true> : flash_bwd_kernel<D, false>;
+  CGK_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::TOTAL));
   const long long ctas = (long long)p.tiles * a.Hk * a.B;
   CGK_REQUIRE(ctas <= 0x7fffffffLL, "cgk_flash_backward: too many tiles");
-  flash_bwd_kernel<D><<<(unsigned)ctas, 512, C::TOTAL, st>>>(tq, tk, tv, tdo, tdq, p);
+  kernel<<<(unsigned)ctas, 512, C::TOTAL, st>>>(tq, tk, tv, tdo, tdq, p);
   CGK_LAUNCH_CHECK();
   return 0;
 }

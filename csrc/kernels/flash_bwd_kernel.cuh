@@ -86,7 +86,9 @@ __device__ __noinline__ void flash_bwd_mask_scores(uint32_t s_tmem, float scale_
 // warps 4..11 compute P / dS (thread = query row x half of the keys), warps 12..15 drain the
 // dQ tile into the fp32 accumulator with bulk tensor reductions.  With 512 threads every thread
 // has 128 registers, which each role fits; no register reallocation is needed.
-template <int D>
+// ALIBI: with position biases; interior tiles add the bias of each column in registers, slope * column as eight constant pairs
+// plus a base per 16 columns.  2 x 3001 x 32 heads of 128, window 1024: 594 -> 463 us.
+template <int D, bool ALIBI>
 __global__ void __launch_bounds__(512, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,

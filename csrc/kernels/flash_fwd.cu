@@ -98,7 +98,10 @@ __device__ __noinline__ void flash_mask_scores(uint32_t s_tmem, float scale_log2
   tmem_st_wait();
 }
 
-template <int D>
+// ALIBI: with position biases.  Interior tiles then add the bias of each column in registers, slope * column as eight
+// constant pairs plus a base per 16 columns; only tiles on a mask edge are rewritten in TMEM.  2 x 3001 x 32 heads of 128,
+// window 1024: 224 -> 180 us.
+template <int D, bool ALIBI>
 __global__ void __launch_bounds__(384, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const FlashFwdDev p) {
@@ -342,7 +345,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (p.block > 0) need_mask |= k0 < tile_q_hi / p.block * p.block;
       // Interior tiles (no mask, no bias) use the raw products; the others are first rewritten in
       // TMEM as final log2-domain scores (-inf where masked), after which the multiplier is 1.
-      const bool fast = !need_mask && !p.alibi && p.scale_log2 > 0.0f;
+      const bool fast = !need_mask && p.scale_log2 > 0.0f;
       if (!fast) {
         // Row-wise visible key range [klo, khi] (empty when khi < klo).  The ALiBi bias of
         // column i of the tile is bias0 + slope * i.
@@ -354,7 +357,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const float bias0 = p.alibi ? slope * (float)(k0 - qk) : 0.0f;
         flash_mask_scores(s_tmem, p.scale_log2, slope, bias0, k0 - klo, span, khi < klo);
       }
-      const float mul = fast ? p.scale_log2 : 1.0f;
+      const float mul = fast && !ALIBI ? p.scale_log2 : 1.0f;
       // The whole S row (128 fp32) comes into registers with four loads in flight and one wait;
       // the accumulator is then free for Q K^T of the next key tile.
       uint32_t r[4][32];
@@ -364,6 +367,25 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       tmem_ld_wait();
       tc_fence_before();
       mbar_arrive_warp(s_free(t));
+      if (ALIBI && fast) {
+        float step[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) step[i] = slope * (float)i;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const float base = fmaf(slope, (float)(k0 - qk + 16 * c), 0.0f);
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            float b0 = step[i], b1 = step[i + 1], x0, x1;
+            fadd2(b0, b1, base, base);
+            uint32_t& u0 = r[c >> 1][(c & 1) * 16 + i];
+            uint32_t& u1 = r[c >> 1][(c & 1) * 16 + i + 1];
+            ffma2(x0, x1, __uint_as_float(u0), __uint_as_float(u1), p.scale_log2, p.scale_log2, b0, b1);
+            u0 = __float_as_uint(x0);
+            u1 = __float_as_uint(x1);
+          }
+        }
+      }
       float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
@@ -558,11 +580,11 @@ static int launch_fwd(const cgk_flash_args& a, const FlashFwdDev& p, cudaStream_
   if ((rc = make_qkv_tmap(&tq, a.q, a.B, a.Tq, a.Hq, D, a.q_bs, a.q_ts, a.q_hs, C::BM))) return rc;
   if ((rc = make_qkv_tmap(&tk, a.k, a.B, a.Tk, a.Hk, D, a.k_bs, a.k_ts, a.k_hs, C::BN))) return rc;
   if ((rc = make_qkv_tmap(&tv, a.v, a.B, a.Tk, a.Hk, D, a.v_bs, a.v_ts, a.v_hs, C::BN))) return rc;
-  CGK_CUDA_CHECK(cudaFuncSetAttribute(flash_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      C::TOTAL));
+  const auto kernel = a.alibi_slopes ? flash_fwd_kernel<D, true> : flash_fwd_kernel<D, false>;
+  CGK_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::TOTAL));
   const long long ctas = (long long)p.tiles * a.Hq * a.B;
   CGK_REQUIRE(ctas <= 0x7fffffffLL, "cgk_flash_forward: too many tiles");
-  flash_fwd_kernel<D><<<(unsigned)ctas, 384, C::TOTAL, st>>>(tq, tk, tv, p);
+  kernel<<<(unsigned)ctas, 384, C::TOTAL, st>>>(tq, tk, tv, p);
   CGK_LAUNCH_CHECK();
   return 0;
 }

@@ -217,6 +217,20 @@ def test_flash_attention_forward_backward(c):
     assert relerr(dq, gq) < 3e-2 and relerr(dk, gk) < 3e-2 and relerr(dv, gv) < 3e-2
 
 
+# biases in interior tiles, on mask edges and both (each head_dim, query groups, ragged ends, another key length), and more heads
+# than one group of the tile order holds, the last group smaller
+@pytest.mark.parametrize("c", [
+    dict(B=2, Tq=700, Tk=700, Hq=8, Hk=2, D=128, causal=True, alibi=True),
+    dict(B=1, Tq=515, Tk=515, Hq=4, Hk=4, D=64, causal=True, window=130, alibi=True),
+    dict(B=1, Tq=600, Tk=600, Hq=4, Hk=1, D=128, causal=False, window=200, alibi=True),
+    dict(B=1, Tq=384, Tk=640, Hq=4, Hk=2, D=64, causal=False, alibi=True),
+    dict(B=50, Tq=130, Tk=130, Hq=12, Hk=12, D=64, causal=True),
+    dict(B=40, Tq=257, Tk=257, Hq=16, Hk=8, D=128, causal=True),
+], ids=lambda c: "-".join(f"{k}{v}" for k, v in c.items()))
+def test_flash_attention_biases_and_tile_order(c):
+    test_flash_attention_forward_backward(c)
+
+
 def test_packed_attention_with_rope_matches_reference():
     from cogito_b200.nn.transformer import packed_attention
     from cogito_b200.ops.misc import rope_tables
