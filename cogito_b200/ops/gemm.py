@@ -199,37 +199,20 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if out.dtype not in (torch.bfloat16, torch.float32):
         raise TypeError("gemm: out must be bf16 or fp32")
 
-    g = _lib.GemmArgs()
-    g.A, g.B, g.out = a.data_ptr(), b.data_ptr(), out3.data_ptr()
-    g.M, g.N, g.K, g.batch = M, N, K, batch
-    g.lda, g.ldb, g.ldc = _ld(a), _ld(b), _ld(out3)
-    if batch > 1:
-        g.strideA, g.strideB, g.strideC = a.stride(0), b.stride(0), out3.stride(0)
-    else:
-        g.strideA = g.strideB = g.strideC = 0
-    g.a_mn, g.b_mn = int(a_mn), int(b_mn)
-    g.out_fp32 = int(out.dtype == torch.float32)
-    g.accumulate = int(accumulate)
-    g.alpha = float(alpha)
-    if bias is not None:
-        if bias.numel() != N:
-            raise ValueError("bias must have N elements")
-        g.bias = bias.data_ptr()
-        g.bias_fp32 = int(bias.dtype == torch.float32)
-    g.act = ACT[act]
-    if residual is not None:
-        assert residual.dtype == torch.bfloat16 and residual.shape[-2:] == (M, N)
-        g.residual, g.ldr = residual.data_ptr(), _ld(residual)
-    if aux_out is not None:
-        assert aux_out.dtype == torch.bfloat16 and aux_out.shape[-2:] == (M, N)
-        g.aux_out, g.ldaux = aux_out.data_ptr(), _ld(aux_out)
-    if aux_in is not None:
-        assert aux_in.dtype == torch.bfloat16 and aux_in.shape[-2:] == (M, N)
-        g.aux_in, g.ldauxin = aux_in.data_ptr(), _ld(aux_in)
-        g.dact = ACT[dact]
-    g.force_simt = int(force_simt)
-    g.max_ctas = int(max_ctas) if max_ctas else _default_max_ctas
-    g.split_k = int(split_k)
+    if bias is not None and bias.numel() != N:
+        raise ValueError("bias must have N elements")
+    for t in (residual, aux_out, aux_in):
+        assert t is None or (t.dtype == torch.bfloat16 and t.shape[-2:] == (M, N))
+    many = batch > 1
+    # the fields in their order, set by one call
+    g = _lib.GemmArgs(a.data_ptr(), b.data_ptr(), out3.data_ptr(), M, N, K, batch, _ld(a), _ld(b), _ld(out3),
+                      a.stride(0) if many else 0, b.stride(0) if many else 0, out3.stride(0) if many else 0, int(a_mn), int(b_mn),
+                      int(out.dtype == torch.float32), int(accumulate), float(alpha),
+                      None if bias is None else bias.data_ptr(), int(bias is not None and bias.dtype == torch.float32), ACT[act],
+                      None if residual is None else residual.data_ptr(), 0 if residual is None else _ld(residual),
+                      None if aux_out is None else aux_out.data_ptr(), 0 if aux_out is None else _ld(aux_out),
+                      None if aux_in is None else aux_in.data_ptr(), 0 if aux_in is None else _ld(aux_in), 0 if aux_in is None else ACT[dact],
+                      int(force_simt), int(max_ctas) if max_ctas else _default_max_ctas, None, None, 0, 0, 0, 0, 0, int(split_k))
     if rope is not None:
         fill_rope(g, rope, a.device)
     _lib.check(_lib.lib().cgk_gemm_bf16(ctypes.byref(g), _lib.stream_ptr()), "cgk_gemm_bf16")
