@@ -402,6 +402,42 @@ __global__ void swiglu_bwd_kernel(const T* __restrict__ x, const T* __restrict__
   }
 }
 
+// The backward pass over bf16 rows in 16-byte pieces, two rows at a time per CTA: six loads in flight per thread, laid out like
+// the forward kernel.  One element per thread and a 64-bit division per element took 2.9 times the traffic's time:
+// 4096 rows of 2 x 11008 203 us, 78 like this (5.8 TB/s).
+constexpr int SWIGLU_BWD_ROWS = 2;
+__global__ void __launch_bounds__(256)
+swiglu_bwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx, long long rows, int H) {
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  if (c >= H) return;
+  for (long long r0 = (long long)blockIdx.x * SWIGLU_BWD_ROWS; r0 < rows; r0 += (long long)gridDim.x * SWIGLU_BWD_ROWS) {
+    uint4 g[SWIGLU_BWD_ROWS], u[SWIGLU_BWD_ROWS], d[SWIGLU_BWD_ROWS];
+#pragma unroll
+    for (int j = 0; j < SWIGLU_BWD_ROWS; ++j) {
+      if (r0 + j >= rows) continue;
+      const __nv_bfloat16* p = x + (r0 + j) * 2 * H + c;
+      g[j] = *reinterpret_cast<const uint4*>(p);
+      u[j] = *reinterpret_cast<const uint4*>(p + H);
+      d[j] = *reinterpret_cast<const uint4*>(dy + (r0 + j) * H + c);
+    }
+#pragma unroll
+    for (int j = 0; j < SWIGLU_BWD_ROWS; ++j) {
+      if (r0 + j >= rows) continue;
+      const uint32_t gw[4] = {g[j].x, g[j].y, g[j].z, g[j].w}, uw[4] = {u[j].x, u[j].y, u[j].z, u[j].w}, dw[4] = {d[j].x, d[j].y, d[j].z, d[j].w};
+      uint32_t og[4], ou[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 a = unpack_bf16x2(gw[e]), b = unpack_bf16x2(uw[e]), t = unpack_bf16x2(dw[e]);
+        og[e] = pack_bf16x2(t.x * b.x * dsilu_stream(a.x), t.y * b.y * dsilu_stream(a.y));
+        ou[e] = pack_bf16x2(t.x * silu_stream(a.x), t.y * silu_stream(a.y));
+      }
+      __nv_bfloat16* o = dx + (r0 + j) * 2 * H + c;
+      *reinterpret_cast<uint4*>(o) = make_uint4(og[0], og[1], og[2], og[3]);
+      *reinterpret_cast<uint4*>(o + H) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+    }
+  }
+}
+
 // ---- 2-D transpose (fp32 / bf16), tiled through shared memory ------------------
 template <typename T>
 __global__ void transpose_kernel(const T* __restrict__ x, T* __restrict__ y, int rows, int cols) {
@@ -751,7 +787,12 @@ CGK_API int cgk_swiglu_backward(int dtype, const void* x, const void* dy, void* 
   CGK_REQUIRE(x && dy && dx && H > 0, "cgk_swiglu_backward: bad argument");
   if (rows == 0) return 0;
   if (dtype == 0) swiglu_bwd_kernel<float><<<ew_grid(rows * H), 256, 0, ST(stream)>>>((const float*)x, (const float*)dy, (float*)dx, rows, H);
-  else swiglu_bwd_kernel<__nv_bfloat16><<<ew_grid(rows * H), 256, 0, ST(stream)>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, rows, H);
+  else if (H % 8 == 0 && (((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx) & 15) == 0) {
+    const dim3 cols = swiglu_rows_grid(rows, H);
+    const long long pairs = (rows + SWIGLU_BWD_ROWS - 1) / SWIGLU_BWD_ROWS, cap = 148 * 16 / (cols.y < 16 ? cols.y : 16);
+    swiglu_bwd_rows_kernel<<<dim3((unsigned)(pairs < cap ? pairs : cap), cols.y), swiglu_rows_threads(H), 0, ST(stream)>>>(
+        (const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, rows, H);
+  } else swiglu_bwd_kernel<__nv_bfloat16><<<ew_grid(rows * H), 256, 0, ST(stream)>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dx, rows, H);
   CGK_LAUNCH_CHECK();
   return 0;
 }

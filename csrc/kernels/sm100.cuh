@@ -651,6 +651,26 @@ __device__ __forceinline__ float dsilu_f(float x) {
   return s * (1.0f + x * (1.0f - s));
 }
 
+// The same without a branch, for kernels that stream bf16: the compiler's division keeps a branch for its rare cases, and a
+// branch per element kept the elements of a thread from overlapping.  The quotient of the approximate reciprocal is corrected by
+// its own remainder (Markstein, IBM J. Res. Dev. 34, 1990).  Where the remainder is not a number (x infinite, or exp(-x)
+// past the range, where the result is 0) or 0 (it would take the sign of -0) the plain quotient stands.  Equal to silu_f
+// in the rounded results of all bf16 inputs.  4096 rows of
+// 2 x 11008: forward 85 -> 57 us, backward 203 -> 78 us.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float corrected_quotient(float x, float d) {
+  const float r = rcp_approx(0.25f * d), q = 0.25f * x * r, rem = fmaf(-q, d, x);       // 1 <= d: 4 / d is never denormal
+  return fabsf(rem) > 0.0f ? fmaf(rem, 0.25f * r, q) : q;
+}
+__device__ __forceinline__ float silu_stream(float x) { return corrected_quotient(x, 1.0f + __expf(-x)); }
+__device__ __forceinline__ float dsilu_stream(float x) {
+  const float s = corrected_quotient(1.0f, 1.0f + __expf(-x));
+  return s * (1.0f + x * (1.0f - s));
+}
 
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;

@@ -9,7 +9,7 @@ constexpr int SWIGLU_ROWS = 4;
 
 enum : int { GATED_SILU = 0, GATED_RELU = 1 };
 template <int ACT>
-__device__ __forceinline__ float gated_act(float x) { return ACT == GATED_RELU ? fmaxf(x, 0.0f) : silu_f(x); }
+__device__ __forceinline__ float gated_act(float x) { return ACT == GATED_RELU ? fmaxf(x, 0.0f) : silu_stream(x); }
 
 template <int ACT = GATED_SILU>
 __device__ __forceinline__ void swiglu_rows_bf16(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ act, long long ldo, long long rows, int F) {
