@@ -446,62 +446,80 @@ norm_bwd_ring_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   }
 }
 
-// The backward pass for rows of more than 1024 elements: a CTA per row, 16 bytes of each tensor per thread, the next row's
-// loads under this row's reduction.  A thread keeps its eight columns from row to row, so dgamma / dbeta stay in registers
-// (a warp per row needs 2 D floats of shared memory per warp, which left one CTA of four warps per SM at D = 4096).
+// The backward pass for rows of more than 1024 elements.  A CTA takes a run of rows, as many at a time as it has warps: first a
+// warp per row forms the row's two sums, then a thread per eight columns goes through the same rows (in L2 by then), so that
+// dgamma / dbeta stay in registers (a warp per row for all of it needs 2 D floats of shared memory per warp, which left one
+// CTA of four warps per SM at D = 4096).  The sums have the order of norm_bwd_kernel, so dx has its bits: a gradient through
+// several layers multiplies a last-bit difference a hundredfold.
+// 4096 x 4096: 140 -> 37 us.
 template <bool RMS>
 __global__ void __launch_bounds__(1024)
 norm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                      const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean_in,
                      const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dres_in,
                      __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, int rows, int D) {
-  __shared__ float sh[2][64];
-  const int c = threadIdx.x;
-  const bool in = c < (D >> 3);
+  __shared__ float4 stat[2][32];                            // mean, rstd and the two means of a row, by warp
+  const int c = threadIdx.x, warp = c >> 5, lane = c & 31, nw = blockDim.x >> 5, nvec = D >> 3;
+  const bool in = c < nvec;
   const uint4 none = make_uint4(0, 0, 0, 0);
-  const uint4 gr = in ? __ldg(reinterpret_cast<const uint4*>(gamma) + c) : none;
-  float accg[8], accb[8];
+  const uint4* gp = reinterpret_cast<const uint4*>(gamma);
+  float g[8], accg[8], accb[8];
+  unpack8(in ? __ldg(gp + c) : none, g);
 #pragma unroll
   for (int j = 0; j < 8; ++j) accg[j] = accb[j] = 0.0f;
-  uint4 xn = none, dn = none, rn = none;
-  float mean_n = 0.0f, rstd_n = 0.0f;
-  auto fetch = [&](long long row) {
-    if (row >= rows) return;
-    mean_n = RMS ? 0.0f : mean_in[row];
-    rstd_n = rstd_in[row];
-    if (!in) return;
-    xn = reinterpret_cast<const uint4*>(x + row * D)[c];
-    dn = reinterpret_cast<const uint4*>(dy + row * D)[c];
-    if (dres_in) rn = reinterpret_cast<const uint4*>(dres_in + row * D)[c];
-  };
-  fetch(blockIdx.x);
+  const long long end = (long long)rows * (blockIdx.x + 1) / gridDim.x;
   int par = 0;
-  for (long long row = blockIdx.x; row < rows; row += gridDim.x, par ^= 1) {
-    const float mean = mean_n, rstd = rstd_n;
-    const uint4 xr = xn, dr = dn, rr = rn;
-    fetch(row + gridDim.x);
-    float h[8], dv[8], t[8], s1 = 0.0f, s2 = 0.0f;
-    unpack8(xr, h);
-    unpack8(dr, dv);
-    unpack8(gr, t);
+  for (long long base = (long long)rows * blockIdx.x / gridDim.x; base < end; base += nw, par ^= 1) {
+    const int n = end - base < nw ? (int)(end - base) : nw;
+    if (warp < n) {
+      const long long row = base + warp;
+      const float mean = RMS ? 0.0f : mean_in[row];
+      const float rstd = rstd_in[row];
+      const uint4* xp = reinterpret_cast<const uint4*>(x + row * D);
+      const uint4* dp = reinterpret_cast<const uint4*>(dy + row * D);
+      float s1 = 0.0f, s2 = 0.0f;
+#pragma unroll 4
+      for (int k = lane; k < nvec; k += 32) {
+        float xv[8], dv[8], gv[8];
+        unpack8(xp[k], xv);
+        unpack8(dp[k], dv);
+        unpack8(__ldg(gp + k), gv);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      h[j] = (h[j] - mean) * rstd;
-      t[j] *= dv[j];
-      s1 += t[j];
-      s2 += t[j] * h[j];
-      accg[j] += dv[j] * h[j];
-      accb[j] += dv[j];
+        for (int j = 0; j < 8; ++j) {
+          const float h = (xv[j] - mean) * rstd;
+          const float t = dv[j] * gv[j];
+          s1 += t;
+          s2 += t * h;
+        }
+      }
+      s1 = RMS ? 0.0f : warp_sum(s1) / D;
+      s2 = warp_sum(s2) / D;
+      if (lane == 0) stat[par][warp] = make_float4(mean, rstd, s1, s2);
     }
-    const float2 sum = block_sum2(s1, in ? s2 : 0.0f, sh[par]);
-    s1 = RMS ? 0.0f : sum.x / D;
-    s2 = sum.y / D;
-    if (in) {
-      float r[8];
-      unpack8(rr, r);
+    __syncthreads();                                        // (one: the next group of rows writes the other half of stat)
+    if (!in) continue;
+#pragma unroll 4
+    for (int k = 0; k < n; ++k) {
+      const long long at = (base + k) * nvec + c;
+      const float4 st = stat[par][k];
+      const float mean = RMS ? 0.0f : st.x, rstd = st.y, s1 = RMS ? 0.0f : st.z, s2 = st.w;
+      float xv[8], dv[8], o[8];
+      unpack8(reinterpret_cast<const uint4*>(x)[at], xv);
+      unpack8(reinterpret_cast<const uint4*>(dy)[at], dv);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) r[j] += rstd * (t[j] - s1 - h[j] * s2);
-      reinterpret_cast<uint4*>(dx + row * D)[c] = pack8(r);
+      for (int j = 0; j < 8; ++j) {
+        const float h = (xv[j] - mean) * rstd;
+        accg[j] += dv[j] * h;
+        accb[j] += dv[j];
+        o[j] = rstd * (dv[j] * g[j] - s1 - h * s2);
+      }
+      if (dres_in) {
+        float r[8];
+        unpack8(reinterpret_cast<const uint4*>(dres_in)[at], r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] += r[j];
+      }
+      reinterpret_cast<uint4*>(dx)[at] = pack8(o);
     }
   }
   if (in) {

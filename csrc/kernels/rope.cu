@@ -85,8 +85,9 @@ rope_apply_vec_kernel(__nv_bfloat16* x, const float* __restrict__ cos_t, const f
   for (int e = 0; e < 4; ++e) {
     const float2 a = unpack_bf16x2(lw[e]), bb = unpack_bf16x2(hw[e]);
     const float ca = cs[2 * e], cb = cs[2 * e + 1], sa = sign * sn[2 * e], sb = sign * sn[2 * e + 1];
-    lr[e] = pack_bf16x2(a.x * ca - bb.x * sa, a.y * cb - bb.y * sb);
-    hr[e] = pack_bf16x2(bb.x * ca + a.x * sa, bb.y * cb + a.y * sb);
+    // the contractions of rope_apply_kernel, written out: the same bits
+    lr[e] = pack_bf16x2(fmaf(a.x, ca, -(bb.x * sa)), fmaf(a.y, cb, -(bb.y * sb)));
+    hr[e] = pack_bf16x2(fmaf(a.x, sa, bb.x * ca), fmaf(a.y, sb, bb.y * cb));
   }
   *reinterpret_cast<uint4*>(p) = make_uint4(lr[0], lr[1], lr[2], lr[3]);
   *reinterpret_cast<uint4*>(p + half) = make_uint4(hr[0], hr[1], hr[2], hr[3]);
