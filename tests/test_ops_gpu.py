@@ -55,6 +55,25 @@ def test_wide_norm_against_64_bits(rows, D, rms):
         assert torch.equal(N.add_rms_norm_(u, r, g, 1e-5), y) and torch.equal(u, s)
 
 
+# a row's result does not depend on how many rows the call has: few rows take a CTA each, many a warp each
+@pytest.mark.parametrize("D", [1032, 1608, 2048, 4096, 8192])
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("with_res", [False, True])
+def test_wide_norm_has_the_same_bits_for_few_rows_and_for_many(D, rms, with_res):
+    from cogito_b200.ops import norm as N
+    torch.manual_seed(D)
+    few, many = 592, 2560                                     # four rows per SM of 148, and more than that
+    x = torch.randn(many, D, device=DEV, dtype=torch.bfloat16) * 3 + 0.5
+    r = torch.randn(many, D, device=DEV, dtype=torch.bfloat16) if with_res else None
+    g = (torch.randn(D, device=DEV) * 0.1 + 1).bfloat16()
+    b = None if rms else torch.randn(D, device=DEV).bfloat16()
+    whole = N.norm_forward_raw(x, g, b, 1e-5, rms, r, True)
+    for part in (slice(0, few), slice(few, few + 1), slice(many - 37, many)):
+        got = N.norm_forward_raw(x[part], g, b, 1e-5, rms, None if r is None else r[part], True)
+        for u, v in zip(got, whole):
+            assert (u is None) == (v is None) and (u is None or torch.equal(u, v[part]))
+
+
 @pytest.mark.parametrize("rows,D", [(64, 768), (33, 128), (1000, 4096), (7, 8)])
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("with_res", [False, True])
