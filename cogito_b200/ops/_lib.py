@@ -96,8 +96,10 @@ def _declare(L: ctypes.CDLL) -> None:
         "cgk_int4_quantize": [vp, ll, i, vp, vp, vp],
         "cgk_int4_dequantize": [vp, vp, ll, i, vp, vp, vp],
         "cgk_int4_gemm": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
+        "cgk_int4_gemm_parts": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
         "cgk_int4_tile_weights": [vp, vp, i, i, i, vp, vp],
         "cgk_int4_wa_gemm": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
+        "cgk_int4_wa_gemm_parts": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
         "cgk_int4_wa_tile_weights": [vp, vp, i, i, i, vp, vp],
         "cgk_kv_int4_append": [vp, vp, vp, i, vp],
         "cgk_kv_int4_append_rows": [vp, vp, vp, ll, ll, ll, i, vp, vp, vp],
@@ -143,6 +145,8 @@ def _declare(L: ctypes.CDLL) -> None:
         "cgk_int4_tiles_bytes": [i, i],
         "cgk_int4_wa_tiles_bytes": [i, i],
         "cgk_int4_gemm_counters": [i, i],
+        "cgk_int4_gemm_parts_floats": [i, i, i, i],
+        "cgk_int4_wa_gemm_parts_floats": [i, i, i, i],
         "cgk_latent_attention_scratch_floats": [i, i, i, i],
         "cgk_kv_rows_scratch_floats": [i, i, i, i],
         "cgk_linear_chunks_scratch_floats": [i, i, i, i],

@@ -72,10 +72,14 @@ class Int4Linear(torch.nn.Module):
 
     # Which tcgen05 kernel multiplies: "wb" keeps the weights as the B operand (converted tile in shared
     # memory, 128 token rows per instruction), "wa" makes them the A operand fed from tensor memory (cost
-    # follows the token count; needs group % 128 == 0).  "auto": "wa" up to 16 token rows, where it measured
-    # faster, "wb" up to two row tiles, and beyond that (prompts) the weights are dequantised to bf16 once per call for the
-    # dense GEMM: "wb" converts every weight tile again for each row tile (4096 x 22016: 111 us against 116 us at 256 rows,
-    # 180 against 136 us at 512).  Each of the two kernels has its own tile-major copy of the weights, made on first use.
+    # follows the token count; needs group % 128 == 0).  "auto": "wa" up to 16 token rows, "wb" up to two row
+    # tiles, and beyond that (prompts) the weights are dequantised to bf16 once per call for the dense GEMM: "wb" converts
+    # every weight tile again for each row tile.  Each of the two kernels has its own tile-major copy of the weights, made on
+    # first use; both sum the parts of a shared tile in a fixed order, so a call gives the same bits every time.
+    # Times (us, layers one after the other) for 4096 x 6144, 4096 x 4096, 4096 x 22016, 11008 x 4096, 4096 x 32000, 2048 x 11264:
+    #   16 rows   "wa" 20.1 14.9 34.7 24.7 44.6 19.2
+    #   17 rows   "wa" 28.2 20.4 54.4 36.9 71.4 25.9 (columns padded to 32)   "wb" 18.9 15.7 43.7 26.3 59.3 17.1
+    #   200 rows  "wb" 31.4 24.9 103 45.9 141 30.5     dense 31.4 26.5 104 61.1 131 32.7 (a third row tile adds half to "wb")
     DENSE_ROWS = 256
     kernel = os.environ.get("COGITO_INT4_KERNEL", "auto")
 
@@ -89,7 +93,7 @@ class Int4Linear(torch.nn.Module):
         self.register_buffer("packed", packed)
         self.register_buffer("scales", scales)
         self.register_buffer("bias", None if bias is None else bias.detach().to(torch.bfloat16))
-        self._acc = None
+        self._counters = None
         self._tiles = {}                      # kernel kind -> tile-major weights
 
     @classmethod
@@ -105,7 +109,7 @@ class Int4Linear(torch.nn.Module):
         self.register_buffer("packed", packed.to(torch.uint8).contiguous())
         self.register_buffer("scales", scales.to(torch.float32).contiguous())
         self.register_buffer("bias", None if bias is None else bias.detach().to(torch.bfloat16))
-        self._acc = None
+        self._counters = None
         self._tiles = {}
         return self
 
@@ -172,16 +176,17 @@ class Int4Linear(torch.nn.Module):
             _lib.check(tile(self.packed.data_ptr(), self.scales.data_ptr(), K, N, self.group,
                             tiles.data_ptr(), _lib.stream_ptr()), "cgk_int4_tile_weights")
             _lib.count_launch()
-        if self._acc is None or self._acc.numel() < M * N or self._acc.device != x2.device:
-            # split-K scratch: zero once, every call leaves it zero again
-            self._acc = torch.zeros(M * N, dtype=torch.float32, device=x2.device)
-            self._counters = torch.zeros(L.cgk_int4_gemm_counters(M, N), dtype=torch.int32, device=x2.device)
+        # for the output tiles that several CTAs share: the parts' own place, and counters (zero once, every call leaves them zero)
+        parts = torch.empty((L.cgk_int4_wa_gemm_parts_floats if wa else L.cgk_int4_gemm_parts_floats)(M, N, K, splits), dtype=torch.float32, device=x2.device)
+        need = L.cgk_int4_gemm_counters(M, N)
+        if self._counters is None or self._counters.numel() < need or self._counters.device != x2.device:
+            self._counters = torch.zeros(need, dtype=torch.int32, device=x2.device)
         if out is None:
             out = torch.empty(M, N, dtype=torch.bfloat16, device=x2.device)
         elif out.dtype != torch.bfloat16 or not out.is_contiguous() or out.numel() != M * N:
             raise ValueError("out must be a contiguous bf16 [rows, out_features] tensor")
-        _lib.check((L.cgk_int4_wa_gemm if wa else L.cgk_int4_gemm)(
-            x2.data_ptr(), K, tiles.data_ptr(), self._acc.data_ptr(), self._counters.data_ptr(),
+        _lib.check((L.cgk_int4_wa_gemm_parts if wa else L.cgk_int4_gemm_parts)(
+            x2.data_ptr(), K, tiles.data_ptr(), parts.data_ptr(), self._counters.data_ptr(),
             out.data_ptr(), N, _lib.ptr(self.bias), M, N, K, splits, _lib.stream_ptr()), "cgk_int4_gemm")
         _lib.count_launch()
         return out.view(*lead, N)

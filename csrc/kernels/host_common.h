@@ -68,4 +68,17 @@ int sm_count(int device);
     }                                       \
   } while (0)
 
+// Runs f(scratch) with `floats` elements from the stream's memory pool, given back in stream order (null: none wanted, or none left).
+template <typename F>
+int with_stream_scratch(long long floats, cudaStream_t stream, F f) {
+  float* p = nullptr;
+  if (floats > 0 && cudaMallocAsync((void**)&p, (size_t)floats * sizeof(float), stream) != cudaSuccess) {
+    (void)cudaGetLastError();
+    p = nullptr;
+  }
+  const int rc = f(p);
+  if (p) CGK_CUDA_CHECK(cudaFreeAsync(p, stream));
+  return rc;
+}
+
 }  // namespace cgk

@@ -18,13 +18,15 @@
 //             stay in the pair order the extraction yields (0,4,1,5,2,6,3,7 within each group
 //             of 8); the epilogue undoes the permutation when it addresses the output.
 //   warp 1    tcgen05.mma, two accumulators in TMEM (128 lanes x 128 columns)
-//   warps 20-23 epilogue.  Whole tile: TMEM -> bias -> bf16 -> global.  Part of a tile: vector red.add
-//             into a zeroed fp32 buffer; the CTA that arrives last at the tile's counter adds
-//             the bias, writes bf16 and leaves buffer and counter zeroed for the next call.
+//   warps 20-23 epilogue.  Whole tile: TMEM -> bias -> bf16 -> global.  Part of a tile: into the part's
+//             own fp32 slot; the CTA that arrives last at the tile's counter sums the slots in the
+//             order of the CTAs, adds the bias, writes bf16 and leaves the counter zeroed for the
+//             next call.  The order is fixed, so a call gives the same bits every time.
 // One CTA per SM.  Each takes as many whole tiles as there are for all of them, then an equal piece of the line of the left-over
 // tiles' steps of 128 k (see int4_gemm_wa.cu).  Whole tiles only left 172 of them (22 016 columns) in two waves on 148 SMs, and a
-// K of 11 008 on 64 CTAs.  80 rows, event times with cold caches: 4096 x 22016 72.6 -> 57.3 us, 11008 x 4096 62.4 -> 38.9, 4096 x 32000 74.7 -> 77.9
-// (two thirds of a wave left over: its tiles meet in the fp32 buffer).
+// K of 11 008 on 64 CTAs.  80 rows, layers one after the other, whole tiles or equal parts of them by atomics / like this: 4096 x 22016
+// 68.8 / 46.5 us, 11008 x 4096 52.1 / 28.7, 4096 x 32000 70.1 / 61.6, 2048 x 11264 (a tile per CTA on 88 SMs) 19.9 / 19.5.
+// The sum of the CTA's last shared tile is work of all its threads: by the epilogue's 128 these took 50.9, 33.3, 64.7 and 24.0.
 #include <cuda_bf16.h>
 #include <stdlib.h>
 
@@ -47,17 +49,48 @@ constexpr int RING_BUDGET = SMEM_BYTES - 1024 - B_STAGES * SUB * B_BYTES - 2048;
 
 struct Int4Dev {
   const uint8_t* w_tiles;          // [N/128][K/64][4608]
-  float* acc;                      // fp32 [M, N], zero between calls (split-K only)
-  int* counters;                   // int32 [m_tiles * n_tiles], zero between calls (split-K only)
+  float4* parts;                   // slots of shared tiles' parts: [m_tiles][sharers][2][32 column quads][a_rows]
+  int* counters;                   // int32 [m_tiles * n_tiles], zero between calls (shared tiles only)
   __nv_bfloat16* out; long long ldo;
   const __nv_bfloat16* bias;
   int M, N, K;
   int a_rows, a_stages;            // rows fetched per X tile (multiple of 8), depth of the X ring
   int raw_stages;                  // depth of the W ring
+  int sharers;                     // CTAs that the left-over tiles are dealt to
   int* status;
 };
 
+// Slot `which` of a sharer: [32 column quads][a_rows] float4s.
+__device__ __forceinline__ float4* part_slot(const Int4Dev& g, int mt, int sharer, int which) {
+  return g.parts + (long long)((mt * g.sharers + sharer) * 2 + which) * ((BN / 4) * g.a_rows);
+}
 
+// The output of a tile out of its parts, summed in the order of the CTAs lo .. hi; `first`: the slot that CTA lo's is in.
+__device__ __forceinline__ void sum_parts(const Int4Dev& g, int mt, int nt, int lo, int hi, int first_slot, int tid, int threads) {
+  __threadfence();
+  const int m0 = mt * BM, n0 = nt * BN, rows = min(BM, g.M - m0), stride = 2 * (BN / 4) * g.a_rows;
+  const float4* first = part_slot(g, mt, lo, first_slot);
+  const float4* others = part_slot(g, mt, lo, 0);
+  for (int e = tid; e < rows * (BN / 8); e += threads) {
+    const int c8 = e / rows, r = e - c8 * rows, at = 2 * c8 * g.a_rows + r, n = n0 + c8 * 8;
+    float4 u = __ldcg(first + at), v = __ldcg(first + at + g.a_rows);
+#pragma unroll 4
+    for (int c = 1; c <= hi - lo; ++c) {
+      const float4* src = others + (long long)c * stride + at;
+      const float4 x = __ldcg(src), y = __ldcg(src + g.a_rows);
+      u.x += x.x; u.y += x.y; u.z += x.z; u.w += x.w;
+      v.x += y.x; v.y += y.y; v.z += y.z; v.w += y.w;
+    }
+    if (g.bias) {
+      u.x += __bfloat162float(g.bias[n]); u.y += __bfloat162float(g.bias[n + 1]);
+      u.z += __bfloat162float(g.bias[n + 2]); u.w += __bfloat162float(g.bias[n + 3]);
+      v.x += __bfloat162float(g.bias[n + 4]); v.y += __bfloat162float(g.bias[n + 5]);
+      v.z += __bfloat162float(g.bias[n + 6]); v.w += __bfloat162float(g.bias[n + 7]);
+    }
+    *reinterpret_cast<uint4*>(g.out + (long long)(m0 + r) * g.ldo + n) =
+        make_uint4(pack_bf16x2(u.x, u.y), pack_bf16x2(u.z, u.w), pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+  }
+}
 
 __global__ void __launch_bounds__(THREADS, 1)
 int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
@@ -84,13 +117,12 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_tiles = g.N / BN, k_tiles = g.K / (SUB * BK), mt = blockIdx.y, m0 = mt * BM;
   // This CTA's steps of 128 k: its `own` steps of whole tiles, then its piece of the line of the tiles that are left over.
-  const long long ctas = gridDim.x, whole = n_tiles / ctas * ctas, rest = (n_tiles - whole) * (long long)k_tiles;
-  const long long sharers = min(ctas, max(1LL, rest / 2));          // of the left-over tiles: at least two steps each
-  const int own = (int)(n_tiles / ctas) * k_tiles;
-  const long long r0 = rest * min((long long)blockIdx.x, sharers) / sharers;
-  const int ksteps = own + (int)(rest * min(blockIdx.x + 1LL, sharers) / sharers - r0), a_stages = g.a_stages, RAW_STAGES = g.raw_stages;
-  auto line = [&](int i) -> long long { return i < own ? (long long)blockIdx.x * own + i : whole * k_tiles + r0 + (i - own); };
-  auto part_steps = [&](int i) -> int { return (int)min((long long)(ksteps - i), k_tiles - line(i) % k_tiles); };
+  const int ctas = gridDim.x, whole = n_tiles / ctas * ctas, own = n_tiles / ctas * k_tiles, sharers = g.sharers;
+  const Pieces pieces((uint32_t)((n_tiles - whole) * k_tiles), (uint32_t)sharers);
+  const int cta = blockIdx.x, r0 = (int)pieces.begin(min(cta, sharers));
+  const int ksteps = own + (int)pieces.begin(min(cta + 1, sharers)) - r0, a_stages = g.a_stages, RAW_STAGES = g.raw_stages;
+  auto line = [&](int i) -> int { return i < own ? cta * own + i : whole * k_tiles + r0 + (i - own); };
+  auto part_steps = [&](int i) -> int { return min(ksteps - i, k_tiles - line(i) % k_tiles); };
   const uint32_t a_bytes = (uint32_t)g.a_rows * 128u;
 
   if (threadIdx.x == 0) {
@@ -119,7 +151,7 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
         if (r % ISSUE_LANES != lane) continue;
         if (!mbar_wait(raw_empty(r), ((i / RAW_STAGES) & 1) ^ 1, dead, g.status, 300)) break;
         mbar_expect_tx(raw_full(r), SUB * RAW_BYTES);
-        bulk_load_1d(sRaw + r * (SUB * RAW_BYTES), g.w_tiles + line(i) * (SUB * RAW_BYTES), SUB * RAW_BYTES, raw_full(r));
+        bulk_load_1d(sRaw + r * (SUB * RAW_BYTES), g.w_tiles + (long long)line(i) * (SUB * RAW_BYTES), SUB * RAW_BYTES, raw_full(r));
       }
     }
   } else if (warp == 3) {
@@ -128,7 +160,7 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
       for (int i = 0; i < ksteps; ++i) {
         const int s = i % a_stages;
         if (s % ISSUE_LANES != lane) continue;
-        const int ks = (int)(line(i) % k_tiles);                      // step within its tile
+        const int ks = line(i) % k_tiles;                             // step within its tile
         if (!mbar_wait(a_empty(s), ((i / a_stages) & 1) ^ 1, dead, g.status, 301)) break;
         mbar_expect_tx(a_full(s), SUB * a_bytes);
 #pragma unroll
@@ -213,10 +245,12 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
     bool ok = true;
     int part = 0;
     for (int i = 0; i < ksteps; ++part) {
-      const int nt = (int)(line(i) / k_tiles), n0 = nt * BN, a = part & 1;
-      // CTAs that share a left-over tile: that of its step x is the largest c with rest c / sharers <= x
-      const long long lo = nt < whole ? 0 : ((nt - whole) * k_tiles * sharers + sharers - 1) / rest;
-      const long long hi = nt < whole ? 0 : ((nt + 1 - whole) * k_tiles * sharers - 1) / rest;
+      const int nt = line(i) / k_tiles, n0 = nt * BN, a = part & 1;
+      // the CTAs that share a left-over tile
+      const uint32_t t0 = (uint32_t)((nt - whole) * k_tiles);
+      const int lo = nt < whole ? 0 : (int)pieces.of(t0), hi = nt < whole ? 0 : (int)pieces.of(t0 + k_tiles - 1);
+      // a CTA's piece may end one shared tile and begin another: slot 0 for the part it begins with, 1 for the other
+      float4* const mine = part_slot(g, mt, cta, i != own) + q * 32 + lane;
       i += part_steps(i);
       ok = __all_sync(0xffffffffu, mbar_wait(acc_full(a), (part >> 1) & 1, dead, g.status, 306)) && ok;
       tc_fence_after();
@@ -227,7 +261,8 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
           __syncwarp();
           tmem_ld32(tmem + a * BN + ((uint32_t)(q * 32) << 16) + c, rr);
           tmem_ld_wait();
-          if (row >= g.M) continue;
+          // a slot takes all its rows, so that no memory sector is written in part (17 rows, 4096 x 22016, cold caches: 55 -> 51 us)
+          if (lo == hi ? row >= g.M : q * 32 + lane >= g.a_rows) continue;
           if (lo == hi) {
             __nv_bfloat16* dstp = g.out + (long long)row * g.ldo + n0 + c;
 #pragma unroll
@@ -242,11 +277,12 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
               *reinterpret_cast<uint4*>(dstp + j) = pk;
             }
           } else {
-            float* dstp = g.acc + (long long)row * g.N + n0 + c;
+            // neighbouring lanes hold neighbouring rows: 16 bytes each, side by side
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
-              red_add_f32x4(dstp + j, __uint_as_float(rr[j]), __uint_as_float(rr[j + 2]), __uint_as_float(rr[j + 4]), __uint_as_float(rr[j + 6]));
-              red_add_f32x4(dstp + j + 4, __uint_as_float(rr[j + 1]), __uint_as_float(rr[j + 3]), __uint_as_float(rr[j + 5]), __uint_as_float(rr[j + 7]));
+              float4* dstp = mine + (c + j) / 4 * g.a_rows;
+              dstp[0] = make_float4(__uint_as_float(rr[j]), __uint_as_float(rr[j + 2]), __uint_as_float(rr[j + 4]), __uint_as_float(rr[j + 6]));
+              dstp[g.a_rows] = make_float4(__uint_as_float(rr[j + 1]), __uint_as_float(rr[j + 3]), __uint_as_float(rr[j + 5]), __uint_as_float(rr[j + 7]));
             }
           }
         }
@@ -255,26 +291,15 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty(a));
       if (lo == hi) continue;
-      // the CTA that arrives last at the tile's counter turns the fp32 sums into the output
+      // the CTA that arrives last at the tile's counter turns the parts into the output
       __threadfence();
       asm volatile("bar.sync 1, 128;" ::: "memory");
       int* counter = g.counters + mt * n_tiles + nt;
-      if (et == 0) *is_last = (atomicAdd(counter, 1) == (int)(hi - lo)) && !*dead;
+      if (et == 0) *is_last = (atomicAdd(counter, 1) == hi - lo) && !*dead;
       asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (i == ksteps) break;                               // the CTA's last part: all its threads take part in the sum, below
       if (*is_last) {
-        __threadfence();
-        const int rows = min(BM, g.M - m0);
-        for (int e = et; e < rows * (BN / 4); e += 128) {
-          const int r = e / (BN / 4), c4 = (e % (BN / 4)) * 4;
-          float4* src = reinterpret_cast<float4*>(g.acc + (long long)(m0 + r) * g.N + n0 + c4);
-          float4 v = __ldcg(src);
-          *src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (g.bias) {
-            v.x += __bfloat162float(g.bias[n0 + c4]); v.y += __bfloat162float(g.bias[n0 + c4 + 1]);
-            v.z += __bfloat162float(g.bias[n0 + c4 + 2]); v.w += __bfloat162float(g.bias[n0 + c4 + 3]);
-          }
-          *reinterpret_cast<uint2*>(g.out + (long long)(m0 + r) * g.ldo + n0 + c4) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
-        }
+        sum_parts(g, mt, nt, lo, hi, pieces.begin(lo) < t0, et, 128);
         if (et == 0) *counter = 0;
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");        // is_last has been read
@@ -284,6 +309,15 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
   tc_fence_before();
   __syncthreads();
   if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, 2 * BN); }
+  if (ksteps > own && *is_last) {
+    const int nt = line(ksteps - 1) / k_tiles;
+    const uint32_t t0 = (uint32_t)((nt - whole) * k_tiles);
+    const int lo = (int)pieces.of(t0), hi = (int)pieces.of(t0 + k_tiles - 1);
+    if (lo != hi) {
+      sum_parts(g, mt, nt, lo, hi, pieces.begin(lo) < t0, threadIdx.x, THREADS);
+      if (threadIdx.x == 0) g.counters[mt * n_tiles + nt] = 0;
+    }
+  }
 }
 
 // packed [K][N/2] bytes + scales (flat groups) -> tiles [N/128][K/64][4608]
@@ -321,30 +355,45 @@ CGK_API int cgk_int4_tile_weights(const void* packed, const float* scales, int K
 }
 CGK_API long long cgk_int4_gemm_counters(int M, int N) { return (long long)((M + BM - 1) / BM) * (N / BN); }
 
-// x bf16 [M, ldx]; w_tiles from cgk_int4_tile_weights; out bf16 [M, ldo]; bias bf16 [N] or null.
-// acc (fp32 [M, N]) and counters (int32 [cgk_int4_gemm_counters]) serve split-K: both must be
-// zero before the first call and are left zero by every call.  splits 0 = chosen here.
-CGK_API int cgk_int4_gemm(const void* x, long long ldx, const void* w_tiles, float* acc, int* counters, void* out, long long ldo,
-                          const void* bias, int M, int N, int K, int splits, void* stream) {
+// How the tiles are dealt out: one CTA per SM (of a row tile's share of them), each with at least two steps of the left-over
+// tiles; given splits: that many equal parts of every tile; without a place for parts: whole tiles.
+struct Deal { long long ctas, sharers; };
+static Deal deal(int sms, int M, int N, int K, int splits, bool parts) {
+  const long long n_tiles = N / BN, m_tiles = (M + BM - 1) / BM, ksteps = K / (SUB * BK);
+  if (splits > 0 || !parts) return {n_tiles * (splits > 0 ? splits : 1), splits > 1 ? n_tiles * splits : 1};
+  long long ctas = sms / m_tiles;
+  if (ctas > n_tiles * ksteps / 2) ctas = n_tiles * ksteps / 2;
+  if (ctas < 1) ctas = 1;
+  // the fewest sharers with the same longest piece: fewer parts to store and to sum
+  const long long rest = n_tiles % ctas * ksteps, most = rest / 2 < 1 ? 1 : rest / 2 < ctas ? rest / 2 : ctas, longest = (rest + most - 1) / most;
+  return {ctas, rest > 0 ? (rest + longest - 1) / longest : 1};
+}
+static int part_rows(int M) { return M > BM ? BM : (M + 7) / 8 * 8; }
+
+CGK_API long long cgk_int4_gemm_parts_floats(int M, int N, int K, int splits) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || M <= 0 || N < BN || K < SUB * BK) return 0;
+  const Deal d = deal(cgk::sm_count(dev), M, N, K, splits, true);
+  return (long long)((M + BM - 1) / BM) * d.sharers * 2 * BN * part_rows(M);
+}
+
+// x bf16 [M, ldx]; w_tiles from cgk_int4_tile_weights; out bf16 [M, ldo]; bias bf16 [N] or null.  parts (fp32
+// [cgk_int4_gemm_parts_floats], any contents) and counters (int32 [cgk_int4_gemm_counters], zero before the first call and left
+// zero by every call) serve tiles shared by several CTAs; without them every tile is computed whole.  splits 0 = chosen here.
+CGK_API int cgk_int4_gemm_parts(const void* x, long long ldx, const void* w_tiles, float* parts, int* counters, void* out, long long ldo,
+                                const void* bias, int M, int N, int K, int splits, void* stream) {
   using namespace cgk;
   CGK_REQUIRE(x && w_tiles && out, "cgk_int4_gemm: null pointer");
   CGK_REQUIRE(M > 0 && N > 0 && K > 0 && N % BN == 0 && K % (SUB * BK) == 0, "cgk_int4_gemm: need N %% 128 == 0 and K %% 128 == 0 (got M=%d N=%d K=%d)", M, N, K);
-  CGK_REQUIRE(ldx % 8 == 0 && ldo % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)w_tiles & 15) == 0 && ((uintptr_t)out & 15) == 0 && ((uintptr_t)acc & 15) == 0,
+  CGK_REQUIRE(ldx % 8 == 0 && ldo % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)w_tiles & 15) == 0 && ((uintptr_t)out & 15) == 0 && ((uintptr_t)parts & 15) == 0,
               "cgk_int4_gemm: operands must be 16-byte aligned with leading dimensions that are multiples of 8");
   int dev = 0;
   CGK_CUDA_CHECK(cudaGetDevice(&dev));
-  const int sms = sm_count(dev), n_tiles = N / BN, m_tiles = (M + BM - 1) / BM, ksteps = K / (SUB * BK);
+  const int m_tiles = (M + BM - 1) / BM, ksteps = K / (SUB * BK);
   CGK_REQUIRE(splits <= 0 || ksteps % splits == 0, "cgk_int4_gemm: K/128 = %d is not divisible by splits = %d", ksteps, splits);
-  CGK_REQUIRE(splits <= 1 || (acc && counters), "cgk_int4_gemm: split-K needs the acc and counters buffers");
-  // one CTA per SM, with at least two steps each; given splits, or no scratch to meet in: whole tiles or equal parts of them
-  const long long total = (long long)n_tiles * ksteps;
-  long long ctas = (long long)n_tiles * (splits > 0 ? splits : 1);
-  if (splits <= 0 && acc && counters) {
-    ctas = sms / m_tiles;
-    if (ctas > total / 2) ctas = total / 2;
-    if (ctas < 1) ctas = 1;
-  }
-  const int a_rows = m_tiles > 1 ? BM : (M + 7) / 8 * 8;
+  CGK_REQUIRE(splits <= 1 || (parts && counters), "cgk_int4_gemm: split-K needs scratch and counters");
+  const Deal d = deal(sm_count(dev), M, N, K, splits, parts && counters);
+  const int a_rows = part_rows(M);
   // X comes from L2 a microsecond after it is asked for: four stages of it, as long as five of W fit beside them (at least 2),
   // and up to a quarter of the ring budget where rows are few
   int a_stages = (RING_BUDGET / 4) / (SUB * a_rows * 128);
@@ -363,9 +412,19 @@ CGK_API int cgk_int4_gemm(const void* x, long long ldx, const void* w_tiles, flo
     CGK_CUDA_CHECK(cudaFuncSetAttribute(int4_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     attr_set[dev] = true;
   }
-  Int4Dev g{(const uint8_t*)w_tiles, acc, counters, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)bias, M, N, K,
-            a_rows, a_stages, raw_stages, device_status(dev)};
-  int4_gemm_kernel<<<dim3((unsigned)ctas, m_tiles), THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(tmX, g);
+  Int4Dev g{(const uint8_t*)w_tiles, (float4*)parts, counters, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)bias, M, N, K,
+            a_rows, a_stages, raw_stages, (int)d.sharers, device_status(dev)};
+  int4_gemm_kernel<<<dim3((unsigned)d.ctas, m_tiles), THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(tmX, g);
   CGK_LAUNCH_CHECK();
   return 0;
+}
+
+// The same for callers that hold an accumulator (fp32 [M, N], zero, left zero) instead of parts, which then come from the stream's
+// memory pool (whole tiles where that has none left).
+CGK_API int cgk_int4_gemm(const void* x, long long ldx, const void* w_tiles, float* acc, int* counters, void* out, long long ldo,
+                          const void* bias, int M, int N, int K, int splits, void* stream) {
+  const bool shared = acc && counters;
+  return cgk::with_stream_scratch(shared ? cgk_int4_gemm_parts_floats(M, N, K, splits) : 0, (cudaStream_t)stream, [&](float* parts) {
+    return cgk_int4_gemm_parts(x, ldx, w_tiles, parts, parts ? counters : nullptr, out, ldo, bias, M, N, K, shared && !parts ? 0 : splits, stream);
+  });
 }

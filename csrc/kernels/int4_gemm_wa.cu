@@ -36,11 +36,12 @@
 // Work is dealt out by steps, not by tiles: the steps of all feature tiles are one line (which is also how the stream lies in
 // memory) and every resident CTA takes an equal piece of it, so that no SM has two tiles while its neighbour has one, and a
 // K of 11 008 (86 steps, whose only power-of-two divisor is 2) fills the machine like any other.  A piece covers the end of
-// one tile and the start of the next; a tile covered by one CTA is written at once, the parts of the others go to an fp32
-// buffer with red.add, and the CTA that arrives last at the tile's counter adds the bias, writes bf16 and leaves buffer and
-// counter zeroed.  The MMA warp runs its loop converged (see umma_f16_lane): eight MMAs of 16 columns a step are few tensor
-// cycles, and issuing them from a one-lane branch took longer than the step's conversion.  16 rows, device time: 11008 x 4096
-// 47.8 -> about 25 us, 4096 x 22016 44.5 -> 38 us.
+// one tile and the start of the next; a tile covered by one CTA is written at once, the parts of the others go to fp32 slots of
+// their own, and the CTA that arrives last at the tile's counter sums them in the order of the CTAs, adds the bias, writes bf16
+// and leaves the counter zeroed.  The order is fixed, so a call gives the same bits every time.  The MMA warp runs its loop
+// converged (see umma_f16_lane): eight MMAs of 16 columns a step are few tensor cycles, and issuing them from a one-lane
+// branch took longer than the step's conversion.  16 rows, layers one after the other: 4096 x 22016 45.2 us by whole tiles, 34.7
+// like this; 11008 x 4096 (two parts per tile) 48.2 and 24.7; 4096 x 4096 in eight parts added by atomics 13.1, 14.9.
 #include <cuda_bf16.h>
 
 #include "host_common.h"
@@ -62,7 +63,8 @@ constexpr int W_MAXCH = 8;                                     // X chunks per t
 struct WaDev {
   const uint8_t* tiles;            // [N/128][K/64][4352]
   const __nv_bfloat16* x; long long ldx;
-  float* acc; int* counters;       // split-K scratch (zero between calls)
+  float* parts;                    // slots of shared tiles' parts: [m_tiles][ctas][2][x_rows][128]
+  int* counters;                   // [m_tiles * n_tiles], zero between calls (shared tiles only)
   __nv_bfloat16* out; long long ldo;
   const __nv_bfloat16* bias;
   int M, N, K;
@@ -77,16 +79,34 @@ __device__ __forceinline__ uint4 ldg_stream_16(const void* p) {     // read once
   return v;
 }
 
-// A part's accumulator (warps 0-3): lane = output feature, column = token.  whole: the part is the tile.
-__device__ __noinline__ void wa_store_part(const WaDev& g, uint32_t tmem, int x_rows, int m0, int nt, const float* xsum_s, bool whole,
-                                           uint32_t acc_full, uint32_t parity, volatile int* dead, bool ok) {
+// The CTAs lo .. hi of a row tile that share feature tile nt.  A CTA's piece may end one shared tile and begin another: its
+// slot 0 is for the part that its piece begins with, slot 1 for the other.  (Worked out in here, out of line: the conversion
+// loop has no registers left.)
+struct WaShare { uint32_t lo, hi, first; };
+__device__ __forceinline__ WaShare wa_share(const WaDev& g, uint32_t nt) {
+  const uint32_t k_tiles = g.K / (WSUB * WK);
+  const Pieces pieces((g.N / WF) * k_tiles, gridDim.x);
+  WaShare w;
+  w.lo = pieces.of(nt * k_tiles);
+  w.hi = pieces.of((nt + 1) * k_tiles - 1);
+  w.first = pieces.begin(w.lo) < nt * k_tiles;               // slot of CTA lo; the others begin with this tile
+  return w;
+}
+__device__ __forceinline__ float* wa_slot(const WaDev& g, uint32_t cta, uint32_t which) {
+  return g.parts + (unsigned long long)((blockIdx.y * gridDim.x + cta) * 2 + which) * (WF * g.x_rows);
+}
+
+// A part's accumulator (warps 0-3): lane = output feature, column = token.
+__device__ __noinline__ void wa_store_part(const WaDev& g, uint32_t tmem, int nt, const float* xsum_s, uint32_t acc_full, uint32_t part, volatile int* dead, bool ok) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp >= 4 || !__all_sync(0xffffffffu, ok && mbar_wait(acc_full, parity, dead, g.status, 331))) return;
+  if (warp >= 4 || !__all_sync(0xffffffffu, ok && mbar_wait(acc_full, part & 1, dead, g.status, 331))) return;
   tc_fence_after();
-  const int fo = nt * WF + warp * 32 + lane;
-  const float bias = (g.bias && whole) ? __bfloat162float(g.bias[fo]) : 0.0f;
+  const WaShare w = wa_share(g, nt);
+  const int f = warp * 32 + lane, fo = nt * WF + f, m0 = blockIdx.y * 128;
+  float* const slot = w.lo == w.hi ? nullptr : wa_slot(g, blockIdx.x, part > 0) + f;
+  const float bias = (g.bias && !slot) ? __bfloat162float(g.bias[fo]) : 0.0f;
 #pragma unroll 1
-  for (int c = 0; c < x_rows; c += 16) {
+  for (int c = 0; c < g.x_rows; c += 16) {
     uint32_t rr[16];
     __syncwarp();
     tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + c, rr);
@@ -96,35 +116,51 @@ __device__ __noinline__ void wa_store_part(const WaDev& g, uint32_t tmem, int x_
       const int t = m0 + c + j;
       if (t < g.M) {
         const float v = __uint_as_float(rr[j]) - 136.0f * xsum_s[c + j];
-        if (whole) g.out[(long long)t * g.ldo + fo] = __float2bfloat16(v + bias);
-        else atomicAdd(g.acc + (long long)t * g.N + fo, v);
+        if (slot) slot[(c + j) * WF] = v;
+        else g.out[(long long)t * g.ldo + fo] = __float2bfloat16(v + bias);
       }
     }
   }
-  if (!whole) __threadfence();
+  if (slot) __threadfence();
 }
 
-// Counts a finished part of a tile that `others` + 1 CTAs share; the last one writes the output.  All conversion threads.
-__device__ __noinline__ void wa_finish_tile(const WaDev& g, int m0, int mt, int nt, int others, volatile int* is_last, volatile int* dead) {
-  const int tid = threadIdx.x, n0 = nt * WF;
-  int* counter = g.counters + mt * (g.N / WF) + nt;
-  if (tid == 0) *is_last = (atomicAdd(counter, 1) == others) && !*dead;
-  asm volatile("bar.sync 1, 256;" ::: "memory");
-  if (!*is_last) return;
+// Counts a finished part of a shared tile (one thread).
+__device__ __forceinline__ void wa_count_part(const WaDev& g, const WaShare& w, int nt, volatile int* is_last, volatile int* dead) {
+  *is_last = (atomicAdd(g.counters + blockIdx.y * (g.N / WF) + nt, 1) == (int)(w.hi - w.lo)) && !*dead;
+}
+// The output of a tile out of its parts, summed in the order of the CTAs; W_CONV_THREADS threads, FETCH parts
+// on their way at once (16 rows, 4096 x 4096: 15.1 us with two, 14.9 with four, 15.9 with eight).
+template <int FETCH>
+__device__ __forceinline__ void wa_sum_parts(const WaDev& g, const WaShare& w, int nt) {
   __threadfence();
+  const int tid = threadIdx.x, n0 = nt * WF, m0 = blockIdx.y * 128, followers = (int)(w.hi - w.lo);
+  const float4* first = reinterpret_cast<const float4*>(wa_slot(g, w.lo, w.first));
+  const float4* next = reinterpret_cast<const float4*>(wa_slot(g, w.lo + 1, 0));
+  const int stride = 2 * (WF / 4) * g.x_rows;
   const int rows = min(128, g.M - m0);
   for (int i = tid; i < rows * (WF / 4); i += W_CONV_THREADS) {
     const int t = i / (WF / 4), c4 = (i % (WF / 4)) * 4;
-    float4* src = reinterpret_cast<float4*>(g.acc + (long long)(m0 + t) * g.N + n0 + c4);
-    float4 v = __ldcg(src);
-    *src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 v = __ldcg(first + i);
+#pragma unroll FETCH
+    for (int c = 0; c < followers; ++c) {
+      const float4 u = __ldcg(next + (long long)c * stride + i);
+      v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+    }
     if (g.bias) {
       v.x += __bfloat162float(g.bias[n0 + c4]); v.y += __bfloat162float(g.bias[n0 + c4 + 1]);
       v.z += __bfloat162float(g.bias[n0 + c4 + 2]); v.w += __bfloat162float(g.bias[n0 + c4 + 3]);
     }
     *reinterpret_cast<uint2*>(g.out + (long long)(m0 + t) * g.ldo + n0 + c4) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
   }
-  if (tid == 0) *counter = 0;
+  if (tid == 0) g.counters[blockIdx.y * (g.N / WF) + nt] = 0;
+}
+// A shared tile that ends inside a CTA's piece: the CTA that has its last part writes the output.  All conversion threads.
+__device__ __noinline__ void wa_finish_tile(const WaDev& g, int nt, volatile int* is_last, volatile int* dead) {
+  const WaShare w = wa_share(g, nt);
+  if (w.lo == w.hi) return;
+  if (threadIdx.x == 0) wa_count_part(g, w, nt, is_last, dead);
+  asm volatile("bar.sync 1, 256;" ::: "memory");
+  if (*is_last) wa_sum_parts<1>(g, w, nt);
 }
 
 template <int NCH>                   // X chunks per thread and step (x_rows * 16 / 256, rounded up)
@@ -148,9 +184,8 @@ int4_wa_kernel(const WaDev g) {
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int n_tiles = g.N / WF, k_tiles = g.K / (WSUB * WK), mt = blockIdx.y, m0 = mt * 128;
-  const long long total = (long long)n_tiles * k_tiles, ctas = gridDim.x;
-  const long long u0 = total * blockIdx.x / ctas;                    // this CTA's steps: [u0, u0 + steps)
-  const int steps = (int)(total * (blockIdx.x + 1) / ctas - u0);
+  const Pieces pieces((uint32_t)(n_tiles * k_tiles), gridDim.x);
+  const int u0 = (int)pieces.begin(blockIdx.x), steps = (int)pieces.begin(blockIdx.x + 1) - u0;     // this CTA's steps: [u0, u0 + steps)
   const uint32_t acc_cols = x_rows <= 32 ? 32u : x_rows <= 64 ? 64u : 128u;
   const uint32_t tmem_cols = acc_cols + W_STAGES * W_ACOLS <= 256 ? 256u : 512u;     // accumulator, then the operand stages
 
@@ -169,7 +204,7 @@ int4_wa_kernel(const WaDev g) {
   const uint32_t tmem = *tmem_slot, tmem_a = tmem + acc_cols;
   // A part of a tile ends at two barriers of all threads: its row sums are complete and its MMAs issued; its accumulator has
   // been read.  Both roles pass them for every part, also after a wait that gave up (later waits then return at once).
-  auto part_steps = [&](int i) -> int { return (int)min((long long)(steps - i), k_tiles - (u0 + i) % k_tiles); };
+  auto part_steps = [&](int i) -> int { return min(steps - i, k_tiles - (u0 + i) % k_tiles); };
 
   if (warp == W_CONV_THREADS / 32) {
     // ---- MMA warp: one lane issues; a stage is free again when its MMAs have completed
@@ -208,7 +243,7 @@ int4_wa_kernel(const WaDev g) {
     // X chunk c = tid + 256 j: block (c / 8) / x_rows, token row (c / 8) % x_rows, piece c % 8 (k = 8 (c % 8) ..)
     const int ch = tid & 7;
     const int chunks = WSUB * x_rows * 8;                              // per step
-    const uint8_t* wsrc = g.tiles + u0 * W_STEP + sub * W_RAW + f * 16;   // k half 0; half 1 is W_NIB / 2 further
+    const uint8_t* wsrc = g.tiles + (long long)u0 * W_STEP + sub * W_RAW + f * 16;   // k half 0; half 1 is W_NIB / 2 further
     constexpr int NB = NCH == 1 ? 1 : WSUB;                          // scale blocks a thread needs (one chunk: one block)
     // Everything that does not change from step to step is worked out once: where each of this thread's
     // X chunks comes from (128 elements a step, from the start again with the next tile) and where it goes inside a stage's X' tile.
@@ -225,7 +260,7 @@ int4_wa_kernel(const WaDev g) {
       xdst[j] = (uint32_t)blk * x_bytes + sw128_offset((uint32_t)t, (uint32_t)ch);
       xsrc[j] = (c < chunks && m0 + t < g.M) ? g.x + (long long)(m0 + t) * g.ldx + blk * WK + ch * 8 : nullptr;
     }
-    const uint8_t* ssrc = g.tiles + u0 * W_STEP + (NCH == 1 ? min((tid >> 3) / x_rows, WSUB - 1) : 0) * W_RAW + W_NIB + ch * 32;
+    const uint8_t* ssrc = g.tiles + (long long)u0 * W_STEP + (NCH == 1 ? min((tid >> 3) / x_rows, WSUB - 1) : 0) * W_RAW + W_NIB + ch * 32;
     uint4 raw[W_PREFETCH][2];
     uint4 xr[2][NCH];                                                // X chunks and scales of the next two steps, by step parity
     float4 sc[2][NB][2];
@@ -234,7 +269,7 @@ int4_wa_kernel(const WaDev g) {
       raw[d][0] = ldg_stream_16(p);
       raw[d][1] = ldg_stream_16(p + W_NIB / 2);
     };
-    int kx = (int)(u0 % k_tiles);                                    // step of its tile that load_x fetches next
+    int kx = u0 % k_tiles;                                           // step of its tile that load_x fetches next
     auto load_x = [&](int p, int step) {
 #pragma unroll
       for (int j = 0; j < NCH; ++j)
@@ -315,17 +350,16 @@ int4_wa_kernel(const WaDev g) {
             xs[j] = 0.0f;
           }
           asm volatile("bar.sync 2, 288;" ::: "memory");
-          const int nt = (int)((u0 + i) / k_tiles);
-          // CTA of step x: the largest c with total c / ctas <= x
-          const long long lo = (((long long)nt * k_tiles + 1) * ctas - 1) / total, hi = ((long long)(nt + 1) * k_tiles * ctas - 1) / total;
-          wa_store_part(g, tmem, x_rows, m0, nt, xsum_s, lo == hi, acc_full, part & 1, dead, ok);
+          const int nt = (u0 + i) / k_tiles;
+          wa_store_part(g, tmem, nt, xsum_s, acc_full, part, dead, ok);
           ++part;
           tc_fence_before();
           asm volatile("bar.sync 2, 288;" ::: "memory");
           if (tid < 128) xsum_s[tid] = 0.0f;
-          if (lo != hi) wa_finish_tile(g, m0, mt, nt, (int)(hi - lo), is_last, dead);
+          if (i + 1 == steps) break;                                 // the CTA's last part: its sum comes below, where registers are free
+          wa_finish_tile(g, nt, is_last, dead);
           asm volatile("bar.sync 1, 256;" ::: "memory");             // row sums and is_last can be used again
-          left = i + 1 < steps ? part_steps(i + 1) : 0;
+          left = part_steps(i + 1);
         }
       }
     }
@@ -334,6 +368,13 @@ int4_wa_kernel(const WaDev g) {
   tc_fence_before();
   __syncthreads();
   if (warp == 0) { tc_fence_after(); tmem_dealloc(tmem, tmem_cols); }
+  if (steps == 0) return;
+  const int nt = (u0 + steps - 1) / k_tiles;
+  const WaShare w = wa_share(g, nt);
+  if (w.lo == w.hi) return;
+  if (tid == 0) wa_count_part(g, w, nt, is_last, dead);
+  __syncthreads();
+  if (*is_last && tid < W_CONV_THREADS) wa_sum_parts<4>(g, w, nt);
 }
 
 // packed [K][N/2] bytes + scales (flat groups along N) -> tiles [N/128][K/64][4352]
@@ -383,35 +424,44 @@ CGK_API int cgk_int4_wa_tile_weights(const void* packed, const float* scales, in
   return 0;
 }
 
-// x bf16 [M, ldx]; tiles from cgk_int4_wa_tile_weights; out bf16 [M, ldo]; bias bf16 [N] or null.
-// acc (fp32 [M, N]) and counters (int32 [cgk_int4_gemm_counters(M, N)]) serve split-K: zero before
-// the first call, left zero by every call.  splits 0 = chosen here.
-CGK_API int cgk_int4_wa_gemm(const void* x, long long ldx, const void* tiles, float* acc, int* counters, void* out, long long ldo,
-                             const void* bias, int M, int N, int K, int splits, void* stream) {
+static int wa_x_rows(int M) { return M > 128 ? 128 : (M + 15) / 16 * 16; }
+static int wa_chunks(int M) { return (WSUB * wa_x_rows(M) * 8 + W_CONV_THREADS - 1) / W_CONV_THREADS; }
+// CTAs per row tile: all that are resident at once (registers and TMEM columns allow two per SM for few rows), with at least
+// three steps each, and of those the fewest with the same longest piece (fewer parts to store and to sum); given splits: that many equal parts of every tile; without a place for parts: whole tiles.
+static long long wa_ctas(int sms, int M, int N, int K, int splits, bool parts) {
+  const long long n_tiles = N / WF, m_tiles = (M + 127) / 128, total = n_tiles * (K / (WSUB * WK));
+  if (splits > 0 || !parts) return n_tiles * (splits > 0 ? splits : 1);
+  long long ctas = (long long)sms * (wa_chunks(M) <= 2 ? 2 : 1) / m_tiles;
+  if (ctas > total / 3) ctas = total / 3;
+  if (ctas < 1) ctas = 1;
+  const long long longest = (total + ctas - 1) / ctas;
+  return (total + longest - 1) / longest;
+}
+
+CGK_API long long cgk_int4_wa_gemm_parts_floats(int M, int N, int K, int splits) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || M <= 0 || N < WF || K < WSUB * WK) return 0;
+  return (long long)((M + 127) / 128) * wa_ctas(cgk::sm_count(dev), M, N, K, splits, true) * 2 * WF * wa_x_rows(M);
+}
+
+// x bf16 [M, ldx]; tiles from cgk_int4_wa_tile_weights; out bf16 [M, ldo]; bias bf16 [N] or null.  parts (fp32
+// [cgk_int4_wa_gemm_parts_floats], any contents) and counters (int32 [cgk_int4_gemm_counters(M, N)], zero before the first call and
+// left zero by every call) serve tiles shared by several CTAs; without them every tile is computed whole.  splits 0 = chosen here.
+CGK_API int cgk_int4_wa_gemm_parts(const void* x, long long ldx, const void* tiles, float* parts, int* counters, void* out, long long ldo,
+                                   const void* bias, int M, int N, int K, int splits, void* stream) {
   using namespace cgk;
   CGK_REQUIRE(x && tiles && out, "cgk_int4_wa_gemm: null pointer");
   CGK_REQUIRE(M > 0 && N > 0 && K > 0 && N % WF == 0 && K % (WSUB * WK) == 0, "cgk_int4_wa_gemm: need N %% 128 == 0 and K %% 128 == 0 (got M=%d N=%d K=%d)", M, N, K);
-  CGK_REQUIRE(ldx % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)tiles & 15) == 0 && ((uintptr_t)acc & 15) == 0 && ldo % 4 == 0 && ((uintptr_t)out & 7) == 0,
+  CGK_REQUIRE(ldx % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)tiles & 15) == 0 && ((uintptr_t)parts & 15) == 0 && ldo % 4 == 0 && ((uintptr_t)out & 7) == 0,
               "cgk_int4_wa_gemm: misaligned operand");
   int dev = 0;
   CGK_CUDA_CHECK(cudaGetDevice(&dev));
-  const int sms = sm_count(dev), n_tiles = N / WF, m_tiles = (M + 127) / 128, ksteps = K / (WSUB * WK);
-  const int x_rows = m_tiles > 1 ? 128 : (M + 15) / 16 * 16;
-  const int nch = (WSUB * x_rows * 8 + W_CONV_THREADS - 1) / W_CONV_THREADS;
-  const int per_sm = nch <= 2 ? 2 : 1;                     // resident CTAs per SM (registers, TMEM columns)
+  const int m_tiles = (M + 127) / 128, ksteps = K / (WSUB * WK), x_rows = wa_x_rows(M), nch = wa_chunks(M);
   CGK_REQUIRE(splits <= 0 || ksteps % splits == 0, "cgk_int4_wa_gemm: K/128 = %d is not divisible by splits = %d", ksteps, splits);
-  CGK_REQUIRE(splits <= 1 || (acc && counters), "cgk_int4_wa_gemm: split-K needs the acc and counters buffers");
-  // CTAs: all that are resident at once, with at least three steps each; given splits, or no scratch to meet in: whole
-  // tiles or equal parts of them
-  const long long total = (long long)n_tiles * ksteps;
-  long long ctas = (long long)n_tiles * (splits > 0 ? splits : 1);
-  if (splits <= 0 && acc && counters) {
-    ctas = (long long)sms * per_sm / m_tiles;
-    if (ctas > total / 3) ctas = total / 3;
-    if (ctas < 1) ctas = 1;
-  }
+  CGK_REQUIRE(splits <= 1 || (parts && counters), "cgk_int4_wa_gemm: split-K needs scratch and counters");
+  const long long ctas = wa_ctas(sm_count(dev), M, N, K, splits, parts && counters);
   const int smem = 1024 + W_STAGES * WSUB * x_rows * 128 + 128 + 512 + 1024;
-  WaDev g{(const uint8_t*)tiles, (const __nv_bfloat16*)x, ldx, acc, counters, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)bias, M, N, K,
+  WaDev g{(const uint8_t*)tiles, (const __nv_bfloat16*)x, ldx, parts, counters, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)bias, M, N, K,
           x_rows, device_status(dev)};
   const dim3 grid((unsigned)ctas, m_tiles);
   cudaStream_t st = (cudaStream_t)stream;
@@ -425,4 +475,13 @@ CGK_API int cgk_int4_wa_gemm(const void* x, long long ldx, const void* tiles, fl
     case 7: return launch_wa<7>(g, grid, smem, st);
     default: return launch_wa<W_MAXCH>(g, grid, smem, st);
   }
+}
+
+// The same for callers that hold an accumulator (see cgk_int4_gemm).
+CGK_API int cgk_int4_wa_gemm(const void* x, long long ldx, const void* tiles, float* acc, int* counters, void* out, long long ldo,
+                             const void* bias, int M, int N, int K, int splits, void* stream) {
+  const bool shared = acc && counters;
+  return cgk::with_stream_scratch(shared ? cgk_int4_wa_gemm_parts_floats(M, N, K, splits) : 0, (cudaStream_t)stream, [&](float* parts) {
+    return cgk_int4_wa_gemm_parts(x, ldx, tiles, parts, parts ? counters : nullptr, out, ldo, bias, M, N, K, shared && !parts ? 0 : splits, stream);
+  });
 }

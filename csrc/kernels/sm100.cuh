@@ -765,6 +765,14 @@ __host__ __forceinline__ int attention_chunk(int tiles, int heads, int sms) {
   return n < heads ? n : heads;
 }
 
+// A line of `total` steps cut into `n` consecutive pieces that differ by one step at most, the longer ones first.
+struct Pieces {
+  uint32_t q, r;
+  __device__ __forceinline__ Pieces(uint32_t total, uint32_t n) : q(total / n), r(total - total / n * n) {}
+  __device__ __forceinline__ uint32_t begin(uint32_t c) const { return c * q + min(c, r); }
+  __device__ __forceinline__ uint32_t of(uint32_t step) const { return step < r * (q + 1) ? step / (q + 1) : r + (step - r * (q + 1)) / q; }
+};
+
 // Counter-based random bits: a hash of (seed, element index).  The dropout kernels draw their
 // keep / drop decision from it, forward and backward alike, so no mask is ever stored.
 __device__ __forceinline__ uint32_t mix32(uint64_t z) {

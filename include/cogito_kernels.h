@@ -216,18 +216,28 @@ int cgk_int4_dequantize(const void* packed, const float* scales, long long n, in
 long long cgk_int4_tiles_bytes(int K, int N);
 int cgk_int4_tile_weights(const void* packed, const float* scales, int K, int N, int group, void* tiles, void* stream);
 /* out[M,N] (bf16, leading dimension ldo) = x[M,K] (bf16) . dequant(w)[K,N] (+ bias).
- * acc (fp32 [M, N]) and counters (int32 [cgk_int4_gemm_counters(M, N)]) serve split-K: zero
- * before the first call, left zero by every call; both may be null, which forces one split.
- * splits 0 = pick so that the SMs are covered in whole waves. */
+ * parts (fp32 [cgk_int4_gemm_parts_floats(M, N, K, splits)], any contents) and counters (int32
+ * [cgk_int4_gemm_counters(M, N)], zero before the first call, left zero by every call) serve output
+ * tiles that several CTAs share; both may be null, which makes every CTA compute whole tiles.  Calls
+ * that may run at the same time need their own.  splits 0 = dealt out so that all SMs have equal
+ * shares, else that many equal parts of every tile.  Parts are summed in a fixed order.
+ * cgk_int4_gemm takes an accumulator (fp32 [M, N], zero, left zero) in the place of parts, which it
+ * allocates from the stream's memory pool. */
 long long cgk_int4_gemm_counters(int M, int N);
+long long cgk_int4_gemm_parts_floats(int M, int N, int K, int splits);
+int cgk_int4_gemm_parts(const void* x, long long ldx, const void* w_tiles, float* parts, int* counters, void* out,
+                        long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
 int cgk_int4_gemm(const void* x, long long ldx, const void* w_tiles, float* acc, int* counters, void* out,
                   long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
 /* The same product with the weights on the M side of the tensor core (time grows with the rows
  * of x instead of always paying for 128), the group scale folded into x and a bit-trick-only
  * nibble conversion.  Needs group % 128 == 0.  Tiles: [N/128][K/64][4352] (4096 bytes of
- * nibbles [feature][8 words], then 64 fp32 scales); acc / counters as for cgk_int4_gemm. */
+ * nibbles [feature][8 words], then 64 fp32 scales); parts / acc / counters as for cgk_int4_gemm. */
 long long cgk_int4_wa_tiles_bytes(int K, int N);
 int cgk_int4_wa_tile_weights(const void* packed, const float* scales, int K, int N, int group, void* tiles, void* stream);
+long long cgk_int4_wa_gemm_parts_floats(int M, int N, int K, int splits);
+int cgk_int4_wa_gemm_parts(const void* x, long long ldx, const void* tiles, float* parts, int* counters, void* out,
+                           long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
 int cgk_int4_wa_gemm(const void* x, long long ldx, const void* tiles, float* acc, int* counters, void* out,
                      long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
 

@@ -64,6 +64,46 @@ def test_int4_gemm_pieces_of_the_weight_stream(M, K, N, kernel):
     _lib.assert_device_ok()
 
 
+# parts of a shared tile are summed in the order of the CTAs, not of their arrival: a call gives the same bits every time
+@pytest.mark.parametrize("M,K,N", [(16, 11008, 4096), (16, 4096, 22016), (80, 4096, 6144), (80, 4096, 22016), (200, 1408, 4096)])
+@pytest.mark.parametrize("kernel", ["wa", "wb"])
+def test_int4_gemm_repeats_itself_to_the_bit(M, K, N, kernel):
+    torch.manual_seed(M + K)
+    lin = Int4Linear.from_packed(torch.randint(0, 256, (K * N // 2,), dtype=torch.uint8), torch.rand(K * N // 128) * 0.01, K, N).to(DEV)
+    lin.kernel = kernel
+    x = torch.randn(M, K, device=DEV, dtype=torch.bfloat16)
+    first = lin(x)
+    for _ in range(20):
+        assert torch.equal(lin(x), first)
+    _lib.assert_device_ok()
+
+
+# the entry points that take an accumulator instead of parts: same bits, accumulator and counters left zero
+@pytest.mark.parametrize("M,K,N,splits", [(5, 512, 1024, 0), (40, 1024, 384, 4), (130, 384, 256, 3), (7, 256, 256, 1)])
+@pytest.mark.parametrize("wa", [False, True])
+def test_int4_gemm_entry_points_with_an_accumulator(M, K, N, splits, wa):
+    torch.manual_seed(M)
+    L = _lib.lib()
+    lin = Int4Linear(torch.randn(N, K) * 0.05, torch.randn(N) * 0.1, 128).to(DEV)
+    lin.kernel = "wa" if wa else "wb"
+    x = torch.randn(M, K, device=DEV, dtype=torch.bfloat16)
+    want = lin(x, splits=splits)
+    acc = torch.zeros(M, N, device=DEV)
+    counters = torch.zeros(L.cgk_int4_gemm_counters(M, N), dtype=torch.int32, device=DEV)
+    run = L.cgk_int4_wa_gemm if wa else L.cgk_int4_gemm
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    args = lambda a, c, s: (x.data_ptr(), K, lin._tiles[wa].data_ptr(), a, c, out.data_ptr(), N, lin.bias.data_ptr(), M, N, K, s, _lib.stream_ptr())
+    for _ in range(2):
+        out.zero_()
+        _lib.check(run(*args(acc.data_ptr(), counters.data_ptr(), splits)))
+        assert torch.equal(out, want) and not acc.any() and not counters.any()
+    _lib.check(run(*args(None, None, 0)))                     # whole tiles
+    # the same terms in another order: fp32 sums of K products, then the rounding to bf16
+    assert ((out.float() - want.float()).norm() / want.float().norm()).item() < 2 ** -8
+    assert run(*args(None, None, 2)) < 0                      # parts without a place for them
+    _lib.assert_device_ok()
+
+
 @pytest.mark.parametrize("n,group", [(8, 8), (1024, 32), (8 * 1031, 8), (128 * 999, 128), (24 * 100, 24)])
 def test_int4_dequantize_by_words(n, group):
     p, s = quantize_int4(torch.randn(n), group)
