@@ -95,6 +95,8 @@ def _declare(L: ctypes.CDLL) -> None:
         "cgk_rope_apply": [i, vp, vp, vp, vp, i, i, i, i, ll, ll, ll, i, i, i, vp],
         "cgk_int4_quantize": [vp, ll, i, vp, vp, vp],
         "cgk_int4_dequantize": [vp, vp, ll, i, vp, vp, vp],
+        "cgk_exchange_capture_mode": [i],
+        "cgk_stream_sync": [vp],
         "cgk_int4_gemm": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
         "cgk_int4_gemm_parts": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
         "cgk_int4_tile_weights": [vp, vp, i, i, i, vp, vp],
@@ -144,6 +146,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "cgk_kv_int4_attention_scratch_floats": [i, i, i, i, i],
         "cgk_int4_tiles_bytes": [i, i],
         "cgk_int4_wa_tiles_bytes": [i, i],
+        "cgk_capture_id": [vp],
         "cgk_int4_gemm_counters": [i, i],
         "cgk_int4_gemm_parts_floats": [i, i, i, i],
         "cgk_int4_wa_gemm_parts_floats": [i, i, i, i],
@@ -192,6 +195,27 @@ def stream_ptr() -> int:
     if torch.cuda.is_initialized():
         return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     return torch.cuda.current_stream().cuda_stream
+
+
+def outside_capture(make):
+    """What ``make`` returns, made on a stream that no graph is being captured from and complete for every stream: for
+    workspaces that outlive a call and may first be needed inside a capture."""
+    if not torch.cuda.is_current_stream_capturing():
+        made = make()
+        check(lib().cgk_stream_sync(stream_ptr()), "cgk_stream_sync")
+        return made
+    relaxed = 2                                            # allocations and waits elsewhere do not break the capture
+    mode = lib().cgk_exchange_capture_mode(relaxed)
+    try:
+        for _ in range(64):                                # streams come from a pool, in turn
+            with torch.cuda.stream(torch.cuda.Stream()):
+                if not torch.cuda.is_current_stream_capturing():
+                    made = make()
+                    check(lib().cgk_stream_sync(stream_ptr()), "cgk_stream_sync")
+                    return made
+    finally:
+        lib().cgk_exchange_capture_mode(mode)
+    raise KernelError("every stream of the pool is being captured")
 
 
 def ptr(t) -> int | None:

@@ -12,6 +12,7 @@ each weight row once; on CPU the same product is computed from the dequantised w
 from __future__ import annotations
 
 import os
+import threading
 
 import torch
 
@@ -67,6 +68,47 @@ def dequantize_int4(packed: torch.Tensor, scales: torch.Tensor, n: int, group: i
     return (q * scales[idx]).to(dtype)
 
 
+class _Counters:
+    """Arrival counters of the tiles that several CTAs share.  Every launch finds its own zero and leaves them zero, so launches
+    that may run at the same time need different ones: a set per stream, and one per stream of a graph capture, which is not
+    replaced when a later call needs more (the graph keeps its address)."""
+    CAPTURES = 32                          # sets for captures; a launch captured beyond that zeroes its own inside the graph
+
+    def __init__(self):
+        self.lock = threading.Lock()
+        self.by_stream, self.by_capture = {}, {}
+        self.spare = None                  # [CAPTURES, the most that one launch needs]
+
+    def __deepcopy__(self, memo):
+        return _Counters()
+
+    def __reduce__(self):
+        return (_Counters, ())
+
+    def prepare(self, most: int, device):
+        """The sets for captures (``most``: counters of the largest launch); the caller holds the lock."""
+        if self.spare is None or self.spare.device != device:
+            self.by_stream, self.by_capture = {}, {}
+            self.spare = _lib.outside_capture(lambda: torch.zeros(self.CAPTURES, most, dtype=torch.int32, device=device))
+
+    def get(self, need: int, most: int, device) -> torch.Tensor:
+        stream = _lib.stream_ptr()
+        if not torch.cuda.is_current_stream_capturing():
+            own = self.by_stream.get(stream)
+            if own is None or own.numel() < need or own.device != device:    # an older set goes back to the allocator in the stream's order
+                own = self.by_stream[stream] = torch.zeros(need, dtype=torch.int32, device=device)
+            return own
+        if need <= most:
+            key = (_lib.lib().cgk_capture_id(stream), stream)
+            with self.lock:
+                self.prepare(most, device)
+                if key not in self.by_capture and len(self.by_capture) < self.CAPTURES:
+                    self.by_capture[key] = len(self.by_capture)
+                if key in self.by_capture:
+                    return self.spare[self.by_capture[key]]
+        return torch.zeros(need, dtype=torch.int32, device=device)
+
+
 class Int4Linear(torch.nn.Module):
     """y = x @ W^T (+ bias) with W stored as packed INT4 of W^T ([in, out], groups along out)."""
 
@@ -93,7 +135,7 @@ class Int4Linear(torch.nn.Module):
         self.register_buffer("packed", packed)
         self.register_buffer("scales", scales)
         self.register_buffer("bias", None if bias is None else bias.detach().to(torch.bfloat16))
-        self._counters = None
+        self._counters = _Counters()
         self._tiles = {}                      # kernel kind -> tile-major weights
 
     @classmethod
@@ -109,7 +151,7 @@ class Int4Linear(torch.nn.Module):
         self.register_buffer("packed", packed.to(torch.uint8).contiguous())
         self.register_buffer("scales", scales.to(torch.float32).contiguous())
         self.register_buffer("bias", None if bias is None else bias.detach().to(torch.bfloat16))
-        self._counters = None
+        self._counters = _Counters()
         self._tiles = {}
         return self
 
@@ -121,6 +163,24 @@ class Int4Linear(torch.nn.Module):
         """W^T as [in, out]."""
         return dequantize_int4(self.packed, self.scales, self.in_features * self.out_features, self.group, dtype) \
             .view(self.in_features, self.out_features)
+
+    def _tile(self, wa: bool, device) -> torch.Tensor:
+        """One-time tile-major reordering of the same quantised values, and the counters that captured calls will need: made
+        before anything is recorded, so that a graph neither repeats the work nor owns the memory."""
+        L, K, N = _lib.lib(), self.in_features, self.out_features
+        nbytes, tile = (L.cgk_int4_wa_tiles_bytes, L.cgk_int4_wa_tile_weights) if wa else (L.cgk_int4_tiles_bytes, L.cgk_int4_tile_weights)
+
+        def make():
+            tiles = torch.empty(nbytes(K, N), dtype=torch.uint8, device=device)
+            _lib.check(tile(self.packed.data_ptr(), self.scales.data_ptr(), K, N, self.group, tiles.data_ptr(), _lib.stream_ptr()), "cgk_int4_tile_weights")
+            _lib.count_launch()
+            return tiles
+
+        with self._counters.lock:
+            self._counters.prepare(L.cgk_int4_gemm_counters(self.DENSE_ROWS, N), device)
+            if self._tiles.get(wa) is None or self._tiles[wa].device != device:
+                self._tiles[wa] = _lib.outside_capture(make)
+            return self._tiles[wa]
 
     def _takes_dense(self, rows: int, splits: int = 0) -> bool:
         return self.kernel == "auto" and splits == 0 and rows > self.DENSE_ROWS
@@ -170,23 +230,16 @@ class Int4Linear(torch.nn.Module):
         wa = (self.kernel == "wa" or (self.kernel == "auto" and M <= 16)) and self.group % 128 == 0 and K % 128 == 0
         tiles = self._tiles.get(wa)
         if tiles is None or tiles.device != x2.device:
-            # one-time tile-major reordering of the same quantised values
-            nbytes, tile = (L.cgk_int4_wa_tiles_bytes, L.cgk_int4_wa_tile_weights) if wa else (L.cgk_int4_tiles_bytes, L.cgk_int4_tile_weights)
-            tiles = self._tiles[wa] = torch.empty(nbytes(K, N), dtype=torch.uint8, device=x2.device)
-            _lib.check(tile(self.packed.data_ptr(), self.scales.data_ptr(), K, N, self.group,
-                            tiles.data_ptr(), _lib.stream_ptr()), "cgk_int4_tile_weights")
-            _lib.count_launch()
-        # for the output tiles that several CTAs share: the parts' own place, and counters (zero once, every call leaves them zero)
+            tiles = self._tile(wa, x2.device)
+        # for the output tiles that several CTAs share: a place for their parts (of this call alone), and counters
         parts = torch.empty((L.cgk_int4_wa_gemm_parts_floats if wa else L.cgk_int4_gemm_parts_floats)(M, N, K, splits), dtype=torch.float32, device=x2.device)
-        need = L.cgk_int4_gemm_counters(M, N)
-        if self._counters is None or self._counters.numel() < need or self._counters.device != x2.device:
-            self._counters = torch.zeros(need, dtype=torch.int32, device=x2.device)
+        counters = self._counters.get(L.cgk_int4_gemm_counters(M, N), L.cgk_int4_gemm_counters(self.DENSE_ROWS, N), x2.device)
         if out is None:
             out = torch.empty(M, N, dtype=torch.bfloat16, device=x2.device)
         elif out.dtype != torch.bfloat16 or not out.is_contiguous() or out.numel() != M * N:
             raise ValueError("out must be a contiguous bf16 [rows, out_features] tensor")
         _lib.check((L.cgk_int4_wa_gemm_parts if wa else L.cgk_int4_gemm_parts)(
-            x2.data_ptr(), K, tiles.data_ptr(), parts.data_ptr(), self._counters.data_ptr(),
+            x2.data_ptr(), K, tiles.data_ptr(), parts.data_ptr(), counters.data_ptr(),
             out.data_ptr(), N, _lib.ptr(self.bias), M, N, K, splits, _lib.stream_ptr()), "cgk_int4_gemm")
         _lib.count_launch()
         return out.view(*lead, N)

@@ -145,3 +145,26 @@ CGK_API int cgk_read_status(int* out, void* stream) {
 }
 
 CGK_API int cgk_version() { return 100; }
+
+// Identity of the graph capture that the stream takes part in; 0: none.
+CGK_API long long cgk_capture_id(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &id) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusActive ? (long long)id : 0;
+}
+
+// What the calling thread may do on streams that are not being captured while one is (cudaStreamCaptureMode); the mode before it.
+CGK_API int cgk_exchange_capture_mode(int mode) {
+  cudaStreamCaptureMode m = (cudaStreamCaptureMode)mode;
+  CGK_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&m));
+  return (int)m;
+}
+
+CGK_API int cgk_stream_sync(void* stream) {
+  CGK_CUDA_CHECK(cudaStreamSynchronize((cudaStream_t)stream));
+  return 0;
+}

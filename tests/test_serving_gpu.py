@@ -78,6 +78,90 @@ def test_int4_gemm_repeats_itself_to_the_bit(M, K, N, kernel):
     _lib.assert_device_ok()
 
 
+def _int4_layer(K=1024, N=2304):
+    g = torch.Generator().manual_seed(K + N)
+    packed = torch.randint(0, 256, (K * N // 2,), dtype=torch.uint8, generator=g)
+    return Int4Linear.from_packed(packed, torch.rand(K * N // 128, generator=g) * 0.01, K, N).to(DEV)
+
+
+# A captured launch keeps the addresses it was given: a later call with more rows must leave them alone, whether the kernel ran
+# before the capture or not.  Memory that such a call gave back would be handed out again and filled.
+@pytest.mark.parametrize("rows", [4, 20, 80])
+@pytest.mark.parametrize("warm", [False, True])
+def test_int4_launch_captured_before_a_larger_call(rows, warm):
+    torch.manual_seed(rows)
+    x, larger, prompt = (torch.randn(n, 1024, device=DEV, dtype=torch.bfloat16) for n in (rows, 200, 300))
+    want, want_larger = _int4_layer()(x), _int4_layer()(larger)
+    lin = _int4_layer()
+    lin(prompt)                                               # goes through the dense product: no workspace yet
+    if warm:
+        lin(x)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = lin(x)
+    if not warm:
+        assert torch.equal(lin(x), want)                      # the layer's own copy of the weights is there before any replay
+    assert torch.equal(lin(larger), want_larger)
+    junk = [torch.full((n,), 0x55555555, dtype=torch.int32, device=DEV) for n in (16, 64, 256, 1024, 1 << 14, 1 << 18, 1 << 20) for _ in range(4)]
+    for _ in range(3):
+        got.zero_()
+        graph.replay()
+        assert torch.equal(got, want)
+    assert torch.equal(lin(larger), want_larger) and torch.equal(lin(x), want)
+    assert all((j == 0x55555555).all() for j in junk)
+    _lib.assert_device_ok()
+
+
+def test_int4_launches_captured_more_often_than_there_are_counters():
+    x = torch.randn(16, 1024, device=DEV, dtype=torch.bfloat16)
+    lin = _int4_layer()
+    want, graphs = lin(x), []
+    for _ in range(lin._counters.CAPTURES + 3):
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = lin(x)
+        graphs.append((graph, got))
+    for graph, got in graphs:
+        for _ in range(2):
+            got.zero_()
+            graph.replay()
+            assert torch.equal(got, want)
+    assert len(lin._counters.by_capture) == lin._counters.CAPTURES
+
+
+# calls of one layer on two streams, eager and captured, run at the same time
+@pytest.mark.parametrize("rows", [16, 20])
+def test_int4_layer_on_two_streams(rows):
+    torch.manual_seed(rows)
+    lin = _int4_layer()
+    xs = [torch.randn(rows, 1024, device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+    want = [lin(x) for x in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    torch.cuda.synchronize()
+    graphs = []
+    for x in xs:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs = [lin(x) for _ in range(20)]
+        graphs.append((graph, outs))
+    torch.cuda.synchronize()
+    eager = [[], []]
+    for _ in range(20):
+        for x, stream, keep in zip(xs, streams, eager):
+            with torch.cuda.stream(stream):
+                keep.append(lin(x))
+    torch.cuda.synchronize()
+    for (graph, _), stream in zip(graphs, streams):
+        with torch.cuda.stream(stream):
+            graph.replay()
+    torch.cuda.synchronize()
+    for w, a, (_, b) in zip(want, eager, graphs):
+        assert all(torch.equal(y, w) for y in a + b)
+    _lib.assert_device_ok()
+
+
 # the entry points that take an accumulator instead of parts: same bits, accumulator and counters left zero
 @pytest.mark.parametrize("M,K,N,splits", [(5, 512, 1024, 0), (40, 1024, 384, 4), (130, 384, 256, 3), (7, 256, 256, 1)])
 @pytest.mark.parametrize("wa", [False, True])
