@@ -116,7 +116,6 @@ class PagedKVCacheInt4(PagedCache):
         self.v_pages = [mk(n_pages, page_size, heads, head_dim // 2, dt=torch.uint8) for _ in range(num_layers)]
         self.k_scales = [mk(n_pages, page_size, heads, G, dt=torch.float32) for _ in range(num_layers)]
         self.v_scales = [mk(n_pages, page_size, heads, G, dt=torch.float32) for _ in range(num_layers)]
-        self._scratch = None
 
     def nbytes(self) -> int:
         return sum(t.numel() * t.element_size() for ts in (self.k_pages, self.v_pages, self.k_scales, self.v_scales) for t in ts)
@@ -199,12 +198,11 @@ class PagedKVCacheInt4(PagedCache):
                 splits = max(1, min(32, 296 // max(1, B * self.heads), (longest + 255) // 256))
             L = _lib.lib()
             need = L.cgk_kv_int4_attention_scratch_floats(B, Hq, Tq, D, splits)
-            if self._scratch is None or self._scratch.numel() < need:
-                self._scratch = torch.empty(need, dtype=torch.float32, device=q.device)
+            scratch = torch.empty(need, dtype=torch.float32, device=q.device)    # of this call: a captured one keeps its address
             out = torch.empty_like(q)
             a = self._args(layer)
             _lib.check(L.cgk_kv_int4_attention(ctypes.byref(a), q.data_ptr(), out.data_ptr(), Tq, Hq, scale, splits,
-                                               self._scratch.data_ptr(), _lib.stream_ptr()), "cgk_kv_int4_attention")
+                                               scratch.data_ptr(), _lib.stream_ptr()), "cgk_kv_int4_attention")
             _lib.count_launch(2)
             return out
         out = torch.empty(B, Tq, Hq, D, dtype=q.dtype)

@@ -372,3 +372,46 @@ def test_engine_and_speculative_decoding_on_gpu():
     seqs, stats = sd.generate(prompts.to(DEV), 10)
     assert stats.acceptance_rate > 0.8 and all(len(s) >= 19 for s in seqs)   # < 1 only through bf16 near-ties
     _lib.assert_device_ok()
+
+
+# the decoding step is captured after the first prompts; prompts of other lengths then run other kernels and larger ones
+def test_speculative_decoding_over_prompts_of_other_lengths():
+    rng.manual_seed(1)
+    cfg = LlamaConfig(vocab_size=1024, n_layer=2, d_model=512, n_head=8, n_kv_head=4, d_ff=1024, max_seq_len=256)
+    target, draft = Llama(cfg).to(DEV).bfloat16(), Llama(cfg).to(DEV).bfloat16()
+    B = 4
+    decoder = lambda: SpeculativeDecoder(LlamaInt4Engine(draft, B, 160), LlamaInt4Engine(target, B, 160), gamma=4, temperature=0.0)
+    sd = decoder()
+    for length in (100, 10, 40, 15, 100):                     # 396 rows through the dense product, 36 and 156 rows, 14 tokens over the cache
+        prompts = torch.randint(0, 1024, (B, length), device=DEV)
+        got, _ = sd.generate(prompts, 12)
+        assert sd._graph is not None
+        fresh = decoder()
+        want, _ = fresh.generate(prompts, 12)
+        fresh.close()
+        assert got == want
+    sd.close()
+    _lib.assert_device_ok()
+
+
+# a captured attention call keeps its scratch although a later call needs more
+def test_kv_attention_captured_before_a_larger_call():
+    torch.manual_seed(5)
+    B, Hk, Hq, D = 2, 2, 8, 128
+    cache = PagedKVCacheInt4(1, B, 512, Hk, D, 32, page_size=64, device=DEV)
+    cache.append(0, *(torch.randn(B, 420, Hk, D, device=DEV).bfloat16() for _ in range(2)))
+    cache.commit(400)
+    q, more = torch.randn(B, 1, Hq, D, device=DEV).bfloat16(), torch.randn(B, 20, Hq, D, device=DEV).bfloat16()
+    want = cache.attention(0, q)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = cache.attention(0, q)
+    cache.attention(0, more)
+    junk = [torch.full((n,), 1e30, device=DEV) for n in (1 << 8, 1 << 12, 1 << 14, 1 << 16, 1 << 18) for _ in range(4)]
+    for _ in range(2):
+        got.zero_()
+        graph.replay()
+        assert torch.equal(got, want)
+    assert all((j == 1e30).all() for j in junk)
+    _lib.assert_device_ok()
