@@ -49,11 +49,17 @@ def norm_forward_raw(x2, gamma, beta, eps, rms, residual2=None, want_sum=False):
 
 
 def add_rms_norm_(x, y, gamma, eps: float):
-    """x += y in place (bf16), and the RMSNorm of the sum, by one kernel on CUDA; x contiguous, not under autograd."""
-    if not (x.is_cuda and x.dtype == y.dtype == gamma.dtype == _BF16 and x.is_contiguous() and y.is_contiguous()):
-        x += y.view_as(x)
-        return rms_norm(x, gamma, eps)
+    """x += y in place (bf16), and the RMSNorm of the sum: by one kernel on CUDA for contiguous operands on 16-byte boundaries that
+    autograd does not follow.  y has x's elements in any shape."""
     D = x.shape[-1]
+    if tuple(gamma.shape) != (D,):
+        raise ValueError(f"add_rms_norm_: gamma has shape {tuple(gamma.shape)}, rows have {D} elements")
+    y = y.view_as(x)                                       # raises for another number of elements
+    ts = (x, y, gamma)
+    if not (all(t.is_cuda and t.device == x.device and t.dtype == _BF16 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in ts)
+            and not (torch.is_grad_enabled() and any(t.requires_grad for t in ts))):
+        x += y
+        return rms_norm(x, gamma, eps)
     out = torch.empty_like(x)
     _lib.check(_lib.lib().cgk_norm_forward(x.data_ptr(), y.data_ptr(), gamma.data_ptr(), None, out.data_ptr(), x.data_ptr(), None, None,
                                            x.numel() // D, D, float(eps), 1, _lib.stream_ptr()), "cgk_norm_forward")

@@ -74,6 +74,29 @@ def test_wide_norm_has_the_same_bits_for_few_rows_and_for_many(D, rms, with_res)
             assert (u is None) == (v is None) and (u is None or torch.equal(u, v[part]))
 
 
+def test_add_rms_norm_refuses_other_shapes_and_takes_any_alignment():
+    from cogito_b200.ops import norm as N
+    torch.manual_seed(3)
+    for dev in ("cpu", DEV):
+        x, y, g = (torch.randn(*s, device=dev).bfloat16() for s in ((3, 2, 64), (6, 64), (64,)))
+        before = x.clone()
+        for bad_y, bad_g in ((y[:5], g), (torch.cat([y, y]), g), (y, g[:56]), (y, torch.cat([g, g]))):
+            with pytest.raises((ValueError, RuntimeError)):
+                N.add_rms_norm_(x, bad_y, bad_g, 1e-5)
+            assert torch.equal(x, before)
+        want_x = before + y.view_as(x)
+        want = N.rms_norm(want_x, g, 1e-5)
+        shifted = torch.cat([y.new_zeros(4), y.reshape(-1)])[4:].view(6, 64)           # contiguous, 8 bytes off a 16-byte boundary
+        wide = torch.cat([y, y], 1)[:, :64].reshape(3, 2, 64).transpose(0, 1).contiguous().transpose(0, 1)     # not contiguous
+        for form in (y, shifted, wide):
+            u = before.clone()
+            assert torch.equal(N.add_rms_norm_(u, form, g, 1e-5), want) and torch.equal(u, want_x)
+        gp = g.clone().requires_grad_()
+        u = before.clone()
+        N.add_rms_norm_(u, y, gp, 1e-5).float().sum().backward()                       # a weight that autograd follows has its gradient
+        assert gp.grad is not None and gp.grad.float().abs().sum() > 0
+
+
 @pytest.mark.parametrize("rows,D", [(64, 768), (33, 128), (1000, 4096), (7, 8)])
 @pytest.mark.parametrize("rms", [False, True])
 @pytest.mark.parametrize("with_res", [False, True])
