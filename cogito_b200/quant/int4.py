@@ -116,7 +116,9 @@ class Int4Linear(torch.nn.Module):
     # memory, 128 token rows per instruction), "wa" makes them the A operand fed from tensor memory (cost
     # follows the token count; needs group % 128 == 0).  "auto": "wa" up to 16 token rows, "wb" up to two row
     # tiles, and beyond that (prompts) the weights are dequantised to bf16 once per call for the dense GEMM: "wb" converts
-    # every weight tile again for each row tile.  Each of the two kernels has its own tile-major copy of the weights, made on
+    # every weight tile again for each row tile.  That copy (2 bytes per weight: 180 MB for 4096 x 22016, 262 MB for
+    # 4096 x 32000) comes from the allocator for the time of the call, one layer's at a time; where there is no room for it,
+    # "wb" takes the call.  Each of the two kernels has its own tile-major copy of the weights, made on
     # first use; both sum the parts of a shared tile in a fixed order, so a call gives the same bits every time.
     # Times (us, layers one after the other) for 4096 x 6144, 4096 x 4096, 4096 x 22016, 11008 x 4096, 4096 x 32000, 2048 x 11264:
     #   16 rows   "wa" 20.1 14.9 34.7 24.7 44.6 19.2
@@ -192,9 +194,12 @@ class Int4Linear(torch.nn.Module):
     def forward_f32(self, x: torch.Tensor) -> torch.Tensor:
         """fp32 result (logits); many rows leave the GEMM in fp32 without a bf16 copy in between."""
         rows = x.numel() // self.in_features
-        if not x.is_cuda or not self._takes_dense(rows):
-            return self.forward(x).float()
-        return self._dense(x.reshape(rows, self.in_features), out_dtype=torch.float32).view(*x.shape[:-1], self.out_features)
+        if x.is_cuda and self._takes_dense(rows):
+            try:
+                return self._dense(x.reshape(rows, self.in_features), out_dtype=torch.float32).view(*x.shape[:-1], self.out_features)
+            except torch.OutOfMemoryError:
+                pass                                       # no room for the weights in bf16: by the streaming kernel
+        return self.forward(x).float()
 
     def forward(self, x: torch.Tensor, splits: int = 0, out: torch.Tensor | None = None) -> torch.Tensor:
         """``out``: an optional contiguous [rows, out_features] buffer for the result (bf16 on CUDA),
@@ -219,11 +224,12 @@ class Int4Linear(torch.nn.Module):
             # shapes the streaming kernel does not cover: dequantise once, then the bf16 GEMM
             return done(self._dense(x2))
         if self._takes_dense(M, splits):
-            if out is None:
-                return self._dense(x2).view(*lead, N)
-            if out.dtype != torch.bfloat16 or not out.is_contiguous() or out.numel() != M * N:
+            if out is not None and (out.dtype != torch.bfloat16 or not out.is_contiguous() or out.numel() != M * N):
                 raise ValueError("out must be a contiguous bf16 [rows, out_features] tensor")
-            return self._dense(x2, out=out.view(M, N)).view(*lead, N)
+            try:
+                return self._dense(x2, out=None if out is None else out.view(M, N)).view(*lead, N)
+            except torch.OutOfMemoryError:
+                pass                                       # no room for the weights in bf16: by the streaming kernel
         x2 = x2.to(torch.bfloat16).contiguous()
         L = _lib.lib()
         # "wa": weights on the M side of the tensor core (needs one scale per k for a 128-feature tile)

@@ -78,6 +78,25 @@ def test_int4_gemm_repeats_itself_to_the_bit(M, K, N, kernel):
     _lib.assert_device_ok()
 
 
+# without room for the weights in bf16 a prompt goes through the streaming kernel, as it did before there was a dense route
+def test_int4_linear_many_rows_without_room_for_the_dense_weights(monkeypatch):
+    torch.manual_seed(9)
+    lin = Int4Linear(torch.randn(384, 256) * 0.05, torch.randn(384) * 0.1, 128).to(DEV)
+    x = torch.randn(300, 256, device=DEV, dtype=torch.bfloat16)
+
+    def no_room(self, dtype=torch.float32):
+        raise torch.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(Int4Linear, "dequantized", no_room)
+    out = torch.empty(300, 384, device=DEV, dtype=torch.bfloat16)
+    lin.kernel = "wb"
+    want = lin(x)
+    lin.kernel = "auto"
+    assert torch.equal(lin(x), want) and torch.equal(lin(x, out=out), want) and torch.equal(out, want)
+    assert torch.equal(lin.forward_f32(x), want.float())
+    _lib.assert_device_ok()
+
+
 def _int4_layer(K=1024, N=2304):
     g = torch.Generator().manual_seed(K + N)
     packed = torch.randint(0, 256, (K * N // 2,), dtype=torch.uint8, generator=g)
