@@ -201,9 +201,13 @@ class Int4Linear(torch.nn.Module):
                 pass                                       # no room for the weights in bf16: by the streaming kernel
         return self.forward(x).float()
 
-    def forward(self, x: torch.Tensor, splits: int = 0, out: torch.Tensor | None = None) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, splits: int = 0, out: torch.Tensor | None = None, f32: bool = False) -> torch.Tensor:
         """``out``: an optional contiguous [rows, out_features] buffer for the result (bf16 on CUDA),
-        e.g. a slot of symmetric memory that a collective kernel reads next."""
+        e.g. a slot of symmetric memory that a collective kernel reads next.  ``f32``: the result of ``forward_f32``."""
+        if f32:
+            if out is not None or splits:
+                raise ValueError("an fp32 result takes neither out nor splits")
+            return self.forward_f32(x)
         lead = x.shape[:-1]
         x2 = x.reshape(-1, self.in_features)
         M = x2.shape[0]

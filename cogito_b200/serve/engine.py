@@ -214,7 +214,7 @@ class LlamaInt4Engine:
             h = self._proj_add_norm(l["proj"], o.reshape(B, Tq, Hq * D), x, l["norm2"])
             nxt = self.layers[i + 1]["norm1"] if i + 1 < len(self.layers) else self.norm_f
             h = self._proj_add_norm(l["down"], M.swiglu(l["gate_up"](h)), x, nxt)
-        logits = self.lm_head(h) if self.tp > 1 else self.lm_head.forward_f32(h)
+        logits = self.lm_head(h) if self.tp > 1 else self.lm_head(h, f32=True)
         if self.tp > 1:
             parts = [torch.empty_like(logits) for _ in range(self.tp)]
             dist.all_gather(parts, logits.contiguous(), group=self.tp_group)

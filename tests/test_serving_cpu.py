@@ -134,3 +134,13 @@ def test_engine_round_trips_through_a_quantised_checkpoint(tmp_path):
     assert torch.equal(eng.forward(ids, commit=True), back.forward(ids, commit=True))
     nxt = torch.randint(0, 256, (2, 1))
     assert torch.equal(eng.forward(nxt), back.forward(nxt))
+
+
+def test_the_engine_calls_its_vocabulary_projection_as_a_module():
+    torch.manual_seed(0)
+    cfg = LlamaConfig(vocab_size=256, n_layer=1, d_model=128, n_head=2, n_kv_head=1, d_ff=128, max_seq_len=32)
+    engine = LlamaInt4Engine(Llama(cfg), 2, 32)
+    seen = []
+    engine.lm_head.register_forward_hook(lambda module, args, out: seen.append(out))
+    logits = engine.forward(torch.randint(0, 256, (2, 5)))
+    assert len(seen) == 1 and torch.equal(seen[0].float(), logits)
