@@ -529,10 +529,17 @@ norm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
     }
   }
   if (in) {
-    float4* og = reinterpret_cast<float4*>(partial + (size_t)blockIdx.x * 2 * D + c * 8);
-    float4* ob = reinterpret_cast<float4*>(partial + (size_t)blockIdx.x * 2 * D + D + c * 8);
-    og[0] = make_float4(accg[0], accg[1], accg[2], accg[3]); og[1] = make_float4(accg[4], accg[5], accg[6], accg[7]);
-    ob[0] = make_float4(accb[0], accb[1], accb[2], accb[3]); ob[1] = make_float4(accb[4], accb[5], accb[6], accb[7]);
+    float* pg = partial + (size_t)blockIdx.x * 2 * D + c * 8;
+    float* pb = pg + D;
+    if ((reinterpret_cast<uintptr_t>(partial) & 15) == 0) {
+      float4* og = reinterpret_cast<float4*>(pg);
+      float4* ob = reinterpret_cast<float4*>(pb);
+      og[0] = make_float4(accg[0], accg[1], accg[2], accg[3]); og[1] = make_float4(accg[4], accg[5], accg[6], accg[7]);
+      ob[0] = make_float4(accb[0], accb[1], accb[2], accb[3]); ob[1] = make_float4(accb[4], accb[5], accb[6], accb[7]);
+    } else {                                                // scratch on any boundary, as for narrower rows
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { pg[j] = accg[j]; pb[j] = accb[j]; }
+    }
   }
 }
 

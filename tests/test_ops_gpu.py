@@ -74,6 +74,22 @@ def test_wide_norm_has_the_same_bits_for_few_rows_and_for_many(D, rms, with_res)
             assert (u is None) == (v is None) and (u is None or torch.equal(u, v[part]))
 
 
+@pytest.mark.parametrize("D", [768, 1608, 4096])
+def test_norm_backward_takes_scratch_on_any_boundary(D):
+    from cogito_b200.ops import _lib
+    L, rows = _lib.lib(), 70
+    torch.manual_seed(D)
+    x, dy = (torch.randn(rows, D, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    g, mean, rstd = torch.ones(D, device=DEV, dtype=torch.bfloat16), torch.zeros(rows, device=DEV), torch.ones(rows, device=DEV)
+    n, results = L.cgk_norm_backward_scratch_elems(rows, D), []
+    for shift in (0, 1, 2, 3):
+        scratch, dx, dg, db = torch.empty(n + 4, device=DEV), torch.empty_like(x), torch.empty(D, device=DEV), torch.empty(D, device=DEV)
+        _lib.check(L.cgk_norm_backward(dy.data_ptr(), x.data_ptr(), g.data_ptr(), mean.data_ptr(), rstd.data_ptr(), None, dx.data_ptr(), dg.data_ptr(),
+                                       db.data_ptr(), scratch[shift:].data_ptr(), rows, D, 0, 0, _lib.stream_ptr()))
+        results.append((dx, dg, db))
+    assert all(torch.equal(a, b) for r in results[1:] for a, b in zip(r, results[0]))
+
+
 def test_add_rms_norm_refuses_other_shapes_and_takes_any_alignment():
     from cogito_b200.ops import norm as N
     torch.manual_seed(3)
