@@ -107,6 +107,30 @@ def test_gemm_split_k_weight_gradient(Mw, Nw, K, split):
     assert relerr(one, ref) < 2e-3
 
 
+# the sliced weight gradient by CTA pairs (more than six row tiles, a long reduction): an odd number of row tiles, a pair whose
+# second CTA has a few rows or none, slices of unequal length, a reduction that ends inside a block
+@pytest.mark.parametrize("Mw,Nw,K,split", [(3072, 768, 8192, 0), (904, 768, 16384, 0), (800, 256, 8192 + 40, 0), (1152, 768, 5000, 3), (2304, 2304, 3072, 5)])
+def test_gemm_split_k_weight_gradient_by_cta_pairs(Mw, Nw, K, split):
+    test_gemm_split_k_weight_gradient(Mw, Nw, K, split)
+
+
+# the rotary epilogue by CTA pairs: rows of the second CTA at their own positions, sequences that end inside a tile
+@pytest.mark.parametrize("D,heads_rot,heads_all,B,T", [(128, 5, 6, 5, 200), (64, 6, 9, 3, 683), (64, 12, 12, 1, 2049)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_gemm_rotary_epilogue_by_cta_pairs(D, heads_rot, heads_all, B, T, inverse):
+    from cogito_b200.ops.gemm import gemm, gemm_reference
+    from cogito_b200.ops.misc import rope_tables
+    torch.manual_seed(4)
+    M, K, N = B * T, 3080, heads_all * D
+    a = torch.randn(M, K, device=DEV, dtype=torch.bfloat16)
+    w = torch.randn(N, K, device=DEV, dtype=torch.bfloat16) * 0.02
+    bias = torch.randn(N, device=DEV, dtype=torch.bfloat16)
+    spec = (*rope_tables(T + 7, D, 10000.0, DEV), heads_rot * D, D, T, 5, inverse)
+    out = gemm(a, w, bias=bias, rope=spec)
+    assert relerr(out, gemm_reference(a, w, bias=bias, rope=spec, out_dtype=torch.float32)) < 1e-2
+    assert torch.equal(out[:, heads_rot * D:], gemm(a, w, bias=bias)[:, heads_rot * D:])
+
+
 @pytest.mark.parametrize("D,heads_rot,heads_all,T", [(64, 6, 9, 128), (128, 5, 6, 96), (64, 3, 3, 64), (128, 2, 3, 50)])
 @pytest.mark.parametrize("inverse", [False, True])
 def test_gemm_rotary_epilogue(D, heads_rot, heads_all, T, inverse):

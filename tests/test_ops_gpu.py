@@ -28,6 +28,28 @@ def test_rope_by_eight_pairs(B, T, H, D, backward):
         assert relerr(got, ref) < 2 ** -8 and torch.equal(got[:, :, 0].cpu(), packed[:, :, 0].cpu()) and torch.equal(got[:, :, -1].cpu(), packed[:, :, -1].cpu())
 
 
+# the vectorised bf16 kernels divide without a branch: every bf16 gate (infinities, NaN, zeros of both signs, denormals) rounds to what
+# the fp32 kernels' division rounds to
+@pytest.mark.parametrize("draw", range(3))
+def test_swiglu_over_all_bf16_gates_has_the_bits_of_the_division(draw):
+    from cogito_b200.ops import _lib
+    L, H = _lib.lib(), 65536
+    g = torch.arange(H, device=DEV, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    torch.manual_seed(draw)
+    one = torch.ones(H, device=DEV, dtype=torch.bfloat16)
+    up, dy = (one, one) if draw == 0 else (torch.randn(H, device=DEV).bfloat16() for _ in range(2))
+    x = torch.cat([g, up])[None].contiguous()
+    got, dgot = torch.empty(1, H, device=DEV, dtype=torch.bfloat16), torch.empty(1, 2 * H, device=DEV, dtype=torch.bfloat16)
+    ref, dref, xf, dyf = torch.empty(1, H, device=DEV), torch.empty(1, 2 * H, device=DEV), x.float(), dy.float()
+    _lib.check(L.cgk_swiglu_forward(1, x.data_ptr(), got.data_ptr(), 1, H, _lib.stream_ptr()))
+    _lib.check(L.cgk_swiglu_forward(0, xf.data_ptr(), ref.data_ptr(), 1, H, _lib.stream_ptr()))
+    _lib.check(L.cgk_swiglu_backward(1, x.data_ptr(), dy.data_ptr(), dgot.data_ptr(), 1, H, _lib.stream_ptr()))
+    _lib.check(L.cgk_swiglu_backward(0, xf.data_ptr(), dyf.data_ptr(), dref.data_ptr(), 1, H, _lib.stream_ptr()))
+    for a, b in ((got, ref.bfloat16()), (dgot, dref.bfloat16())):
+        assert torch.equal(a.isnan(), b.isnan())
+        assert torch.equal(a.view(torch.int16)[~a.isnan()], b.view(torch.int16)[~b.isnan()])
+
+
 # rows of more than 1024 elements take a CTA each: the smallest and largest, a width that fills no whole warp, more rows than CTAs
 @pytest.mark.parametrize("rows,D", [(1, 1032), (5, 8192), (700, 1608), (1300, 2048)])
 @pytest.mark.parametrize("rms", [False, True])
