@@ -6,6 +6,7 @@ package goes through :func:`lib`.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from ctypes import POINTER, Structure, c_char_p, c_float, c_int, c_int32, c_int64, c_longlong, c_void_p, c_ulonglong
@@ -96,7 +97,6 @@ def _declare(L: ctypes.CDLL) -> None:
         "cgk_int4_quantize": [vp, ll, i, vp, vp, vp],
         "cgk_int4_dequantize": [vp, vp, ll, i, vp, vp, vp],
         "cgk_exchange_capture_mode": [i],
-        "cgk_stream_sync": [vp],
         "cgk_int4_gemm": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
         "cgk_int4_gemm_parts": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
         "cgk_int4_tile_weights": [vp, vp, i, i, i, vp, vp],
@@ -197,25 +197,54 @@ def stream_ptr() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
-def outside_capture(make):
-    """What ``make`` returns, made on a stream that no graph is being captured from and complete for every stream: for
-    workspaces that outlive a call and may first be needed inside a capture."""
-    if not torch.cuda.is_current_stream_capturing():
-        made = make()
-        check(lib().cgk_stream_sync(stream_ptr()), "cgk_stream_sync")
-        return made
-    relaxed = 2                                            # allocations and waits elsewhere do not break the capture
+class Made:
+    """Something that outlives a call (``value``, what ``make`` returns) and is filled by launches.  They run on the current stream,
+    or, if that is being captured, on another one at once, so that a graph neither repeats them nor owns the memory.  ``here``
+    orders the current stream behind them."""
+
+    def __init__(self, make):
+        self.event = None                                  # None: over
+        if not torch.cuda.is_current_stream_capturing():
+            self.value, self.stream, event = make(), stream_ptr(), torch.cuda.Event()
+            event.record()
+            self.event = event
+            return
+        with uncaptured():
+            for _ in range(64):                            # streams come from a pool, in turn
+                with torch.cuda.stream(torch.cuda.Stream()):
+                    if not torch.cuda.is_current_stream_capturing():
+                        self.value = make()
+                        torch.cuda.current_stream().synchronize()
+                        return
+        raise KernelError("every stream of the pool is being captured")
+
+    def here(self):
+        event = self.event
+        if event is not None:
+            with uncaptured():
+                if torch.cuda.is_current_stream_capturing():
+                    event.synchronize()                    # a graph may be replayed anywhere
+                if event.query():
+                    self.event = None
+                elif stream_ptr() != self.stream:
+                    torch.cuda.current_stream().wait_event(event)
+        return self.value
+
+    def __getstate__(self):
+        if self.event is not None:
+            self.event.synchronize()
+        return {"value": self.value, "event": None}
+
+
+@contextlib.contextmanager
+def uncaptured():
+    """Allocations and waits of this thread on other streams do not break a capture that is under way."""
+    relaxed = 2
     mode = lib().cgk_exchange_capture_mode(relaxed)
     try:
-        for _ in range(64):                                # streams come from a pool, in turn
-            with torch.cuda.stream(torch.cuda.Stream()):
-                if not torch.cuda.is_current_stream_capturing():
-                    made = make()
-                    check(lib().cgk_stream_sync(stream_ptr()), "cgk_stream_sync")
-                    return made
+        yield
     finally:
         lib().cgk_exchange_capture_mode(mode)
-    raise KernelError("every stream of the pool is being captured")
 
 
 def ptr(t) -> int | None:

@@ -87,9 +87,9 @@ class _Counters:
 
     def prepare(self, most: int, device):
         """The sets for captures (``most``: counters of the largest launch); the caller holds the lock."""
-        if self.spare is None or self.spare.device != device:
+        if self.spare is None or self.spare.value.device != device:
             self.by_stream, self.by_capture = {}, {}
-            self.spare = _lib.outside_capture(lambda: torch.zeros(self.CAPTURES, most, dtype=torch.int32, device=device))
+            self.spare = _lib.Made(lambda: torch.zeros(self.CAPTURES, most, dtype=torch.int32, device=device))
 
     def get(self, need: int, most: int, device) -> torch.Tensor:
         stream = _lib.stream_ptr()
@@ -105,7 +105,7 @@ class _Counters:
                 if key not in self.by_capture and len(self.by_capture) < self.CAPTURES:
                     self.by_capture[key] = len(self.by_capture)
                 if key in self.by_capture:
-                    return self.spare[self.by_capture[key]]
+                    return self.spare.here()[self.by_capture[key]]
         return torch.zeros(need, dtype=torch.int32, device=device)
 
 
@@ -138,7 +138,7 @@ class Int4Linear(torch.nn.Module):
         self.register_buffer("scales", scales)
         self.register_buffer("bias", None if bias is None else bias.detach().to(torch.bfloat16))
         self._counters = _Counters()
-        self._tiles = {}                      # kernel kind -> tile-major weights
+        self._tiles, self._tiled = {}, {}     # kernel kind -> tile-major weights, and their making until it is known to be over
 
     @classmethod
     def from_packed(cls, packed: torch.Tensor, scales: torch.Tensor, in_features: int, out_features: int, group: int = 128,
@@ -154,7 +154,7 @@ class Int4Linear(torch.nn.Module):
         self.register_buffer("scales", scales.to(torch.float32).contiguous())
         self.register_buffer("bias", None if bias is None else bias.detach().to(torch.bfloat16))
         self._counters = _Counters()
-        self._tiles = {}
+        self._tiles, self._tiled = {}, {}
         return self
 
     @classmethod
@@ -181,7 +181,8 @@ class Int4Linear(torch.nn.Module):
         with self._counters.lock:
             self._counters.prepare(L.cgk_int4_gemm_counters(self.DENSE_ROWS, N), device)
             if self._tiles.get(wa) is None or self._tiles[wa].device != device:
-                self._tiles[wa] = _lib.outside_capture(make)
+                made = _lib.Made(make)
+                self._tiled[wa], self._tiles[wa] = made, made.value
             return self._tiles[wa]
 
     def _takes_dense(self, rows: int, splits: int = 0) -> bool:
@@ -241,6 +242,11 @@ class Int4Linear(torch.nn.Module):
         tiles = self._tiles.get(wa)
         if tiles is None or tiles.device != x2.device:
             tiles = self._tile(wa, x2.device)
+        made = self._tiled.get(wa)
+        if made is not None:
+            made.here()
+            if made.event is None:
+                self._tiled.pop(wa, None)
         # for the output tiles that several CTAs share: a place for their parts (of this call alone), and counters
         parts = torch.empty((L.cgk_int4_wa_gemm_parts_floats if wa else L.cgk_int4_gemm_parts_floats)(M, N, K, splits), dtype=torch.float32, device=x2.device)
         counters = self._counters.get(L.cgk_int4_gemm_counters(M, N), L.cgk_int4_gemm_counters(self.DENSE_ROWS, N), x2.device)

@@ -163,8 +163,3 @@ CGK_API int cgk_exchange_capture_mode(int mode) {
   CGK_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&m));
   return (int)m;
 }
-
-CGK_API int cgk_stream_sync(void* stream) {
-  CGK_CUDA_CHECK(cudaStreamSynchronize((cudaStream_t)stream));
-  return 0;
-}

@@ -1,4 +1,6 @@
 """Serving kernels on the GPU against their host restatements (fp32 PyTorch / the C library)."""
+import copy
+
 import pytest
 import torch
 
@@ -148,6 +150,32 @@ def test_int4_launches_captured_more_often_than_there_are_counters():
             graph.replay()
             assert torch.equal(got, want)
     assert len(lin._counters.by_capture) == lin._counters.CAPTURES
+
+
+# a layer's first call on one stream and the next on another, while the first stream is still busy
+@pytest.mark.parametrize("captured", [False, True])
+def test_int4_layer_first_used_on_a_busy_stream(captured):
+    x = torch.randn(16, 1024, device=DEV, dtype=torch.bfloat16)
+    want, lin, busy = _int4_layer()(x), _int4_layer(), torch.cuda.Stream()
+    a = torch.randn(4096, 4096, device=DEV)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(busy):
+        for _ in range(20):
+            a = a @ a * 1e-2
+        first = lin(x)
+    if captured:
+        graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            graph.capture_begin(capture_error_mode="thread_local")
+            second = lin(x)
+            graph.capture_end()
+            graph.replay()
+        side.synchronize()
+    else:
+        second = lin(x)
+    torch.cuda.synchronize()
+    assert torch.equal(first, want) and torch.equal(second, want)
+    assert torch.equal(copy.deepcopy(lin)(x), want) and torch.equal(lin(x), want)
 
 
 # calls of one layer on two streams, eager and captured, run at the same time
