@@ -355,8 +355,8 @@ constexpr int SAMPLE_SHORT_K = 512;
 // keys.  80 rows of 32 000 fp32 logits, top-k 50,
 // top-p 0.9: 55.3 us with 32 counting rounds of three barriers, serial sums and the zeros written last; 26.6 us like this.
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-sample_kernel(const void* __restrict__ logits, int logits_bf16, long long ld, int V, float temperature, int top_k, float top_p,
-              unsigned long long seed, const long long* __restrict__ step, int* __restrict__ tokens, float* __restrict__ probs_out) {
+sample_kernel(const void* logits, int logits_bf16, long long ld, int V, float temperature, int top_k, float top_p,
+              unsigned long long seed, const long long* __restrict__ step, int* __restrict__ tokens, float* probs_out, int in_place) {
   extern __shared__ uint32_t s_keys[];
   __shared__ uint32_t s_count, s_cnt[2][32];
   __shared__ float s_red[32], s_mass;
@@ -379,14 +379,16 @@ sample_kernel(const void* __restrict__ logits, int logits_bf16, long long ld, in
     for (int i = SAMPLE_IN_REGS + tid; i < V; i += SAMPLE_THREADS) s_keys[i - SAMPLE_IN_REGS] = float_key(load(i));
   }
   if (tid == 0) s_count = 0;
-  // the zeros of the distribution leave while the selection runs; the kept probabilities are written over them at the end
-  if (probs_out) {
+  // the zeros of the distribution leave while the selection runs (if they do not cover logits that it still reads); the kept
+  // probabilities are written over them at the end
+  auto zeros = [&]() {
     float* out = probs_out + (long long)row * V;
     if ((V & 3) == 0 && (reinterpret_cast<uintptr_t>(probs_out) & 15) == 0)
       for (int i = tid; i < V / 4; i += SAMPLE_THREADS) reinterpret_cast<float4*>(out)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     else
       for (int i = tid; i < V; i += SAMPLE_THREADS) out[i] = 0.0f;
-  }
+  };
+  if (probs_out && !in_place) zeros();
   auto each = [&](auto f) {                                  // a thread's own keys
     if (kept) {
 #pragma unroll
@@ -462,6 +464,7 @@ sample_kernel(const void* __restrict__ logits, int logits_bf16, long long ld, in
   float e = tid < n ? __expf(cand_v[tid] - mx) : 0.0f;
   const float total = block_sum(e);
   if (tid < n) cand_v[tid] = e / total;
+  if (probs_out && in_place) zeros();
   __syncthreads();
   if (tid == 0) {
     // sums in the order of the candidates, eight values fetched ahead of the chain of additions
@@ -690,7 +693,9 @@ CGK_API int cgk_sample(const void* logits, int logits_bf16, long long ld, int ro
   // keys beyond those in registers: 4 bytes each, for rows that are kept at all
   const int smem = V > SAMPLE_IN_REGS && V <= SAMPLE_IN_REGS + SAMPLE_IN_SMEM ? (V - SAMPLE_IN_REGS) * 4 : 0;
   if (smem > 32 * 1024) CGK_CUDA_CHECK(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_IN_SMEM * 4));
-  sample_kernel<<<rows, SAMPLE_THREADS, smem, (cudaStream_t)stream>>>(logits, logits_bf16, ld, V, temperature, top_k, top_p, seed, step, tokens, probs_out);
+  const char* from = (const char*)logits, * to = from + ((long long)(rows - 1) * ld + V) * (logits_bf16 ? 2 : 4), * probs = (const char*)probs_out;
+  const int in_place = probs && probs < to && from < probs + (long long)rows * V * 4;
+  sample_kernel<<<rows, SAMPLE_THREADS, smem, (cudaStream_t)stream>>>(logits, logits_bf16, ld, V, temperature, top_k, top_p, seed, step, tokens, probs_out, in_place);
   CGK_LAUNCH_CHECK();
   return 0;
 }

@@ -261,7 +261,8 @@ long long cgk_kv_int4_attention_scratch_floats(int batch, int Hq, int Tq, int D,
 int cgk_kv_int4_attention(const cgk_kv_args* a, const void* q, void* out, int Tq, int Hq, float scale,
                           int splits, float* scratch, void* stream);
 /* Per row: logits / temperature -> top_k (1..1024, 0 = 1024) -> top_p -> sample.  temperature
- * <= 0: argmax.  Random stream = (seed, row, *step).  probs_out: fp32 [rows, V] or null. */
+ * <= 0: argmax.  Random stream = (seed, row, *step).  probs_out: fp32 [rows, V] or null; it may
+ * be the logits (fp32, ld = V). */
 int cgk_sample(const void* logits, int logits_bf16, long long ld, int rows, int V, float temperature, int top_k,
                float top_p, unsigned long long seed, const long long* step, int* tokens, float* probs_out,
                void* stream);

@@ -364,6 +364,19 @@ def test_sampling_selection_at_its_edges(V, k):
             assert (probs.cpu().gather(1, tok.cpu().long()[:, None]) > 0).all()
 
 
+# the distribution may take the place of its logits: rows kept in registers, in shared memory too, and read again
+@pytest.mark.parametrize("V", [1000, 32000, 50257, 90000])
+@pytest.mark.parametrize("k", [50, 0])
+def test_sampling_in_place(V, k):
+    torch.manual_seed(V + k)
+    x = torch.randn(5, V, device=DEV) * 3
+    step = torch.tensor([2], device=DEV)
+    want_tok, want = sample(x, 0.8, k, 0.9, seed=3, step=step, return_probs=True)
+    tok = torch.empty(5, dtype=torch.int32, device=DEV)
+    _lib.check(_lib.lib().cgk_sample(x.data_ptr(), 0, V, 5, V, 0.8, k, 0.9, 3, step.data_ptr(), tok.data_ptr(), x.data_ptr(), _lib.stream_ptr()))
+    assert torch.equal(tok, want_tok) and torch.equal(x, want)
+
+
 def test_sampling_takes_the_first_of_equal_values():
     x = torch.zeros(1, 1000)
     x[0, [5, 900, 17]] = 1.0
