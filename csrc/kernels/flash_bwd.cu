@@ -196,7 +196,7 @@ CGK_API int cgk_flash_backward(const cgk_flash_args* pa, void* stream) {
   p.status = device_status(dev);
   p.tiles = (a.Tk + 127) / 128;
   // head_dim 64 keeps a head's tiles together (64 x 12 heads of 2048: 2.29 ms, 2.36 in groups): its tiles are shorter, and the
-  // key tiles of a head then add to dQ in the same staggered order from run to run
+  // key tiles of a head mostly add to dQ in the same staggered order from run to run (the adds are asynchronous: nothing fixes it)
   p.chunk = a.D == 64 ? 1 : attention_chunk(p.tiles, a.B * a.Hk, sm_count(dev));
   int rc = (a.D == 64) ? launch_bwd<64>(a, p, st) : launch_bwd<128>(a, p, st);
   if (rc) return rc;

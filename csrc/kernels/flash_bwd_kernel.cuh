@@ -31,7 +31,7 @@ struct BwdCfg {
   static constexpr int PS_BYTES = BM * BN * 2;     // P and dS tiles
   // Q / dO slots: a slot is held from a step's S / dP until its dK / dV.  At head_dim 128 there is room for three tiles: they
   // are a ring of single tiles, Q and dO in turn, so that the next Q arrives a step ahead and the next dO as soon as dK has
-  // read this Q.With
+  // read this Q.  With
   // one slot of both, loads began when a step's last MMA had read it: 32 query on 8 key heads, 4096 tokens: 773 us, 598 now
   // (together with the earlier release of dQ, below).
   static constexpr bool SPLIT = (D == 128);

@@ -343,8 +343,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (p.causal) need_mask |= (k0 + C::BN - 1 > tile_q_lo);
       if (p.window >= 0) need_mask |= (k0 < tile_q_hi - p.window) || (!p.causal && k0 + C::BN - 1 > tile_q_lo + p.window);
       if (p.block > 0) need_mask |= k0 < tile_q_hi / p.block * p.block;
-      // Interior tiles (no mask, no bias) use the raw products; the others are first rewritten in
-      // TMEM as final log2-domain scores (-inf where masked), after which the multiplier is 1.
+      // Interior tiles use the raw products (with biases, added in registers below, scaled there);
+      // tiles on a mask edge are first rewritten in TMEM as final log2-domain scores (biases
+      // included, -inf where masked).  The multiplier of the row loop is then 1.
       const bool fast = !need_mask && p.scale_log2 > 0.0f;
       if (!fast) {
         // Row-wise visible key range [klo, khi] (empty when khi < klo).  The ALiBi bias of
