@@ -576,12 +576,17 @@ norm_bwd_reduce_kernel(const float* __restrict__ partial, int nparts, int D,
 using namespace cgk;
 
 static int wide_threads(int D) { return (D / 8 + 31) / 32 * 32; }
-// CTAs of the wide backward kernel: 64 registers a thread, up to four of them per SM
+// CTAs of the wide backward kernel: 64 registers a thread, up to four of them per SM, with NORM_WIDE_RUN rows or more each
+// once half the SMs have one: a CTA's partial sums are 2 D floats that the second kernel reads.  Rows of 2048, both kernels, a row per
+// CTA / four: 4 rows 5.9 / 6.6 us, 80 rows 6.7 / 6.6, 300 rows 10.1 / 7.3, 592 rows 13.9 / 8.3, 1200 rows 13.9 / 11.0.
+constexpr int NORM_WIDE_RUN = 4;
 static int norm_bwd_wide_grid(int dev, int rows, int D) {
   int per_sm = 1024 / wide_threads(D);
   if (per_sm > 4) per_sm = 4;
-  const int cap = sm_count(dev) * per_sm;
-  return rows < cap ? rows : cap;
+  const int sms = sm_count(dev), cap = sms * per_sm, few = rows < sms / 2 ? rows : sms / 2;
+  int ctas = (rows + NORM_WIDE_RUN - 1) / NORM_WIDE_RUN;
+  if (ctas < few) ctas = few;
+  return ctas < cap ? ctas : cap;
 }
 
 // CTAs of the backward kernel: as many as fit an SM by shared memory (each holds 2 * D floats per
