@@ -405,7 +405,9 @@ __global__ void swiglu_bwd_kernel(const T* __restrict__ x, const T* __restrict__
 // The backward pass over bf16 rows in 16-byte pieces, two rows at a time per CTA: six loads in flight per thread, laid out like
 // the forward kernel.  One element per thread and a 64-bit division per element took 2.9 times the traffic's time:
 // 4096 rows of 2 x 11008 203 us, 78 like this (5.8 TB/s).
-constexpr int SWIGLU_BWD_ROWS = 2;
+// Narrow rows and small products stay with that kernel (it / this, us): 65536 x 8 4.7 / 21.1, x 64 17.0 / 21.2, x 128 32.1 / 21.9;
+// 7 x 2816 1.8 / 2.2, 80 x 1408 (113 K elements) 2.1 / 2.2, 512 x 256 (131 K) 2.3 / 2.0.
+constexpr int SWIGLU_BWD_ROWS = 2, SWIGLU_BWD_WIDTH = 128, SWIGLU_BWD_ELEMS = 128 * 1024;
 __global__ void __launch_bounds__(256)
 swiglu_bwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx, long long rows, int H) {
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
@@ -787,7 +789,7 @@ CGK_API int cgk_swiglu_backward(int dtype, const void* x, const void* dy, void* 
   CGK_REQUIRE(x && dy && dx && H > 0, "cgk_swiglu_backward: bad argument");
   if (rows == 0) return 0;
   if (dtype == 0) swiglu_bwd_kernel<float><<<ew_grid(rows * H), 256, 0, ST(stream)>>>((const float*)x, (const float*)dy, (float*)dx, rows, H);
-  else if (H % 8 == 0 && (((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx) & 15) == 0) {
+  else if (H % 8 == 0 && H >= SWIGLU_BWD_WIDTH && rows * H >= SWIGLU_BWD_ELEMS && (((uintptr_t)x | (uintptr_t)dy | (uintptr_t)dx) & 15) == 0) {
     const dim3 cols = swiglu_rows_grid(rows, H);
     const long long pairs = (rows + SWIGLU_BWD_ROWS - 1) / SWIGLU_BWD_ROWS, cap = 148 * 16 / (cols.y < 16 ? cols.y : 16);
     swiglu_bwd_rows_kernel<<<dim3((unsigned)(pairs < cap ? pairs : cap), cols.y), swiglu_rows_threads(H), 0, ST(stream)>>>(

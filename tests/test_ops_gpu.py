@@ -28,6 +28,19 @@ def test_rope_by_eight_pairs(B, T, H, D, backward):
         assert relerr(got, ref) < 2 ** -8 and torch.equal(got[:, :, 0].cpu(), packed[:, :, 0].cpu()) and torch.equal(got[:, :, -1].cpu(), packed[:, :, -1].cpu())
 
 
+# both sides of the line between the backward kernels: narrow rows and small products, element by element; the others by rows
+@pytest.mark.parametrize("rows,H", [(1, 8), (1100, 120), (1024, 128), (1023, 128), (513, 256), (129, 1016)])
+def test_swiglu_backward_on_both_sides_of_its_line(rows, H):
+    from cogito_b200.ops import _lib
+    L = _lib.lib()
+    torch.manual_seed(H)
+    x, dy = torch.randn(rows, 2 * H, device=DEV).bfloat16(), torch.randn(rows, H, device=DEV).bfloat16()
+    got, ref, xf, dyf = torch.empty_like(x), torch.empty(rows, 2 * H, device=DEV), x.float(), dy.float()
+    _lib.check(L.cgk_swiglu_backward(1, x.data_ptr(), dy.data_ptr(), got.data_ptr(), rows, H, _lib.stream_ptr()))
+    _lib.check(L.cgk_swiglu_backward(0, xf.data_ptr(), dyf.data_ptr(), ref.data_ptr(), rows, H, _lib.stream_ptr()))
+    assert torch.equal(got, ref.bfloat16())
+
+
 # the vectorised bf16 kernels divide without a branch: every bf16 gate (infinities, NaN, zeros of both signs, denormals) rounds to what
 # the fp32 kernels' division rounds to
 @pytest.mark.parametrize("draw", range(3))
@@ -38,13 +51,14 @@ def test_swiglu_over_all_bf16_gates_has_the_bits_of_the_division(draw):
     torch.manual_seed(draw)
     one = torch.ones(H, device=DEV, dtype=torch.bfloat16)
     up, dy = (one, one) if draw == 0 else (torch.randn(H, device=DEV).bfloat16() for _ in range(2))
-    x = torch.cat([g, up])[None].contiguous()
-    got, dgot = torch.empty(1, H, device=DEV, dtype=torch.bfloat16), torch.empty(1, 2 * H, device=DEV, dtype=torch.bfloat16)
-    ref, dref, xf, dyf = torch.empty(1, H, device=DEV), torch.empty(1, 2 * H, device=DEV), x.float(), dy.float()
-    _lib.check(L.cgk_swiglu_forward(1, x.data_ptr(), got.data_ptr(), 1, H, _lib.stream_ptr()))
-    _lib.check(L.cgk_swiglu_forward(0, xf.data_ptr(), ref.data_ptr(), 1, H, _lib.stream_ptr()))
-    _lib.check(L.cgk_swiglu_backward(1, x.data_ptr(), dy.data_ptr(), dgot.data_ptr(), 1, H, _lib.stream_ptr()))
-    _lib.check(L.cgk_swiglu_backward(0, xf.data_ptr(), dyf.data_ptr(), dref.data_ptr(), 1, H, _lib.stream_ptr()))
+    rows = 2                                                  # the backward kernel by rows starts at 128 K elements
+    x, dy = torch.cat([g, up]).repeat(rows, 1), dy.repeat(rows, 1)
+    got, dgot = torch.empty(rows, H, device=DEV, dtype=torch.bfloat16), torch.empty(rows, 2 * H, device=DEV, dtype=torch.bfloat16)
+    ref, dref, xf, dyf = torch.empty(rows, H, device=DEV), torch.empty(rows, 2 * H, device=DEV), x.float(), dy.float()
+    _lib.check(L.cgk_swiglu_forward(1, x.data_ptr(), got.data_ptr(), rows, H, _lib.stream_ptr()))
+    _lib.check(L.cgk_swiglu_forward(0, xf.data_ptr(), ref.data_ptr(), rows, H, _lib.stream_ptr()))
+    _lib.check(L.cgk_swiglu_backward(1, x.data_ptr(), dy.data_ptr(), dgot.data_ptr(), rows, H, _lib.stream_ptr()))
+    _lib.check(L.cgk_swiglu_backward(0, xf.data_ptr(), dyf.data_ptr(), dref.data_ptr(), rows, H, _lib.stream_ptr()))
     for a, b in ((got, ref.bfloat16()), (dgot, dref.bfloat16())):
         assert torch.equal(a.isnan(), b.isnan())
         assert torch.equal(a.view(torch.int16)[~a.isnan()], b.view(torch.int16)[~b.isnan()])
