@@ -277,7 +277,8 @@ CGK_API int cgk_adam_step(float* p, float* m, float* v, const float* g, void* p1
   CGK_REQUIRE(p && m && v && g, "cgk_adam_step: null pointer");
   if (n == 0) return 0;
   AdamHyper h{lr, beta1, beta2, eps, weight_decay, max_grad_norm};
-  const int vec = (((uintptr_t)p | (uintptr_t)m | (uintptr_t)v | (uintptr_t)g) & 15) == 0 && ((uintptr_t)p16 & 7) == 0;
+  // few elements: one per thread is over sooner (1000: 2.0 us, 2.5 by fours; 65 536: 2.4 and 2.6; 100 000: 2.8 and 2.6)
+  const int vec = n >= 80 * 1024 && (((uintptr_t)p | (uintptr_t)m | (uintptr_t)v | (uintptr_t)g) & 15) == 0 && ((uintptr_t)p16 & 7) == 0;
   adam_step_kernel<<<flat_grid(vec ? (n + 3) / 4 : n, 256), 256, 0, (cudaStream_t)stream>>>(
       p, m, v, g, (__nv_bfloat16*)p16, n, vec, h, (const ScalerState*)state);
   CGK_LAUNCH_CHECK();

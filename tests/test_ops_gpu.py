@@ -110,6 +110,25 @@ def test_wide_norm_has_the_same_bits_for_few_rows_and_for_many(D, rms, with_res)
             assert (u is None) == (v is None) and (u is None or torch.equal(u, v[part]))
 
 
+# one element per access below 80 K elements or off a 16-byte boundary, four above
+@pytest.mark.parametrize("n", [1, 1000, 81919, 81920, 81923, 200001])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_adam_step_by_one_and_by_four(n, shift):
+    from cogito_b200.ops import _lib
+    torch.manual_seed(n)
+    p, m, v, g = (torch.rand(n + 4, device=DEV)[shift:shift + n] for _ in range(4))
+    p16 = torch.empty(n + 4, device=DEV, dtype=torch.bfloat16)[shift:shift + n]
+    lr, b1, b2, eps, wd = 1e-2, 0.9, 0.99, 1e-8, 0.1
+    pd, md, vd, gd = (t.double() for t in (p, m, v, g))
+    md, vd = b1 * md + (1 - b1) * gd, b2 * vd + (1 - b2) * gd * gd
+    pd = pd * (1 - lr * wd) - lr * (md / (1 - b1)) / ((vd / (1 - b2)).sqrt() + eps)
+    _lib.check(_lib.lib().cgk_adam_step(p.data_ptr(), m.data_ptr(), v.data_ptr(), g.data_ptr(), p16.data_ptr(), n, lr, b1, b2, eps, wd, 0.0, None, _lib.stream_ptr()))
+    # a handful of fp32 roundings each; 1 - b2 and 1 - b1 are fp32 differences of rounded constants: 2^-24 / 0.01 at most
+    for got, ref in ((m, md), (v, vd), (p, pd)):
+        assert ((got.double() - ref).abs() <= ref.abs() * 1e-5 + 1e-6).all()
+    assert torch.equal(p16, p.bfloat16())
+
+
 @pytest.mark.parametrize("D", [768, 1608, 4096])
 def test_norm_backward_takes_scratch_on_any_boundary(D):
     from cogito_b200.ops import _lib
