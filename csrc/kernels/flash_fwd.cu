@@ -124,10 +124,17 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   int qblk, h;
-  attention_tile(blockIdx.x, p.tiles, p.B * p.Hq, p.chunk, qblk, h);
+  int b;
+  if (p.chunk == 0) {                           // the grid's own order
+    qblk = blockIdx.x;
+    h = blockIdx.y;
+    b = blockIdx.z;
+  } else {
+    attention_tile(blockIdx.x, p.tiles, p.B * p.Hq, p.chunk, qblk, h);
+    b = h / p.Hq;
+    h -= b * p.Hq;
+  }
   qblk = p.tiles - 1 - qblk;                    // heavy (late) causal blocks first
-  const int b = h / p.Hq;
-  h -= b * p.Hq;
   const int hk = (int)(((long long)h * p.Hk) / p.Hq);
   const int q0 = qblk * 2 * C::BM;
   const int off = p.Tk - p.Tq;  // causal alignment: key k visible to query q iff k <= q + off
@@ -585,7 +592,7 @@ static int launch_fwd(const cgk_flash_args& a, const FlashFwdDev& p, cudaStream_
   CGK_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::TOTAL));
   const long long ctas = (long long)p.tiles * a.Hq * a.B;
   CGK_REQUIRE(ctas <= 0x7fffffffLL, "cgk_flash_forward: too many tiles");
-  kernel<<<(unsigned)ctas, 384, C::TOTAL, st>>>(tq, tk, tv, p);
+  kernel<<<p.chunk ? dim3((unsigned)ctas) : dim3(p.tiles, a.Hq, a.B), 384, C::TOTAL, st>>>(tq, tk, tv, p);
   CGK_LAUNCH_CHECK();
   return 0;
 }
@@ -622,7 +629,10 @@ CGK_API int cgk_flash_forward(const cgk_flash_args* pa, void* stream) {
   p.o_vec = o_vec;
   p.status = device_status(dev);
   p.tiles = (a.Tq + 255) / 256;                 // pairs of 128-row query tiles
-  p.chunk = attention_chunk(p.tiles, a.B * a.Hq, sm_count(dev));
+  // Tiles of equal length, and grids that start at once, take the grid's own order (0), without the divisions of the other:
+  // 2 sequences of 93 tokens, 40 heads of 128, 9.2 -> 8.8 us; 2 x 718 tokens without a mask 44.1 -> 43.2.
+  const bool own_order = !a.causal || (long long)p.tiles * a.Hq * a.B <= sm_count(dev);
+  p.chunk = own_order && a.Hq <= 65535 && a.B <= 65535 ? 0 : attention_chunk(p.tiles, a.B * a.Hq, sm_count(dev));
   if (a.D == 64) return launch_fwd<64>(a, p, (cudaStream_t)stream);
   return launch_fwd<128>(a, p, (cudaStream_t)stream);
 }
