@@ -219,11 +219,13 @@ int launch(const cgk_gemm_args& a, GemmDev g, int S, cudaStream_t stream) {
 // Where the line lies (times with cold caches and about 7 us of event and launch in each, 128 x 64 tiles here / persistent kernel):
 //   one row tile, while 128-column tiles fit two to an SM: 32 x 768 x 2048 13.1 / 18.4 us, x 2048 x 2048 14.3 / 19.2,
 //   x 2048 x 5632 18.4 / 36.9, x 32000 x 2048 (128 columns, no split) 39.6 / 47.1;
-//   several row tiles, if the K range is long enough (24 blocks) for at least four CTAs per tile: 256 x 2048 x 2048 16.4 / 19.5,
+//   several row tiles, if the K range is long enough (32 blocks) for at least four CTAs per tile: 256 x 2048 x 2048 16.4 / 19.5,
 //   512 x 768 x 3072 18.4 / 24.6, 2048 x 64 x 2048 15.2 / 18.4; with two CTAs per tile (512 x 2048 x 2048) both take 20.4, and
-//   256 x 3072 x 768 (12 blocks) 16.4 / 14.3;
+//   256 x 3072 x 768 (12 blocks) 16.4 / 14.3, warm 2089 x 128 x 1584 (25 blocks in eight parts) 13.8 / 11.9;
 //   a column count that is no multiple of 32, whose last tiles the persistent kernel stores element by element: weight
-//   gradient 512 x 784 x 256 14.5 / 47.1.
+//   gradient 512 x 784 x 256 14.5 / 47.1.  With one CTA per tile its longer loop over 64 columns has to be short (warm: 2811 x 808 x 784
+//   15.6 / 25.7, but 6635 x 200 x 1064 19.5 / 18.8, 7321 x 136 x 1976 28.0 / 23.6), or the sum is added to the output, which costs the other
+//   kernel a read per element too (1248 x 1272 over 2936 rows 32.8 / 46.7, 1672 x 968 over 4840 rows 55.6 / 46.0).
 bool gemm_few_plan(const cgk_gemm_args& a, int ctas, FewPlan* p) {
   if (a.rope_cos || a.split_k > 1) return false;
   const long long tm = (long long)a.batch * ((a.M + BM - 1) / BM), slots = a.max_ctas > 0 ? ctas : 2LL * ctas;
@@ -237,8 +239,9 @@ bool gemm_few_plan(const cgk_gemm_args& a, int ctas, FewPlan* p) {
   }
   p->bn = 64;
   p->split = split(tiles(64));
-  if (a.N % 32 != 0 && a.N % 4 == 0 && a.N > 32) return tiles(64) * p->split <= slots;
-  return kb >= 24 && p->split >= 4 && tiles(64) * p->split <= slots;
+  if (a.N % 32 != 0 && a.N % 4 == 0 && a.N > 32)
+    return tiles(64) * p->split <= slots && (p->split > 1 || kb <= 16 || (a.accumulate && kb <= 64));
+  return kb >= 32 && p->split >= 4 && tiles(64) * p->split <= slots;
 }
 
 int launch_gemm_few(const cgk_gemm_args& a, const GemmDev& g, const FewPlan& p, cudaStream_t stream) {

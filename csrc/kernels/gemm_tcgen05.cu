@@ -269,13 +269,15 @@ static int launch_wide(const cgk_gemm_args& a, const GemmDev& g0, int ctas, cuda
 // Pairs or single CTAs for a 256-wide tile (single / pair, us, timed in turn).  Pairs where the main loop is what a tile waits
 // for: 8176 x 22016 x 4096 1029 / 929, weight gradient 3072 x 768 over 131 072 rows 450 / 421; with K below 1024 where the
 // epilogue is light and there are tiles for two rounds: 131072 x 2304 x 768 409 / 372, 32768 x 50304 x 768 2154 / 1911, but
-// with GELU' 613 / 650 and 5555 x 768 x 768 19.4 / 21.2.  A single round of tiles pays for a pair's longer start unless K is long
+// with GELU' 613 / 650 and 5555 x 768 x 768 19.4 / 21.2, and with columns that are no multiple of 32, which take the general
+// epilogue, from K = 720 on (warm: 32751 x 368 x 192 55 / 70, 31750 x 1624 x 592 131 / 151, 3609 x 3096 x 688 52 / 56, but
+// 27264 x 3224 x 736 192 / 183, 9952 x 4520 x 824 152 / 140).  A single round of tiles pays for a pair's longer start unless K is long
 // (5555 x 768 x 2304 24.6 / 26.7, x 3072 31.7 / 31.8, 1000 x 4096 x 11008 87 / 77), and few rows for its taller tile
 // (300 x 22016 x 4096 70.5 / 79.9, 520 rows 95 / 101, 1000 rows 151 / 132).
 static bool by_pairs(const cgk_gemm_args& a, int ctas) {
   if (ctas < 2 || a.M <= 6 * BM) return false;
   const long long tiles = (long long)a.batch * ((a.M + 2 * BM - 1) / (2 * BM)) * ((a.N + PAIR_BN - 1) / PAIR_BN), pairs = ctas / 2;
-  if (a.K < 1024) return !a.act && !a.aux_in && !a.aux_out && tiles >= 2 * pairs;
+  if (a.K < 1024) return !a.act && !a.aux_in && !a.aux_out && (a.N % 32 == 0 || a.K >= 720) && tiles >= 2 * pairs;
   return tiles > pairs || a.K >= 3072;
 }
 
