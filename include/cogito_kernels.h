@@ -18,6 +18,10 @@ const char* cgk_last_error(void);
 int cgk_version(void);
 /* out[4] = {code, where, block, aux}; synchronises `stream`; clears the word. */
 int cgk_read_status(int* out, void* stream);
+/* Identity of the graph capture that the stream takes part in (0: none), and what the calling thread may do elsewhere while one
+ * is under way (a cudaStreamCaptureMode; returns the mode before). */
+long long cgk_capture_id(void* stream);
+int cgk_exchange_capture_mode(int mode);
 
 /* ---- GEMM ------------------------------------------------------------- */
 enum { CGK_ACT_NONE = 0, CGK_ACT_GELU = 1, CGK_ACT_RELU = 2, CGK_ACT_SILU = 3,
