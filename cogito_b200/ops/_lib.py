@@ -102,6 +102,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "cgk_int4_tile_weights": [vp, vp, i, i, i, vp, vp],
         "cgk_int4_wa_gemm": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
         "cgk_int4_wa_gemm_parts": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
+        "cgk_int4_wa_gemm_parts_f32": [vp, ll, vp, vp, vp, vp, ll, vp, i, i, i, i, vp],
         "cgk_int4_wa_tile_weights": [vp, vp, i, i, i, vp, vp],
         "cgk_kv_int4_append": [vp, vp, vp, i, vp],
         "cgk_kv_int4_append_rows": [vp, vp, vp, ll, ll, ll, i, vp, vp, vp],

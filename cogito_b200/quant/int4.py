@@ -112,19 +112,20 @@ class _Counters:
 class Int4Linear(torch.nn.Module):
     """y = x @ W^T (+ bias) with W stored as packed INT4 of W^T ([in, out], groups along out)."""
 
-    # Which tcgen05 kernel multiplies: "wb" keeps the weights as the B operand (converted tile in shared
-    # memory, 128 token rows per instruction), "wa" makes them the A operand fed from tensor memory (cost
-    # follows the token count; needs group % 128 == 0).  "auto": "wa" up to 16 token rows, "wb" up to two row
+    # Which kernel multiplies: "wb" keeps the weights as the B operand of tcgen05 MMAs (converted tile in shared
+    # memory, 128 token rows per instruction), "wa" makes them the A operand of warp-level MMAs, fed from registers (cost
+    # follows the token count; needs group % 128 == 0).  "auto": "wa" up to 32 token rows, "wb" up to two row
     # tiles, and beyond that (prompts) the weights are dequantised to bf16 once per call for the dense GEMM: "wb" converts
     # every weight tile again for each row tile.  That copy (2 bytes per weight: 180 MB for 4096 x 22016, 262 MB for
     # 4096 x 32000) comes from the allocator for the time of the call, one layer's at a time; where there is no room for it,
     # "wb" takes the call.  Each of the two kernels has its own tile-major copy of the weights, made on
     # first use; both sum the parts of a shared tile in a fixed order, so a call gives the same bits every time.
     # Times (us, layers one after the other) for 4096 x 6144, 4096 x 4096, 4096 x 22016, 11008 x 4096, 4096 x 32000, 2048 x 11264:
-    #   16 rows   "wa" 20.1 14.9 34.7 24.7 44.6 19.2
-    #   17 rows   "wa" 28.2 20.4 54.4 36.9 71.4 25.9 (columns padded to 32)   "wb" 18.9 15.7 43.7 26.3 59.3 17.1
-    #   200 rows  "wb" 31.4 24.9 103 45.9 141 30.5     dense 31.4 26.5 104 61.1 131 32.7 (a third row tile adds half to "wb")
-    DENSE_ROWS = 256
+    #   16 rows   "wa" 8.4 6.5 20.6 11.0 25.9 10.3      (before, through tensor memory: 20.1 14.9 34.7 24.7 44.6 19.2)
+    #   32 rows   "wa" 12.8 9.0 31.5 15.7 39.8 15.5     "wb" 19.2 15.8 43.3 25.9 58.4 17.4
+    #   80 rows   "wa" 27.4 22.4 75.4 40.5 107 28.4     "wb" 21.0 18.3 45.8 28.1 60.4 19.3 (three passes over the weights)
+    #   200 rows  "wb" 31.4 24.9 103 45.9 141 30.5      dense 31.4 26.5 104 61.1 131 32.7 (a third row tile adds half to "wb")
+    FEW_ROWS, DENSE_ROWS = 32, 256
     kernel = os.environ.get("COGITO_INT4_KERNEL", "auto")
 
     def __init__(self, weight: torch.Tensor, bias: torch.Tensor | None = None, group: int = 128):
@@ -193,13 +194,15 @@ class Int4Linear(torch.nn.Module):
         return gemm(x2.to(torch.bfloat16).contiguous(), self.dequantized(torch.bfloat16), b_mn=True, bias=self.bias, **kw)
 
     def forward_f32(self, x: torch.Tensor) -> torch.Tensor:
-        """fp32 result (logits); many rows leave the GEMM in fp32 without a bf16 copy in between."""
+        """fp32 result (logits); few rows and prompts leave the GEMM in fp32 without a bf16 copy in between."""
         rows = x.numel() // self.in_features
         if x.is_cuda and self._takes_dense(rows):
             try:
                 return self._dense(x.reshape(rows, self.in_features), out_dtype=torch.float32).view(*x.shape[:-1], self.out_features)
             except torch.OutOfMemoryError:
                 pass                                       # no room for the weights in bf16: by the streaming kernel
+        if x.is_cuda and rows and self._streams_few(rows):
+            return self._stream(x.reshape(rows, self.in_features), f32=True).view(*x.shape[:-1], self.out_features)
         return self.forward(x).float()
 
     def forward(self, x: torch.Tensor, splits: int = 0, out: torch.Tensor | None = None, f32: bool = False) -> torch.Tensor:
@@ -235,10 +238,19 @@ class Int4Linear(torch.nn.Module):
                 return self._dense(x2, out=None if out is None else out.view(M, N)).view(*lead, N)
             except torch.OutOfMemoryError:
                 pass                                       # no room for the weights in bf16: by the streaming kernel
+        return self._stream(x2, splits, out).view(*lead, N)
+
+    def _streams_few(self, rows: int) -> bool:
+        """"wa" (needs one scale per k for a 128-feature tile)."""
+        return (self.kernel == "wa" or (self.kernel == "auto" and rows <= self.FEW_ROWS)) and self.group % 128 == 0 \
+            and self.in_features % 128 == 0 and self.out_features % 128 == 0
+
+    def _stream(self, x2: torch.Tensor, splits: int = 0, out: torch.Tensor | None = None, f32: bool = False) -> torch.Tensor:
+        """[rows, in] through "wa" or "wb"; ``f32``: an fp32 result ("wa" only)."""
         x2 = x2.to(torch.bfloat16).contiguous()
         L = _lib.lib()
-        # "wa": weights on the M side of the tensor core (needs one scale per k for a 128-feature tile)
-        wa = (self.kernel == "wa" or (self.kernel == "auto" and M <= 16)) and self.group % 128 == 0 and K % 128 == 0
+        M, N, K = x2.shape[0], self.out_features, self.in_features
+        wa = self._streams_few(M)
         tiles = self._tiles.get(wa)
         if tiles is None or tiles.device != x2.device:
             tiles = self._tile(wa, x2.device)
@@ -251,11 +263,11 @@ class Int4Linear(torch.nn.Module):
         parts = torch.empty((L.cgk_int4_wa_gemm_parts_floats if wa else L.cgk_int4_gemm_parts_floats)(M, N, K, splits), dtype=torch.float32, device=x2.device)
         counters = self._counters.get(L.cgk_int4_gemm_counters(M, N), L.cgk_int4_gemm_counters(self.DENSE_ROWS, N), x2.device)
         if out is None:
-            out = torch.empty(M, N, dtype=torch.bfloat16, device=x2.device)
+            out = torch.empty(M, N, dtype=torch.float32 if f32 else torch.bfloat16, device=x2.device)
         elif out.dtype != torch.bfloat16 or not out.is_contiguous() or out.numel() != M * N:
             raise ValueError("out must be a contiguous bf16 [rows, out_features] tensor")
-        _lib.check((L.cgk_int4_wa_gemm_parts if wa else L.cgk_int4_gemm_parts)(
-            x2.data_ptr(), K, tiles.data_ptr(), parts.data_ptr(), counters.data_ptr(),
-            out.data_ptr(), N, _lib.ptr(self.bias), M, N, K, splits, _lib.stream_ptr()), "cgk_int4_gemm")
+        entry = (L.cgk_int4_wa_gemm_parts_f32 if f32 else L.cgk_int4_wa_gemm_parts) if wa else L.cgk_int4_gemm_parts
+        _lib.check(entry(x2.data_ptr(), K, tiles.data_ptr(), parts.data_ptr(), counters.data_ptr(),
+                         out.data_ptr(), N, _lib.ptr(self.bias), M, N, K, splits, _lib.stream_ptr()), "cgk_int4_gemm")
         _lib.count_launch()
-        return out.view(*lead, N)
+        return out

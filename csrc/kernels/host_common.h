@@ -68,6 +68,26 @@ int sm_count(int device);
     }                                       \
   } while (0)
 
+// Launches a kernel that may start while its predecessor in the stream is still running (programmatic dependent launch): every
+// thread of it passes pdl_wait() before it touches memory that another kernel writes or reads.  cluster: CTAs along x, 0 for none.
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 0 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Runs f(scratch) with `floats` elements from the stream's memory pool, given back in stream order (null: none wanted, or none left).
 template <typename F>
 int with_stream_scratch(long long floats, cudaStream_t stream, F f) {

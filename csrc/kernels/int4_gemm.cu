@@ -353,7 +353,8 @@ CGK_API int cgk_int4_tile_weights(const void* packed, const float* scales, int K
   CGK_LAUNCH_CHECK();
   return 0;
 }
-CGK_API long long cgk_int4_gemm_counters(int M, int N) { return (long long)((M + BM - 1) / BM) * (N / BN); }
+// one per output tile; the smallest tiles of cgk_int4_wa_gemm are 32 x 32
+CGK_API long long cgk_int4_gemm_counters(int M, int N) { return (long long)((M + 31) / 32) * (N / 32); }
 
 // How the tiles are dealt out: one CTA per SM (of a row tile's share of them), each with at least two steps of the left-over
 // tiles; given splits: that many equal parts of every tile; without a place for parts: whole tiles.

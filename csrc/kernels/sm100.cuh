@@ -14,6 +14,20 @@
 namespace cgk {
 
 // ---------------------------------------------------------------------------
+// launches that overlap their predecessor (launch_overlapped on the host)
+// ---------------------------------------------------------------------------
+// Everything that the kernels before this one in the stream wrote is visible behind pdl_wait(), and they have ended; every thread
+// of a kernel that is launched so passes it, also the ones that find nothing to do (a successor counts on this kernel's
+// end to be behind its predecessor's).  pdl_trigger() lets the next kernel's CTAs take the resources that this one leaves; it comes
+// after a CTA has taken its own tensor memory.  Both do nothing in a kernel launched the usual way.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// bytes: a multiple of 16, from a 16-byte boundary
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+// ---------------------------------------------------------------------------
 // status reporting
 // ---------------------------------------------------------------------------
 // One int4 in global memory per library instance: {code, where, block, aux}.

@@ -233,15 +233,17 @@ int cgk_int4_gemm_parts(const void* x, long long ldx, const void* w_tiles, float
                         long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
 int cgk_int4_gemm(const void* x, long long ldx, const void* w_tiles, float* acc, int* counters, void* out,
                   long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
-/* The same product with the weights on the M side of the tensor core (time grows with the rows
- * of x instead of always paying for 128), the group scale folded into x and a bit-trick-only
- * nibble conversion.  Needs group % 128 == 0.  Tiles: [N/128][K/64][4352] (4096 bytes of
- * nibbles [feature][8 words], then 64 fp32 scales); parts / acc / counters as for cgk_int4_gemm. */
+/* The same product for few rows: warp-level MMAs fed from registers (rows 32 at a time, time grows
+ * with them), the group scale folded into x and a bit-trick-only nibble conversion.  Needs
+ * group % 128 == 0.  Tiles: [N/128][K/32][2176] (2048 bytes of nibbles in the order of the MMA's
+ * fragments, then 32 fp32 scales); parts / acc / counters as for cgk_int4_gemm.  _f32: fp32 output. */
 long long cgk_int4_wa_tiles_bytes(int K, int N);
 int cgk_int4_wa_tile_weights(const void* packed, const float* scales, int K, int N, int group, void* tiles, void* stream);
 long long cgk_int4_wa_gemm_parts_floats(int M, int N, int K, int splits);
 int cgk_int4_wa_gemm_parts(const void* x, long long ldx, const void* tiles, float* parts, int* counters, void* out,
                            long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
+int cgk_int4_wa_gemm_parts_f32(const void* x, long long ldx, const void* tiles, float* parts, int* counters, float* out,
+                               long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
 int cgk_int4_wa_gemm(const void* x, long long ldx, const void* tiles, float* acc, int* counters, void* out,
                      long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
 

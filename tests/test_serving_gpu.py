@@ -66,6 +66,38 @@ def test_int4_gemm_pieces_of_the_weight_stream(M, K, N, kernel):
     _lib.assert_device_ok()
 
 
+# few rows: 8, 16 and 32 columns of MMAs, one unit of 64 k per warp and fewer, clusters of eight down to two and pieces of the line,
+# an fp32 result; rows of X and of the output that lie further apart than they are long are the C entry's
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 31, 33, 65])
+@pytest.mark.parametrize("K,N", [(128, 256), (512, 128), (1024, 640), (4096, 2176), (1664, 6144), (1152, 9600)])
+def test_int4_gemm_few_rows(M, K, N):
+    torch.manual_seed(M + K)
+    lin = Int4Linear(torch.randn(N, K) * 0.05, torch.randn(N) * 0.1, 128).to(DEV)
+    lin.kernel = "wa"
+    x = (torch.randn(M, K) + 0.5).bfloat16().to(DEV)
+    ref = x.double() @ lin.dequantized().double() + lin.bias.double()
+    full = lin(x, f32=True)
+    assert full.dtype == torch.float32
+    # x' is rounded to bf16 once per element (2^-9 of the terms' norm), sums are fp32 with terms 17 times as large as the weights
+    assert ((full.double() - ref).norm() / ref.norm()).item() < 2 ** -8
+    assert torch.equal(full.bfloat16(), lin(x)) and torch.equal(full, lin(x, f32=True))
+    _lib.assert_device_ok()
+
+
+@pytest.mark.parametrize("N", [256, 22016])
+def test_int4_gemm_few_rows_strided(N):
+    L, M, K = _lib.lib(), 19, 1024
+    lin = _int4_layer(K, N)
+    lin.kernel = "wa"
+    wide = torch.randn(M, K + 24, device=DEV, dtype=torch.bfloat16)
+    want, out = lin(wide[:, 8:8 + K].contiguous()), torch.full((M, N + 4), 7.0, device=DEV, dtype=torch.bfloat16)
+    parts = torch.empty(L.cgk_int4_wa_gemm_parts_floats(M, N, K, 0), device=DEV)
+    counters = torch.zeros(L.cgk_int4_gemm_counters(M, N), dtype=torch.int32, device=DEV)
+    _lib.check(L.cgk_int4_wa_gemm_parts(wide[:, 8:].data_ptr(), K + 24, lin._tiles[True].data_ptr(), parts.data_ptr(), counters.data_ptr(), out.data_ptr(), N + 4,
+                                        None, M, N, K, 0, _lib.stream_ptr()), "cgk_int4_wa_gemm_parts")
+    assert torch.equal(out[:, :N], want) and (out[:, N:] == 7).all() and not counters.any()
+
+
 # parts of a shared tile are summed in the order of the CTAs, not of their arrival: a call gives the same bits every time
 @pytest.mark.parametrize("M,K,N", [(16, 11008, 4096), (16, 4096, 22016), (80, 4096, 6144), (80, 4096, 22016), (200, 1408, 4096)])
 @pytest.mark.parametrize("kernel", ["wa", "wb"])
