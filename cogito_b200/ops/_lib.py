@@ -107,6 +107,8 @@ def _declare(L: ctypes.CDLL) -> None:
         "cgk_kv_int4_append": [vp, vp, vp, i, vp],
         "cgk_kv_int4_append_rows": [vp, vp, vp, ll, ll, ll, i, vp, vp, vp],
         "cgk_kv_int4_attention": [vp, vp, vp, i, i, f, i, vp, vp],
+        "cgk_kv_int4_attention_few": [vp, i, i],
+        "cgk_kv_int4_attention_strided": [vp, vp, ll, ll, ll, vp, i, i, f, i, vp],
         "cgk_sample": [vp, i, ll, i, i, f, i, f, c_ulonglong, vp, vp, vp, vp],
         "cgk_spec_accept": [vp, vp, vp, i, i, i, c_ulonglong, vp, vp, vp, vp, vp, vp],
         "cgk_tree_mask": [vp, i, i, vp, vp, vp],

@@ -210,7 +210,7 @@ class LlamaInt4Engine:
                 kq, vq = kept if kept is not None else (self._fake_quant(t) for t in (k, v))
                 o = flash_forward(qkv[:, :, :Hq], kq, vq, causal=True)[0]
             else:
-                o = self.cache.attention(i, qkv[:, :, :Hq].contiguous())
+                o = self.cache.attention(i, qkv[:, :, :Hq])
             h = self._proj_add_norm(l["proj"], o.reshape(B, Tq, Hq * D), x, l["norm2"])
             nxt = self.layers[i + 1]["norm1"] if i + 1 < len(self.layers) else self.norm_f
             h = self._proj_add_norm(l["down"], M.swiglu(l["gate_up"](h)), x, nxt)

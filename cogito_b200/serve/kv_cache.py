@@ -192,15 +192,25 @@ class PagedKVCacheInt4(PagedCache):
         B, Tq, Hq, D = q.shape
         scale = 1.0 / math.sqrt(D)
         if q.is_cuda:
-            q = q.to(torch.bfloat16).contiguous()
+            q = q.to(torch.bfloat16)
+            L, a, longest = _lib.lib(), self._args(layer), self.max_pages * self.page_size
+            if L.cgk_kv_int4_attention_few(ctypes.byref(a), Tq, Hq):
+                # rows are read where they lie (a slice of a packed projection); CTAs that share a head's keys take at least a block of 16 per warp
+                if q.stride(3) != 1 or any(s % 8 for s in q.stride()[:3]) or q.data_ptr() % 16:
+                    q = q.contiguous()
+                if splits <= 0:
+                    splits = max(1, min(8, 296 // max(1, B * self.heads), (longest + 63) // 64))
+                out = torch.empty(B, Tq, Hq, D, dtype=q.dtype, device=q.device)
+                _lib.check(L.cgk_kv_int4_attention_strided(ctypes.byref(a), q.data_ptr(), q.stride(0), q.stride(1), q.stride(2), out.data_ptr(), Tq, Hq, scale,
+                                                           splits, _lib.stream_ptr()), "cgk_kv_int4_attention_strided")
+                _lib.count_launch()
+                return out
+            q = q.contiguous()
             if splits <= 0:
-                longest = self.max_pages * self.page_size
                 splits = max(1, min(32, 296 // max(1, B * self.heads), (longest + 255) // 256))
-            L = _lib.lib()
             need = L.cgk_kv_int4_attention_scratch_floats(B, Hq, Tq, D, splits)
             scratch = torch.empty(need, dtype=torch.float32, device=q.device)    # of this call: a captured one keeps its address
             out = torch.empty_like(q)
-            a = self._args(layer)
             _lib.check(L.cgk_kv_int4_attention(ctypes.byref(a), q.data_ptr(), out.data_ptr(), Tq, Hq, scale, splits,
                                                scratch.data_ptr(), _lib.stream_ptr()), "cgk_kv_int4_attention")
             _lib.count_launch(2)

@@ -40,7 +40,7 @@
 #include <atomic>
 
 #include "host_common.h"
-#include "sm100.cuh"
+#include "mma_sync.cuh"
 #include "cogito_kernels.h"
 
 namespace {
@@ -86,35 +86,12 @@ __device__ __forceinline__ WaShare wa_share(uint32_t k_units, const Pieces& piec
   return w;
 }
 
-__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_16_or_zero(uint32_t dst, const void* src, uint32_t bytes) {     // bytes: 16, or 0 for zeros
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t mapped) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(mapped) : "memory");
-  return v;
-}
 // One thread's arrival for its CTA behind a barrier: what the CTA wrote before is visible to whoever finds it counted.
 __device__ __forceinline__ int arrive_acq_rel(int* counter) {
   int old;
   asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
   return old;
 }
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-// (v & mask) | magic in one instruction: only one of two constants fits into it, so both come from registers
-__device__ __forceinline__ uint32_t pick(uint32_t v, uint32_t mask, uint32_t magic) {
-  uint32_t r;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(v), "r"(mask), "r"(magic));
-  return r;
-}
-
 template <int NT>
 __global__ void __launch_bounds__(W_THREADS, 1)
 int4_wa_kernel(const WaDev g) {
@@ -174,7 +151,7 @@ int4_wa_kernel(const WaDev g) {
       fs += C::STAGE;
       if (fs == ring_end) fs = ring;
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");                    // an empty group past the end: the count below stays right
+    cp_async_commit();                    // an empty group past the end: the count below stays right
   };
 #pragma unroll
   for (int i = 0; i < C::STAGES - 1; ++i) fetch();
@@ -194,7 +171,7 @@ int4_wa_kernel(const WaDev g) {
       }
     }
     for (; u < to; u += W_WARPS) {
-      asm volatile("cp.async.wait_group %0;" ::"n"(C::STAGES - 2) : "memory");
+      cp_async_wait<C::STAGES - 2>();
       __syncwarp();                                                         // the scales came through the first lanes; the slot fetched next was read by all
       const uint8_t* src = stages + slot * C::STAGE;
       slot = slot + 1 == C::STAGES ? 0 : slot + 1;

@@ -1,0 +1,318 @@
+// Attention of few query rows over the paged INT4 KV cache (head_dim 128): decoding and the verify pass of speculative decoding.
+//
+// A kv head has R = Tq * (Hq / Hk) query rows, 4 for one new token and 20 for five with four query heads per kv head.  tcgen05 tiles
+// of 128 keys (kv_attn_tc.cu) spent 12 us per 128 keys on writing converted tiles to shared memory and on two hand-overs to the
+// MMA-issuing thread; here every warp works through its own blocks of 16 keys with mma.sync, from the nibbles to its part of the
+// result, and meets the others only at the end:
+//   * S[rows, 16 keys] = Q . K^T: lane (g, q) holds the 32 elements 32 q .. 32 q + 31 of keys g and g + 8, 16 bytes of nibbles each,
+//     which are its fragments of eight MMAs; the elements' order in a word (0,4,1,5,2,6,3,7) is given to Q's fragments instead;
+//   * O[rows, 128] += P . V: the sums of S are the A fragments of P; lane (g, q) holds elements 16 g .. 16 g + 15 of keys 2 q, 2 q + 1,
+//     2 q + 8, 2 q + 9, and column g of the MMAs' eight columns j is element 16 g + j;
+//   * a lane copies (cp.async, a ring of four blocks) exactly what it converts; the pages of the next 32 blocks are held one by lane.
+// The parts (row maximum, sum, O) of the warps of a cluster of CTAs that share a (sequence, kv head) meet over distributed shared
+// memory, in the order of the ranks and warps.
+// Values are those of kv_attn_tc.cu: K and V as bf16(q * bf16(scale)), P rounded to bf16 before it is summed.
+//
+// 16 sequences of 641 tokens, 32 query and 8 kv heads, one new token: PLACE us (24.7 + 2.7 for the kernel that combined the splits before);
+// five: PLACE (37.4 + 5.2).  10.5 MB of cache are 1.6 us at HBM rate; the rest is start, the chain of a warp's five blocks and the merge.
+#include <cuda_bf16.h>
+
+#include "host_common.h"
+#include "kv_dev.cuh"
+#include "mma_sync.cuh"
+
+namespace cgk {
+namespace {
+
+constexpr int KM_WARPS = 4, KM_THREADS = KM_WARPS * 32, KM_D = 128, KM_KB = 16, KM_STAGES = 4, KM_MAX_CLUSTER = 8;
+constexpr int KM_STAGE = 32 * (2 * 16 + 4 * 8 + 2 * 4 + 4 * 4);       // a warp's block: K, V, K scales, V scales, all by lane
+constexpr int KM_LD = KM_D + 4;                                       // row of a part: rows start in different banks
+
+template <int MT>                                                      // 16-row tiles of Q
+struct KmSmem {
+  static constexpr int ROWS = 16 * MT;
+  static constexpr int RING = KM_WARPS * KM_STAGES * KM_STAGE;
+  static constexpr int PART = ROWS * KM_LD * 4;                        // a warp's O
+  static constexpr int O_BYTES = KM_WARPS * PART;                      // overlays the rings once the loop is over
+  static constexpr int BODY = RING > O_BYTES ? RING : O_BYTES;
+  static constexpr int OFF_ML = BODY;                                  // float [warp][2][ROWS]: maximum, sum
+  static constexpr int OFF_W = OFF_ML + KM_WARPS * 2 * ROWS * 4;       // float [KM_MAX_CLUSTER * KM_WARPS][ROWS]: weights of all parts
+  static constexpr int OFF_Q = OFF_W + KM_MAX_CLUSTER * KM_WARPS * ROWS * 4;
+  static constexpr int TOTAL = OFF_Q + (MT > 1 ? MT * 8 * 512 : 0);    // Q fragments of more than one tile: [tile][MMA][lane] 16 bytes
+};
+
+// eight nibbles -> four pairs of bf16 (elements 0,4 1,5 2,6 3,7), times the group scale
+__device__ __forceinline__ void km_convert(uint32_t w, __nv_bfloat162 s2, uint32_t mask, uint32_t magic, uint32_t (&o)[4]) {
+  const uint32_t v = w ^ 0x88888888u, c136 = 0x43084308u;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t x = pick(v >> (4 * j), mask, magic);                // 128 + (nibble ^ 8) in both halves
+    const __nv_bfloat162 h = __hmul2(__hsub2(*reinterpret_cast<const __nv_bfloat162*>(&x), *reinterpret_cast<const __nv_bfloat162*>(&c136)), s2);
+    o[j] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+
+template <int MT>
+__global__ void __launch_bounds__(KM_THREADS, 2)
+kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long q_bs, long long q_ts, long long q_hs, int Tq, int Hq, float scale_log2,
+                        __nv_bfloat16* __restrict__ out) {
+  using S = KmSmem<MT>;
+  constexpr int ROWS = S::ROWS;
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, qq = lane & 3;
+  const int splits = gridDim.x, rank = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+  const int rep = Hq / c.heads, R = Tq * rep, G = KM_D / c.group;
+  pdl_trigger();
+  pdl_wait();
+  const int len = c.lengths[b] + Tq;                                   // the Tq new tokens were appended before the call
+  const int blocks = (len + KM_KB - 1) / KM_KB, stride = splits * KM_WARPS;
+  const int first = rank * KM_WARPS + warp;                            // this warp's blocks of 16 keys: first, first + stride, ..
+  const int mine = first < blocks ? (blocks - first + stride - 1) / stride : 0;
+  const bool one_page = c.page_size % KM_KB == 0;                      // a block never crosses pages
+
+  const uint32_t ring = smem_u32(smem) + warp * (KM_STAGES * KM_STAGE);
+  int held = 0;                                                        // lane l: the page of block (next multiple of 32 blocks) + l
+  auto page_of = [&](int key) { return c.page_table[CGK_IDX(b * c.max_pages + key / c.page_size, c.batch * c.max_pages)]; };
+  auto fetch = [&](int i) {
+    if (i < mine) {
+      const int kb = (first + i * stride) * KM_KB;
+      if ((i & 31) == 0) {
+        const int j = i + lane;
+        held = one_page && j < mine ? page_of((first + j * stride) * KM_KB) : 0;
+      }
+      const int page = __shfl_sync(0xffffffffu, held, i & 31);
+      const long long base = (long long)page * c.page_size + kb % c.page_size;
+      auto token = [&](int k) -> long long {                           // key kb + k, inside the sequence
+        if (one_page) return (base + k) * c.heads + hk;
+        return ((long long)page_of(kb + k) * c.page_size + (kb + k) % c.page_size) * c.heads + hk;
+      };
+      const uint32_t dst = ring + (i % KM_STAGES) * KM_STAGE;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int k = gq + 8 * h;
+        const bool in = kb + k < len;
+        const long long t = in ? token(k) : 0;
+        cp_async_16_or_zero(dst + h * 512 + lane * 16, c.k_pages + t * (KM_D / 2) + qq * 16, in ? 16 : 0);
+        cp_async_or_zero<4>(dst + 2048 + h * 128 + lane * 4, c.k_scales + t * G + qq * 32 / c.group, in ? 4 : 0);
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const int k = 2 * qq + (h & 1) + 8 * (h >> 1);
+        const bool in = kb + k < len;
+        const long long t = in ? token(k) : 0;
+        cp_async_or_zero<8>(dst + 1024 + h * 256 + lane * 8, c.v_pages + t * (KM_D / 2) + gq * 8, in ? 8 : 0);
+        cp_async_or_zero<4>(dst + 2304 + h * 128 + lane * 4, c.v_scales + t * G + gq * 16 / c.group, in ? 4 : 0);
+      }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int i = 0; i < KM_STAGES - 1; ++i) fetch(i);
+
+  // Q: fragment register 0 / 2 (row g) and 1 / 3 (row g + 8) of MMA 2 w and 2 w + 1 are elements 32 q + 8 w ..
+  uint32_t qf[MT == 1 ? 8 : 1][4];
+  uint4* const q_s = reinterpret_cast<uint4*>(smem + S::OFF_Q);
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) {
+    if (MT > 1 && warp >= MT && mt == 0) break;
+    if (MT > 1 && warp != mt) continue;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      uint32_t p[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = mt * 16 + gq + 8 * h;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (r < R) v = *reinterpret_cast<const uint4*>(q + b * q_bs + r / rep * q_ts + (hk * rep + r % rep) * q_hs + qq * 32 + w * 8);
+        p[h][0] = __byte_perm(v.x, v.z, 0x5410); p[h][1] = __byte_perm(v.x, v.z, 0x7632);
+        p[h][2] = __byte_perm(v.y, v.w, 0x5410); p[h][3] = __byte_perm(v.y, v.w, 0x7632);
+      }
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        if constexpr (MT == 1) {
+          qf[2 * w + s][0] = p[0][2 * s]; qf[2 * w + s][1] = p[1][2 * s]; qf[2 * w + s][2] = p[0][2 * s + 1]; qf[2 * w + s][3] = p[1][2 * s + 1];
+        } else {
+          q_s[(mt * 8 + 2 * w + s) * 32 + lane] = make_uint4(p[0][2 * s], p[1][2 * s], p[0][2 * s + 1], p[1][2 * s + 1]);
+        }
+      }
+    }
+  }
+  if (MT > 1) __syncthreads();
+
+  float o[MT][16][4], m[MT][2], l[MT][2];
+  int last[MT][2];                                                     // the last key that a row sees
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      m[mt][h] = -INFINITY;
+      l[mt][h] = 0.0f;
+      last[mt][h] = len - Tq + min((mt * 16 + gq + 8 * h) / rep, Tq - 1);      // causal among the new tokens
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[mt][j][e] = 0.0f;
+  }
+  uint32_t mask = 0x000F000Fu, magic = 0x43004300u;
+  asm volatile("" : "+r"(mask), "+r"(magic));
+
+  for (int i = 0; i < mine; ++i) {
+    cp_async_wait<KM_STAGES - 2>();
+    fetch(i + KM_STAGES - 1);
+    const uint8_t* src = smem + warp * (KM_STAGES * KM_STAGE) + (i % KM_STAGES) * KM_STAGE;
+    const int kb = (first + i * stride) * KM_KB;
+    float s[MT][2][4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {                                      // keys g and g + 8: the columns of two MMAs
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[mt][h][e] = 0.0f;
+      const uint4 raw = *reinterpret_cast<const uint4*>(src + h * 512 + lane * 16);
+      const __nv_bfloat162 s2 = __float2bfloat162_rn(*reinterpret_cast<const float*>(src + 2048 + h * 128 + lane * 4));
+      const uint32_t w4[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        uint32_t k[4];
+        km_convert(w4[w], s2, mask, magic, k);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if constexpr (MT == 1) {
+              mma_bf16(s[0][h], qf[2 * w + t][0], qf[2 * w + t][1], qf[2 * w + t][2], qf[2 * w + t][3], k[2 * t], k[2 * t + 1]);
+            } else {
+              const uint4 a = q_s[(mt * 8 + 2 * w + t) * 32 + lane];
+              mma_bf16(s[mt][h], a.x, a.y, a.z, a.w, k[2 * t], k[2 * t + 1]);
+            }
+          }
+      }
+    }
+    uint32_t p[MT][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {                                    // rows g and g + 8; values 2 h, 2 h + 1 of both tiles
+        float x[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int key = kb + (e >> 1) * 8 + 2 * qq + (e & 1);
+          x[e] = key <= last[mt][h] ? s[mt][e >> 1][2 * h + (e & 1)] * scale_log2 : -INFINITY;
+        }
+        float mx = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float mo = m[mt][h], mn = fmaxf(mo, mx);
+        if (__any_sync(0xffffffffu, mn > mo)) {
+          const float corr = mo > -INFINITY ? fast_exp2(mo - mn) : (mn > -INFINITY ? 0.0f : 1.0f);
+          l[mt][h] *= corr;
+          m[mt][h] = mn;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) { o[mt][j][2 * h] *= corr; o[mt][j][2 * h + 1] *= corr; }
+        }
+        float e4[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) e4[e] = x[e] > -INFINITY ? fast_exp2(x[e] - mn) : 0.0f;
+        const uint32_t lo = pack_bf16x2(e4[0], e4[1]), hi = pack_bf16x2(e4[2], e4[3]);
+        const float2 a = unpack_bf16x2(lo), d = unpack_bf16x2(hi);
+        l[mt][h] += (a.x + a.y) + (d.x + d.y);
+        p[mt][h] = lo;                                                 // A registers 0 / 1: keys 2 q, 2 q + 1
+        p[mt][2 + h] = hi;                                             // 2 / 3: eight more
+      }
+    }
+    // V: two words (elements 16 g .. 16 g + 7, 8 more) of each of four keys
+    uint2 raw[4];
+    __nv_bfloat162 s2[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      raw[h] = *reinterpret_cast<const uint2*>(src + 1024 + h * 256 + lane * 8);
+      s2[h] = __float2bfloat162_rn(*reinterpret_cast<const float*>(src + 2304 + h * 128 + lane * 4));
+    }
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      uint32_t v[4][4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) km_convert(w ? raw[h].y : raw[h].x, s2[h], mask, magic, v[h]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {                                    // elements 8 w + j (low halves) and 8 w + 4 + j (high halves)
+        const uint32_t b0 = __byte_perm(v[0][j], v[1][j], 0x5410), b1 = __byte_perm(v[2][j], v[3][j], 0x5410);
+        const uint32_t c0 = __byte_perm(v[0][j], v[1][j], 0x7632), c1 = __byte_perm(v[2][j], v[3][j], 0x7632);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          mma_bf16(o[mt][8 * w + j], p[mt][0], p[mt][1], p[mt][2], p[mt][3], b0, b1);
+          mma_bf16(o[mt][8 * w + 4 + j], p[mt][0], p[mt][1], p[mt][2], p[mt][3], c0, c1);
+        }
+      }
+    }
+  }
+  cp_async_wait<0>();
+  __syncthreads();                                                     // the rings make room for the parts
+  // sum j's columns 2 q and 2 q + 1 are elements 16 (2 q) + j and 16 (2 q + 1) + j
+  float* const part = reinterpret_cast<float*>(smem) + warp * (S::PART / 4);
+  float* const ml = reinterpret_cast<float*>(smem + S::OFF_ML);
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = mt * 16 + gq + 8 * h;
+      float sum = l[mt][h];
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      if (qq == 0) { ml[warp * 2 * ROWS + r] = m[mt][h]; ml[warp * 2 * ROWS + ROWS + r] = sum; }
+#pragma unroll
+      for (int col = 0; col < 2; ++col)
+#pragma unroll
+        for (int j = 0; j < 16; j += 4)
+          *reinterpret_cast<float4*>(part + r * KM_LD + 16 * (2 * qq + col) + j) =
+              make_float4(o[mt][j][2 * h + col], o[mt][j + 1][2 * h + col], o[mt][j + 2][2 * h + col], o[mt][j + 3][2 * h + col]);
+    }
+  if (splits > 1) cluster_sync_all();
+  else __syncthreads();
+  // every CTA writes its share of the rows: weights 2^(m_part - m) / sum of all parts, then the weighted sum
+  const int parts = splits * KM_WARPS, r0 = min(R, ROWS) * rank / splits, r1 = min(R, ROWS) * (rank + 1) / splits;
+  float* const wts = reinterpret_cast<float*>(smem + S::OFF_W);
+  auto at = [&](uint32_t addr, int p) { return splits > 1 ? cluster_map(addr, p / KM_WARPS) : addr; };
+  for (int r = r0 + warp; r < r1; r += KM_WARPS) {
+    float pm = -INFINITY, pl = 0.0f;
+    if (lane < parts) {
+      const uint32_t a = at(smem_u32(ml + lane % KM_WARPS * 2 * ROWS + r), lane);
+      pm = splits > 1 ? ld_cluster_f1(a) : ml[lane % KM_WARPS * 2 * ROWS + r];
+      pl = splits > 1 ? ld_cluster_f1(a + ROWS * 4) : ml[lane % KM_WARPS * 2 * ROWS + ROWS + r];
+    }
+    const float top = warp_max(pm), w = pm > -INFINITY ? fast_exp2(pm - top) : 0.0f, total = warp_sum(w * pl);
+    if (lane < parts) wts[lane * ROWS + r] = total > 0.0f ? w / total : 0.0f;
+    __syncwarp();
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int p = 0; p < parts; ++p) {
+      const float* src = reinterpret_cast<const float*>(smem) + p % KM_WARPS * (S::PART / 4) + r * KM_LD + lane * 4;
+      const float4 v = splits > 1 ? ld_cluster_f4(at(smem_u32(src), p)) : *reinterpret_cast<const float4*>(src);
+      const float wp = wts[p * ROWS + r];
+      acc.x += wp * v.x; acc.y += wp * v.y; acc.z += wp * v.z; acc.w += wp * v.w;
+    }
+    const int t = r / rep, h = hk * rep + r % rep;
+    *reinterpret_cast<uint2*>(out + (((long long)b * Tq + t) * Hq + h) * KM_D + lane * 4) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
+  }
+  if (splits > 1) cluster_sync_all();                                  // nobody leaves while its parts are read
+}
+
+template <int MT>
+cudaError_t launch_mt(const KvDev& c, const __nv_bfloat16* q, long long bs, long long ts, long long hs, int Tq, int Hq, float scale, int splits, __nv_bfloat16* out,
+                      cudaStream_t stream) {
+  const cudaError_t e = cudaFuncSetAttribute(kv_attention_mma_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, KmSmem<MT>::TOTAL);
+  if (e != cudaSuccess) return e;
+  return launch_overlapped(kv_attention_mma_kernel<MT>, dim3(splits, c.heads, c.batch), dim3(KM_THREADS), KmSmem<MT>::TOTAL, stream, splits > 1 ? splits : 0,
+                           c, q, bs, ts, hs, Tq, Hq, scale * 1.44269504089f, out);
+}
+}  // namespace
+
+// R = Tq * (Hq / heads) <= 32.  splits: CTAs per (sequence, kv head), at most 8 are used.
+cudaError_t launch_kv_attention_mma(const KvDev& c, const __nv_bfloat16* q, long long bs, long long ts, long long hs, int Tq, int Hq, float scale, int splits,
+                                    __nv_bfloat16* out, cudaStream_t stream) {
+  const int s = splits < KM_MAX_CLUSTER ? splits : KM_MAX_CLUSTER;
+  if (Tq * (Hq / c.heads) <= 16) return launch_mt<1>(c, q, bs, ts, hs, Tq, Hq, scale, s, out, stream);
+  return launch_mt<2>(c, q, bs, ts, hs, Tq, Hq, scale, s, out, stream);
+}
+}  // namespace cgk
+
+CGK_BOUNDS_READER(kv_attn_mma)

@@ -654,6 +654,19 @@ CGK_API int cgk_kv_int4_append_rows(const cgk_kv_args* a, const void* k_new, con
 CGK_API long long cgk_kv_int4_attention_scratch_floats(int batch, int Hq, int Tq, int D, int splits) {
   return (long long)batch * Hq * Tq * splits * (D + 2);
 }
+CGK_API int cgk_kv_int4_attention_few(const cgk_kv_args* a, int Tq, int Hq) {
+  return a && a->heads > 0 && a->D == 128 && a->group % 32 == 0 && Hq % a->heads == 0 && (long long)Tq * (Hq / a->heads) <= KV_FEW_ROWS;
+}
+// The few-row kernel over rows of q that lie bs, ts, hs elements apart (cgk_kv_int4_attention_few says whether it takes the call).
+CGK_API int cgk_kv_int4_attention_strided(const cgk_kv_args* a, const void* q, long long bs, long long ts, long long hs, void* out, int Tq, int Hq, float scale,
+                                          int splits, void* stream) {
+  if (int rc = check_kv(a, "cgk_kv_int4_attention")) return rc;
+  CGK_REQUIRE(q && out && Tq > 0 && splits > 0 && cgk_kv_int4_attention_few(a, Tq, Hq), "cgk_kv_int4_attention_strided: bad argument");
+  CGK_REQUIRE(((bs | ts | hs) & 7) == 0 && (((uintptr_t)q | (uintptr_t)a->k_pages) & 15) == 0 && ((uintptr_t)a->v_pages & 7) == 0 && ((uintptr_t)out & 7) == 0,
+              "cgk_kv_int4_attention_strided: misaligned rows");
+  CGK_CUDA_CHECK(launch_kv_attention_mma(kv_dev(a), (const __nv_bfloat16*)q, bs, ts, hs, Tq, Hq, scale, splits, (__nv_bfloat16*)out, (cudaStream_t)stream));
+  return 0;
+}
 // q, out: bf16 [batch, Tq, Hq, D]; the Tq newest tokens must already be in the cache (positions
 // lengths[b] .. lengths[b] + Tq - 1).  scratch: cgk_kv_int4_attention_scratch_floats floats.
 CGK_API int cgk_kv_int4_attention(const cgk_kv_args* a, const void* q, void* out, int Tq, int Hq, float scale, int splits, float* scratch, void* stream) {
@@ -667,6 +680,8 @@ CGK_API int cgk_kv_int4_attention(const cgk_kv_args* a, const void* q, void* out
   const dim3 grid(splits, a->heads, a->batch);
   const long long rows = (long long)a->batch * Hq * Tq;
   const int cblocks = (int)((rows * D + 255) / 256 < 1184 ? (rows * D + 255) / 256 : 1184);
+  if (cgk_kv_int4_attention_few(a, Tq, Hq) && (((uintptr_t)q | (uintptr_t)a->k_pages) & 15) == 0 && (((uintptr_t)a->v_pages | (uintptr_t)out) & 7) == 0)
+    return cgk_kv_int4_attention_strided(a, q, (long long)Tq * Hq * D, (long long)Hq * D, D, out, Tq, Hq, scale, splits, stream);
   if (D == 128 && a->group % 32 == 0) {
     // tensor-core path (kv_attn_tc.cu); the CUDA-core kernel below covers the other shapes
     int dev = 0;

@@ -333,6 +333,34 @@ def test_kv_append_of_strided_rows(D, group, Hk, T):
     _lib.assert_device_ok()
 
 
+# up to 32 query rows per kv head: one and two row tiles with rows that are padding, a history of less than a block, of blocks that cross pages,
+# of more blocks per warp than it holds pages for, more CTAs per head than blocks; rows read out of a packed projection
+@pytest.mark.parametrize("group,page,Hk,Hq,Tq,hist", [(32, 64, 2, 2, 1, 0), (32, 16, 2, 8, 1, 15), (64, 20, 1, 8, 2, 150), (128, 48, 3, 12, 5, 333), (32, 64, 1, 4, 8, 4999),
+                                                      (32, 64, 1, 17, 1, 2100), (64, 7, 2, 8, 8, 64)])
+def test_kv_attention_of_few_rows(group, page, Hk, Hq, Tq, hist):
+    torch.manual_seed(hist + Tq)
+    B, D, room = 2, 128, hist + 64
+    gpu = PagedKVCacheInt4(1, B, room, Hk, D, group, page_size=page, device=DEV)
+    cpu = PagedKVCacheInt4(1, B, room, Hk, D, group, page_size=page)
+    perm = torch.randperm(gpu.page_table.numel()).view_as(gpu.page_table).int()
+    gpu.page_table.copy_(perm); cpu.page_table.copy_(perm)
+    kn, vn = (torch.randn(B, Tq, Hk, D).bfloat16() for _ in range(2))
+    packed = torch.randn(B, Tq, Hq + 3, D).bfloat16()
+    k, v = (torch.randn(B, hist, Hk, D).bfloat16() for _ in range(2))
+    for c, d in ((gpu, DEV), (cpu, "cpu")):
+        if hist:
+            c.append(0, k.to(d), v.to(d))
+            c.commit(torch.tensor([hist, hist // 3], dtype=torch.int32, device=d))
+        c.append(0, kn.to(d), vn.to(d))
+    ref, q = cpu.attention(0, packed[:, :, 2:2 + Hq].float()), packed.to(DEV)[:, :, 2:2 + Hq]
+    for splits in (1, 3, 8, 0):
+        got = gpu.attention(0, q, splits=splits)
+        # K, V and P are rounded to bf16 (2^-9 each), the results as well
+        assert ((got.float().cpu() - ref).norm() / ref.norm()).item() < 2 ** -7
+        assert torch.equal(got, gpu.attention(0, q.contiguous(), splits=splits))
+    _lib.assert_device_ok()
+
+
 def test_kv_attention_long_history_many_key_blocks():
     torch.manual_seed(3)
     B, hist, Hk, Hq, D, Tq = 2, 700, 2, 8, 128, 5
