@@ -199,7 +199,7 @@ class PagedKVCacheInt4(PagedCache):
                 if q.stride(3) != 1 or any(s % 8 for s in q.stride()[:3]) or q.data_ptr() % 16:
                     q = q.contiguous()
                 if splits <= 0:
-                    splits = max(1, min(8, 296 // max(1, B * self.heads), (longest + 63) // 64))
+                    splits = max(1, min(4, 148 // max(1, B * self.heads), (longest + 127) // 128))
                 out = torch.empty(B, Tq, Hq, D, dtype=q.dtype, device=q.device)
                 _lib.check(L.cgk_kv_int4_attention_strided(ctypes.byref(a), q.data_ptr(), q.stride(0), q.stride(1), q.stride(2), out.data_ptr(), Tq, Hq, scale,
                                                            splits, _lib.stream_ptr()), "cgk_kv_int4_attention_strided")

@@ -1,20 +1,23 @@
 // Attention of few query rows over the paged INT4 KV cache (head_dim 128): decoding and the verify pass of speculative decoding.
 //
 // A kv head has R = Tq * (Hq / Hk) query rows, 4 for one new token and 20 for five with four query heads per kv head.  tcgen05 tiles
-// of 128 keys (kv_attn_tc.cu) spent 12 us per 128 keys on writing converted tiles to shared memory and on two hand-overs to the
-// MMA-issuing thread; here every warp works through its own blocks of 16 keys with mma.sync, from the nibbles to its part of the
+// of 128 keys (kv_attn_tc.cu) spent some 4 us per tile on writing the converted values to shared memory and on two hand-overs to the
+// MMA-issuing thread; here every warp works through its own blocks of 32 keys with mma.sync, from the nibbles to its part of the
 // result, and meets the others only at the end:
-//   * S[rows, 16 keys] = Q . K^T: lane (g, q) holds the 32 elements 32 q .. 32 q + 31 of keys g and g + 8, 16 bytes of nibbles each,
+//   * S[rows, 8 keys] = Q . K^T: lane (g, q) holds the 32 elements 32 q .. 32 q + 31 of key g, 16 bytes of nibbles,
 //     which are its fragments of eight MMAs; the elements' order in a word (0,4,1,5,2,6,3,7) is given to Q's fragments instead;
 //   * O[rows, 128] += P . V: the sums of S are the A fragments of P; lane (g, q) holds elements 16 g .. 16 g + 15 of keys 2 q, 2 q + 1,
 //     2 q + 8, 2 q + 9, and column g of the MMAs' eight columns j is element 16 g + j;
-//   * a lane copies (cp.async, a ring of four blocks) exactly what it converts; the pages of the next 32 blocks are held one by lane.
+//   * raw rows come by cp.async into a ring of the warp, two blocks ahead; where the next 32 groups of 16 keys start is held one by
+//     lane.  Scales come as one copy per key: with a copy per lane and scale the copies of a block (a tag per key and instruction)
+//     took as long as its arithmetic (16 sequences, one token: 15.7 us).
 // The parts (row maximum, sum, O) of the warps of a cluster of CTAs that share a (sequence, kv head) meet over distributed shared
 // memory, in the order of the ranks and warps.
 // Values are those of kv_attn_tc.cu: K and V as bf16(q * bf16(scale)), P rounded to bf16 before it is summed.
 //
-// 16 sequences of 641 tokens, 32 query and 8 kv heads, one new token: PLACE us (24.7 + 2.7 for the kernel that combined the splits before);
-// five: PLACE (37.4 + 5.2).  10.5 MB of cache are 1.6 us at HBM rate; the rest is start, the chain of a warp's five blocks and the merge.
+// 16 sequences of 641 tokens, 32 query and 8 kv heads, one new token: 11.1 us (24.7 + 2.7 for the kernel that combined the splits before);
+// five: 16.3 (37.4 + 5.2).  10.5 MB of cache are 1.6 us at HBM rate.  The rest is the chain lengths -> page -> keys at the start (3 us),
+// three blocks of some 1.5 us per warp (conversion and MMAs of two warps per scheduler), and the merge (1 us).
 #include <cuda_bf16.h>
 
 #include "host_common.h"
@@ -24,9 +27,10 @@
 namespace cgk {
 namespace {
 
-constexpr int KM_WARPS = 4, KM_THREADS = KM_WARPS * 32, KM_D = 128, KM_KB = 16, KM_STAGES = 4, KM_MAX_CLUSTER = 8;
-constexpr int KM_STAGE = 32 * (2 * 16 + 4 * 8 + 2 * 4 + 4 * 4);       // a warp's block: K, V, K scales, V scales, all by lane
-constexpr int KM_LD = KM_D + 4;                                       // row of a part: rows start in different banks
+constexpr int KM_WARPS = 8, KM_THREADS = KM_WARPS * 32, KM_D = 128, KM_NK = 2, KM_KB = 16 * KM_NK, KM_STAGES = 3, KM_MAX_CLUSTER = 32 / KM_WARPS;   // a lane per part
+// a warp's 16 keys: K by lane, V rows of 64 bytes (80 apart: the lanes of a load in different banks), four scales per key of K and of V
+constexpr int KM_V = 1024, KM_VLD = 80, KM_S = KM_V + 16 * KM_VLD, KM_GROUP = KM_S + 2 * 16 * 16, KM_STAGE = KM_NK * KM_GROUP;
+constexpr int KM_LD = 8 * 20 + 4;                                     // row of a part: eight pieces of 16 elements, 20 apart: no two lanes of a store share banks
 
 template <int MT>                                                      // 16-row tiles of Q
 struct KmSmem {
@@ -53,7 +57,7 @@ __device__ __forceinline__ void km_convert(uint32_t w, __nv_bfloat162 s2, uint32
 }
 
 template <int MT>
-__global__ void __launch_bounds__(KM_THREADS, 2)
+__global__ void __launch_bounds__(KM_THREADS, 1)
 kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long q_bs, long long q_ts, long long q_hs, int Tq, int Hq, float scale_log2,
                         __nv_bfloat16* __restrict__ out) {
   using S = KmSmem<MT>;
@@ -65,65 +69,72 @@ kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long 
   pdl_trigger();
   pdl_wait();
   const int len = c.lengths[b] + Tq;                                   // the Tq new tokens were appended before the call
+  // Q rows of this warp's tile (all warps: the only tile; else one warp per tile): asked for before the chain of page and keys
+  const bool loads_q = MT == 1 || warp < MT;
+  uint4 qr[2][4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = (MT == 1 ? 0 : warp * 16) + gq + 8 * h, t = r / rep;
+    const __nv_bfloat16* p = q + b * q_bs + t * q_ts + (hk * rep + r - t * rep) * q_hs + qq * 32;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) qr[h][w] = loads_q && r < R ? *reinterpret_cast<const uint4*>(p + w * 8) : make_uint4(0, 0, 0, 0);
+  }
   const int blocks = (len + KM_KB - 1) / KM_KB, stride = splits * KM_WARPS;
   const int first = rank * KM_WARPS + warp;                            // this warp's blocks of 16 keys: first, first + stride, ..
   const int mine = first < blocks ? (blocks - first + stride - 1) / stride : 0;
-  const bool one_page = c.page_size % KM_KB == 0;                      // a block never crosses pages
+  const bool one_page = c.page_size % 16 == 0;                         // 16 keys never cross pages
 
   const uint32_t ring = smem_u32(smem) + warp * (KM_STAGES * KM_STAGE);
-  int held = 0;                                                        // lane l: the page of block (next multiple of 32 blocks) + l
-  auto page_of = [&](int key) { return c.page_table[CGK_IDX(b * c.max_pages + key / c.page_size, c.batch * c.max_pages)]; };
+  auto token = [&](int key) {                                          // a key's place in the pool, in tokens
+    const int lp = key / c.page_size;
+    return c.page_table[CGK_IDX(b * c.max_pages + lp, c.batch * c.max_pages)] * c.page_size + key - lp * c.page_size;
+  };
+  const uint8_t* const k_src = c.k_pages + hk * (KM_D / 2) + qq * 16;
+  const uint8_t* const v_src = c.v_pages + hk * (KM_D / 2) + qq * 16;
+  const float* const s_src = (lane < 16 ? c.k_scales : c.v_scales) + hk * G;
+  const int row_bytes = c.heads * (KM_D / 2), row_scales = c.heads * G;
+  int held = 0;                                                        // lane l: where group (last multiple of 32) + l of 16 keys starts
   auto fetch = [&](int i) {
     if (i < mine) {
-      const int kb = (first + i * stride) * KM_KB;
-      if ((i & 31) == 0) {
-        const int j = i + lane;
-        held = one_page && j < mine ? page_of((first + j * stride) * KM_KB) : 0;
-      }
-      const int page = __shfl_sync(0xffffffffu, held, i & 31);
-      const long long base = (long long)page * c.page_size + kb % c.page_size;
-      auto token = [&](int k) -> long long {                           // key kb + k, inside the sequence
-        if (one_page) return (base + k) * c.heads + hk;
-        return ((long long)page_of(kb + k) * c.page_size + (kb + k) % c.page_size) * c.heads + hk;
-      };
-      const uint32_t dst = ring + (i % KM_STAGES) * KM_STAGE;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int k = gq + 8 * h;
-        const bool in = kb + k < len;
-        const long long t = in ? token(k) : 0;
-        cp_async_16_or_zero(dst + h * 512 + lane * 16, c.k_pages + t * (KM_D / 2) + qq * 16, in ? 16 : 0);
-        cp_async_or_zero<4>(dst + 2048 + h * 128 + lane * 4, c.k_scales + t * G + qq * 32 / c.group, in ? 4 : 0);
-      }
+      for (int n = 0; n < KM_NK; ++n) {
+        const int group = i * KM_NK + n, kb = (first + i * stride) * KM_KB + n * 16, left = len - kb;      // keys from here on
+        if (one_page && (group & 31) == 0) {
+          const int j = group + lane, key = (first + j / KM_NK * stride) * KM_KB + j % KM_NK * 16;
+          held = key < len ? token(key) : 0;
+        }
+        const int base = __shfl_sync(0xffffffffu, held, group & 31);
+        auto place = [&](int k) -> long long { return k >= left ? base : one_page ? base + k : token(kb + k); };   // beyond the end nothing is read
+        const uint32_t dst = ring + (i % KM_STAGES) * KM_STAGE + n * KM_GROUP;
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const int k = 2 * qq + (h & 1) + 8 * (h >> 1);
-        const bool in = kb + k < len;
-        const long long t = in ? token(k) : 0;
-        cp_async_or_zero<8>(dst + 1024 + h * 256 + lane * 8, c.v_pages + t * (KM_D / 2) + gq * 8, in ? 8 : 0);
-        cp_async_or_zero<4>(dst + 2304 + h * 128 + lane * 4, c.v_scales + t * G + gq * 16 / c.group, in ? 4 : 0);
+        for (int h = 0; h < 2; ++h) {
+          const int k = gq + 8 * h;
+          const long long t = place(k);
+          cp_async_16_or_zero(dst + h * 512 + lane * 16, k_src + t * row_bytes, k < left ? 16 : 0);
+          cp_async_16_or_zero(dst + KM_V + k * KM_VLD + qq * 16, v_src + t * row_bytes, k < left ? 16 : 0);
+        }
+        const int k = lane & 15;                                       // lanes 0-15: the scales of K, 16-31: of V
+        const float* src = s_src + place(k) * row_scales;
+        if (G == 4) cp_async_16_or_zero(dst + KM_S + lane * 16, src, k < left ? 16 : 0);
+        else if (G == 2) cp_async_or_zero<8>(dst + KM_S + lane * 16, src, k < left ? 8 : 0);
+        else cp_async_or_zero<4>(dst + KM_S + lane * 16, src, k < left ? 4 : 0);
       }
     }
     cp_async_commit();
   };
-#pragma unroll
+#pragma unroll 1
   for (int i = 0; i < KM_STAGES - 1; ++i) fetch(i);
 
-  // Q: fragment register 0 / 2 (row g) and 1 / 3 (row g + 8) of MMA 2 w and 2 w + 1 are elements 32 q + 8 w ..
+  // Fragment registers 0 / 2 (row g) and 1 / 3 (row g + 8) of MMAs 2 w and 2 w + 1 are elements 32 q + 8 w ..
   uint32_t qf[MT == 1 ? 8 : 1][4];
   uint4* const q_s = reinterpret_cast<uint4*>(smem + S::OFF_Q);
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt) {
-    if (MT > 1 && warp >= MT && mt == 0) break;
-    if (MT > 1 && warp != mt) continue;
+  if (loads_q) {
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       uint32_t p[2][4];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int r = mt * 16 + gq + 8 * h;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (r < R) v = *reinterpret_cast<const uint4*>(q + b * q_bs + r / rep * q_ts + (hk * rep + r % rep) * q_hs + qq * 32 + w * 8);
+        const uint4 v = qr[h][w];
         p[h][0] = __byte_perm(v.x, v.z, 0x5410); p[h][1] = __byte_perm(v.x, v.z, 0x7632);
         p[h][2] = __byte_perm(v.y, v.w, 0x5410); p[h][3] = __byte_perm(v.y, v.w, 0x7632);
       }
@@ -132,7 +143,7 @@ kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long 
         if constexpr (MT == 1) {
           qf[2 * w + s][0] = p[0][2 * s]; qf[2 * w + s][1] = p[1][2 * s]; qf[2 * w + s][2] = p[0][2 * s + 1]; qf[2 * w + s][3] = p[1][2 * s + 1];
         } else {
-          q_s[(mt * 8 + 2 * w + s) * 32 + lane] = make_uint4(p[0][2 * s], p[1][2 * s], p[0][2 * s + 1], p[1][2 * s + 1]);
+          q_s[(warp * 8 + 2 * w + s) * 32 + lane] = make_uint4(p[0][2 * s], p[1][2 * s], p[0][2 * s + 1], p[1][2 * s + 1]);
         }
       }
     }
@@ -154,23 +165,27 @@ kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long 
 #pragma unroll
       for (int e = 0; e < 4; ++e) o[mt][j][e] = 0.0f;
   }
+  const int k_group = qq * 32 / c.group, v_group = gq * 16 / c.group;
   uint32_t mask = 0x000F000Fu, magic = 0x43004300u;
   asm volatile("" : "+r"(mask), "+r"(magic));
 
   for (int i = 0; i < mine; ++i) {
     cp_async_wait<KM_STAGES - 2>();
+    __syncwarp();
     fetch(i + KM_STAGES - 1);
     const uint8_t* src = smem + warp * (KM_STAGES * KM_STAGE) + (i % KM_STAGES) * KM_STAGE;
     const int kb = (first + i * stride) * KM_KB;
-    float s[MT][2][4];
+    float s[MT][2 * KM_NK][4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {                                      // keys g and g + 8: the columns of two MMAs
+    for (int h = 0; h < 2 * KM_NK; ++h) {                              // keys 8 h + g: the columns of an MMA
+      float odd[MT][4];                                                // two chains of four MMAs instead of one of eight
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[mt][h][e] = 0.0f;
-      const uint4 raw = *reinterpret_cast<const uint4*>(src + h * 512 + lane * 16);
-      const __nv_bfloat162 s2 = __float2bfloat162_rn(*reinterpret_cast<const float*>(src + 2048 + h * 128 + lane * 4));
+        for (int e = 0; e < 4; ++e) s[mt][h][e] = odd[mt][e] = 0.0f;
+      const uint8_t* group = src + h / 2 * KM_GROUP;
+      const uint4 raw = *reinterpret_cast<const uint4*>(group + h % 2 * 512 + lane * 16);
+      const __nv_bfloat162 s2 = __float2bfloat162_rn(*reinterpret_cast<const float*>(group + KM_S + (h % 2 * 8 + gq) * 16 + k_group * 4));
       const uint32_t w4[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
@@ -181,67 +196,79 @@ kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long 
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             if constexpr (MT == 1) {
-              mma_bf16(s[0][h], qf[2 * w + t][0], qf[2 * w + t][1], qf[2 * w + t][2], qf[2 * w + t][3], k[2 * t], k[2 * t + 1]);
+              mma_bf16(t ? odd[0] : s[0][h], qf[2 * w + t][0], qf[2 * w + t][1], qf[2 * w + t][2], qf[2 * w + t][3], k[2 * t], k[2 * t + 1]);
             } else {
               const uint4 a = q_s[(mt * 8 + 2 * w + t) * 32 + lane];
-              mma_bf16(s[mt][h], a.x, a.y, a.z, a.w, k[2 * t], k[2 * t + 1]);
+              mma_bf16(t ? odd[mt] : s[mt][h], a.x, a.y, a.z, a.w, k[2 * t], k[2 * t + 1]);
             }
           }
       }
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[mt][h][e] += odd[mt][e];
     }
-    uint32_t p[MT][4];
+    uint32_t p[MT][KM_NK][4];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {                                    // rows g and g + 8; values 2 h, 2 h + 1 of both tiles
-        float x[4];
+      for (int h = 0; h < 2; ++h) {                                    // rows g and g + 8; values 2 h, 2 h + 1 of all tiles
+        float x[4 * KM_NK], mx = -INFINITY;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
+        for (int e = 0; e < 4 * KM_NK; ++e) {
           const int key = kb + (e >> 1) * 8 + 2 * qq + (e & 1);
           x[e] = key <= last[mt][h] ? s[mt][e >> 1][2 * h + (e & 1)] * scale_log2 : -INFINITY;
+          mx = fmaxf(mx, x[e]);
         }
-        float mx = fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         const float mo = m[mt][h], mn = fmaxf(mo, mx);
         if (__any_sync(0xffffffffu, mn > mo)) {
-          const float corr = mo > -INFINITY ? fast_exp2(mo - mn) : (mn > -INFINITY ? 0.0f : 1.0f);
+          const float corr = mo > -INFINITY ? fast_exp2(mo - mn) : 1.0f;       // nothing summed yet: nothing to rescale
           l[mt][h] *= corr;
           m[mt][h] = mn;
 #pragma unroll
           for (int j = 0; j < 16; ++j) { o[mt][j][2 * h] *= corr; o[mt][j][2 * h + 1] *= corr; }
         }
-        float e4[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) e4[e] = x[e] > -INFINITY ? fast_exp2(x[e] - mn) : 0.0f;
-        const uint32_t lo = pack_bf16x2(e4[0], e4[1]), hi = pack_bf16x2(e4[2], e4[3]);
-        const float2 a = unpack_bf16x2(lo), d = unpack_bf16x2(hi);
-        l[mt][h] += (a.x + a.y) + (d.x + d.y);
-        p[mt][h] = lo;                                                 // A registers 0 / 1: keys 2 q, 2 q + 1
-        p[mt][2 + h] = hi;                                             // 2 / 3: eight more
+        for (int n = 0; n < KM_NK; ++n) {
+          float e4[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) e4[e] = x[4 * n + e] > -INFINITY ? fast_exp2(x[4 * n + e] - mn) : 0.0f;
+          const uint32_t lo = pack_bf16x2(e4[0], e4[1]), hi = pack_bf16x2(e4[2], e4[3]);
+          const float2 a = unpack_bf16x2(lo), d = unpack_bf16x2(hi);
+          l[mt][h] += (a.x + a.y) + (d.x + d.y);
+          p[mt][n][h] = lo;                                            // A registers 0 / 1: keys 2 q, 2 q + 1
+          p[mt][n][2 + h] = hi;                                        // 2 / 3: eight more
+        }
       }
     }
     // V: two words (elements 16 g .. 16 g + 7, 8 more) of each of four keys
-    uint2 raw[4];
-    __nv_bfloat162 s2[4];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      raw[h] = *reinterpret_cast<const uint2*>(src + 1024 + h * 256 + lane * 8);
-      s2[h] = __float2bfloat162_rn(*reinterpret_cast<const float*>(src + 2304 + h * 128 + lane * 4));
-    }
+    for (int n = 0; n < KM_NK; ++n) {
+      const uint8_t* group = src + n * KM_GROUP;
+      uint2 raw[4];
+      __nv_bfloat162 s2[4];
 #pragma unroll
-    for (int w = 0; w < 2; ++w) {
-      uint32_t v[4][4];
+      for (int h = 0; h < 4; ++h) {
+        const int k = 2 * qq + (h & 1) + 8 * (h >> 1);
+        raw[h] = *reinterpret_cast<const uint2*>(group + KM_V + k * KM_VLD + gq * 8);
+        s2[h] = __float2bfloat162_rn(*reinterpret_cast<const float*>(group + KM_S + 256 + k * 16 + v_group * 4));
+      }
 #pragma unroll
-      for (int h = 0; h < 4; ++h) km_convert(w ? raw[h].y : raw[h].x, s2[h], mask, magic, v[h]);
+      for (int w = 0; w < 2; ++w) {
+        uint32_t v[4][4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {                                    // elements 8 w + j (low halves) and 8 w + 4 + j (high halves)
-        const uint32_t b0 = __byte_perm(v[0][j], v[1][j], 0x5410), b1 = __byte_perm(v[2][j], v[3][j], 0x5410);
-        const uint32_t c0 = __byte_perm(v[0][j], v[1][j], 0x7632), c1 = __byte_perm(v[2][j], v[3][j], 0x7632);
+        for (int h = 0; h < 4; ++h) km_convert(w ? raw[h].y : raw[h].x, s2[h], mask, magic, v[h]);
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          mma_bf16(o[mt][8 * w + j], p[mt][0], p[mt][1], p[mt][2], p[mt][3], b0, b1);
-          mma_bf16(o[mt][8 * w + 4 + j], p[mt][0], p[mt][1], p[mt][2], p[mt][3], c0, c1);
+        for (int j = 0; j < 4; ++j) {                                  // elements 8 w + j (low halves) and 8 w + 4 + j (high halves)
+          const uint32_t b0 = __byte_perm(v[0][j], v[1][j], 0x5410), b1 = __byte_perm(v[2][j], v[3][j], 0x5410);
+          const uint32_t c0 = __byte_perm(v[0][j], v[1][j], 0x7632), c1 = __byte_perm(v[2][j], v[3][j], 0x7632);
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            mma_bf16(o[mt][8 * w + j], p[mt][n][0], p[mt][n][1], p[mt][n][2], p[mt][n][3], b0, b1);
+            mma_bf16(o[mt][8 * w + 4 + j], p[mt][n][0], p[mt][n][1], p[mt][n][2], p[mt][n][3], c0, c1);
+          }
         }
       }
     }
@@ -264,7 +291,7 @@ kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long 
       for (int col = 0; col < 2; ++col)
 #pragma unroll
         for (int j = 0; j < 16; j += 4)
-          *reinterpret_cast<float4*>(part + r * KM_LD + 16 * (2 * qq + col) + j) =
+          *reinterpret_cast<float4*>(part + r * KM_LD + 20 * (2 * qq + col) + j) =
               make_float4(o[mt][j][2 * h + col], o[mt][j + 1][2 * h + col], o[mt][j + 2][2 * h + col], o[mt][j + 3][2 * h + col]);
     }
   if (splits > 1) cluster_sync_all();
@@ -284,8 +311,9 @@ kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long 
     if (lane < parts) wts[lane * ROWS + r] = total > 0.0f ? w / total : 0.0f;
     __syncwarp();
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 8
     for (int p = 0; p < parts; ++p) {
-      const float* src = reinterpret_cast<const float*>(smem) + p % KM_WARPS * (S::PART / 4) + r * KM_LD + lane * 4;
+      const float* src = reinterpret_cast<const float*>(smem) + p % KM_WARPS * (S::PART / 4) + r * KM_LD + (lane >> 2) * 20 + (lane & 3) * 4;
       const float4 v = splits > 1 ? ld_cluster_f4(at(smem_u32(src), p)) : *reinterpret_cast<const float4*>(src);
       const float wp = wts[p * ROWS + r];
       acc.x += wp * v.x; acc.y += wp * v.y; acc.z += wp * v.z; acc.w += wp * v.w;
@@ -306,7 +334,7 @@ cudaError_t launch_mt(const KvDev& c, const __nv_bfloat16* q, long long bs, long
 }
 }  // namespace
 
-// R = Tq * (Hq / heads) <= 32.  splits: CTAs per (sequence, kv head), at most 8 are used.
+// R = Tq * (Hq / heads) <= 32.  splits: CTAs per (sequence, kv head), at most four are used.
 cudaError_t launch_kv_attention_mma(const KvDev& c, const __nv_bfloat16* q, long long bs, long long ts, long long hs, int Tq, int Hq, float scale, int splits,
                                     __nv_bfloat16* out, cudaStream_t stream) {
   const int s = splits < KM_MAX_CLUSTER ? splits : KM_MAX_CLUSTER;
