@@ -385,6 +385,8 @@ __global__ void swiglu_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, lo
 template <int ACT>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_rows_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long long ldo, long long rows, int H) {
+  pdl_trigger();
+  pdl_wait();
   swiglu_rows_bf16<ACT>(x, y, ldo, rows, H);
 }
 template <typename T>
@@ -770,7 +772,7 @@ static int launch_gated(int dtype, const void* x, void* y, long long ldo, long l
   typedef __nv_bfloat16 bf;
   if (dtype == 0) swiglu_fwd_kernel<float, ACT><<<ew_grid(rows * H), 256, 0, st>>>((const float*)x, (float*)y, ldo, rows, H);
   else if (H % 8 == 0 && ldo % 8 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0)
-    swiglu_fwd_rows_kernel<ACT><<<swiglu_rows_grid(rows, H), swiglu_rows_threads(H), 0, st>>>((const bf*)x, (bf*)y, ldo, rows, H);
+    CGK_CUDA_CHECK(launch_overlapped(swiglu_fwd_rows_kernel<ACT>, swiglu_rows_grid(rows, H), dim3(swiglu_rows_threads(H)), 0, st, 0, (const bf*)x, (bf*)y, ldo, rows, H));
   else swiglu_fwd_kernel<bf, ACT><<<ew_grid(rows * H), 256, 0, st>>>((const bf*)x, (bf*)y, ldo, rows, H);
   CGK_LAUNCH_CHECK();
   return 0;

@@ -135,9 +135,13 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
     mbar_fence_init();
   }
   if (warp == 2) { tmem_alloc(smem_u32(tmem_slot), 2 * BN); tmem_relinquish(); }
+  // the first weights (no earlier kernel's business) start on their way to L2 while the predecessor still runs
+  if (warp == 0 && blockIdx.y == 0 && lane < min(ksteps, 14)) prefetch_l2(g.w_tiles + (long long)line(lane) * (SUB * RAW_BYTES), SUB * RAW_BYTES);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();
+  pdl_wait();
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
@@ -415,8 +419,7 @@ CGK_API int cgk_int4_gemm_parts(const void* x, long long ldx, const void* w_tile
   }
   Int4Dev g{(const uint8_t*)w_tiles, (float4*)parts, counters, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)bias, M, N, K,
             a_rows, a_stages, raw_stages, (int)d.sharers, device_status(dev)};
-  int4_gemm_kernel<<<dim3((unsigned)d.ctas, m_tiles), THREADS, SMEM_BYTES, (cudaStream_t)stream>>>(tmX, g);
-  CGK_LAUNCH_CHECK();
+  CGK_CUDA_CHECK(launch_overlapped(int4_gemm_kernel, dim3((unsigned)d.ctas, m_tiles), dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, 0, tmX, g));
   return 0;
 }
 

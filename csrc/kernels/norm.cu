@@ -45,6 +45,8 @@ norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ residu
                 float eps) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = D >> 3;  // uint4 vectors per row
+  pdl_trigger();
+  pdl_wait();
   for (long long row = (long long)blockIdx.x * NORM_WARPS + warp; row < rows;
        row += (long long)gridDim.x * NORM_WARPS) {
     const uint4* xp = reinterpret_cast<const uint4*>(x + row * D);
@@ -142,6 +144,8 @@ norm_fwd_wide_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ r
   float f[8], g[8], b[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) f[j] = g[j] = b[j] = 0.0f;
+  pdl_trigger();
+  pdl_wait();
   if (in) {
     uint4 a = reinterpret_cast<const uint4*>(x + row * D)[c];
     unpack8(__ldg(reinterpret_cast<const uint4*>(gamma) + c), g);
@@ -612,9 +616,9 @@ CGK_API int cgk_norm_forward(const void* x, const void* residual, const void* ga
   CGK_CUDA_CHECK(cudaGetDevice(&dev));
   if (D > NORM_WIDE && rows <= sm_count(dev) * NORM_WIDE_ROWS_PER_SM) {
     const auto kernel = rms ? norm_fwd_wide_kernel<true> : norm_fwd_wide_kernel<false>;
-    kernel<<<rows, wide_threads(D), 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)gamma,
-                                             rms ? nullptr : (const __nv_bfloat16*)beta, (__nv_bfloat16*)y, (__nv_bfloat16*)sum_out, mean, rstd, D, eps);
-    CGK_LAUNCH_CHECK();
+    CGK_CUDA_CHECK(launch_overlapped(kernel, dim3(rows), dim3(wide_threads(D)), 0, st, 0, (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual,
+                                     (const __nv_bfloat16*)gamma, rms ? nullptr : (const __nv_bfloat16*)beta, (__nv_bfloat16*)y, (__nv_bfloat16*)sum_out,
+                                     mean, rstd, D, eps));
     return 0;
   }
   int grid = (rows + NORM_WARPS - 1) / NORM_WARPS;
@@ -622,15 +626,10 @@ CGK_API int cgk_norm_forward(const void* x, const void* residual, const void* ga
   if (grid > cap) grid = cap;
   const int need = (D / 8 + 31) / 32;
 #define LAUNCH(MAXV)                                                                          \
-  if (rms)                                                                                    \
-    norm_fwd_kernel<MAXV, true><<<grid, NORM_WARPS * 32, 0, st>>>(                            \
+  CGK_CUDA_CHECK(launch_overlapped(rms ? norm_fwd_kernel<MAXV, true> : norm_fwd_kernel<MAXV, false>, dim3(grid), dim3(NORM_WARPS * 32), 0, st, 0,     \
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)gamma, \
-        nullptr, (__nv_bfloat16*)y, (__nv_bfloat16*)sum_out, mean, rstd, rows, D, eps);       \
-  else                                                                                        \
-    norm_fwd_kernel<MAXV, false><<<grid, NORM_WARPS * 32, 0, st>>>(                           \
-        (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)gamma, \
-        (const __nv_bfloat16*)beta, (__nv_bfloat16*)y, (__nv_bfloat16*)sum_out, mean, rstd,   \
-        rows, D, eps);
+        rms ? nullptr : (const __nv_bfloat16*)beta, (__nv_bfloat16*)y, (__nv_bfloat16*)sum_out, mean, rstd, \
+        rows, D, eps));
   if (need <= 1) { LAUNCH(1) }
   else if (need <= 2) { LAUNCH(2) }
   else if (need <= 4) { LAUNCH(4) }

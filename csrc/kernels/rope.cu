@@ -67,6 +67,8 @@ __global__ void __launch_bounds__(256)
 rope_apply_vec_kernel(__nv_bfloat16* x, const float* __restrict__ cos_t, const float* __restrict__ sin_t, const int* __restrict__ positions,
                       int units, int Tn, int H, int half, long long bs, long long ts, long long hs, int pos_offset, int max_seq, float sign) {
   const int u = blockIdx.x * 256 + threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (u >= units) return;
   const int upr = half >> 3, row = u / upr, j = (u - row * upr) * 8, bt = row / H, h = row - bt * H, b = bt / Tn, t = bt - b * Tn;
   int pos = positions ? positions[bt] : pos_offset + t;
@@ -122,9 +124,8 @@ CGK_API int cgk_rope_apply(int dtype, void* x, const float* cos_t, const float* 
   const float sign = backward ? -1.0f : 1.0f;
   if (dtype != 0 && D % 16 == 0 && ((bs | ts | hs) & 7) == 0 && n / 8 <= 0x7fffff00LL &&
       (((uintptr_t)x | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15) == 0) {
-    rope_apply_vec_kernel<<<(unsigned)((n / 8 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-        (__nv_bfloat16*)x, cos_t, sin_t, positions, (int)(n / 8), T, H, D / 2, bs, ts, hs, pos_offset, max_seq, sign);
-    CGK_LAUNCH_CHECK();
+    CGK_CUDA_CHECK(launch_overlapped(rope_apply_vec_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, 0,
+                                     (__nv_bfloat16*)x, cos_t, sin_t, positions, (int)(n / 8), T, H, D / 2, bs, ts, hs, pos_offset, max_seq, sign));
     return 0;
   }
   if (dtype == 0)

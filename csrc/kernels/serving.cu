@@ -133,6 +133,8 @@ struct KvRows { const __nv_bfloat16* src[2]; __nv_bfloat16* out[2]; long long bs
 __global__ void __launch_bounds__(256)
 kv_append_rows_kernel(KvDev c, const KvRows r, int T, int group_lanes, int* status) {
   const int which = blockIdx.y, upr = c.D >> 3;                       // units of eight elements per row
+  pdl_trigger();
+  pdl_wait();
   const long long units = (long long)c.batch * T * c.heads * upr;
   const long long u = (long long)blockIdx.x * 256 + threadIdx.x;
   const bool in = u < units;
@@ -647,8 +649,8 @@ CGK_API int cgk_kv_int4_append_rows(const cgk_kv_args* a, const void* k_new, con
   CGK_CUDA_CHECK(cudaGetDevice(&dev));
   const long long units = (long long)a->batch * T * a->heads * (a->D / 8);
   const KvRows r{{(const __nv_bfloat16*)k_new, (const __nv_bfloat16*)v_new}, {(__nv_bfloat16*)k_out, (__nv_bfloat16*)v_out}, bs, ts, hs};
-  kv_append_rows_kernel<<<dim3((unsigned)((units + 255) / 256), 2), 256, 0, (cudaStream_t)stream>>>(kv_dev(a), r, T, gl, device_status(dev));
-  CGK_LAUNCH_CHECK();
+  CGK_CUDA_CHECK(launch_overlapped(kv_append_rows_kernel, dim3((unsigned)((units + 255) / 256), 2), dim3(256), 0, (cudaStream_t)stream, 0, kv_dev(a), r, T, gl,
+                                   device_status(dev)));
   return 0;
 }
 CGK_API long long cgk_kv_int4_attention_scratch_floats(int batch, int Hq, int Tq, int D, int splits) {
