@@ -21,6 +21,7 @@ constexpr int FEW_SMEM = 1024 + FEW_RING + 256;
 struct FewDev {
   int a_rows, stages;                            // rows of A per stage (multiple of 8), depth of the rings
   int vec4;                                      // the output takes four elements per store
+  const __nv_bfloat16* b; long long ldb, strideB;
 };
 
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t mapped) {
@@ -93,10 +94,18 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     tmem_alloc(smem_u32(tmem_holder), BN);
     tmem_relinquish();
   }
+  // B is a weight matrix where few rows meet it: this CTA's part of it (as much as its rings hold) starts on its way to L2 while the
+  // predecessor still runs.  A prefetch has no result, so it does not matter who wrote the operand.
+  if (warp >= 4 && !g.b_mn) {
+    const int row = n0 + (int)threadIdx.x - 128, k = kb0 * BK, len = min(g.K, min(kb1, kb0 + FEW_MAX_STAGES) * BK) - k;
+    if (row < min(g.N, n0 + BN) && len >= 8) prefetch_l2(f.b + b * f.strideB + (long long)row * f.ldb + k, (uint32_t)(len / 8 * 16));
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_holder;
+  pdl_trigger();
+  pdl_wait();
 
   if (warp == 0) {
     if (elect_one()) {
@@ -194,23 +203,13 @@ int launch(const cgk_gemm_args& a, GemmDev g, int S, cudaStream_t stream) {
   const int stage = f.a_rows * 128 + BN * 128;
   f.stages = FEW_RING / stage < FEW_MAX_STAGES ? FEW_RING / stage : FEW_MAX_STAGES;
   const uintptr_t out = (uintptr_t)a.out;
+  f.b = (const __nv_bfloat16*)a.B; f.ldb = a.ldb; f.strideB = a.strideB;
   f.vec4 = a.ldc % 4 == 0 && (a.batch == 1 || a.strideC % 4 == 0) && (out & (a.out_fp32 ? 15 : 7)) == 0;
   CUtensorMap tmA, tmB;
   int rc = make_gemm_tmaps(a, BN, &tmA, &tmB, f.a_rows);
   if (rc) return rc;
   CGK_CUDA_CHECK(cudaFuncSetAttribute(gemm_few_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(g.batch * g.tiles_m * g.tiles_n * S));
-  cfg.blockDim = dim3(FEW_THREADS);
-  cfg.dynamicSmemBytes = FEW_SMEM;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr = {};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = S;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  CGK_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_few_kernel<BN>, tmA, tmB, g, f));
+  CGK_CUDA_CHECK(launch_overlapped(gemm_few_kernel<BN>, dim3((unsigned)(g.batch * g.tiles_m * g.tiles_n * S)), dim3(FEW_THREADS), FEW_SMEM, stream, S, tmA, tmB, g, f));
   return 0;
 }
 

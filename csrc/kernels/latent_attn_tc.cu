@@ -88,6 +88,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_pages, const Latent
   const int split = blockIdx.x % a.splits, h0 = (int)(blockIdx.x / a.splits) * NP;
   const long long t = blockIdx.y;
   const int nh = min(NP, c.heads - h0);
+  pdl_wait();
   const int len = (int)CGK_IDX(c.pos[t], (long long)c.max_pages * c.page_size) + 1;
   const int per = ((len + a.splits - 1) / a.splits + LT_KB - 1) / LT_KB * LT_KB;
   const int k_begin = split * per, k_end = min(len, k_begin + per);
@@ -132,6 +133,7 @@ latent_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_pages, const Latent
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 8) {
@@ -348,8 +350,7 @@ int launch_np(const CUtensorMap& tm, const LatentTcDev& a, int rows, cudaStream_
   const uint32_t smem = LtSmem<NP>::total(a.slots_c, a.ns);
   CGK_CUDA_CHECK(cudaFuncSetAttribute(latent_attn_tc_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const dim3 grid(a.splits * ((a.c.heads + NP - 1) / NP), rows);
-  latent_attn_tc_kernel<NP><<<grid, LT_THREADS, smem, st>>>(tm, a);
-  CGK_LAUNCH_CHECK();
+  CGK_CUDA_CHECK(launch_overlapped(latent_attn_tc_kernel<NP>, grid, dim3(LT_THREADS), smem, st, 0, tm, a));
   return 0;
 }
 

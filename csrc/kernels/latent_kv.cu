@@ -27,6 +27,8 @@ latent_norm_append_kernel(const TI* __restrict__ in, long long ld, const float* 
   __shared__ float red[64];
   const long long t = blockIdx.x;
   const int n = q_rank + R, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  pdl_trigger();
+  pdl_wait();
   const int p = (int)CGK_IDX(pos[t], (long long)max_pages * page_size), s = (int)CGK_IDX(slot[t], slots);
   const long long page = CGK_IDX(page_table[(long long)s * max_pages + p / page_size], n_pages);
   float sq = 0.0f, sc = 0.0f;
@@ -144,6 +146,8 @@ __global__ void latent_merge_kernel(const float* __restrict__ part, const float*
   const long long row = blockIdx.x;
   const int lane = threadIdx.x & 31, r = blockIdx.y * blockDim.x + threadIdx.x;
   const float* p = part + row * splits * R + r;
+  pdl_trigger();
+  pdl_wait();
   float e[16];                                       // the first ranges' sums travel while the weights are worked out
 #pragma unroll
   for (int s = 0; s < 16; ++s) e[s] = (s < splits && r < R) ? p[(long long)s * R] : 0.0f;
@@ -197,8 +201,7 @@ int fill_latent(const cgk_latent_args& a, LatentDev* d) {
 }  // namespace
 
 cudaError_t launch_latent_merge(const float* part, const float* ml, __nv_bfloat16* out, int rows, int splits, int R, cudaStream_t st) {
-  latent_merge_kernel<<<dim3(rows, (R + 127) / 128), 128, 0, st>>>(part, ml, out, splits, R);
-  return cudaGetLastError();
+  return launch_overlapped(latent_merge_kernel, dim3(rows, (R + 127) / 128), dim3(128), 0, st, 0, part, ml, out, splits, R);
 }
 
 }  // namespace cgk
@@ -222,13 +225,13 @@ CGK_API int cgk_latent_norm_append(const cgk_latent_args* pa, const void* in, in
 #define CGK_LNA(TI, T)                                                                                                              \
   do {                                                                                                                             \
     if (vec)                                                                                                                       \
-      latent_norm_append_kernel<TI, T, 4><<<rows, nt, smem, st>>>((const TI*)in, ld, (const float*)wq, (const float*)wc, q_rank,   \
-                                                                  d.R, eps, (T*)cq, (T*)c_out, (T*)d.pages, d.slot, d.pos,         \
-                                                                  d.page_table, d.slots, d.max_pages, d.page_size, d.n_pages);     \
+      CGK_CUDA_CHECK(launch_overlapped(latent_norm_append_kernel<TI, T, 4>, dim3(rows), dim3(nt), smem, st, 0, (const TI*)in, ld,       \
+                                       (const float*)wq, (const float*)wc, q_rank, d.R, eps, (T*)cq, (T*)c_out, (T*)d.pages, d.slot,   \
+                                       d.pos, d.page_table, d.slots, d.max_pages, d.page_size, d.n_pages));                           \
     else                                                                                                                           \
-      latent_norm_append_kernel<TI, T, 1><<<rows, nt, smem, st>>>((const TI*)in, ld, (const float*)wq, (const float*)wc, q_rank,   \
-                                                                  d.R, eps, (T*)cq, (T*)c_out, (T*)d.pages, d.slot, d.pos,         \
-                                                                  d.page_table, d.slots, d.max_pages, d.page_size, d.n_pages);     \
+      CGK_CUDA_CHECK(launch_overlapped(latent_norm_append_kernel<TI, T, 1>, dim3(rows), dim3(nt), smem, st, 0, (const TI*)in, ld,       \
+                                       (const float*)wq, (const float*)wc, q_rank, d.R, eps, (T*)cq, (T*)c_out, (T*)d.pages, d.slot,   \
+                                       d.pos, d.page_table, d.slots, d.max_pages, d.page_size, d.n_pages));                           \
   } while (0)
   if (pa->fp32) {
     CGK_REQUIRE(in_fp32, "cgk_latent_norm_append: the fp32 form takes fp32 inputs");

@@ -20,6 +20,8 @@ __global__ void embed_sinusoid_kernel(const long long* __restrict__ ids, const i
                                       float scale, const double* __restrict__ freq, float* __restrict__ x,
                                       TH* __restrict__ h, int D, int vocab) {
   const long long row = blockIdx.x;
+  pdl_trigger();
+  pdl_wait();
   const long long id = CGK_IDX(ids[row], vocab);
   const double p = (double)pos[row];
   const int pairs = (D + 1) / 2;
@@ -126,6 +128,8 @@ __global__ void __launch_bounds__(512)
 stream_update_regs_kernel(const UpdateDev a) {
   __shared__ float red[16];
   const long long t = blockIdx.x;
+  pdl_trigger();
+  pdl_wait();
   const TY* y = reinterpret_cast<const TY*>(a.y);
   const TP* pairs = reinterpret_cast<const TP*>(a.pairs);
   float* x = a.x + t * a.D;
@@ -204,6 +208,8 @@ stream_norms_kernel(const NormsDev a) {
   extern __shared__ float row_buf[];
   __shared__ float red[33];
   const long long t = blockIdx.x;
+  pdl_trigger();
+  pdl_wait();
   float* x = a.x + t * a.D;
   const TE* e = a.ids ? reinterpret_cast<const TE*>(a.table) + CGK_IDX(a.ids[t], a.vocab) * a.D : nullptr;
   const TY* y = reinterpret_cast<const TY*>(a.y) + t * a.ldy;
@@ -280,6 +286,8 @@ __global__ void rms_rows_kernel(const float* __restrict__ x, const long long* __
                                 TO* __restrict__ out, int D, float eps) {
   __shared__ float red[33];
   const long long i = blockIdx.x;
+  pdl_trigger();
+  pdl_wait();
   const float* xr = x + CGK_IDX(rows ? rows[i] : i, n_rows) * D;
   float ss = 0.0f;
   for (int c = threadIdx.x; c < D; c += blockDim.x) ss = fmaf(xr[c], xr[c], ss);
@@ -297,10 +305,8 @@ int launch_update(const UpdateDev& d, int rows, bool vec, cudaStream_t st) {
   if (d.D % 8 == 0 && d.D <= 512 * 8 * 4 && a16(d.y, d.ldy * sizeof(TY)) && a16(d.pairs, d.ldp * sizeof(TP)) && a16(d.x, 0) && a16(d.w, 0) &&
       a16(d.h, 0)) {
     const int vecs = d.D / 8, iter = vecs <= 512 ? 1 : (vecs <= 1024 ? 2 : 4), nt = ((vecs + iter - 1) / iter + 31) / 32 * 32;
-    if (iter == 1) stream_update_regs_kernel<TY, TP, TH, 1><<<rows, nt, 0, st>>>(d);
-    else if (iter == 2) stream_update_regs_kernel<TY, TP, TH, 2><<<rows, nt, 0, st>>>(d);
-    else stream_update_regs_kernel<TY, TP, TH, 4><<<rows, nt, 0, st>>>(d);
-    CGK_LAUNCH_CHECK();
+    const auto kernel = iter == 1 ? stream_update_regs_kernel<TY, TP, TH, 1> : iter == 2 ? stream_update_regs_kernel<TY, TP, TH, 2> : stream_update_regs_kernel<TY, TP, TH, 4>;
+    CGK_CUDA_CHECK(launch_overlapped(kernel, dim3(rows), dim3(nt), 0, st, 0, d));
     return 0;
   }
   const int smem = d.D * 4;
@@ -322,9 +328,8 @@ template <typename TE, typename TY, typename TH>
 int launch_norms(const NormsDev& d, int rows, bool vec, cudaStream_t st) {
   if (vec && d.D <= 512 * 8 * 4) {
     const int vecs = d.D / 8, iter = vecs <= 512 ? 1 : (vecs <= 1024 ? 2 : 4), nt = ((vecs + iter - 1) / iter + 31) / 32 * 32;
-    if (iter == 1) stream_norms_kernel<TE, TY, TH, 8, 1><<<rows, nt, 0, st>>>(d);
-    else if (iter == 2) stream_norms_kernel<TE, TY, TH, 8, 2><<<rows, nt, 0, st>>>(d);
-    else stream_norms_kernel<TE, TY, TH, 8, 4><<<rows, nt, 0, st>>>(d);
+    const auto kernel = iter == 1 ? stream_norms_kernel<TE, TY, TH, 8, 1> : iter == 2 ? stream_norms_kernel<TE, TY, TH, 8, 2> : stream_norms_kernel<TE, TY, TH, 8, 4>;
+    CGK_CUDA_CHECK(launch_overlapped(kernel, dim3(rows), dim3(nt), 0, st, 0, d));
   } else {
     const int smem = d.D * 4;
     if (smem > 48 * 1024)
@@ -379,10 +384,10 @@ CGK_API int cgk_embed_sinusoid(const void* ids, const void* pos, const void* tab
   const int* p = (const int*)pos;
   const double* f = (const double*)freq;
   if (table_fp32 && h_fp32)
-    embed_sinusoid_kernel<float, float><<<rows, nt, 0, st>>>(i, p, (const float*)table, scale, f, (float*)x, (float*)h, D, vocab);
+    CGK_CUDA_CHECK(launch_overlapped(embed_sinusoid_kernel<float, float>, dim3(rows), dim3(nt), 0, st, 0, i, p, (const float*)table, scale, f, (float*)x, (float*)h, D, vocab));
   else if (!table_fp32 && !h_fp32)
-    embed_sinusoid_kernel<__nv_bfloat16, __nv_bfloat16><<<rows, nt, 0, st>>>(i, p, (const __nv_bfloat16*)table, scale, f, (float*)x,
-                                                                             (__nv_bfloat16*)h, D, vocab);
+    CGK_CUDA_CHECK(launch_overlapped(embed_sinusoid_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(rows), dim3(nt), 0, st, 0, i, p, (const __nv_bfloat16*)table, scale, f,
+                                     (float*)x, (__nv_bfloat16*)h, D, vocab));
   else
     CGK_REQUIRE(false, "cgk_embed_sinusoid: table and operand copy must have one type");
   CGK_LAUNCH_CHECK();
@@ -420,10 +425,10 @@ CGK_API int cgk_rms_rows(const void* x, const void* rows, int n_out, int n_rows,
   cudaStream_t st = (cudaStream_t)stream;
   const int nt = row_threads(D);
   if (out_fp32)
-    rms_rows_kernel<float><<<n_out, nt, 0, st>>>((const float*)x, (const long long*)rows, n_rows, (const float*)w, (float*)out, D, eps);
+    CGK_CUDA_CHECK(launch_overlapped(rms_rows_kernel<float>, dim3(n_out), dim3(nt), 0, st, 0, (const float*)x, (const long long*)rows, n_rows, (const float*)w, (float*)out, D, eps));
   else
-    rms_rows_kernel<__nv_bfloat16><<<n_out, nt, 0, st>>>((const float*)x, (const long long*)rows, n_rows, (const float*)w,
-                                                        (__nv_bfloat16*)out, D, eps);
+    CGK_CUDA_CHECK(launch_overlapped(rms_rows_kernel<__nv_bfloat16>, dim3(n_out), dim3(nt), 0, st, 0, (const float*)x, (const long long*)rows, n_rows, (const float*)w,
+                                     (__nv_bfloat16*)out, D, eps));
   CGK_LAUNCH_CHECK();
   return 0;
 }
