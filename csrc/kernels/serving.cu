@@ -351,34 +351,69 @@ constexpr int SAMPLE_SHORT_K = 512;
 
 // One CTA per row.  A row is read once; what remains is a chain of short dependent steps, so the time is the number of
 // block barriers and the instructions between them.  Up to SAMPLE_SHORT_K wanted values: the kk-th largest of the 1024
-// threads' own maxima is a lower bound of the kk-th largest value (at least kk values reach it), found by 32 barriers that
-// count one comparison per thread; the few values at or above it are sorted, which also picks the wanted ones.  More
-// wanted values, or a row whose large values lie with few threads (over 1024 reach the bound): 32 counting rounds over all
-// keys.  80 rows of 32 000 fp32 logits, top-k 50,
-// top-p 0.9: 55.3 us with 32 counting rounds of three barriers, serial sums and the zeros written last; 26.6 us like this.
-__global__ void __launch_bounds__(SAMPLE_THREADS)
+// threads' own maxima is a lower bound of the kk-th largest value (at least kk values reach it), found to 20 bits by barriers that
+// count one comparison per thread.  The threads compare the logits as they are: v -> v / temperature keeps their order, so only the
+// bound and the few values near it are divided (a division per logit was 3 us of a row), and a value is taken if its quotient
+// reaches the bound's, as if all had been divided.  The few values taken are ranked, which also picks the wanted ones.  More
+// wanted values, or a row whose large values lie with few threads (over 1024 reach the bound): 32 counting rounds over the quotients
+// of all logits.  80 rows of 32 000 fp32 logits, top-k 50,
+// top-p 0.9: 55.3 us with 32 counting rounds of three barriers, serial sums and the zeros written last; 26.6 us with bounds by
+// maxima; 15.6 us with 16-byte loads, no divisions, ranks instead of a sort and one chain of sums instead of two.
+// FOURS: fours of neighbours per thread (rows that allow 16-byte loads), else single logits.  QUOTIENTS: every logit is divided as it is read
+// (more wanted values than are bounded by maxima; infinite temperatures, whose quotient of infinities ends on top).
+template <bool FOURS, bool QUOTIENTS>
+__global__ void __launch_bounds__(SAMPLE_THREADS, 1)
 sample_kernel(const void* logits, int logits_bf16, long long ld, int V, float temperature, int top_k, float top_p,
               unsigned long long seed, const long long* __restrict__ step, int* __restrict__ tokens, float* probs_out, int in_place) {
-  extern __shared__ uint32_t s_keys[];
+  extern __shared__ __align__(16) uint32_t s_keys[];
   __shared__ uint32_t s_count, s_cnt[2][32];
-  __shared__ float s_red[32], s_mass;
+  __shared__ float s_red[32], s_mass, s_u;
   __shared__ int s_keep;
   __shared__ float cand_v[MAX_TOPK];
   __shared__ int cand_i[MAX_TOPK];
+  __shared__ float prefix_s[MAX_TOPK];                       // sums of the candidates' probabilities; before that, scratch of the ranking
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  auto load = [&](int i) -> float {
-    const float v = logits_bf16 ? __bfloat162float(((const __nv_bfloat16*)logits)[row * ld + i]) : ((const float*)logits)[row * ld + i];
-    return temperature > 0.0f ? v / temperature : v;
+  pdl_trigger();
+  pdl_wait();
+  const bool scaled = temperature > 0.0f, scale = scaled && !QUOTIENTS;     // scale: keys are those of the logits as they are
+  // sort key of a logit; a NaN has that of its quotient, whatever the division makes of it
+  float nan = __int_as_float(0x7fc00000);
+  asm volatile("" : "+f"(nan));
+  const uint32_t nan_key = float_key(nan / temperature), negative_nan_key = float_key(-nan / temperature);
+  auto raw_key = [&](float v) -> uint32_t {
+    if (QUOTIENTS) return float_key(scaled ? v / temperature : v);
+    return scaled && v != v ? (__float_as_int(v) < 0 ? negative_nan_key : nan_key) : float_key(v);
+  };
+  auto divided = [&](uint32_t key) -> uint32_t { return key == nan_key || key == negative_nan_key ? key : float_key(key_float(key) / temperature); };
+  auto load = [&](int i) -> uint32_t {
+    return raw_key(logits_bf16 ? __bfloat162float(((const __nv_bfloat16*)logits)[row * ld + i]) : ((const float*)logits)[row * ld + i]);
   };
   auto block_sum = [&](float v) { v = warp_sum(v); if (lane == 0) s_red[warp] = v; __syncthreads(); v = s_red[lane]; v = warp_sum(v); __syncthreads(); return v; };
-  const int k = temperature > 0.0f ? (top_k <= 0 || top_k > MAX_TOPK ? MAX_TOPK : top_k) : 1;
+  const int k = scaled ? (top_k <= 0 || top_k > MAX_TOPK ? MAX_TOPK : top_k) : 1;
   const int kk = k < V ? k : V;
   const bool kept = V <= SAMPLE_IN_REGS + SAMPLE_IN_SMEM;
+  auto place = [&](int j) { return FOURS ? (tid + (j >> 2) * SAMPLE_THREADS) * 4 + (j & 3) : tid + j * SAMPLE_THREADS; };
   uint32_t key[SAMPLE_REGS];                                 // 0 stands for "no element": it is below the key of any float
-  if (kept) {
+  if (FOURS && kept) {
+    const float4* src = reinterpret_cast<const float4*>((const float*)logits + row * ld);
 #pragma unroll
-    for (int j = 0; j < SAMPLE_REGS; ++j) { const int i = tid + j * SAMPLE_THREADS; key[j] = i < V ? float_key(load(i)) : 0u; }
-    for (int i = SAMPLE_IN_REGS + tid; i < V; i += SAMPLE_THREADS) s_keys[i - SAMPLE_IN_REGS] = float_key(load(i));
+    for (int j = 0; j < SAMPLE_REGS / 4; ++j) {
+      const int i = tid + j * SAMPLE_THREADS;
+      const bool in = i < V / 4;
+      const float4 v = in ? src[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      key[4 * j] = in ? raw_key(v.x) : 0u;
+      key[4 * j + 1] = in ? raw_key(v.y) : 0u;
+      key[4 * j + 2] = in ? raw_key(v.z) : 0u;
+      key[4 * j + 3] = in ? raw_key(v.w) : 0u;
+    }
+    for (int i = SAMPLE_IN_REGS / 4 + tid; i < V / 4; i += SAMPLE_THREADS) {
+      const float4 v = src[i];
+      reinterpret_cast<uint4*>(s_keys)[i - SAMPLE_IN_REGS / 4] = make_uint4(raw_key(v.x), raw_key(v.y), raw_key(v.z), raw_key(v.w));
+    }
+  } else if (kept) {
+#pragma unroll
+    for (int j = 0; j < SAMPLE_REGS; ++j) { const int i = tid + j * SAMPLE_THREADS; key[j] = i < V ? load(i) : 0u; }
+    for (int i = SAMPLE_IN_REGS + tid; i < V; i += SAMPLE_THREADS) s_keys[i - SAMPLE_IN_REGS] = load(i);
   }
   if (tid == 0) s_count = 0;
   // the zeros of the distribution leave while the selection runs (if they do not cover logits that it still reads); the kept
@@ -391,35 +426,67 @@ sample_kernel(const void* logits, int logits_bf16, long long ld, int V, float te
       for (int i = tid; i < V; i += SAMPLE_THREADS) out[i] = 0.0f;
   };
   if (probs_out && !in_place) zeros();
-  auto each = [&](auto f) {                                  // a thread's own keys
+  // a thread's own keys: of the logits until they are divided in place (rows that are not kept: at every look); index >= V: no element
+  bool as_they_are = true;
+  auto each = [&](auto f) {
     if (kept) {
 #pragma unroll
-      for (int j = 0; j < SAMPLE_REGS; ++j) f(key[j], tid + j * SAMPLE_THREADS);
-      for (int i = SAMPLE_IN_REGS + tid; i < V; i += SAMPLE_THREADS) f(s_keys[i - SAMPLE_IN_REGS], i);
+      for (int j = 0; j < SAMPLE_REGS; ++j) f(key[j], place(j));
+      if (FOURS) {
+        for (int i = SAMPLE_IN_REGS + tid * 4; i < V; i += SAMPLE_THREADS * 4) {
+          const uint4 v = *reinterpret_cast<const uint4*>(s_keys + i - SAMPLE_IN_REGS);
+          f(v.x, i); f(v.y, i + 1); f(v.z, i + 2); f(v.w, i + 3);
+        }
+      } else {
+        for (int i = SAMPLE_IN_REGS + tid; i < V; i += SAMPLE_THREADS) f(s_keys[i - SAMPLE_IN_REGS], i);
+      }
     } else {
-      for (int i = tid; i < V; i += SAMPLE_THREADS) f(float_key(load(i)), i);
+      for (int i = tid; i < V; i += SAMPLE_THREADS) f(as_they_are ? load(i) : divided(load(i)), i);
     }
   };
-  auto take = [&](uint32_t kv, int i) {
+  auto take = [&](uint32_t quotient, int i) {
     if (i >= V) return;
     const uint32_t slot = atomicAdd(&s_count, 1u);
-    if (slot < (uint32_t)MAX_TOPK) { cand_v[slot] = key_float(kv); cand_i[slot] = i; }
+    if (slot < (uint32_t)MAX_TOPK) { cand_v[slot] = key_float(quotient); cand_i[slot] = i; }
   };
   int n = 0;
   if (kk <= SAMPLE_SHORT_K) {
     uint32_t mine = 0;
     each([&](uint32_t kv, int) { mine = max(mine, kv); });
     uint32_t bound = 0;
-    for (int bit = 31; bit >= 0; --bit) {
+#pragma unroll 1
+    for (int bit = 31; bit >= 12; --bit) {
       const uint32_t want = bound | (1u << bit);
       if (__syncthreads_count(mine >= want) >= kk) bound = want;
     }
-    if (mine >= bound) each([&](uint32_t kv, int i) { if (kv >= bound) take(kv, i); });
+    // Below `near` no quotient reaches the bound's: normal quotients that round to the same value have logits within two steps of
+    // each other; in the ranges where more of them fall together the limit is a loose one.
+    const uint32_t least = scale ? divided(bound) : bound;
+    const float q = key_float(least), size = fabsf(q);
+    uint32_t near = bound;
+    if (scale) {
+      if (size > 1e-30f && size < 1e38f) near = bound > 8u ? bound - 8u : 1u;
+      else if (size <= 1e-30f) near = float_key(-2e-30f * temperature);
+      else near = q < 0.0f ? 1u : float_key(0.5e38f * temperature);
+    }
+    if (mine >= near)
+      each([&](uint32_t kv, int i) {
+        if (kv >= near) { const uint32_t quotient = scale ? divided(kv) : kv; if (quotient >= least) take(quotient, i); }
+      });
     __syncthreads();
     n = s_count <= (uint32_t)MAX_TOPK ? (int)s_count : 0;    // 0: too many, the general way
     __syncthreads();
   }
   if (n == 0) {
+    if (scale) {                                             // from here on the quotients are compared
+      as_they_are = false;
+      if (kept) {
+#pragma unroll
+        for (int j = 0; j < SAMPLE_REGS; ++j) key[j] = key[j] ? divided(key[j]) : 0u;
+        for (int i = SAMPLE_IN_REGS + tid; i < V; i += SAMPLE_THREADS) s_keys[i - SAMPLE_IN_REGS] = divided(s_keys[i - SAMPLE_IN_REGS]);
+        __syncthreads();                                     // (by other threads than they belong to)
+      }
+    }
     uint32_t prefix = 0;                                     // becomes the key of the kk-th largest value
     for (int bit = 31; bit >= 0; --bit) {
       const uint32_t want = prefix | (1u << bit);
@@ -439,72 +506,91 @@ sample_kernel(const void* logits, int logits_bf16, long long ld, int V, float te
     __syncthreads();
     n = (int)min(s_count, (uint32_t)kk);
   }
-  // bitonic sort, descending by (value, then smaller index first) so that the result is deterministic; zeros of both signs
+  // descending by (value, then smaller index first) so that the result is deterministic; zeros of both signs
   // are equal, NaN has a place in the order, and padding comes after everything
-  int n2 = 1; while (n2 < n) n2 <<= 1;
   auto order = [&](int i) -> uint32_t { return cand_i[i] == 0x7fffffff ? 0u : float_key(cand_v[i] + 0.0f); };
-  for (int i = n + tid; i < n2; i += SAMPLE_THREADS) { cand_v[i] = -INFINITY; cand_i[i] = 0x7fffffff; }
-  __syncthreads();
-  for (int size = 2; size <= n2; size <<= 1)
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = tid; i < n2; i += SAMPLE_THREADS) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool desc = (i & size) == 0;
-          const uint32_t ki = order(i), kj = order(j);
-          const bool i_first = ki > kj || (ki == kj && cand_i[i] < cand_i[j]);
-          if (i_first != desc) { const float tv = cand_v[i]; cand_v[i] = cand_v[j]; cand_v[j] = tv; const int ti = cand_i[i]; cand_i[i] = cand_i[j]; cand_i[j] = ti; }
-        }
-      }
-      if (n2 > 32) __syncthreads();
-      else __syncwarp();                                     // one warp holds all of them
+  if (n <= 128) {
+    // few: a candidate's place is the number of those before it, counted by 8 to 32 lanes
+    unsigned long long* const both = reinterpret_cast<unsigned long long*>(prefix_s);
+    if (tid < n) both[tid] = (unsigned long long)order(tid) << 32 | (uint32_t)~cand_i[tid];
+    __syncthreads();
+    const int per = n <= 32 ? 32 : n <= 64 ? 16 : 8, c = tid / per;
+    int before = 0;
+    if (c < n) {
+      const unsigned long long own = both[c];
+      for (int j = tid % per; j < n; j += per) before += both[j] > own;
     }
-  if (n2 <= 32) __syncthreads();
+    for (int o = per >> 1; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (c < n && tid % per == 0) {                           // beyond the 128 keys that are still being read
+      prefix_s[512 + before] = cand_v[c];
+      prefix_s[768 + before] = __int_as_float(cand_i[c]);
+    }
+    __syncthreads();
+    if (tid < n) { cand_v[tid] = prefix_s[512 + tid]; cand_i[tid] = __float_as_int(prefix_s[768 + tid]); }
+    __syncthreads();
+  } else {
+    int n2 = 1; while (n2 < n) n2 <<= 1;
+    for (int i = n + tid; i < n2; i += SAMPLE_THREADS) { cand_v[i] = -INFINITY; cand_i[i] = 0x7fffffff; }
+    __syncthreads();
+    for (int size = 2; size <= n2; size <<= 1)
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        for (int i = tid; i < n2; i += SAMPLE_THREADS) {
+          const int j = i ^ stride;
+          if (j > i) {
+            const bool desc = (i & size) == 0;
+            const uint32_t ki = order(i), kj = order(j);
+            const bool i_first = ki > kj || (ki == kj && cand_i[i] < cand_i[j]);
+            if (i_first != desc) { const float tv = cand_v[i]; cand_v[i] = cand_v[j]; cand_v[j] = tv; const int ti = cand_i[i]; cand_i[i] = cand_i[j]; cand_i[j] = ti; }
+          }
+        }
+        __syncthreads();
+      }
+  }
   n = min(n, kk);
   // softmax over the candidates, nucleus cut, sample
   const float mx = cand_v[0];
   float e = tid < n ? __expf(cand_v[tid] - mx) : 0.0f;
   const float total = block_sum(e);
   if (tid < n) cand_v[tid] = e / total;
+  if (tid == 32) {
+    const Philox rnd = philox(seed, (uint64_t)row, step ? (uint64_t)*step : 0ull);
+    s_u = u01(rnd.c[0]);
+  }
   if (probs_out && in_place) zeros();
   __syncthreads();
-  if (tid == 0) {
-    // sums in the order of the candidates, eight values fetched ahead of the chain of additions
-    // (reads past n stay inside the array and are not used)
-    int keep = n;
-    float mass = 0.0f;
-    const bool cut = top_p > 0.0f && top_p < 1.0f;
-    bool done = false;
-    for (int b = 0; b < n && !done; b += 8) {
-      float v[8];
+  if (warp == 0) {
+    if (lane == 0) {
+      // sums in the order of the candidates, eight values fetched ahead of the chain of additions
+      // (reads past n stay inside the array and are not used)
+      int keep = n;
+      float mass = 0.0f;
+      const bool cut = top_p > 0.0f && top_p < 1.0f;
+      bool done = false;
+      for (int b = 0; b < n && !done; b += 8) {
+        float v[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = cand_v[b + j];
+        for (int j = 0; j < 8; ++j) v[j] = cand_v[b + j];
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (!done && b + j < n) {
-          mass += v[j];
-          if (cut && mass >= top_p) { keep = b + j + 1; done = true; }
-        }
+        for (int j = 0; j < 8; ++j)
+          if (!done && b + j < n) {
+            mass += v[j];
+            prefix_s[b + j] = mass;
+            if (cut && mass >= top_p) { keep = b + j + 1; done = true; }
+          }
+      }
+      s_keep = keep;
+      s_mass = mass;
     }
-    const Philox rnd = philox(seed, (uint64_t)row, step ? (uint64_t)*step : 0ull);
-    const float u = u01(rnd.c[0]) * mass;
-    float acc = 0.0f;
+    __syncwarp();
+    // the first candidate whose sum exceeds the drawn share of the mass
+    const int keep = s_keep;
+    const float u = s_u * s_mass;
     int pick = keep - 1;
-    done = false;
-    for (int b = 0; b < keep && !done; b += 8) {
-      float v[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = cand_v[b + j];
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (!done && b + j < keep) {
-          acc += v[j];
-          if (u < acc) { pick = b + j; done = true; }
-        }
+    for (int b = 0; b < keep; b += 32) {
+      const uint32_t above = __ballot_sync(0xffffffffu, b + lane < keep && u < prefix_s[b + lane]);
+      if (above) { pick = b + __ffs(above) - 1; break; }
     }
-    tokens[row] = cand_i[CGK_IDX(pick, keep)];
-    s_keep = keep;
-    s_mass = mass;
+    if (lane == 0) tokens[row] = cand_i[CGK_IDX(pick, keep)];
   }
   if (!probs_out) return;
   __syncthreads();
@@ -709,11 +795,15 @@ CGK_API int cgk_sample(const void* logits, int logits_bf16, long long ld, int ro
   CGK_REQUIRE(logits && tokens && rows > 0 && V > 0 && ld >= V, "cgk_sample: bad argument");
   // keys beyond those in registers: 4 bytes each, for rows that are kept at all
   const int smem = V > SAMPLE_IN_REGS && V <= SAMPLE_IN_REGS + SAMPLE_IN_SMEM ? (V - SAMPLE_IN_REGS) * 4 : 0;
-  if (smem > 32 * 1024) CGK_CUDA_CHECK(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_IN_SMEM * 4));
   const char* from = (const char*)logits, * to = from + ((long long)(rows - 1) * ld + V) * (logits_bf16 ? 2 : 4), * probs = (const char*)probs_out;
   const int in_place = probs && probs < to && from < probs + (long long)rows * V * 4;
-  sample_kernel<<<rows, SAMPLE_THREADS, smem, (cudaStream_t)stream>>>(logits, logits_bf16, ld, V, temperature, top_k, top_p, seed, step, tokens, probs_out, in_place);
-  CGK_LAUNCH_CHECK();
+  const bool fours = !logits_bf16 && ((V | ld) & 3) == 0 && ((uintptr_t)logits & 15) == 0;
+  const int k = temperature > 0.0f ? (top_k <= 0 || top_k > MAX_TOPK ? MAX_TOPK : top_k) : 1;
+  const bool quotients = (k < V ? k : V) > SAMPLE_SHORT_K || !(temperature < 1e30f);
+  const auto kernel = fours ? (quotients ? sample_kernel<true, true> : sample_kernel<true, false>) : (quotients ? sample_kernel<false, true> : sample_kernel<false, false>);
+  if (smem > 32 * 1024) CGK_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SAMPLE_IN_SMEM * 4));
+  CGK_CUDA_CHECK(launch_overlapped(kernel, dim3(rows), dim3(SAMPLE_THREADS), smem, (cudaStream_t)stream, 0, logits, logits_bf16, ld, V, temperature, top_k, top_p, seed,
+                                   step, tokens, probs_out, in_place));
   return 0;
 }
 CGK_API int cgk_spec_accept(const int* draft_tokens, const float* q, const float* p, int batch, int gamma, int V, unsigned long long seed,

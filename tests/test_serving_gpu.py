@@ -444,6 +444,47 @@ def test_sampling_takes_the_first_of_equal_values():
     assert probs[0].nonzero().view(-1).tolist() == [0, 5, 17, 900]
 
 
+# logits are selected as they are and only the few near the bound are divided by the temperature: the tokens kept are those of the
+# quotients, the first of equal ones, also where neighbours fall together (rounding, subnormal quotients, overflow) or are no numbers (of more than 1024 equal ones, any are kept)
+@pytest.mark.parametrize("V", [33, 1000, 32000, 50257])
+@pytest.mark.parametrize("temperature", [0.7, 1.0, 3.0, 1e-6, 1e6, 1e30, 1e-40])
+@pytest.mark.parametrize("kind", ["normal", "neighbours", "zeros", "tiny", "huge", "negative", "nan"])
+def test_sampling_keeps_the_largest_quotients(V, temperature, kind):
+    g = torch.Generator().manual_seed(V)
+    x = torch.randn(3, V, generator=g)
+    if kind == "neighbours":                                   # 16 neighbouring floats, many times each
+        x = (torch.randint(0, 16, (3, V), generator=g, dtype=torch.int32) + 0x40490000).view(torch.float32)
+    elif kind == "zeros":
+        x[:, 3:] = torch.where(torch.rand(3, V - 3, generator=g) < 0.5, 0.0, -1.0)
+    elif kind == "tiny":
+        x = x * 1e-39
+    elif kind == "huge":
+        x = x * 1e38
+    elif kind == "negative":
+        x = -x.abs() * 1e37
+        x[:, ::3] = float("-inf")
+    elif kind == "nan":
+        x[:, V // 2], x[:, 1] = float("nan"), float("-inf")
+    x = x.to(DEV)
+    k, t = 9, torch.tensor(temperature, device=DEV)
+    quotient = x / t
+    if kind == "nan":                                          # no number comes behind all numbers
+        quotient[:, V // 2] = float("-inf")
+    if V > 1024 and any(int((q == q.sort(descending=True)[0][k - 1]).sum()) > 512 for q in quotient):
+        pytest.skip("more equal values than are ranked")
+    quotient = torch.where((quotient == 0) & quotient.signbit(), -1e-45, quotient)     # a negative zero comes behind the others
+    order = torch.sort(quotient, dim=-1, descending=True, stable=True)[1][:, :k]
+    _, probs = sample(x, temperature, k, 1.0, return_probs=True)
+    for r in range(3):
+        best = quotient[r, order[r, 0]]
+        if not torch.isfinite(best):                           # a sum of infinities or NaN: no distribution to compare
+            continue
+        want = torch.softmax(quotient[r, order[r]].double(), 0)
+        assert (probs[r].nonzero().view(-1).tolist() == sorted(order[r][want.float() > 0].tolist()))
+        assert (probs[r, order[r]].double() - want).abs().max() < 1e-6
+    _lib.assert_device_ok()
+
+
 def test_spec_accept_rule_and_commit():
     B, g, V = 64, 4, 512
     torch.manual_seed(2)
