@@ -461,10 +461,12 @@ sample_kernel(const void* logits, int logits_bf16, long long ld, int V, float te
     }
     // Below `near` no quotient reaches the bound's: normal quotients that round to the same value have logits within two steps of
     // each other; in the ranges where more of them fall together the limit is a loose one.
-    const uint32_t least = scale ? divided(bound) : bound;
+    constexpr uint32_t lowest = 0x007FFFFFu;                 // key of -infinity: the 20 bits of a bound may lie below it, at no number's key
+    if (bound != 0 && bound < lowest) bound = lowest;
+    const uint32_t least = scale && bound != 0 ? divided(bound) : bound;
     const float q = key_float(least), size = fabsf(q);
     uint32_t near = bound;
-    if (scale) {
+    if (scale && bound != 0) {
       if (size > 1e-30f && size < 1e38f) near = bound > 8u ? bound - 8u : 1u;
       else if (size <= 1e-30f) near = float_key(-2e-30f * temperature);
       else near = q < 0.0f ? 1u : float_key(0.5e38f * temperature);

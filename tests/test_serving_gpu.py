@@ -485,6 +485,13 @@ def test_sampling_keeps_the_largest_quotients(V, temperature, kind):
     _lib.assert_device_ok()
 
 
+# as many wanted as there are, minus infinity among them: the bound's 20 bits lie below its key
+def test_sampling_keeps_minus_infinity_when_all_are_wanted():
+    x = torch.tensor([[1.0, float("-inf"), 3.0, float("-inf"), 2.0]])
+    tok, probs = sample(x.to(DEV), 0.5, 5, 1.0, return_probs=True)
+    assert torch.allclose(probs.cpu(), torch.softmax(x / 0.5, -1))
+
+
 def test_spec_accept_rule_and_commit():
     B, g, V = 64, 4, 512
     torch.manual_seed(2)
