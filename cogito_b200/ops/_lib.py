@@ -200,6 +200,15 @@ def stream_ptr() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+def to_device(host: torch.Tensor, device) -> torch.Tensor:
+    """A small host tensor on the device, in the order of the current stream and without a wait: a copy from pageable memory holds the
+    host until everything before it in the stream is done (a prompt step of the layer-stack engine has six, and the GPU idled
+    behind the last of them until the launches went on).  The pinned block is handed out again only when its copy is over."""
+    if torch.device(device).type != "cuda" or torch.cuda.is_current_stream_capturing():
+        return host.to(device)
+    return host.pin_memory().to(device, non_blocking=True)
+
+
 class Made:
     """Something that outlives a call (``value``, what ``make`` returns) and is filled by launches.  They run on the current stream,
     or, if that is being captured, on another one at once, so that a graph neither repeats them nor owns the memory.  ``here``

@@ -141,7 +141,7 @@ def _advance_chunks(a: LinearStateArgs, rule: StateRule, batch, rows: int, devic
     if key not in batch.memo:
         first = [g.start + i * g.count for g in batch.prompts for i in range(g.sequences)]
         items, run_items, cut = stretches([g.count for g in batch.prompts for _ in range(g.sequences)], rule.heads, first)
-        flat = torch.tensor([v for t in items + run_items for v in t], dtype=torch.int32).to(device)
+        flat = _lib.to_device(torch.tensor([v for t in items + run_items for v in t], dtype=torch.int32), device)
         batch.memo[key] = flat, len(items), len(run_items), cut
     flat, n, runs, cut = batch.memo[key]
     L, scratch = _lib.lib(), None

@@ -94,7 +94,7 @@ class PagedCache:
             raise RuntimeError(f"the page pool is exhausted: {need - len(own)} pages wanted, {len(self._free_pages)} free")
         first = len(own)
         own.extend(self._free_pages.pop() for _ in range(need - first))
-        self.page_table[slot, first:need] = torch.tensor(own[first:], dtype=torch.int32).to(self.device)
+        self.page_table[slot, first:need] = _lib.to_device(torch.tensor(own[first:], dtype=torch.int32), self.device)
 
     def close(self, slot: int):
         """Returns the slot and its pages."""

@@ -109,34 +109,36 @@ class StackEngine:
         if self.use_graph and keep is None and all(len(t) == 1 for _, t, _ in entries):
             logits = self._decode_graph(entries)
             rows = [i for i, (_, _, w) in enumerate(entries) for _ in w]
-            out = logits[torch.tensor(rows, dtype=torch.int64, device=self.device)] if rows != list(range(len(entries))) else logits.clone()
+            out = logits[_lib.to_device(torch.tensor(rows, dtype=torch.int64), self.device)] if rows != list(range(len(entries))) else logits.clone()
         else:
             # prompt portions first; the caller's order of the wanted logits is kept by the row list
             order = sorted(range(len(entries)), key=lambda i: len(entries[i][1]) < self.PROMPT_MIN)
-            ids, pos, slot, segs, runs, single = [], [], [], [], [], None
+            segs, runs, single, start, longest = [], [], None, 0, 0
             first = {}
+            host = torch.empty(3, sum(len(t) for _, t, _ in entries), dtype=torch.int64)      # token, position, slot
             for i in order:
                 s, toks, _ = entries[i]
                 n, begin = len(toks), self.cached[s]
-                first[i] = len(ids)
+                first[i] = start
                 if n >= self.PROMPT_MIN:
-                    segs.append(Segment(len(ids), 1, n, s, begin))
+                    segs.append(Segment(start, 1, n, s, begin))
                 elif single is None:
-                    single = len(ids)
-                runs.append((len(ids), n))
-                ids += toks
-                pos += range(begin, begin + n)
-                slot += [s] * n
-            host = torch.tensor([ids, pos, slot], dtype=torch.int64)
-            dev = host.to(self.device)
+                    single = start
+                runs.append((start, n))
+                host[0, start:start + n] = torch.tensor(toks, dtype=torch.int64)
+                torch.arange(begin, begin + n, out=host[1, start:start + n])
+                host[2, start:start + n] = s
+                start += n
+                longest = max(longest, begin + n)
+            dev = _lib.to_device(host, self.device)
             small = dev[1:].to(torch.int32)
-            batch = TokenBatch(dev[0], small[0], small[1], segs, len(ids) if single is None else single, max(pos) + 1,
-                               torch.tensor(runs, dtype=torch.int32).to(self.device))
+            batch = TokenBatch(dev[0], small[0], small[1], segs, start if single is None else single, longest,
+                               _lib.to_device(torch.tensor(runs, dtype=torch.int32), self.device))
             x = self.model.stream(batch, self.cache, **({} if keep is None else {"keep": keep}))
             rows = [first[i] + w for i, (_, _, want) in enumerate(entries) for w in want]
             out = torch.empty(0, V, device=self.device)
             if rows:
-                out = self.model.logits(x, torch.tensor(rows, dtype=torch.int64).to(self.device))
+                out = self.model.logits(x, _lib.to_device(torch.tensor(rows, dtype=torch.int64), self.device))
         for s, toks, _ in entries:
             self.cached[s] += len(toks)
         assert out.shape[0] == wanted
@@ -156,7 +158,7 @@ class StackEngine:
         pad = size - n
         host = torch.tensor([[t[0] for _, t, _ in entries] + [0] * pad, [self.cached[s] for s, _, _ in entries] + [0] * pad,
                              [s for s, _, _ in entries] + [self._pad_slot] * pad], dtype=torch.int64)
-        g["in"].copy_(host)
+        g["in"].copy_(host.pin_memory(), non_blocking=True)
         g["graph"].replay()
         _lib.count_launch(g["launches"])
         return g["logits"][:n]
