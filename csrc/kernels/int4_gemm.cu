@@ -31,7 +31,7 @@
 #include <stdlib.h>
 
 #include "host_common.h"
-#include "sm100.cuh"
+#include "mma_sync.cuh"
 #include "cogito_kernels.h"
 
 namespace {
@@ -40,7 +40,8 @@ using namespace cgk;
 constexpr int BM = 128, BN = 128, BK = 64;
 constexpr int ISSUE_LANES = 8;                                // threads of a producer warp that issue copies
 constexpr int SUB = 2;                                        // 64-row sub-tiles per pipeline step (a step covers 128 k)
-constexpr int B_STAGES = 2, MAX_RAW_STAGES = 16, MAX_A_STAGES = 8, CONVERT_WARPS = 16;
+constexpr int B_STAGES = 3, MAX_RAW_STAGES = 16, MAX_A_STAGES = 8;
+constexpr int GROUPS = 2, GROUP_WARPS = 8, CONVERT_WARPS = GROUPS * GROUP_WARPS;     // converting warps: groups that take the steps in turn
 constexpr int B_BYTES = BK * BN * 2;
 constexpr int NIB_BYTES = BK * BN / 2, SCALE_BYTES = BK * 2 * 4, RAW_BYTES = NIB_BYTES + SCALE_BYTES;   // 4096 + 512
 constexpr int EPI_WARP0 = 4 + CONVERT_WARPS, THREADS = 32 * (EPI_WARP0 + 4);
@@ -127,8 +128,8 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < MAX_A_STAGES; ++s) { mbar_init(a_full(s), 1); mbar_init(a_empty(s), 1); }
-    for (int s = 0; s < B_STAGES; ++s) { mbar_init(b_full(s), CONVERT_WARPS); mbar_init(b_empty(s), 1); }
-    for (int s = 0; s < MAX_RAW_STAGES; ++s) { mbar_init(raw_full(s), 1); mbar_init(raw_empty(s), CONVERT_WARPS); }
+    for (int s = 0; s < B_STAGES; ++s) { mbar_init(b_full(s), GROUP_WARPS); mbar_init(b_empty(s), 1); }
+    for (int s = 0; s < MAX_RAW_STAGES; ++s) { mbar_init(raw_full(s), 1); mbar_init(raw_empty(s), GROUP_WARPS); }
     for (int a = 0; a < 2; ++a) { mbar_init(acc_full(a), 1); mbar_init(acc_empty(a), 4); }
     *dead = 0;
     *is_last = 0;
@@ -150,22 +151,30 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
     // belongs to the same lane: its uses are then waited for in order, which the one-bit phase
     // parity of an mbarrier requires.
     if (lane < ISSUE_LANES) {
+      int r = 0;
+      uint32_t par = 1;
       for (int i = 0; i < ksteps; ++i) {
-        const int r = i % RAW_STAGES;
-        if (r % ISSUE_LANES != lane) continue;
-        if (!mbar_wait(raw_empty(r), ((i / RAW_STAGES) & 1) ^ 1, dead, g.status, 300)) break;
-        mbar_expect_tx(raw_full(r), SUB * RAW_BYTES);
-        bulk_load_1d(sRaw + r * (SUB * RAW_BYTES), g.w_tiles + (long long)line(i) * (SUB * RAW_BYTES), SUB * RAW_BYTES, raw_full(r));
+        const int here = r;
+        const uint32_t phase = par;
+        if (++r == RAW_STAGES) { r = 0; par ^= 1; }
+        if (here % ISSUE_LANES != lane) continue;
+        if (!mbar_wait(raw_empty(here), phase, dead, g.status, 300)) break;
+        mbar_expect_tx(raw_full(here), SUB * RAW_BYTES);
+        bulk_load_1d(sRaw + here * (SUB * RAW_BYTES), g.w_tiles + (long long)line(i) * (SUB * RAW_BYTES), SUB * RAW_BYTES, raw_full(here));
       }
     }
   } else if (warp == 3) {
     if (lane < ISSUE_LANES) {
       if (lane == 0) tma_prefetch_desc(&tmX);
+      int next = 0;
+      uint32_t par = 1;
       for (int i = 0; i < ksteps; ++i) {
-        const int s = i % a_stages;
+        const int s = next;
+        const uint32_t phase = par;
+        if (++next == a_stages) { next = 0; par ^= 1; }
         if (s % ISSUE_LANES != lane) continue;
         const int ks = line(i) % k_tiles;                             // step within its tile
-        if (!mbar_wait(a_empty(s), ((i / a_stages) & 1) ^ 1, dead, g.status, 301)) break;
+        if (!mbar_wait(a_empty(s), phase, dead, g.status, 301)) break;
         mbar_expect_tx(a_full(s), SUB * a_bytes);
 #pragma unroll
         for (int sub = 0; sub < SUB; ++sub)
@@ -178,16 +187,18 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
       bool ok = true;
       int left = 0, part = -1;
       bool first = true;
+      int sa = 0, sb = 0;
+      uint32_t pa = 0, pb = 0;
       for (int i = 0; i < ksteps && ok; ++i) {
-        const int sa = i % a_stages, sb = i % B_STAGES;
         if (left == 0) {
           left = part_steps(i);
           first = true;
           ++part;
           if (!mbar_wait(acc_empty(part & 1), ((part >> 1) & 1) ^ 1, dead, g.status, 307)) { ok = false; break; }
         }
-        if (!mbar_wait(a_full(sa), (i / a_stages) & 1, dead, g.status, 302) ||
-            !mbar_wait(b_full(sb), (i / B_STAGES) & 1, dead, g.status, 303)) { ok = false; break; }
+        // both polls are under way together: an answer takes some 200 cycles, also where it is yes
+        const uint32_t a_there = mbar_try_wait(a_full(sa), pa), b_there = mbar_try_wait(b_full(sb), pb);
+        if (!(a_there & b_there) && (!mbar_wait(a_full(sa), pa, dead, g.status, 302) || !mbar_wait(b_full(sb), pb, dead, g.status, 303))) { ok = false; break; }
         tc_fence_after();
         const uint32_t d = tmem + (uint32_t)(part & 1) * BN;
 #pragma unroll
@@ -201,45 +212,68 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
         first = false;
         umma_commit(a_empty(sa));
         umma_commit(b_empty(sb));
+        if (++sa == a_stages) { sa = 0; pa ^= 1; }
+        if (++sb == B_STAGES) { sb = 0; pb ^= 1; }
         if (--left == 0) umma_commit(acc_full(part & 1));
       }
     }
   } else if (warp >= 4 && warp < EPI_WARP0) {
-    const int tid = threadIdx.x - 128;                 // 0 .. 32*CONVERT_WARPS-1
-    constexpr int WORDS_PER_THREAD = (SUB * BK * BN / 8) / (32 * CONVERT_WARPS);
-    bool ok = true;
-    for (int i = 0; i < ksteps && ok; ++i) {
-      const int r = i % RAW_STAGES, s = i % B_STAGES;
-      // one lane polls for the warp (256+ threads hammering one barrier word cost ~150 cycles a wait)
-      int got = 1;
-      if (lane == 0) got = mbar_wait(raw_full(r), (i / RAW_STAGES) & 1, dead, g.status, 304) &&
-                           mbar_wait(b_empty(s), ((i / B_STAGES) & 1) ^ 1, dead, g.status, 305);
-      got = __shfl_sync(0xffffffffu, got, 0);
-      if (!got) { ok = false; break; }
+    // Group gi has steps gi, gi + 2, ..: while one waits for its buffers or for the answers to its polls, the other converts.
+    const int gi = (warp - 4) / GROUP_WARPS, tid = threadIdx.x - 128 - gi * (32 * GROUP_WARPS);
+    constexpr int WORDS = BK * BN / 8 / (32 * GROUP_WARPS);            // per thread and 64-row sub-tile: rows 16 apart, the same 8 columns
+    const int k0 = tid >> 4, jw = tid & 15;
+    const uint8_t* const raw0 = raw_s + tid * 4;
+    const uint8_t* const scale0 = raw_s + NIB_BYTES + k0 * 8 + (jw >> 3) * 4;
+    const uint32_t dst0 = sB + (jw >> 3) * 8192u + sw128_offset((uint32_t)k0, (uint32_t)(jw & 7));    // 16 rows on: 2048 bytes
+    uint32_t mask = 0x000F000Fu, magic = 0x43004300u;
+    asm volatile("" : "+r"(mask), "+r"(magic));
+    const __nv_bfloat162 off = __float2bfloat162_rn(136.0f);
+    int r = gi, s = gi;
+    uint32_t pr = 0, ps = 1;
+    if (r >= RAW_STAGES) { r -= RAW_STAGES; pr ^= 1; }
+    for (int i = gi; i < ksteps; i += GROUPS) {
+      // one lane polls for the warp (256+ threads hammering one barrier word cost ~150 cycles a wait), both barriers at once
+      uint32_t got = 1;
+      if (lane == 0) {
+        const uint32_t raw_there = mbar_try_wait(raw_full(r), pr), b_there = mbar_try_wait(b_empty(s), ps);
+        got = raw_there & b_there;
+        if (!got) got = mbar_wait(raw_full(r), pr, dead, g.status, 304) && mbar_wait(b_empty(s), ps, dead, g.status, 305);
+      }
+      if (!__shfl_sync(0xffffffffu, got, 0)) break;
+      const uint8_t* raw = raw0 + r * (SUB * RAW_BYTES);
+      const uint8_t* scales = scale0 + r * (SUB * RAW_BYTES);
+      const uint32_t dst = dst0 + s * (SUB * B_BYTES);
 #pragma unroll
-      for (int it = 0; it < WORDS_PER_THREAD; ++it) {
-        // word of the step: sub-tile, then row k = w / 16 (16 words = 128 columns), 8 columns per word
-        const int wi = it * (32 * CONVERT_WARPS) + tid, sub = wi >> 10, w = wi & 1023, k = w >> 4, jw = w & 15;
-        const uint8_t* tile = raw_s + (r * SUB + sub) * RAW_BYTES;
-        const uint32_t* raw = reinterpret_cast<const uint32_t*>(tile);
-        const float* scale = reinterpret_cast<const float*>(tile + NIB_BYTES);
-        const uint32_t b_addr = sB + (s * SUB + sub) * B_BYTES;
-        const uint32_t v = raw[w] ^ 0x88888888u;         // two's complement -> q + 8
-        const __nv_bfloat162 off = __float2bfloat162_rn(136.0f), sc = __float2bfloat162_rn(scale[2 * k + (jw >> 3)]);
-        uint32_t t[4];
+      for (int sub = 0; sub < SUB; ++sub) {
+        uint32_t v[WORDS];
+        float sc[WORDS];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint32_t u = ((v >> (4 * j)) & 0x000F000Fu) | 0x43004300u;      // bf16 (128 + q + 8) for columns j and j + 4
-          __nv_bfloat162 h = __hmul2(__hsub2(*reinterpret_cast<__nv_bfloat162*>(&u), off), sc);
-          t[j] = *reinterpret_cast<uint32_t*>(&h);
+        for (int it = 0; it < WORDS; ++it) {
+          v[it] = *reinterpret_cast<const uint32_t*>(raw + sub * RAW_BYTES + it * (32 * GROUP_WARPS * 4));
+          sc[it] = *reinterpret_cast<const float*>(scales + sub * RAW_BYTES + it * (16 * 8));
         }
-        // positions 0..7 of the chunk hold columns 0,4,1,5,2,6,3,7
-        const uint32_t dst = b_addr + (jw >> 3) * 8192u + sw128_offset((uint32_t)k, (uint32_t)(jw & 7));
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");
+#pragma unroll
+        for (int it = 0; it < WORDS; ++it) {
+          const uint32_t w = v[it] ^ 0x88888888u;          // two's complement -> q + 8
+          const __nv_bfloat162 sc2 = __float2bfloat162_rn(sc[it]);
+          uint32_t t[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t u = pick(w >> (4 * j), mask, magic);           // bf16 (128 + q + 8) for columns j and j + 4
+            const __nv_bfloat162 h = __hmul2(__hsub2(*reinterpret_cast<const __nv_bfloat162*>(&u), off), sc2);
+            t[j] = *reinterpret_cast<const uint32_t*>(&h);
+          }
+          // positions 0..7 of the chunk hold columns 0,4,1,5,2,6,3,7
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + sub * B_BYTES + it * 2048), "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");
+        }
       }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) { mbar_arrive(b_full(s)); mbar_arrive(raw_empty(r)); }
+      r += GROUPS;
+      if (r >= RAW_STAGES) { r -= RAW_STAGES; pr ^= 1; }
+      s += GROUPS;
+      if (s >= B_STAGES) { s -= B_STAGES; ps ^= 1; }
     }
   } else if (warp >= EPI_WARP0) {
     // ---- epilogue: lane = output row inside the 128-row tile.
