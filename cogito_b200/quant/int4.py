@@ -122,9 +122,9 @@ class Int4Linear(torch.nn.Module):
     # first use; both sum the parts of a shared tile in a fixed order, so a call gives the same bits every time.
     # Times (us, layers one after the other) for 4096 x 6144, 4096 x 4096, 4096 x 22016, 11008 x 4096, 4096 x 32000, 2048 x 11264:
     #   16 rows   "wa" 8.4 6.5 20.6 11.0 25.9 10.3      (before, through tensor memory: 20.1 14.9 34.7 24.7 44.6 19.2)
-    #   32 rows   "wa" 12.8 9.0 31.5 15.7 39.8 15.5     "wb" 19.2 15.8 43.3 25.9 58.4 17.4
-    #   80 rows   "wa" 27.4 22.4 75.4 40.5 107 28.4     "wb" 21.0 18.3 45.8 28.1 60.4 19.3 (three passes over the weights)
-    #   200 rows  "wb" 31.4 24.9 103 45.9 141 30.5      dense 31.4 26.5 104 61.1 131 32.7 (a third row tile adds half to "wb")
+    #   32 rows   "wa" 12.8 9.0 31.5 15.7 39.8 15.5     "wb" 14.7 12.4 29.7 18.8 39.1 13.3
+    #   80 rows   "wa" 27.4 22.4 75.4 40.5 107 28.4     "wb" 17.7 14.5 32.1 20.8 44.8 15.0 (three passes over the weights)
+    #   200 rows  "wb" 24.7 20.6 83.4 35.1 111 24.3     dense 31.4 26.5 104 61.1 131 32.7 (a third row tile adds half to "wb")
     FEW_ROWS, DENSE_ROWS = 32, 256
     kernel = os.environ.get("COGITO_INT4_KERNEL", "auto")
 
@@ -194,14 +194,14 @@ class Int4Linear(torch.nn.Module):
         return gemm(x2.to(torch.bfloat16).contiguous(), self.dequantized(torch.bfloat16), b_mn=True, bias=self.bias, **kw)
 
     def forward_f32(self, x: torch.Tensor) -> torch.Tensor:
-        """fp32 result (logits); few rows and prompts leave the GEMM in fp32 without a bf16 copy in between."""
+        """fp32 result (logits); the result leaves the GEMM in fp32 without a bf16 copy in between."""
         rows = x.numel() // self.in_features
         if x.is_cuda and self._takes_dense(rows):
             try:
                 return self._dense(x.reshape(rows, self.in_features), out_dtype=torch.float32).view(*x.shape[:-1], self.out_features)
             except torch.OutOfMemoryError:
                 pass                                       # no room for the weights in bf16: by the streaming kernel
-        if x.is_cuda and rows and self._streams_few(rows):
+        if x.is_cuda and 0 < rows <= self.DENSE_ROWS and self._streams():
             return self._stream(x.reshape(rows, self.in_features), f32=True).view(*x.shape[:-1], self.out_features)
         return self.forward(x).float()
 
@@ -228,8 +228,7 @@ class Int4Linear(torch.nn.Module):
                 y = y + self.bias.float()
             return done(y.to(x.dtype))
         N, K = self.out_features, self.in_features
-        if N % 128 or K % 64 or self.group % 64:
-            # shapes the streaming kernel does not cover: dequantise once, then the bf16 GEMM
+        if not self._streams():
             return done(self._dense(x2))
         if self._takes_dense(M, splits):
             if out is not None and (out.dtype != torch.bfloat16 or not out.is_contiguous() or out.numel() != M * N):
@@ -240,13 +239,17 @@ class Int4Linear(torch.nn.Module):
                 pass                                       # no room for the weights in bf16: by the streaming kernel
         return self._stream(x2, splits, out).view(*lead, N)
 
+    def _streams(self) -> bool:
+        """A shape that the streaming kernels cover; for others the weights are dequantised, then the bf16 GEMM."""
+        return self.out_features % 128 == 0 and self.in_features % 64 == 0 and self.group % 64 == 0
+
     def _streams_few(self, rows: int) -> bool:
         """"wa" (needs one scale per k for a 128-feature tile)."""
         return (self.kernel == "wa" or (self.kernel == "auto" and rows <= self.FEW_ROWS)) and self.group % 128 == 0 \
             and self.in_features % 128 == 0 and self.out_features % 128 == 0
 
     def _stream(self, x2: torch.Tensor, splits: int = 0, out: torch.Tensor | None = None, f32: bool = False) -> torch.Tensor:
-        """[rows, in] through "wa" or "wb"; ``f32``: an fp32 result ("wa" only)."""
+        """[rows, in] through "wa" or "wb"; ``f32``: an fp32 result."""
         x2 = x2.to(torch.bfloat16).contiguous()
         L = _lib.lib()
         M, N, K = x2.shape[0], self.out_features, self.in_features
@@ -266,7 +269,10 @@ class Int4Linear(torch.nn.Module):
             out = torch.empty(M, N, dtype=torch.float32 if f32 else torch.bfloat16, device=x2.device)
         elif out.dtype != torch.bfloat16 or not out.is_contiguous() or out.numel() != M * N:
             raise ValueError("out must be a contiguous bf16 [rows, out_features] tensor")
-        entry = (L.cgk_int4_wa_gemm_parts_f32 if f32 else L.cgk_int4_wa_gemm_parts) if wa else L.cgk_int4_gemm_parts
+        if wa:
+            entry = L.cgk_int4_wa_gemm_parts_f32 if f32 else L.cgk_int4_wa_gemm_parts
+        else:
+            entry = L.cgk_int4_gemm_parts_f32 if f32 else L.cgk_int4_gemm_parts
         _lib.check(entry(x2.data_ptr(), K, tiles.data_ptr(), parts.data_ptr(), counters.data_ptr(),
                          out.data_ptr(), N, _lib.ptr(self.bias), M, N, K, splits, _lib.stream_ptr()), "cgk_int4_gemm")
         _lib.count_launch()

@@ -52,9 +52,9 @@ struct Int4Dev {
   const uint8_t* w_tiles;          // [N/128][K/64][4608]
   float4* parts;                   // slots of shared tiles' parts: [m_tiles][sharers][2][32 column quads][a_rows]
   int* counters;                   // int32 [m_tiles * n_tiles], zero between calls (shared tiles only)
-  __nv_bfloat16* out; long long ldo;
+  void* out; long long ldo;        // bf16, or fp32 with out_f32
   const __nv_bfloat16* bias;
-  int M, N, K;
+  int M, N, K, out_f32;
   int a_rows, a_stages;            // rows fetched per X tile (multiple of 8), depth of the X ring
   int raw_stages;                  // depth of the W ring
   int sharers;                     // CTAs that the left-over tiles are dealt to
@@ -64,6 +64,17 @@ struct Int4Dev {
 // Slot `which` of a sharer: [32 column quads][a_rows] float4s.
 __device__ __forceinline__ float4* part_slot(const Int4Dev& g, int mt, int sharer, int which) {
   return g.parts + (long long)((mt * g.sharers + sharer) * 2 + which) * ((BN / 4) * g.a_rows);
+}
+
+// Eight neighbouring elements of the output.
+__device__ __forceinline__ void store8(const Int4Dev& g, long long at, const float4& u, const float4& v) {
+  if (g.out_f32) {
+    float4* p = reinterpret_cast<float4*>((float*)g.out + at);
+    p[0] = u;
+    p[1] = v;
+  } else {
+    *reinterpret_cast<uint4*>((__nv_bfloat16*)g.out + at) = make_uint4(pack_bf16x2(u.x, u.y), pack_bf16x2(u.z, u.w), pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+  }
 }
 
 // The output of a tile out of its parts, summed in the order of the CTAs lo .. hi; `first`: the slot that CTA lo's is in.
@@ -88,8 +99,7 @@ __device__ __forceinline__ void sum_parts(const Int4Dev& g, int mt, int nt, int 
       v.x += __bfloat162float(g.bias[n + 4]); v.y += __bfloat162float(g.bias[n + 5]);
       v.z += __bfloat162float(g.bias[n + 6]); v.w += __bfloat162float(g.bias[n + 7]);
     }
-    *reinterpret_cast<uint4*>(g.out + (long long)(m0 + r) * g.ldo + n) =
-        make_uint4(pack_bf16x2(u.x, u.y), pack_bf16x2(u.z, u.w), pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+    store8(g, (long long)(m0 + r) * g.ldo + n, u, v);
   }
 }
 
@@ -302,7 +312,6 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
           // a slot takes all its rows, so that no memory sector is written in part (17 rows, 4096 x 22016, cold caches: 55 -> 51 us)
           if (lo == hi ? row >= g.M : q * 32 + lane >= g.a_rows) continue;
           if (lo == hi) {
-            __nv_bfloat16* dstp = g.out + (long long)row * g.ldo + n0 + c;
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               float v[8] = {__uint_as_float(rr[j]), __uint_as_float(rr[j + 2]), __uint_as_float(rr[j + 4]), __uint_as_float(rr[j + 6]),
@@ -311,8 +320,7 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] += __bfloat162float(g.bias[n0 + c + j + e]);
               }
-              uint4 pk = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
-              *reinterpret_cast<uint4*>(dstp + j) = pk;
+              store8(g, (long long)row * g.ldo + n0 + c + j, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]));
             }
           } else {
             // neighbouring lanes hold neighbouring rows: 16 bytes each, side by side
@@ -416,11 +424,8 @@ CGK_API long long cgk_int4_gemm_parts_floats(int M, int N, int K, int splits) {
   return (long long)((M + BM - 1) / BM) * d.sharers * 2 * BN * part_rows(M);
 }
 
-// x bf16 [M, ldx]; w_tiles from cgk_int4_tile_weights; out bf16 [M, ldo]; bias bf16 [N] or null.  parts (fp32
-// [cgk_int4_gemm_parts_floats], any contents) and counters (int32 [cgk_int4_gemm_counters], zero before the first call and left
-// zero by every call) serve tiles shared by several CTAs; without them every tile is computed whole.  splits 0 = chosen here.
-CGK_API int cgk_int4_gemm_parts(const void* x, long long ldx, const void* w_tiles, float* parts, int* counters, void* out, long long ldo,
-                                const void* bias, int M, int N, int K, int splits, void* stream) {
+static int wb_gemm(const void* x, long long ldx, const void* w_tiles, float* parts, int* counters, void* out, long long ldo,
+                   const void* bias, int M, int N, int K, int splits, int out_f32, void* stream) {
   using namespace cgk;
   CGK_REQUIRE(x && w_tiles && out, "cgk_int4_gemm: null pointer");
   CGK_REQUIRE(M > 0 && N > 0 && K > 0 && N % BN == 0 && K % (SUB * BK) == 0, "cgk_int4_gemm: need N %% 128 == 0 and K %% 128 == 0 (got M=%d N=%d K=%d)", M, N, K);
@@ -451,10 +456,23 @@ CGK_API int cgk_int4_gemm_parts(const void* x, long long ldx, const void* w_tile
     CGK_CUDA_CHECK(cudaFuncSetAttribute(int4_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     attr_set[dev] = true;
   }
-  Int4Dev g{(const uint8_t*)w_tiles, (float4*)parts, counters, (__nv_bfloat16*)out, ldo, (const __nv_bfloat16*)bias, M, N, K,
+  Int4Dev g{(const uint8_t*)w_tiles, (float4*)parts, counters, out, ldo, (const __nv_bfloat16*)bias, M, N, K, out_f32,
             a_rows, a_stages, raw_stages, (int)d.sharers, device_status(dev)};
   CGK_CUDA_CHECK(launch_overlapped(int4_gemm_kernel, dim3((unsigned)d.ctas, m_tiles), dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, 0, tmX, g));
   return 0;
+}
+
+// x bf16 [M, ldx]; w_tiles from cgk_int4_tile_weights; out bf16 [M, ldo]; bias bf16 [N] or null.  parts (fp32
+// [cgk_int4_gemm_parts_floats], any contents) and counters (int32 [cgk_int4_gemm_counters], zero before the first call and left
+// zero by every call) serve tiles shared by several CTAs; without them every tile is computed whole.  splits 0 = chosen here.
+CGK_API int cgk_int4_gemm_parts(const void* x, long long ldx, const void* w_tiles, float* parts, int* counters, void* out, long long ldo,
+                                const void* bias, int M, int N, int K, int splits, void* stream) {
+  return wb_gemm(x, ldx, w_tiles, parts, counters, out, ldo, bias, M, N, K, splits, 0, stream);
+}
+// The same with an fp32 output (logits).
+CGK_API int cgk_int4_gemm_parts_f32(const void* x, long long ldx, const void* w_tiles, float* parts, int* counters, float* out, long long ldo,
+                                    const void* bias, int M, int N, int K, int splits, void* stream) {
+  return wb_gemm(x, ldx, w_tiles, parts, counters, out, ldo, bias, M, N, K, splits, 1, stream);
 }
 
 // The same for callers that hold an accumulator (fp32 [M, N], zero, left zero) instead of parts, which then come from the stream's
@@ -463,6 +481,6 @@ CGK_API int cgk_int4_gemm(const void* x, long long ldx, const void* w_tiles, flo
                           const void* bias, int M, int N, int K, int splits, void* stream) {
   const bool shared = acc && counters;
   return cgk::with_stream_scratch(shared ? cgk_int4_gemm_parts_floats(M, N, K, splits) : 0, (cudaStream_t)stream, [&](float* parts) {
-    return cgk_int4_gemm_parts(x, ldx, w_tiles, parts, parts ? counters : nullptr, out, ldo, bias, M, N, K, shared && !parts ? 0 : splits, stream);
+    return wb_gemm(x, ldx, w_tiles, parts, parts ? counters : nullptr, out, ldo, bias, M, N, K, shared && !parts ? 0 : splits, 0, stream);
   });
 }

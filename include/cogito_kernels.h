@@ -226,11 +226,13 @@ int cgk_int4_tile_weights(const void* packed, const float* scales, int K, int N,
  * that may run at the same time need their own.  splits 0 = dealt out so that all SMs have equal
  * shares, else that many equal parts of every tile.  Parts are summed in a fixed order.
  * cgk_int4_gemm takes an accumulator (fp32 [M, N], zero, left zero) in the place of parts, which it
- * allocates from the stream's memory pool. */
+ * allocates from the stream's memory pool.  _f32: fp32 output. */
 long long cgk_int4_gemm_counters(int M, int N);
 long long cgk_int4_gemm_parts_floats(int M, int N, int K, int splits);
 int cgk_int4_gemm_parts(const void* x, long long ldx, const void* w_tiles, float* parts, int* counters, void* out,
                         long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
+int cgk_int4_gemm_parts_f32(const void* x, long long ldx, const void* w_tiles, float* parts, int* counters, float* out,
+                            long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
 int cgk_int4_gemm(const void* x, long long ldx, const void* w_tiles, float* acc, int* counters, void* out,
                   long long ldo, const void* bias, int M, int N, int K, int splits, void* stream);
 /* The same product for few rows: warp-level MMAs fed from registers (rows 32 at a time, time grows

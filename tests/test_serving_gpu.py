@@ -84,6 +84,21 @@ def test_int4_gemm_few_rows(M, K, N):
     _lib.assert_device_ok()
 
 
+# an fp32 result of "wb": whole tiles and parts of tiles, rows that end inside a warp, an odd number of steps for the two converting groups
+@pytest.mark.parametrize("M,K,N,group", [(33, 128, 128, 64), (80, 384, 22016, 128), (97, 4096, 640, 128), (130, 1152, 19072, 64)])
+def test_int4_gemm_in_fp32_by_row_tiles(M, K, N, group):
+    torch.manual_seed(M + K)
+    lin = Int4Linear(torch.randn(N, K) * 0.05, torch.randn(N) * 0.1, group).to(DEV)
+    lin.kernel = "wb"
+    x = torch.randn(M, K).bfloat16().to(DEV)
+    ref = x.double() @ lin.dequantized().double() + lin.bias.double()
+    full = lin(x, f32=True)
+    # scale, then weight rounded to bf16 (2^-9 of the terms' norm each), fp32 sums
+    assert full.dtype == torch.float32 and ((full.double() - ref).norm() / ref.norm()).item() < 2 ** -7
+    assert torch.equal(full.bfloat16(), lin(x)) and torch.equal(full, lin(x, f32=True))
+    _lib.assert_device_ok()
+
+
 @pytest.mark.parametrize("N", [256, 22016])
 def test_int4_gemm_few_rows_strided(N):
     L, M, K = _lib.lib(), 19, 1024
