@@ -2,31 +2,31 @@
 //
 // W holds the reference's quantised values (src/quantize/int4.c:10-59, 90-114: row-major [K,N],
 // 4-bit two's complement, even column in the low nibble, one fp32 scale per flat group of
-// `group` elements), reordered tile-major without re-quantising: for n-tile nt (128 columns)
-// and k-step ks (64 rows) one contiguous 4608-byte block holds the tile's 64 rows of 64 bytes
-// followed by the tile's scales as fp32 [64 rows][2 column halves].  A CTA's slab is then one
-// sequential stream, which is what keeps HBM efficient (64-byte pieces of the row-major
-// layout are not); cgk_int4_tile_weights does the reordering.
+// `group` elements), reordered tile-major without re-quantising (cgk_int4_tile_weights): per 128 columns ("features") and 64 k one
+// block of 4352 bytes: for each half of the k 16 bytes of nibbles (q + 8) a feature, nibbles j and j + 4 of a word for k 2 j and
+// 2 j + 1; then, for each half of the features, the 64 k's scales rounded to bf16, which is what the product takes them as.  A CTA's
+// share is then one sequential stream, which is what keeps HBM efficient (64-byte pieces of the row-major layout are not).
 //
-// The shape is weight-bandwidth bound (M <= 128 rows against megabytes of weights):
-//   warp 0    bulk copies of W blocks into a 12-deep ring (bytes in flight cover HBM latency)
-//   warp 3    TMA: X tiles [rows, 64 k] into their own ring of up to 12 stages; only
-//             round_up(M, 8) rows are fetched — the tensor core still multiplies 128 rows, the
-//             others hold whatever shared memory held and only feed output rows nobody stores
-//   warps 4-19 nibbles -> bf16: exact integer (magic-number trick), one multiply by the scale,
-//             stored in the 128-byte-swizzled MN-major operand layout tcgen05 reads.  Columns
-//             stay in the pair order the extraction yields (0,4,1,5,2,6,3,7 within each group
-//             of 8); the epilogue undoes the permutation when it addresses the output.
-//   warp 1    tcgen05.mma, two accumulators in TMEM (128 lanes x 128 columns)
-//   warps 20-23 epilogue.  Whole tile: TMEM -> bias -> bf16 -> global.  Part of a tile: into the part's
+// The weights are the A operand (128 features) and come from tensor memory, the rows of X are the B operand.  The shape is bound by
+// the weights' bytes and by what turns them into an operand.  With the weights written to and read from shared memory that was the
+// limit (1080 of 1110 cycles a step of 128 k, of which 512 for weights and 256 for 128 rows of X however many there are); a thread
+// that has one feature stores its k straight into its lane of tensor memory, its scales are read by all lanes of a warp at once.
+//   warp 0    bulk copies of W blocks into a ring as deep as shared memory allows (bytes in flight cover HBM latency)
+//   warp 3    TMA: X tiles [rows, 64 k] into their own ring of up to 6 stages; round_up(M, 16) rows.  One lane issues: eight lanes,
+//             each with its own ring slots, held one another up in their waits (80 rows of 4096 x 32000: 47 -> 37 us)
+//   warps 4-19 two groups: nibbles -> bf16: exact integer (magic-number trick), one multiply by the scale, to tensor memory
+//   warp 1    tcgen05.mma, two accumulators in TMEM (128 lanes x up to 128 columns)
+//   warps 20-23 epilogue, a lane a feature.  Whole tile: TMEM -> bias -> bf16 (or fp32) -> global.  Part of a tile: into the part's
 //             own fp32 slot; the CTA that arrives last at the tile's counter sums the slots in the
-//             order of the CTAs, adds the bias, writes bf16 and leaves the counter zeroed for the
+//             order of the CTAs, adds the bias, writes the output and leaves the counter zeroed for the
 //             next call.  The order is fixed, so a call gives the same bits every time.
-// One CTA per SM.  Each takes as many whole tiles as there are for all of them, then an equal piece of the line of the left-over
-// tiles' steps of 128 k (see int4_gemm_wa.cu).  Whole tiles only left 172 of them (22 016 columns) in two waves on 148 SMs, and a
-// K of 11 008 on 64 CTAs.  80 rows, layers one after the other, whole tiles or equal parts of them by atomics / like this: 4096 x 22016
-// 68.8 / 46.5 us, 11008 x 4096 52.1 / 28.7, 4096 x 32000 70.1 / 61.6, 2048 x 11264 (a tile per CTA on 88 SMs) 19.9 / 19.5.
-// The sum of the CTA's last shared tile is work of all its threads: by the epilogue's 128 these took 50.9, 33.3, 64.7 and 24.0.
+// 80 rows, layers one after the other, operand through shared / through tensor memory (the deal below included): 4096 x 6144
+// 17.7 / 11.4 us, 4096 x 4096 14.5 / 10.2, 4096 x 22016 32.1 / 24.8, 11008 x 4096 20.8 / 17.2, 4096 x 32000 44.8 / 34.3,
+// 2048 x 11264 15.0 / 11.3.  A step takes some 850 cycles: eight MMAs of 16 k with A in tensor memory (70 to 90 each, whatever the
+// rows), issue slots that the converting warps share with the MMA warp, and from 128 rows on the 32 KB of X.
+// One CTA per SM.  Each takes as many whole tiles as there are for all of them; the tiles that are left over are shared (deal, below).
+// The sum of the CTA's last shared tile is work of all its threads; four of a thread's quads are on their way at a time (one: 22016
+// columns took 45 us instead of 32).
 #include <cuda_bf16.h>
 #include <stdlib.h>
 
@@ -38,68 +38,84 @@ namespace {
 using namespace cgk;
 
 constexpr int BM = 128, BN = 128, BK = 64;
-constexpr int ISSUE_LANES = 8;                                // threads of a producer warp that issue copies
 constexpr int SUB = 2;                                        // 64-row sub-tiles per pipeline step (a step covers 128 k)
-constexpr int B_STAGES = 3, MAX_RAW_STAGES = 16, MAX_A_STAGES = 8;
+constexpr int B_STAGES = 4, MAX_RAW_STAGES = 16, MAX_A_STAGES = 8;
+constexpr int ACC_COLS = 2 * BM, W_COLS = SUB * BK / 2, TMEM_COLS = 512;              // two accumulators, then B_STAGES operands of W_COLS columns
 constexpr int GROUPS = 2, GROUP_WARPS = 8, CONVERT_WARPS = GROUPS * GROUP_WARPS;     // converting warps: groups that take the steps in turn
-constexpr int B_BYTES = BK * BN * 2;
-constexpr int NIB_BYTES = BK * BN / 2, SCALE_BYTES = BK * 2 * 4, RAW_BYTES = NIB_BYTES + SCALE_BYTES;   // 4096 + 512
+constexpr int NIB_BYTES = BK * BN / 2, SCALE_BYTES = BK * 2 * 2, RAW_BYTES = NIB_BYTES + SCALE_BYTES;   // 4096 + 256
 constexpr int EPI_WARP0 = 4 + CONVERT_WARPS, THREADS = 32 * (EPI_WARP0 + 4);
-constexpr int SMEM_BYTES = 226 * 1024;                       // alignment slack | X ring | B ring | W ring | barriers
-constexpr int RING_BUDGET = SMEM_BYTES - 1024 - B_STAGES * SUB * B_BYTES - 2048;   // shared by the X and W rings
+constexpr int SMEM_BYTES = 226 * 1024;                       // alignment slack | X ring | W ring | barriers
+constexpr int RING_BUDGET = SMEM_BYTES - 1024 - 2048;        // shared by the X and W rings
 
 struct Int4Dev {
-  const uint8_t* w_tiles;          // [N/128][K/64][4608]
-  float4* parts;                   // slots of shared tiles' parts: [m_tiles][sharers][2][32 column quads][a_rows]
+  const uint8_t* w_tiles;          // [N/128][K/64][4352]
+  float4* parts;                   // slots of shared tiles' parts: [m_tiles][sharers][2][a_rows][32 column quads]
   int* counters;                   // int32 [m_tiles * n_tiles], zero between calls (shared tiles only)
   void* out; long long ldo;        // bf16, or fp32 with out_f32
   const __nv_bfloat16* bias;
   int M, N, K, out_f32;
-  int a_rows, a_stages;            // rows fetched per X tile (multiple of 8), depth of the X ring
+  int a_rows, a_stages;            // rows fetched per X tile (multiple of 16: columns of the MMA), depth of the X ring
   int raw_stages;                  // depth of the W ring
-  int sharers;                     // CTAs that the left-over tiles are dealt to
+  int sharers, per_tile;           // CTAs that the left-over tiles are dealt to; with per_tile: that many to each of them
+  int piece, longer;               // steps of a sharer's piece; how many have one more
   int* status;
 };
 
-// Slot `which` of a sharer: [32 column quads][a_rows] float4s.
+// The steps of the left-over tiles, dealt to the sharers in order, in pieces that differ by one step at most: of the whole line, or
+// (per_tile > 0) of each tile.
+struct Shares {
+  uint32_t per_tile, k_tiles, q, r;                          // a line is q steps for each piece and one more for the first r
+  __device__ __forceinline__ explicit Shares(const Int4Dev& g, uint32_t k_tiles) : per_tile(g.per_tile), k_tiles(k_tiles), q(g.piece), r(g.longer) {}
+  __device__ __forceinline__ uint32_t begin(uint32_t c) const {
+    const uint32_t t = per_tile ? c / per_tile : 0, j = c - t * per_tile;
+    return t * k_tiles + j * q + min(j, r);
+  }
+  // the sharers that left-over tile t begins and ends with
+  __device__ __forceinline__ int first(uint32_t t) const { return per_tile ? t * per_tile : of(t * k_tiles); }
+  __device__ __forceinline__ int last(uint32_t t) const { return per_tile ? t * per_tile + per_tile - 1 : of((t + 1) * k_tiles - 1); }
+  __device__ __forceinline__ uint32_t of(uint32_t step) const { return step < r * (q + 1) ? step / (q + 1) : r + (step - r * (q + 1)) / q; }
+};
+
+// Slot `which` of a sharer: [a_rows][32 column quads] float4s.
 __device__ __forceinline__ float4* part_slot(const Int4Dev& g, int mt, int sharer, int which) {
   return g.parts + (long long)((mt * g.sharers + sharer) * 2 + which) * ((BN / 4) * g.a_rows);
 }
 
-// Eight neighbouring elements of the output.
-__device__ __forceinline__ void store8(const Int4Dev& g, long long at, const float4& u, const float4& v) {
-  if (g.out_f32) {
-    float4* p = reinterpret_cast<float4*>((float*)g.out + at);
-    p[0] = u;
-    p[1] = v;
-  } else {
-    *reinterpret_cast<uint4*>((__nv_bfloat16*)g.out + at) = make_uint4(pack_bf16x2(u.x, u.y), pack_bf16x2(u.z, u.w), pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
-  }
+// Four neighbouring elements of the output.
+__device__ __forceinline__ void store4(const Int4Dev& g, long long at, const float4& v) {
+  if (g.out_f32) *reinterpret_cast<float4*>((float*)g.out + at) = v;
+  else *reinterpret_cast<uint2*>((__nv_bfloat16*)g.out + at) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
 }
 
 // The output of a tile out of its parts, summed in the order of the CTAs lo .. hi; `first`: the slot that CTA lo's is in.
 __device__ __forceinline__ void sum_parts(const Int4Dev& g, int mt, int nt, int lo, int hi, int first_slot, int tid, int threads) {
-  __threadfence();
   const int m0 = mt * BM, n0 = nt * BN, rows = min(BM, g.M - m0), stride = 2 * (BN / 4) * g.a_rows;
   const float4* first = part_slot(g, mt, lo, first_slot);
   const float4* others = part_slot(g, mt, lo, 0);
-  for (int e = tid; e < rows * (BN / 8); e += threads) {
-    const int c8 = e / rows, r = e - c8 * rows, at = 2 * c8 * g.a_rows + r, n = n0 + c8 * 8;
-    float4 u = __ldcg(first + at), v = __ldcg(first + at + g.a_rows);
-#pragma unroll 4
-    for (int c = 1; c <= hi - lo; ++c) {
-      const float4* src = others + (long long)c * stride + at;
-      const float4 x = __ldcg(src), y = __ldcg(src + g.a_rows);
-      u.x += x.x; u.y += x.y; u.z += x.z; u.w += x.w;
-      v.x += y.x; v.y += y.y; v.z += y.z; v.w += y.w;
+  constexpr int U = 4;                                     // quads of a thread on their way at a time, times two parts
+  const int quads = rows * (BN / 4), c1 = hi - lo;
+  for (int e0 = tid; e0 < quads; e0 += U * threads) {
+    float4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = __ldcg(first + min(e0 + u * threads, quads - 1));
+#pragma unroll 2
+    for (int c = 1; c <= c1; ++c) {
+      float4 x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) x[u] = __ldcg(others + (long long)c * stride + min(e0 + u * threads, quads - 1));
+#pragma unroll
+      for (int u = 0; u < U; ++u) { v[u].x += x[u].x; v[u].y += x[u].y; v[u].z += x[u].z; v[u].w += x[u].w; }
     }
-    if (g.bias) {
-      u.x += __bfloat162float(g.bias[n]); u.y += __bfloat162float(g.bias[n + 1]);
-      u.z += __bfloat162float(g.bias[n + 2]); u.w += __bfloat162float(g.bias[n + 3]);
-      v.x += __bfloat162float(g.bias[n + 4]); v.y += __bfloat162float(g.bias[n + 5]);
-      v.z += __bfloat162float(g.bias[n + 6]); v.w += __bfloat162float(g.bias[n + 7]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = e0 + u * threads, t = e / (BN / 4), n = n0 + e % (BN / 4) * 4;
+      if (e >= quads) break;
+      if (g.bias) {
+        v[u].x += __bfloat162float(g.bias[n]); v[u].y += __bfloat162float(g.bias[n + 1]);
+        v[u].z += __bfloat162float(g.bias[n + 2]); v[u].w += __bfloat162float(g.bias[n + 3]);
+      }
+      store4(g, (long long)(m0 + t) * g.ldo + n, v[u]);
     }
-    store8(g, (long long)(m0 + r) * g.ldo + n, u, v);
   }
 }
 
@@ -108,9 +124,8 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t sA = base;                                         // a_stages x (a_rows * 128 B); reads of 128 rows may run into sB
-  const uint32_t sB = sA + (uint32_t)g.a_stages * SUB * (uint32_t)g.a_rows * 128u;   // B_STAGES x SUB x 16 KiB
-  const uint32_t sRaw = sB + B_STAGES * SUB * B_BYTES;              // raw_stages x SUB x 4608 B
+  const uint32_t sA = base;                                         // a_stages x SUB x (a_rows * 128 B)
+  const uint32_t sRaw = sA + (uint32_t)g.a_stages * SUB * (uint32_t)g.a_rows * 128u;   // raw_stages x SUB x 4352 B
   const uint32_t sBar = base + SMEM_BYTES - 2048;
   const uint8_t* raw_s = gen + (sRaw - base);
   volatile int* dead = reinterpret_cast<volatile int*>(gen + (sBar - base) + 960);
@@ -129,7 +144,7 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
   const int n_tiles = g.N / BN, k_tiles = g.K / (SUB * BK), mt = blockIdx.y, m0 = mt * BM;
   // This CTA's steps of 128 k: its `own` steps of whole tiles, then its piece of the line of the tiles that are left over.
   const int ctas = gridDim.x, whole = n_tiles / ctas * ctas, own = n_tiles / ctas * k_tiles, sharers = g.sharers;
-  const Pieces pieces((uint32_t)((n_tiles - whole) * k_tiles), (uint32_t)sharers);
+  const Shares pieces(g, (uint32_t)k_tiles);
   const int cta = blockIdx.x, r0 = (int)pieces.begin(min(cta, sharers));
   const int ksteps = own + (int)pieces.begin(min(cta + 1, sharers)) - r0, a_stages = g.a_stages, RAW_STAGES = g.raw_stages;
   auto line = [&](int i) -> int { return i < own ? cta * own + i : whole * k_tiles + r0 + (i - own); };
@@ -145,7 +160,7 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
     *is_last = 0;
     mbar_fence_init();
   }
-  if (warp == 2) { tmem_alloc(smem_u32(tmem_slot), 2 * BN); tmem_relinquish(); }
+  if (warp == 2) { tmem_alloc(smem_u32(tmem_slot), TMEM_COLS); tmem_relinquish(); }
   // the first weights (no earlier kernel's business) start on their way to L2 while the predecessor still runs
   if (warp == 0 && blockIdx.y == 0 && lane < min(ksteps, 14)) prefetch_l2(g.w_tiles + (long long)line(lane) * (SUB * RAW_BYTES), SUB * RAW_BYTES);
   tc_fence_before();
@@ -156,44 +171,34 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    // A thread's bulk copies run one after the other (measured: ~0.43 us each, whatever the ring
-    // depth), so several lanes issue, each with its own copies in flight.  A ring slot always
-    // belongs to the same lane: its uses are then waited for in order, which the one-bit phase
-    // parity of an mbarrier requires.
-    if (lane < ISSUE_LANES) {
+    if (lane == 0) {
       int r = 0;
       uint32_t par = 1;
       for (int i = 0; i < ksteps; ++i) {
-        const int here = r;
-        const uint32_t phase = par;
+        if (!mbar_wait(raw_empty(r), par, dead, g.status, 300)) break;
+        mbar_expect_tx(raw_full(r), SUB * RAW_BYTES);
+        bulk_load_1d(sRaw + r * (SUB * RAW_BYTES), g.w_tiles + (long long)line(i) * (SUB * RAW_BYTES), SUB * RAW_BYTES, raw_full(r));
         if (++r == RAW_STAGES) { r = 0; par ^= 1; }
-        if (here % ISSUE_LANES != lane) continue;
-        if (!mbar_wait(raw_empty(here), phase, dead, g.status, 300)) break;
-        mbar_expect_tx(raw_full(here), SUB * RAW_BYTES);
-        bulk_load_1d(sRaw + here * (SUB * RAW_BYTES), g.w_tiles + (long long)line(i) * (SUB * RAW_BYTES), SUB * RAW_BYTES, raw_full(here));
       }
     }
   } else if (warp == 3) {
-    if (lane < ISSUE_LANES) {
-      if (lane == 0) tma_prefetch_desc(&tmX);
-      int next = 0;
+    if (lane == 0) {
+      tma_prefetch_desc(&tmX);
+      int s = 0;
       uint32_t par = 1;
       for (int i = 0; i < ksteps; ++i) {
-        const int s = next;
-        const uint32_t phase = par;
-        if (++next == a_stages) { next = 0; par ^= 1; }
-        if (s % ISSUE_LANES != lane) continue;
         const int ks = line(i) % k_tiles;                             // step within its tile
-        if (!mbar_wait(a_empty(s), phase, dead, g.status, 301)) break;
+        if (!mbar_wait(a_empty(s), par, dead, g.status, 301)) break;
         mbar_expect_tx(a_full(s), SUB * a_bytes);
 #pragma unroll
         for (int sub = 0; sub < SUB; ++sub)
           tma_load_2d(sA + (s * SUB + sub) * a_bytes, &tmX, a_full(s), (ks * SUB + sub) * BK, m0);
+        if (++s == a_stages) { s = 0; par ^= 1; }
       }
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(BM, BN, 0, 1);
+      const uint32_t idesc = make_idesc_bf16(BN, g.a_rows, 0, 0);
       bool ok = true;
       int left = 0, part = -1;
       bool first = true;
@@ -210,14 +215,13 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
         const uint32_t a_there = mbar_try_wait(a_full(sa), pa), b_there = mbar_try_wait(b_full(sb), pb);
         if (!(a_there & b_there) && (!mbar_wait(a_full(sa), pa, dead, g.status, 302) || !mbar_wait(b_full(sb), pb, dead, g.status, 303))) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d = tmem + (uint32_t)(part & 1) * BN;
+        const uint32_t d = tmem + (uint32_t)(part & 1) * BM, w = tmem + ACC_COLS + (uint32_t)sb * W_COLS;
 #pragma unroll
         for (int sub = 0; sub < SUB; ++sub) {
-          const uint32_t a_addr = sA + (sa * SUB + sub) * a_bytes, b_addr = sB + (sb * SUB + sub) * B_BYTES;
+          const uint32_t a_addr = sA + (sa * SUB + sub) * a_bytes;
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk)
-            umma_f16(d, make_smem_desc_sw128(a_addr + kk * 32, 16u, 1024u), make_smem_desc_sw128(b_addr + kk * 2048, 8192u, 1024u), idesc,
-                     (!first || (sub | kk) != 0) ? 1u : 0u);
+          for (int kk = 0; kk < BK / 16; ++kk)             // 16 k: 8 columns of W, 32 bytes along a row of X
+            umma_f16_ts(d, w + (sub * (BK / 16) + kk) * 8, make_smem_desc_sw128(a_addr + kk * 32, 16u, 1024u), idesc, (!first || (sub | kk) != 0) ? 1u : 0u);
         }
         first = false;
         umma_commit(a_empty(sa));
@@ -229,12 +233,11 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
     }
   } else if (warp >= 4 && warp < EPI_WARP0) {
     // Group gi has steps gi, gi + 2, ..: while one waits for its buffers or for the answers to its polls, the other converts.
-    const int gi = (warp - 4) / GROUP_WARPS, tid = threadIdx.x - 128 - gi * (32 * GROUP_WARPS);
-    constexpr int WORDS = BK * BN / 8 / (32 * GROUP_WARPS);            // per thread and 64-row sub-tile: rows 16 apart, the same 8 columns
-    const int k0 = tid >> 4, jw = tid & 15;
-    const uint8_t* const raw0 = raw_s + tid * 4;
-    const uint8_t* const scale0 = raw_s + NIB_BYTES + k0 * 8 + (jw >> 3) * 4;
-    const uint32_t dst0 = sB + (jw >> 3) * 8192u + sw128_offset((uint32_t)k0, (uint32_t)(jw & 7));    // 16 rows on: 2048 bytes
+    // A thread has one feature (a lane of tensor memory) and one 64-k block of a step.
+    const int gi = (warp - 4) / GROUP_WARPS, quad = warp & 3, sub = ((warp - 4) >> 2) & 1, f = quad * 32 + lane;
+    const uint8_t* const raw0 = raw_s + sub * RAW_BYTES + f * 16;
+    const uint8_t* const scale0 = raw_s + sub * RAW_BYTES + NIB_BYTES + (quad >> 1) * (BK * 2);
+    const uint32_t dst0 = tmem + ((uint32_t)(quad * 32) << 16) + ACC_COLS + sub * (BK / 2);
     uint32_t mask = 0x000F000Fu, magic = 0x43004300u;
     asm volatile("" : "+r"(mask), "+r"(magic));
     const __nv_bfloat162 off = __float2bfloat162_rn(136.0f);
@@ -250,34 +253,30 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
         if (!got) got = mbar_wait(raw_full(r), pr, dead, g.status, 304) && mbar_wait(b_empty(s), ps, dead, g.status, 305);
       }
       if (!__shfl_sync(0xffffffffu, got, 0)) break;
+      tc_fence_after();
       const uint8_t* raw = raw0 + r * (SUB * RAW_BYTES);
       const uint8_t* scales = scale0 + r * (SUB * RAW_BYTES);
-      const uint32_t dst = dst0 + s * (SUB * B_BYTES);
 #pragma unroll
-      for (int sub = 0; sub < SUB; ++sub) {
-        uint32_t v[WORDS];
-        float sc[WORDS];
+      for (int half = 0; half < 2; ++half) {
+        const uint4 w4 = *reinterpret_cast<const uint4*>(raw + half * (NIB_BYTES / 2));
+        const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+        uint32_t t[16];
 #pragma unroll
-        for (int it = 0; it < WORDS; ++it) {
-          v[it] = *reinterpret_cast<const uint32_t*>(raw + sub * RAW_BYTES + it * (32 * GROUP_WARPS * 4));
-          sc[it] = *reinterpret_cast<const float*>(scales + sub * RAW_BYTES + it * (16 * 8));
-        }
-#pragma unroll
-        for (int it = 0; it < WORDS; ++it) {
-          const uint32_t w = v[it] ^ 0x88888888u;          // two's complement -> q + 8
-          const __nv_bfloat162 sc2 = __float2bfloat162_rn(sc[it]);
-          uint32_t t[4];
+        for (int c = 0; c < 4; ++c) {
+          const uint4 s4 = *reinterpret_cast<const uint4*>(scales + (half * 4 + c) * 16);      // of eight k, for all lanes
+          const uint32_t sc[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const uint32_t u = pick(w >> (4 * j), mask, magic);           // bf16 (128 + q + 8) for columns j and j + 4
-            const __nv_bfloat162 h = __hmul2(__hsub2(*reinterpret_cast<const __nv_bfloat162*>(&u), off), sc2);
-            t[j] = *reinterpret_cast<const uint32_t*>(&h);
+            const uint32_t u = pick(w[c] >> (4 * j), mask, magic);        // bf16 (128 + q + 8) of k 2 j and 2 j + 1
+            const __nv_bfloat162 h = __hmul2(__hsub2(*reinterpret_cast<const __nv_bfloat162*>(&u), off), *reinterpret_cast<const __nv_bfloat162*>(&sc[j]));
+            t[4 * c + j] = *reinterpret_cast<const uint32_t*>(&h);
           }
-          // positions 0..7 of the chunk hold columns 0,4,1,5,2,6,3,7
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + sub * B_BYTES + it * 2048), "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");
         }
+        __syncwarp();
+        tmem_st16(dst0 + s * W_COLS + half * 16, t);
       }
-      fence_proxy_async_smem();
+      tmem_st_wait();
+      tc_fence_before();
       __syncwarp();
       if (lane == 0) { mbar_arrive(b_full(s)); mbar_arrive(raw_empty(r)); }
       r += GROUPS;
@@ -286,49 +285,42 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
       if (s >= B_STAGES) { s -= B_STAGES; ps ^= 1; }
     }
   } else if (warp >= EPI_WARP0) {
-    // ---- epilogue: lane = output row inside the 128-row tile.
-    // Accumulator positions j..j+7 of a group of 8 are columns j + {0,4,1,5,2,6,3,7}.
+    // ---- epilogue: lane = output feature of the tile, accumulator column = row of X.
     // Every thread goes through every part and its barriers, also after a wait that gave up (later waits return at once).
-    const int q = warp & 3, et = threadIdx.x - 32 * EPI_WARP0, row = m0 + q * 32 + lane;
+    const int q = warp & 3, et = threadIdx.x - 32 * EPI_WARP0, f = q * 32 + lane;
     bool ok = true;
     int part = 0;
     for (int i = 0; i < ksteps; ++part) {
       const int nt = line(i) / k_tiles, n0 = nt * BN, a = part & 1;
       // the CTAs that share a left-over tile
       const uint32_t t0 = (uint32_t)((nt - whole) * k_tiles);
-      const int lo = nt < whole ? 0 : (int)pieces.of(t0), hi = nt < whole ? 0 : (int)pieces.of(t0 + k_tiles - 1);
+      const int lo = nt < whole ? 0 : pieces.first(nt - whole), hi = nt < whole ? 0 : pieces.last(nt - whole);
       // a CTA's piece may end one shared tile and begin another: slot 0 for the part it begins with, 1 for the other
-      float4* const mine = part_slot(g, mt, cta, i != own) + q * 32 + lane;
+      float* const mine = lo == hi ? nullptr : reinterpret_cast<float*>(part_slot(g, mt, cta, i != own)) + f;
+      const float bias = g.bias && !mine ? __bfloat162float(g.bias[n0 + f]) : 0.0f;
       i += part_steps(i);
       ok = __all_sync(0xffffffffu, mbar_wait(acc_full(a), (part >> 1) & 1, dead, g.status, 306)) && ok;
       tc_fence_after();
       if (ok) {
+        const int rows = min(g.a_rows, g.M - m0);
+        float* const out_f = (float*)g.out + (long long)m0 * g.ldo + n0 + f;
+        __nv_bfloat16* const out_b = (__nv_bfloat16*)g.out + (long long)m0 * g.ldo + n0 + f;
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t rr[32];
+        for (int c = 0; c < g.a_rows; c += 16) {
+          uint32_t rr[16];
           __syncwarp();
-          tmem_ld32(tmem + a * BN + ((uint32_t)(q * 32) << 16) + c, rr);
+          tmem_ld16(tmem + a * BM + ((uint32_t)(q * 32) << 16) + c, rr);
           tmem_ld_wait();
-          // a slot takes all its rows, so that no memory sector is written in part (17 rows, 4096 x 22016, cold caches: 55 -> 51 us)
-          if (lo == hi ? row >= g.M : q * 32 + lane >= g.a_rows) continue;
-          if (lo == hi) {
+          if (mine) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              float v[8] = {__uint_as_float(rr[j]), __uint_as_float(rr[j + 2]), __uint_as_float(rr[j + 4]), __uint_as_float(rr[j + 6]),
-                            __uint_as_float(rr[j + 1]), __uint_as_float(rr[j + 3]), __uint_as_float(rr[j + 5]), __uint_as_float(rr[j + 7])};
-              if (g.bias) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] += __bfloat162float(g.bias[n0 + c + j + e]);
-              }
-              store8(g, (long long)row * g.ldo + n0 + c + j, make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]));
-            }
+            for (int j = 0; j < 16; ++j) mine[(c + j) * BN] = __uint_as_float(rr[j]);
           } else {
-            // neighbouring lanes hold neighbouring rows: 16 bytes each, side by side
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              float4* dstp = mine + (c + j) / 4 * g.a_rows;
-              dstp[0] = make_float4(__uint_as_float(rr[j]), __uint_as_float(rr[j + 2]), __uint_as_float(rr[j + 4]), __uint_as_float(rr[j + 6]));
-              dstp[g.a_rows] = make_float4(__uint_as_float(rr[j + 1]), __uint_as_float(rr[j + 3]), __uint_as_float(rr[j + 5]), __uint_as_float(rr[j + 7]));
+            for (int j = 0; j < 16; ++j) {
+              const float v = __uint_as_float(rr[j]) + bias;
+              if (c + j >= rows) break;
+              if (g.out_f32) out_f[(c + j) * g.ldo] = v;
+              else out_b[(c + j) * g.ldo] = __float2bfloat16(v);
             }
           }
         }
@@ -338,10 +330,13 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
       if (lane == 0) mbar_arrive(acc_empty(a));
       if (lo == hi) continue;
       // the CTA that arrives last at the tile's counter turns the parts into the output
-      __threadfence();
       asm volatile("bar.sync 1, 128;" ::: "memory");
       int* counter = g.counters + mt * n_tiles + nt;
-      if (et == 0) *is_last = (atomicAdd(counter, 1) == hi - lo) && !*dead;
+      if (et == 0) {                                        // the barriers hand the others' parts to this thread and its view to them
+        int before;
+        asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+        *is_last = before == hi - lo && !*dead;
+      }
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (i == ksteps) break;                               // the CTA's last part: all its threads take part in the sum, below
       if (*is_last) {
@@ -354,11 +349,11 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
   if (*dead) __nanosleep(100000);
   tc_fence_before();
   __syncthreads();
-  if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, 2 * BN); }
+  if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem, TMEM_COLS); }
   if (ksteps > own && *is_last) {
     const int nt = line(ksteps - 1) / k_tiles;
     const uint32_t t0 = (uint32_t)((nt - whole) * k_tiles);
-    const int lo = (int)pieces.of(t0), hi = (int)pieces.of(t0 + k_tiles - 1);
+    const int lo = pieces.first(nt - whole), hi = pieces.last(nt - whole);
     if (lo != hi) {
       sum_parts(g, mt, nt, lo, hi, pieces.begin(lo) < t0, threadIdx.x, THREADS);
       if (threadIdx.x == 0) g.counters[mt * n_tiles + nt] = 0;
@@ -366,7 +361,7 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
   }
 }
 
-// packed [K][N/2] bytes + scales (flat groups) -> tiles [N/128][K/64][4608]
+// packed [K][N/2] bytes + scales (flat groups) -> tiles [N/128][K/64][4352]
 __global__ void int4_tile_kernel(const uint8_t* __restrict__ packed, const float* __restrict__ scales, int K, int N, int group,
                                  uint8_t* __restrict__ tiles) {
   const int k_tiles = K / BK;
@@ -374,13 +369,20 @@ __global__ void int4_tile_kernel(const uint8_t* __restrict__ packed, const float
   for (long long blk = blockIdx.x; blk < blocks; blk += gridDim.x) {
     const int nt = (int)(blk / k_tiles), ks = (int)(blk % k_tiles);
     uint8_t* dst = tiles + blk * RAW_BYTES;
-    for (int i = threadIdx.x; i < NIB_BYTES / 4; i += blockDim.x) {
-      const int k = i >> 4, wj = i & 15;
-      reinterpret_cast<uint32_t*>(dst)[i] = *reinterpret_cast<const uint32_t*>(packed + ((long long)(ks * BK + k) * N + nt * BN) / 2 + wj * 4);
+    for (int i = threadIdx.x; i < NIB_BYTES / 4; i += blockDim.x) {       // word i: k half i / 512, feature (i % 512) / 4, word i % 4
+      const int f = nt * BN + ((i & 511) >> 2), k0 = ks * BK + (i >> 9) * 32 + (i & 3) * 8;
+      uint32_t word = 0;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {                                       // nibbles j and j + 4: k 2 j and 2 j + 1
+        const uint8_t byte = packed[((long long)(k0 + e) * N + f) >> 1];
+        const uint32_t nib = ((f & 1) ? (byte >> 4) : (byte & 0xF)) ^ 8u;
+        word |= nib << (4 * ((e >> 1) + 4 * (e & 1)));
+      }
+      reinterpret_cast<uint32_t*>(dst)[i] = word;
     }
     for (int i = threadIdx.x; i < BK * 2; i += blockDim.x) {
-      const int k = i >> 1, half = i & 1;
-      reinterpret_cast<float*>(dst + NIB_BYTES)[i] = scales[((long long)(ks * BK + k) * N + nt * BN + half * 64) / group];
+      const int half = i / BK, k = i % BK;
+      reinterpret_cast<__nv_bfloat16*>(dst + NIB_BYTES)[i] = __float2bfloat16(scales[((long long)(ks * BK + k) * N + nt * BN + half * 64) / group]);
     }
   }
 }
@@ -404,18 +406,30 @@ CGK_API long long cgk_int4_gemm_counters(int M, int N) { return (long long)((M +
 
 // How the tiles are dealt out: one CTA per SM (of a row tile's share of them), each with at least two steps of the left-over
 // tiles; given splits: that many equal parts of every tile; without a place for parts: whole tiles.
-struct Deal { long long ctas, sharers; };
+// The left-over tiles, by the fewest steps of: each tile's steps in p pieces of its own (1: the tile stays whole), 2 p steps' worth of
+// time for storing and summing the parts; or the line of all their steps in equal pieces, 10 for parts of two tiles in most CTAs and
+// tiles that wait for CTAs which have another one to end first.  80 rows, line / own pieces: 4096 x 4096 (4 pieces) 12.1 / 10.2 us,
+// 4096 x 22016 (4) 31.4 / 24.8, 4096 x 6144 (3) 13.1 / 11.4, 2048 x 11264 (whole, 88 CTAs) 12.0 / 11.3; 11008 x 4096 stays a line
+// (17.0 / 17.0), 4096 x 32000 has 102 whole tiles (35.2 / 34.3).
+struct Deal { long long ctas, sharers; int per_tile; };
 static Deal deal(int sms, int M, int N, int K, int splits, bool parts) {
   const long long n_tiles = N / BN, m_tiles = (M + BM - 1) / BM, ksteps = K / (SUB * BK);
-  if (splits > 0 || !parts) return {n_tiles * (splits > 0 ? splits : 1), splits > 1 ? n_tiles * splits : 1};
+  if (splits > 0 || !parts) return {n_tiles * (splits > 0 ? splits : 1), splits > 1 ? n_tiles * splits : 1, splits > 1 ? splits : 0};
   long long ctas = sms / m_tiles;
   if (ctas > n_tiles * ksteps / 2) ctas = n_tiles * ksteps / 2;
   if (ctas < 1) ctas = 1;
-  // the fewest sharers with the same longest piece: fewer parts to store and to sum
-  const long long rest = n_tiles % ctas * ksteps, most = rest / 2 < 1 ? 1 : rest / 2 < ctas ? rest / 2 : ctas, longest = (rest + most - 1) / most;
-  return {ctas, rest > 0 ? (rest + longest - 1) / longest : 1};
+  const long long left = n_tiles % ctas, rest = left * ksteps;
+  if (left == 0) return {ctas, 1, 0};
+  const long long most = rest / 2 < 1 ? 1 : rest / 2 < ctas ? rest / 2 : ctas, longest = (rest + most - 1) / most;
+  long long best = longest + 10;
+  Deal d = {ctas, (rest + longest - 1) / longest, 0};                        // the fewest sharers with the same longest piece
+  for (long long p = ctas / left < ksteps / 2 ? ctas / left : ksteps / 2; p >= 1; --p) {
+    const long long cost = (ksteps + p - 1) / p + (p > 1 ? 2 * p : 0);
+    if (cost <= best) { best = cost; d = {ctas, left * p, (int)p}; }
+  }
+  return d;
 }
-static int part_rows(int M) { return M > BM ? BM : (M + 7) / 8 * 8; }
+static int part_rows(int M) { return M > BM ? BM : (M + 15) / 16 * 16; }
 
 CGK_API long long cgk_int4_gemm_parts_floats(int M, int N, int K, int splits) {
   int dev = 0;
@@ -438,11 +452,9 @@ static int wb_gemm(const void* x, long long ldx, const void* w_tiles, float* par
   CGK_REQUIRE(splits <= 1 || (parts && counters), "cgk_int4_gemm: split-K needs scratch and counters");
   const Deal d = deal(sm_count(dev), M, N, K, splits, parts && counters);
   const int a_rows = part_rows(M);
-  // X comes from L2 a microsecond after it is asked for: four stages of it, as long as five of W fit beside them (at least 2),
-  // and up to a quarter of the ring budget where rows are few
-  int a_stages = (RING_BUDGET / 4) / (SUB * a_rows * 128);
-  if (a_stages < 4) a_stages = 4;
-  while (a_stages > 2 && RING_BUDGET - a_stages * SUB * a_rows * 128 < 5 * SUB * RAW_BYTES) --a_stages;
+  // X comes from L2 a microsecond after it is asked for: six stages of it, at least three, as long as eight of W fit beside them
+  int a_stages = 6;
+  while (a_stages > 3 && RING_BUDGET - a_stages * SUB * a_rows * 128 < 8 * SUB * RAW_BYTES) --a_stages;
   if (a_stages > MAX_A_STAGES) a_stages = MAX_A_STAGES;
   int raw_stages = (RING_BUDGET - a_stages * SUB * a_rows * 128) / (SUB * RAW_BYTES);
   if (raw_stages > MAX_RAW_STAGES) raw_stages = MAX_RAW_STAGES;
@@ -456,8 +468,10 @@ static int wb_gemm(const void* x, long long ldx, const void* w_tiles, float* par
     CGK_CUDA_CHECK(cudaFuncSetAttribute(int4_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
     attr_set[dev] = true;
   }
+  // a line to deal (each left-over tile's, or all of theirs) and its pieces
+  const long long steps = (long long)(d.per_tile ? 1 : N / BN % d.ctas) * ksteps, pieces = d.per_tile ? d.per_tile : d.sharers;
   Int4Dev g{(const uint8_t*)w_tiles, (float4*)parts, counters, out, ldo, (const __nv_bfloat16*)bias, M, N, K, out_f32,
-            a_rows, a_stages, raw_stages, (int)d.sharers, device_status(dev)};
+            a_rows, a_stages, raw_stages, (int)d.sharers, d.per_tile, (int)(steps / pieces), (int)(steps % pieces), device_status(dev)};
   CGK_CUDA_CHECK(launch_overlapped(int4_gemm_kernel, dim3((unsigned)d.ctas, m_tiles), dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream, 0, tmX, g));
   return 0;
 }

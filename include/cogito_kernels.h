@@ -215,8 +215,8 @@ int cgk_int4_quantize(const float* x, long long n, int group, void* packed, floa
 int cgk_int4_dequantize(const void* packed, const float* scales, long long n, int group, float* out_f32,
                         void* out_bf16, void* stream);
 /* Tile-major reordering of reference-format weights for cgk_int4_gemm: packed [K, N/2] bytes +
- * fp32 scales per flat group -> [N/128][K/64][4608] (64 rows of 64 bytes, then fp32 scales
- * [64][2]).  N % 128 == 0, K % 64 == 0, group a multiple of 64 dividing N. */
+ * fp32 scales per flat group -> [N/128][K/64][4352] (two halves of 32 k: 16 bytes of nibbles for each of
+ * 128 columns; then bf16 scales [2 column halves][64 k]).  N % 128 == 0, K % 64 == 0, group a multiple of 64 dividing N. */
 long long cgk_int4_tiles_bytes(int K, int N);
 int cgk_int4_tile_weights(const void* packed, const float* scales, int K, int N, int group, void* tiles, void* stream);
 /* out[M,N] (bf16, leading dimension ldo) = x[M,K] (bf16) . dequant(w)[K,N] (+ bias).

@@ -99,6 +99,21 @@ def test_int4_gemm_in_fp32_by_row_tiles(M, K, N, group):
     _lib.assert_device_ok()
 
 
+# left-over tiles in pieces of their own (uneven ones too), in equal pieces of their line, whole, and one of a single step; rows about a multiple of 16
+@pytest.mark.parametrize("K,N", [(1152, 6144), (1408, 4096), (5504, 4096), (256, 11264), (128, 640)])
+@pytest.mark.parametrize("M", [47, 48, 113, 129])
+def test_int4_gemm_by_ways_to_deal_tiles(M, K, N):
+    torch.manual_seed(M + K)
+    lin = Int4Linear(torch.randn(N, K) * 0.05, torch.randn(N) * 0.1, 64).to(DEV)
+    lin.kernel = "wb"
+    x = torch.randn(M, K).bfloat16().to(DEV)
+    ref = x.double() @ lin.dequantized().double() + lin.bias.double()
+    # scale, then weight rounded to bf16 (2^-9 of the terms' norm each), fp32 sums; a bf16 result 2^-9 of its own
+    got = lin(x, f32=True)
+    assert ((got.double() - ref).norm() / ref.norm()).item() < 2 ** -7 and torch.equal(got.bfloat16(), lin(x))
+    _lib.assert_device_ok()
+
+
 @pytest.mark.parametrize("N", [256, 22016])
 def test_int4_gemm_few_rows_strided(N):
     L, M, K = _lib.lib(), 19, 1024
