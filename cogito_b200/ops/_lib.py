@@ -23,7 +23,7 @@ if not _DEBUG and not _LIB_PATH.exists() and (_LIB_DIR / "libcogito_kernels_serv
 _lib = None
 # source files that carry index checks in the debug build (one recorded violation each)
 _BOUNDS_FILES = ("gemm_tcgen05", "gemm_few", "softmax_ce", "serving", "elementwise", "flash_fwd", "flash_bwd", "residual_stream", "latent_kv",
-                 "latent_attn_tc", "moe", "kv_rows", "linear_state", "linear_state_tc")
+                 "latent_attn_tc", "moe", "kv_rows", "kv_attn_mma", "linear_state", "linear_state_tc")
 
 
 class KernelError(RuntimeError):

@@ -112,20 +112,22 @@ class _Counters:
 class Int4Linear(torch.nn.Module):
     """y = x @ W^T (+ bias) with W stored as packed INT4 of W^T ([in, out], groups along out)."""
 
-    # Which kernel multiplies: "wb" keeps the weights as the B operand of tcgen05 MMAs (converted tile in shared
-    # memory, 128 token rows per instruction), "wa" makes them the A operand of warp-level MMAs, fed from registers (cost
-    # follows the token count; needs group % 128 == 0).  "auto": "wa" up to 32 token rows, "wb" up to two row
+    # Which kernel multiplies: "wb" makes the weights the A operand of tcgen05 MMAs (converted tile in tensor
+    # memory, up to 128 token rows per instruction), "wa" makes them the A operand of warp-level MMAs, fed from registers (cost
+    # follows the token count; needs group % 128 == 0).  "auto": "wa" up to 16 token rows, "wb" up to two row
     # tiles, and beyond that (prompts) the weights are dequantised to bf16 once per call for the dense GEMM: "wb" converts
     # every weight tile again for each row tile.  That copy (2 bytes per weight: 180 MB for 4096 x 22016, 262 MB for
     # 4096 x 32000) comes from the allocator for the time of the call, one layer's at a time; where there is no room for it,
     # "wb" takes the call.  Each of the two kernels has its own tile-major copy of the weights, made on
     # first use; both sum the parts of a shared tile in a fixed order, so a call gives the same bits every time.
     # Times (us, layers one after the other) for 4096 x 6144, 4096 x 4096, 4096 x 22016, 11008 x 4096, 4096 x 32000, 2048 x 11264:
-    #   16 rows   "wa" 8.4 6.5 20.6 11.0 25.9 10.3      (before, through tensor memory: 20.1 14.9 34.7 24.7 44.6 19.2)
-    #   32 rows   "wa" 12.8 9.0 31.5 15.7 39.8 15.5     "wb" 14.7 12.4 29.7 18.8 39.1 13.3
-    #   80 rows   "wa" 27.4 22.4 75.4 40.5 107 28.4     "wb" 17.7 14.5 32.1 20.8 44.8 15.0 (three passes over the weights)
-    #   200 rows  "wb" 24.7 20.6 83.4 35.1 111 24.3     dense 31.4 26.5 104 61.1 131 32.7 (a third row tile adds half to "wb")
-    FEW_ROWS, DENSE_ROWS = 32, 256
+    #   16 rows   "wa" 8.5 6.5 21.0 11.1 26.3 10.4      "wb" 9.6 8.4 22.5 14.3 30.7 9.3
+    #   17 rows   "wa" 12.6 9.1 31.3 15.8 39.4 15.4     "wb" 9.8 8.6 22.6 14.7 30.8 9.5    (four columns of MMAs instead of two)
+    #   32 rows   "wa" 12.9 9.1 31.8 15.9 40.1 15.6     "wb" 10.1 8.9 23.3 15.0 31.5 9.8
+    #   80 rows                                         "wb" 11.4 10.2 24.8 17.2 34.3 11.3
+    #   200 rows  "wb" 19.5 14.6 44.7 27.2 63.3 18.8    dense 31.4 26.5 104 61.1 131 32.7
+    # The line to the dense GEMM stays where the weights would be rounded once more than there.
+    FEW_ROWS, DENSE_ROWS = 16, 256
     kernel = os.environ.get("COGITO_INT4_KERNEL", "auto")
 
     def __init__(self, weight: torch.Tensor, bias: torch.Tensor | None = None, group: int = 128):
