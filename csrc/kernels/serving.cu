@@ -744,16 +744,19 @@ CGK_API int cgk_kv_int4_append_rows(const cgk_kv_args* a, const void* k_new, con
 CGK_API long long cgk_kv_int4_attention_scratch_floats(int batch, int Hq, int Tq, int D, int splits) {
   return (long long)batch * Hq * Tq * splits * (D + 2);
 }
+// The few-row kernel copies K and V 16 bytes at a time and the scales of a key and head (4, 8 or 16 bytes) in one piece: pools
+// that lie on smaller boundaries are for the kernels that read single words.
 CGK_API int cgk_kv_int4_attention_few(const cgk_kv_args* a, int Tq, int Hq) {
-  return a && a->heads > 0 && a->D == 128 && a->group % 32 == 0 && Hq % a->heads == 0 && (long long)Tq * (Hq / a->heads) <= KV_FEW_ROWS;
+  if (!a || a->heads <= 0 || a->D != 128 || a->group < 32 || a->group % 32 != 0 || Hq % a->heads != 0 || (long long)Tq * (Hq / a->heads) > KV_FEW_ROWS) return 0;
+  return (((uintptr_t)a->k_pages | (uintptr_t)a->v_pages) & 15) == 0 &&
+         (((uintptr_t)a->k_scales | (uintptr_t)a->v_scales) & (uintptr_t)(4 * (a->D / a->group) - 1)) == 0;
 }
 // The few-row kernel over rows of q that lie bs, ts, hs elements apart (cgk_kv_int4_attention_few says whether it takes the call).
 CGK_API int cgk_kv_int4_attention_strided(const cgk_kv_args* a, const void* q, long long bs, long long ts, long long hs, void* out, int Tq, int Hq, float scale,
                                           int splits, void* stream) {
   if (int rc = check_kv(a, "cgk_kv_int4_attention")) return rc;
   CGK_REQUIRE(q && out && Tq > 0 && splits > 0 && cgk_kv_int4_attention_few(a, Tq, Hq), "cgk_kv_int4_attention_strided: bad argument");
-  CGK_REQUIRE(((bs | ts | hs) & 7) == 0 && (((uintptr_t)q | (uintptr_t)a->k_pages) & 15) == 0 && ((uintptr_t)a->v_pages & 7) == 0 && ((uintptr_t)out & 7) == 0,
-              "cgk_kv_int4_attention_strided: misaligned rows");
+  CGK_REQUIRE(((bs | ts | hs) & 7) == 0 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)out & 7) == 0, "cgk_kv_int4_attention_strided: misaligned rows");
   CGK_CUDA_CHECK(launch_kv_attention_mma(kv_dev(a), (const __nv_bfloat16*)q, bs, ts, hs, Tq, Hq, scale, splits, (__nv_bfloat16*)out, (cudaStream_t)stream));
   return 0;
 }
@@ -762,6 +765,7 @@ CGK_API int cgk_kv_int4_attention_strided(const cgk_kv_args* a, const void* q, l
 CGK_API int cgk_kv_int4_attention(const cgk_kv_args* a, const void* q, void* out, int Tq, int Hq, float scale, int splits, float* scratch, void* stream) {
   if (int rc = check_kv(a, "cgk_kv_int4_attention")) return rc;
   CGK_REQUIRE(q && out && scratch && Tq > 0 && Hq % a->heads == 0 && splits > 0 && splits <= 256, "cgk_kv_int4_attention: bad argument");
+  CGK_REQUIRE((((uintptr_t)a->k_pages | (uintptr_t)a->v_pages | (uintptr_t)a->k_scales | (uintptr_t)a->v_scales) & 3) == 0, "cgk_kv_int4_attention: misaligned pools");
   const int D = a->D;
   const size_t smem = sizeof(float) * ((size_t)KV_MAXR * D + 4 * 32 * (D + 1) + 4 * KV_MAXR * 32 + 4 * KV_MAXR * (2 + D));
   float* part_acc = scratch;
@@ -770,10 +774,11 @@ CGK_API int cgk_kv_int4_attention(const cgk_kv_args* a, const void* q, void* out
   const dim3 grid(splits, a->heads, a->batch);
   const long long rows = (long long)a->batch * Hq * Tq;
   const int cblocks = (int)((rows * D + 255) / 256 < 1184 ? (rows * D + 255) / 256 : 1184);
-  if (cgk_kv_int4_attention_few(a, Tq, Hq) && (((uintptr_t)q | (uintptr_t)a->k_pages) & 15) == 0 && (((uintptr_t)a->v_pages | (uintptr_t)out) & 7) == 0)
+  if (cgk_kv_int4_attention_few(a, Tq, Hq) && ((uintptr_t)q & 15) == 0 && ((uintptr_t)out & 7) == 0)
     return cgk_kv_int4_attention_strided(a, q, (long long)Tq * Hq * D, (long long)Hq * D, D, out, Tq, Hq, scale, splits, stream);
-  if (D == 128 && a->group % 32 == 0) {
-    // tensor-core path (kv_attn_tc.cu); the CUDA-core kernel below covers the other shapes
+  if (D == 128 && a->group % 32 == 0 && (((uintptr_t)q | (uintptr_t)a->k_pages | (uintptr_t)a->v_pages) & 15) == 0) {
+    // tensor-core path (kv_attn_tc.cu: K, V and q 16 bytes at a time, single scales); the CUDA-core kernel below covers the
+    // other shapes and pools, which it reads by 32-bit words
     int dev = 0;
     CGK_CUDA_CHECK(cudaGetDevice(&dev));
     CGK_CUDA_CHECK(launch_kv_attention_tc(kv_dev(a), (const __nv_bfloat16*)q, Tq, Hq, scale, splits, part_acc, part_ml, device_status(dev), st));

@@ -266,13 +266,14 @@ int cgk_kv_int4_append_rows(const cgk_kv_args* a, const void* k_new, const void*
 long long cgk_kv_int4_attention_scratch_floats(int batch, int Hq, int Tq, int D, int splits);
 /* q, out: bf16 [batch, Tq, Hq, D]; the Tq newest tokens are already in the cache; query t sees
  * keys 0 .. lengths[b] + t.  Hq a multiple of heads (grouped-query attention). */
-/* Up to 32 query rows per kv head (Tq * Hq / heads), D 128 and group % 32 == 0: _few says so, and _strided takes rows of q bs, ts, hs
- * elements apart (multiples of 8) and needs no scratch. */
+int cgk_kv_int4_attention(const cgk_kv_args* a, const void* q, void* out, int Tq, int Hq, float scale,
+                          int splits, float* scratch, void* stream);
+/* Up to 32 query rows per kv head (Tq * Hq / heads), D 128, group % 32 == 0, pages on 16-byte boundaries and scales on boundaries of
+ * 4 * D / group bytes: _few says so, and _strided takes rows of q bs, ts, hs elements apart (multiples of 8; q on a 16-byte, out on an
+ * 8-byte boundary) and needs no scratch.  cgk_kv_int4_attention takes pages and scales on any 4-byte boundary. */
 int cgk_kv_int4_attention_few(const cgk_kv_args* a, int Tq, int Hq);
 int cgk_kv_int4_attention_strided(const cgk_kv_args* a, const void* q, long long bs, long long ts, long long hs, void* out, int Tq,
                                   int Hq, float scale, int splits, void* stream);
-int cgk_kv_int4_attention(const cgk_kv_args* a, const void* q, void* out, int Tq, int Hq, float scale,
-                          int splits, float* scratch, void* stream);
 /* Per row: logits / temperature -> top_k (1..1024, 0 = 1024) -> top_p -> sample.  temperature
  * <= 0: argmax.  Random stream = (seed, row, *step).  probs_out: fp32 [rows, V] or null; it may
  * be the logits (fp32, ld = V). */

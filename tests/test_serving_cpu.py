@@ -1,10 +1,14 @@
 """Serving stack on the host path: INT4 packing against the C library, paged KV cache,
 sampling composition, speculative decoding."""
+import ctypes
+
 import numpy as np
+import pytest
 import torch
 
 from capi_defs import L, T, cg
 from cogito_b200.models.llama import Llama, LlamaConfig, llama_tiny
+from cogito_b200.ops import _lib
 from cogito_b200.quant.int4 import Int4Linear, dequantize_int4, quantize_int4
 from cogito_b200.serve.engine import LlamaInt4Engine, SpeculativeDecoder
 from cogito_b200.serve.kv_cache import PagedKVCacheInt4
@@ -144,3 +148,18 @@ def test_the_engine_calls_its_vocabulary_projection_as_a_module():
     engine.lm_head.register_forward_hook(lambda module, args, out: seen.append(out))
     logits = engine.forward(torch.randint(0, 256, (2, 5)))
     assert len(seen) == 1 and torch.equal(seen[0].float(), logits)
+
+
+# the few-row kernel copies K and V in 16 bytes and a (token, head)'s scales in one piece of 4 * D / group: its rule asks for those boundaries
+@pytest.mark.skipif(not _lib.available(), reason="the kernel library has not been built")
+@pytest.mark.parametrize("group", [32, 64, 128])
+def test_rule_of_the_few_row_cache_attention_asks_for_its_boundaries(group):
+    cache, few = PagedKVCacheInt4(1, 2, 64, 2, 128, group), _lib.lib().cgk_kv_int4_attention_few
+    piece = 4 * 128 // group
+    for pool, boundary in (("k_pages", 16), ("v_pages", 16), ("k_scales", piece), ("v_scales", piece)):
+        for offset in range(0, 36, 4):
+            a = cache._args(0)
+            for name in ("k_pages", "v_pages", "k_scales", "v_scales"):
+                setattr(a, name, 1 << 20)
+            setattr(a, pool, (1 << 20) + offset)
+            assert few(ctypes.byref(a), 2, 8) == (offset % boundary == 0), (pool, offset)

@@ -391,6 +391,34 @@ def test_kv_attention_of_few_rows(group, page, Hk, Hq, Tq, hist):
     _lib.assert_device_ok()
 
 
+# pools on smaller boundaries than the few-row kernel's copies: its rule leaves them to the kernels that read single scales, or words
+@pytest.mark.parametrize("group", [32, 64, 128])
+@pytest.mark.parametrize("pages,scales", [(0, 4), (0, 8), (8, 0), (4, 4)])
+def test_kv_attention_of_pools_on_small_boundaries(group, pages, scales):
+    torch.manual_seed(group + pages)
+    B, hist, Hk, Hq, D, Tq = 2, 150, 2, 8, 128, 3
+    gpu = PagedKVCacheInt4(1, B, 256, Hk, D, group, page_size=16, device=DEV)
+    cpu = PagedKVCacheInt4(1, B, 256, Hk, D, group, page_size=16)
+
+    def moved(t, by):                                          # the same pool, `by` bytes off a boundary of 256
+        room = torch.empty(t.numel() + 64, dtype=t.dtype, device=t.device)
+        return room[by // t.element_size():][:t.numel()].view_as(t).copy_(t)
+    for pools, by in ((gpu.k_pages, 0), (gpu.v_pages, pages), (gpu.k_scales, scales), (gpu.v_scales, scales)):
+        pools[0] = moved(pools[0], by)
+    k, v = (torch.randn(B, hist, Hk, D).bfloat16() for _ in range(2))
+    kn, vn, q = (torch.randn(B, Tq, h, D).bfloat16() for h in (Hk, Hk, Hq))
+    for c, d in ((gpu, DEV), (cpu, "cpu")):
+        c.append(0, k.to(d), v.to(d))
+        c.commit(torch.tensor([hist, hist - 41], dtype=torch.int32, device=d))
+        c.append(0, kn.to(d), vn.to(d))
+    ref = cpu.attention(0, q.float())
+    for splits in (1, 3, 0):
+        got = gpu.attention(0, q.to(DEV), splits=splits).float().cpu()
+        # K, V and P are rounded to bf16 (2^-9 each), the results as well
+        assert ((got - ref).norm() / ref.norm()).item() < 2 ** -7
+    _lib.assert_device_ok()
+
+
 def test_kv_attention_long_history_many_key_blocks():
     torch.manual_seed(3)
     B, hist, Hk, Hq, D, Tq = 2, 700, 2, 8, 128, 5
