@@ -371,7 +371,8 @@ sample_kernel(const void* logits, int logits_bf16, long long ld, int V, float te
   __shared__ int s_keep;
   __shared__ float cand_v[MAX_TOPK];
   __shared__ int cand_i[MAX_TOPK];
-  __shared__ float prefix_s[MAX_TOPK];                       // sums of the candidates' probabilities; before that, scratch of the ranking
+  __shared__ __align__(16) float prefix_s[MAX_TOPK];         // sums of the candidates' probabilities; before that, scratch of the ranking
+  static_assert(__alignof__(prefix_s) >= sizeof(unsigned long long), "the ranking keeps 64-bit keys in it");
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_trigger();
   pdl_wait();
