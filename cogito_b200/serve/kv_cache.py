@@ -186,6 +186,15 @@ class PagedKVCacheInt4(PagedCache):
             out.append(q * s.repeat_interleave(self.group, -1))
         return out
 
+    @staticmethod
+    def _sharers(longest: int, pairs: int) -> int:
+        """CTAs that share the keys of a (sequence, kv head) in the few-row kernel: its eight warps hold a block of 32 keys each, so 256
+        keys are one CTA's; more than four pay for their wider merge from three rounds of four on, 16 from three of eight on (one
+        sequence, 8 kv heads, one token, us: 120 keys 4.4 by one, 5.9 by two; 2000 9.6 by four, 10.2 by eight; 3000 11.7 and 11.2;
+        8000 22.4 and 15.5; one kv head: 4000 10.5 by eight, 12.0 by 16; 8000 14.6 and 13.2; 32 000 38.5 and 25.4)."""
+        wanted = 16 if longest > 4608 else 8 if longest > 2304 else min(4, (longest + 255) // 256)
+        return max(1, min(wanted, 148 // max(1, pairs)))
+
     def attention(self, layer: int, q: torch.Tensor, splits: int = 0) -> torch.Tensor:
         """q: [batch, Tq, Hq, D], the Tq newest tokens (already appended, not yet committed).
         Query t sees keys 0 .. lengths[b] + t."""
@@ -195,11 +204,11 @@ class PagedKVCacheInt4(PagedCache):
             q = q.to(torch.bfloat16)
             L, a, longest = _lib.lib(), self._args(layer), self.max_pages * self.page_size
             if L.cgk_kv_int4_attention_few(ctypes.byref(a), Tq, Hq):
-                # rows are read where they lie (a slice of a packed projection); CTAs that share a head's keys take at least a block of 16 per warp
+                # rows are read where they lie (a slice of a packed projection)
                 if q.stride(3) != 1 or any(s % 8 for s in q.stride()[:3]) or q.data_ptr() % 16:
                     q = q.contiguous()
                 if splits <= 0:
-                    splits = max(1, min(4, 148 // max(1, B * self.heads), (longest + 127) // 128))
+                    splits = self._sharers(longest, B * self.heads)
                 out = torch.empty(B, Tq, Hq, D, dtype=q.dtype, device=q.device)
                 _lib.check(L.cgk_kv_int4_attention_strided(ctypes.byref(a), q.data_ptr(), q.stride(0), q.stride(1), q.stride(2), out.data_ptr(), Tq, Hq, scale,
                                                            splits, _lib.stream_ptr()), "cgk_kv_int4_attention_strided")

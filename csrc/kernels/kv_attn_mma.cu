@@ -18,7 +18,12 @@
 // 16 sequences of 641 tokens, 32 query and 8 kv heads, one new token: 11.1 us (24.7 + 2.7 for the kernel that combined the splits before);
 // five: 16.3 (37.4 + 5.2).  10.5 MB of cache are 1.6 us at HBM rate.  The rest is the chain lengths -> page -> keys at the start (3 us),
 // three blocks of some 1.5 us per warp (conversion and MMAs of two warps per scheduler), and the merge (1 us).
+// Long histories of few heads are shared by up to 16 CTAs, if that many clusters run at once.  One sequence of 32 000 tokens, 8 kv heads:
+// 40.8 us (by four CTAs 70.8, tcgen05 with combined splits 66.4), five tokens 64.4 (110; 87.9); one kv head 25.4 (68.5; 35.8), five
+// tokens 38.9 (106; 44.7).
 #include <cuda_bf16.h>
+
+#include <atomic>
 
 #include "host_common.h"
 #include "kv_dev.cuh"
@@ -27,21 +32,24 @@
 namespace cgk {
 namespace {
 
-constexpr int KM_WARPS = 8, KM_THREADS = KM_WARPS * 32, KM_D = 128, KM_NK = 2, KM_KB = 16 * KM_NK, KM_STAGES = 3, KM_MAX_CLUSTER = 32 / KM_WARPS;   // a lane per part
+constexpr int KM_WARPS = 8, KM_THREADS = KM_WARPS * 32, KM_D = 128, KM_NK = 2, KM_KB = 16 * KM_NK, KM_STAGES = 3;
 // a warp's 16 keys: K by lane, V rows of 64 bytes (80 apart: the lanes of a load in different banks), four scales per key of K and of V
 constexpr int KM_V = 1024, KM_VLD = 80, KM_S = KM_V + 16 * KM_VLD, KM_GROUP = KM_S + 2 * 16 * 16, KM_STAGE = KM_NK * KM_GROUP;
 constexpr int KM_LD = 8 * 20 + 4;                                     // row of a part: eight pieces of 16 elements, 20 apart: no two lanes of a store share banks
 
-template <int MT>                                                      // 16-row tiles of Q
+// MT: 16-row tiles of Q.  LP: parts that a lane weighs, so up to 4 * LP CTAs (with four parts a lane in every launch, the compiler kept
+// values of the loop over two row tiles in local memory: 16 sequences, five tokens, 15.7 -> 16.6 us)
+template <int MT, int LP>
 struct KmSmem {
+  static constexpr int MAX_CLUSTER = LP * 32 / KM_WARPS;
   static constexpr int ROWS = 16 * MT;
   static constexpr int RING = KM_WARPS * KM_STAGES * KM_STAGE;
   static constexpr int PART = ROWS * KM_LD * 4;                        // a warp's O
   static constexpr int O_BYTES = KM_WARPS * PART;                      // overlays the rings once the loop is over
   static constexpr int BODY = RING > O_BYTES ? RING : O_BYTES;
   static constexpr int OFF_ML = BODY;                                  // float [warp][2][ROWS]: maximum, sum
-  static constexpr int OFF_W = OFF_ML + KM_WARPS * 2 * ROWS * 4;       // float [KM_MAX_CLUSTER * KM_WARPS][ROWS]: weights of all parts
-  static constexpr int OFF_Q = OFF_W + KM_MAX_CLUSTER * KM_WARPS * ROWS * 4;
+  static constexpr int OFF_W = OFF_ML + KM_WARPS * 2 * ROWS * 4;       // float [MAX_CLUSTER * KM_WARPS][ROWS]: weights of all parts
+  static constexpr int OFF_Q = OFF_W + MAX_CLUSTER * KM_WARPS * ROWS * 4;
   static constexpr int TOTAL = OFF_Q + (MT > 1 ? MT * 8 * 512 : 0);    // Q fragments of more than one tile: [tile][MMA][lane] 16 bytes
 };
 
@@ -56,11 +64,11 @@ __device__ __forceinline__ void km_convert(uint32_t w, __nv_bfloat162 s2, uint32
   }
 }
 
-template <int MT>
+template <int MT, int LP>
 __global__ void __launch_bounds__(KM_THREADS, 1)
 kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long q_bs, long long q_ts, long long q_hs, int Tq, int Hq, float scale_log2,
                         __nv_bfloat16* __restrict__ out) {
-  using S = KmSmem<MT>;
+  using S = KmSmem<MT, LP>;
   constexpr int ROWS = S::ROWS;
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, qq = lane & 3;
@@ -80,7 +88,7 @@ kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long 
     for (int w = 0; w < 4; ++w) qr[h][w] = loads_q && r < R ? *reinterpret_cast<const uint4*>(p + w * 8) : make_uint4(0, 0, 0, 0);
   }
   const int blocks = (len + KM_KB - 1) / KM_KB, stride = splits * KM_WARPS;
-  const int first = rank * KM_WARPS + warp;                            // this warp's blocks of 16 keys: first, first + stride, ..
+  const int first = rank * KM_WARPS + warp;                            // this warp's blocks of keys: first, first + stride, ..
   const int mine = first < blocks ? (blocks - first + stride - 1) / stride : 0;
   const bool one_page = c.page_size % 16 == 0;                         // 16 keys never cross pages
 
@@ -296,19 +304,36 @@ kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long 
     }
   if (splits > 1) cluster_sync_all();
   else __syncthreads();
-  // every CTA writes its share of the rows: weights 2^(m_part - m) / sum of all parts, then the weighted sum
-  const int parts = splits * KM_WARPS, r0 = min(R, ROWS) * rank / splits, r1 = min(R, ROWS) * (rank + 1) / splits;
+  // every CTA writes its share of the rows: weights 2^(m_part - m) / sum of all parts, then the weighted sum; part p is that of warp
+  // p % KM_WARPS of CTA p / KM_WARPS, which began with block p: those beyond the last block are empty
+  const int parts = LP == 1 ? splits * KM_WARPS : min(splits * KM_WARPS, (len + KM_KB - 1) / KM_KB), r0 = min(R, ROWS) * rank / splits, r1 = min(R, ROWS) * (rank + 1) / splits;
   float* const wts = reinterpret_cast<float*>(smem + S::OFF_W);
   auto at = [&](uint32_t addr, int p) { return splits > 1 ? cluster_map(addr, p / KM_WARPS) : addr; };
   for (int r = r0 + warp; r < r1; r += KM_WARPS) {
-    float pm = -INFINITY, pl = 0.0f;
-    if (lane < parts) {
-      const uint32_t a = at(smem_u32(ml + lane % KM_WARPS * 2 * ROWS + r), lane);
-      pm = splits > 1 ? ld_cluster_f1(a) : ml[lane % KM_WARPS * 2 * ROWS + r];
-      pl = splits > 1 ? ld_cluster_f1(a + ROWS * 4) : ml[lane % KM_WARPS * 2 * ROWS + ROWS + r];
+    float pm[LP], pl[LP], top = -INFINITY, total = 0.0f;
+#pragma unroll
+    for (int i = 0; i < LP; ++i) {
+      const int p = lane + 32 * i;
+      pm[i] = -INFINITY;
+      pl[i] = 0.0f;
+      if (p < parts) {
+        const float* src = ml + p % KM_WARPS * 2 * ROWS + r;
+        const uint32_t a = at(smem_u32(src), p);
+        pm[i] = splits > 1 ? ld_cluster_f1(a) : src[0];
+        pl[i] = splits > 1 ? ld_cluster_f1(a + ROWS * 4) : src[ROWS];
+      }
+      top = fmaxf(top, pm[i]);
     }
-    const float top = warp_max(pm), w = pm > -INFINITY ? fast_exp2(pm - top) : 0.0f, total = warp_sum(w * pl);
-    if (lane < parts) wts[lane * ROWS + r] = total > 0.0f ? w / total : 0.0f;
+    top = warp_max(top);
+#pragma unroll
+    for (int i = 0; i < LP; ++i) {
+      pm[i] = pm[i] > -INFINITY ? fast_exp2(pm[i] - top) : 0.0f;
+      total += pm[i] * pl[i];
+    }
+    total = warp_sum(total);
+#pragma unroll
+    for (int i = 0; i < LP; ++i)
+      if (lane + 32 * i < parts) wts[(lane + 32 * i) * ROWS + r] = total > 0.0f ? pm[i] / total : 0.0f;
     __syncwarp();
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 8
@@ -324,22 +349,67 @@ kv_attention_mma_kernel(KvDev c, const __nv_bfloat16* __restrict__ q, long long 
   if (splits > 1) cluster_sync_all();                                  // nobody leaves while its parts are read
 }
 
+// The clusters of S CTAs that a device runs at once, 0 if none (asked for once; concurrent callers would store the same value).
+template <int MT, int LP>
+cudaError_t clusters_at_once(int S, int* fit) {
+  static std::atomic<int> known[64][KmSmem<MT, LP>::MAX_CLUSTER + 1];
+  int dev = 0;
+  if (cudaError_t e = cudaGetDevice(&dev)) return e;
+  if (dev < 64 && known[dev][S].load(std::memory_order_relaxed)) {
+    *fit = known[dev][S].load(std::memory_order_relaxed) - 1;
+    return cudaSuccess;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)S);
+  cfg.blockDim = dim3(KM_THREADS);
+  cfg.dynamicSmemBytes = KmSmem<MT, LP>::TOTAL;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = S;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(fit, kv_attention_mma_kernel<MT, LP>, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    *fit = 0;
+  }
+  if (dev < 64) known[dev][S].store(*fit + 1, std::memory_order_relaxed);
+  return cudaSuccess;
+}
+
+template <int MT, int LP>
+cudaError_t launch_cluster(const KvDev& c, const __nv_bfloat16* q, long long bs, long long ts, long long hs, int Tq, int Hq, float scale, int s, __nv_bfloat16* out,
+                           cudaStream_t stream) {
+  const cudaError_t e = cudaFuncSetAttribute(kv_attention_mma_kernel<MT, LP>, cudaFuncAttributeMaxDynamicSharedMemorySize, KmSmem<MT, LP>::TOTAL);
+  if (e != cudaSuccess) return e;
+  return launch_overlapped(kv_attention_mma_kernel<MT, LP>, dim3(s, c.heads, c.batch), dim3(KM_THREADS), KmSmem<MT, LP>::TOTAL, stream, s > 1 ? s : 0,
+                           c, q, bs, ts, hs, Tq, Hq, scale * 1.44269504089f, out);
+}
+
 template <int MT>
 cudaError_t launch_mt(const KvDev& c, const __nv_bfloat16* q, long long bs, long long ts, long long hs, int Tq, int Hq, float scale, int splits, __nv_bfloat16* out,
                       cudaStream_t stream) {
-  const cudaError_t e = cudaFuncSetAttribute(kv_attention_mma_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, KmSmem<MT>::TOTAL);
-  if (e != cudaSuccess) return e;
-  return launch_overlapped(kv_attention_mma_kernel<MT>, dim3(splits, c.heads, c.batch), dim3(KM_THREADS), KmSmem<MT>::TOTAL, stream, splits > 1 ? splits : 0,
-                           c, q, bs, ts, hs, Tq, Hq, scale * 1.44269504089f, out);
+  constexpr int FEW = KmSmem<MT, 1>::MAX_CLUSTER, MANY = KmSmem<MT, 4>::MAX_CLUSTER;
+  if (splits > FEW) {
+    cudaError_t e = cudaFuncSetAttribute(kv_attention_mma_kernel<MT, 4>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kv_attention_mma_kernel<MT, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, KmSmem<MT, 4>::TOTAL);
+    if (e != cudaSuccess) return e;
+    // as many as run at once in clusters: a cluster lies in one GPC, whose SMs it may not fill
+    for (int s = splits < MANY ? splits : MANY; s > FEW; s = s > 8 ? 8 : FEW) {
+      int fit = 0;
+      if ((e = clusters_at_once<MT, 4>(s, &fit)) != cudaSuccess) return e;
+      if (fit >= (long long)c.heads * c.batch) return launch_cluster<MT, 4>(c, q, bs, ts, hs, Tq, Hq, scale, s, out, stream);
+    }
+  }
+  return launch_cluster<MT, 1>(c, q, bs, ts, hs, Tq, Hq, scale, splits < FEW ? splits : FEW, out, stream);
 }
 }  // namespace
 
-// R = Tq * (Hq / heads) <= 32.  splits: CTAs per (sequence, kv head), at most four are used.
+// R = Tq * (Hq / heads) <= 32.  splits: CTAs per (sequence, kv head), at most 16 are used.
 cudaError_t launch_kv_attention_mma(const KvDev& c, const __nv_bfloat16* q, long long bs, long long ts, long long hs, int Tq, int Hq, float scale, int splits,
                                     __nv_bfloat16* out, cudaStream_t stream) {
-  const int s = splits < KM_MAX_CLUSTER ? splits : KM_MAX_CLUSTER;
-  if (Tq * (Hq / c.heads) <= 16) return launch_mt<1>(c, q, bs, ts, hs, Tq, Hq, scale, s, out, stream);
-  return launch_mt<2>(c, q, bs, ts, hs, Tq, Hq, scale, s, out, stream);
+  if (Tq * (Hq / c.heads) <= 16) return launch_mt<1>(c, q, bs, ts, hs, Tq, Hq, scale, splits, out, stream);
+  return launch_mt<2>(c, q, bs, ts, hs, Tq, Hq, scale, splits, out, stream);
 }
 }  // namespace cgk
 

@@ -16,7 +16,7 @@ struct KvDev {
 
 // Attention over the cache for head_dim 128, a quantisation group that is a multiple of 32 and at most KV_FEW_ROWS query rows per kv
 // head (Tq * Hq / heads): q rows of 128 contiguous elements at b * bs + t * ts + h * hs, all multiples of 8, on a 16-byte boundary; pages on
-// 16-byte boundaries, a (token, head)'s scales on a boundary of their own size.  At most four CTAs per (sequence, kv head) share the keys; no scratch.
+// 16-byte boundaries, a (token, head)'s scales on a boundary of their own size.  At most 16 CTAs per (sequence, kv head) share the keys; no scratch.
 constexpr int KV_FEW_ROWS = 32;
 cudaError_t launch_kv_attention_mma(const KvDev& c, const __nv_bfloat16* q, long long bs, long long ts, long long hs, int Tq, int Hq, float scale, int splits,
                                     __nv_bfloat16* out, cudaStream_t stream);

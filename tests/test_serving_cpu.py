@@ -163,3 +163,10 @@ def test_rule_of_the_few_row_cache_attention_asks_for_its_boundaries(group):
                 setattr(a, name, 1 << 20)
             setattr(a, pool, (1 << 20) + offset)
             assert few(ctypes.byref(a), 2, 8) == (offset % boundary == 0), (pool, offset)
+
+
+# long histories of few heads are shared by more CTAs than four, short ones take no more than have a block for every warp
+def test_sharers_of_a_history_in_the_few_row_cache_attention():
+    sharers = PagedKVCacheInt4._sharers
+    assert [sharers(n, 1) for n in (1, 256, 257, 1024, 2304, 2305, 4608, 4609, 1 << 20)] == [1, 1, 2, 4, 4, 8, 8, 16, 16]
+    assert sharers(32768, 8) == 16 and sharers(32768, 16) == 9 and sharers(32768, 128) == 1 and sharers(32768, 1000) == 1

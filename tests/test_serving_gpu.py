@@ -391,6 +391,33 @@ def test_kv_attention_of_few_rows(group, page, Hk, Hq, Tq, hist):
     _lib.assert_device_ok()
 
 
+# a head's keys shared by up to 16 CTAs: parts that are all empty but one, a last block of few keys, histories of other lengths side by side,
+# and more CTAs than there are rows to write
+@pytest.mark.parametrize("Hk,Hq,Tq", [(1, 4, 1), (2, 8, 5), (1, 1, 1), (1, 32, 1)])
+@pytest.mark.parametrize("hist", [0, 40, 1030, 4500])
+def test_kv_attention_shared_by_many_ctas(Hk, Hq, Tq, hist):
+    torch.manual_seed(hist + Hq)
+    B, D = 2, 128
+    gpu = PagedKVCacheInt4(1, B, hist + 64, Hk, D, 32, page_size=64, device=DEV)
+    cpu = PagedKVCacheInt4(1, B, hist + 64, Hk, D, 32, page_size=64)
+    kn, vn, q = (torch.randn(B, Tq, h, D).bfloat16() for h in (Hk, Hk, Hq))
+    k, v = (torch.randn(B, hist, Hk, D).bfloat16() for _ in range(2))
+    q[0] *= 4                                                  # a few keys hold the mass of one sequence
+    for c, d in ((gpu, DEV), (cpu, "cpu")):
+        if hist:
+            c.append(0, k.to(d), v.to(d))
+            c.commit(torch.tensor([hist, hist // 5], dtype=torch.int32, device=d))
+        c.append(0, kn.to(d), vn.to(d))
+    ref, q = cpu.attention(0, q.float()), q.to(DEV)
+    for splits in (5, 8, 12, 16, 40, 0):
+        got = gpu.attention(0, q, splits=splits)
+        # a score of the first sequence is a sum of products with deviation 4: rounding K to bf16 (2^-9 of each product at most) moves it,
+        # and so its key's weight by that share, by 4 * 2^-9 = 2^-7 in the mean square; V, P and the results are rounded too (2^-9 each)
+        assert ((got.float().cpu() - ref).norm() / ref.norm()).item() < 2 ** -6
+        assert torch.equal(got, gpu.attention(0, q, splits=splits))
+    _lib.assert_device_ok()
+
+
 # pools on smaller boundaries than the few-row kernel's copies: its rule leaves them to the kernels that read single scales, or words
 @pytest.mark.parametrize("group", [32, 64, 128])
 @pytest.mark.parametrize("pages,scales", [(0, 4), (0, 8), (8, 0), (4, 4)])
@@ -435,6 +462,27 @@ def test_kv_attention_long_history_many_key_blocks():
     for splits in (1, 3, 0):
         got = gpu.attention(0, q.to(DEV), splits=splits).float().cpu()
         assert (got - ref).abs().max().item() < 2e-2
+    _lib.assert_device_ok()
+
+
+# more than 32 rows per kv head: the tcgen05 kernel over many blocks of 128 keys, one and two passes over the rows
+@pytest.mark.parametrize("Tq", [9, 20])
+def test_kv_attention_of_more_rows_over_many_key_blocks(Tq):
+    torch.manual_seed(Tq)
+    B, hist, Hk, Hq, D = 2, 1500, 2, 8, 128
+    gpu = PagedKVCacheInt4(1, B, 1600, Hk, D, 32, page_size=32, device=DEV)
+    cpu = PagedKVCacheInt4(1, B, 1600, Hk, D, 32, page_size=32)
+    k, v = (torch.randn(B, hist, Hk, D).bfloat16() for _ in range(2))
+    kn, vn, q = (torch.randn(B, Tq, h, D).bfloat16() for h in (Hk, Hk, Hq))
+    for c, d in ((gpu, DEV), (cpu, "cpu")):
+        c.append(0, k.to(d), v.to(d))
+        c.commit(torch.tensor([hist, hist - 801], dtype=torch.int32, device=d))
+        c.append(0, kn.to(d), vn.to(d))
+    ref = cpu.attention(0, q.float())
+    for splits in (1, 3, 0):
+        got = gpu.attention(0, q.to(DEV), splits=splits).float().cpu()
+        # K, V and P are rounded to bf16 (2^-9 each), the results as well
+        assert ((got - ref).norm() / ref.norm()).item() < 2 ** -7
     _lib.assert_device_ok()
 
 
