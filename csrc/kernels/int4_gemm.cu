@@ -42,10 +42,15 @@ constexpr int SUB = 2;                                        // 64-row sub-tile
 constexpr int B_STAGES = 4, MAX_RAW_STAGES = 16, MAX_A_STAGES = 8;
 constexpr int ACC_COLS = 2 * BM, W_COLS = SUB * BK / 2, TMEM_COLS = 512;              // two accumulators, then B_STAGES operands of W_COLS columns
 constexpr int GROUPS = 2, GROUP_WARPS = 8, CONVERT_WARPS = GROUPS * GROUP_WARPS;     // converting warps: groups that take the steps in turn
+// A group waits for a ring slot by the parity of its phase, which also holds while the slot's last step but one has not arrived (with an
+// odd depth that step is the other group's).  Before it comes to step i it has ended step i - GROUPS, for which step i - GROUPS - B_STAGES
+// was multiplied and so all steps before it were converted: a ring of this many steps or more is safe.
+constexpr int MIN_RAW_STAGES = GROUPS + B_STAGES;
 constexpr int NIB_BYTES = BK * BN / 2, SCALE_BYTES = BK * 2 * 2, RAW_BYTES = NIB_BYTES + SCALE_BYTES;   // 4096 + 256
 constexpr int EPI_WARP0 = 4 + CONVERT_WARPS, THREADS = 32 * (EPI_WARP0 + 4);
 constexpr int SMEM_BYTES = 226 * 1024;                       // alignment slack | X ring | W ring | barriers
 constexpr int RING_BUDGET = SMEM_BYTES - 1024 - 2048;        // shared by the X and W rings
+static_assert((RING_BUDGET - 3 * SUB * BM * 128) / (SUB * RAW_BYTES) >= MIN_RAW_STAGES, "the W ring beside the least X ring");
 
 struct Int4Dev {
   const uint8_t* w_tiles;          // [N/128][K/64][4352]
@@ -460,6 +465,7 @@ static int wb_gemm(const void* x, long long ldx, const void* w_tiles, float* par
   if (raw_stages > MAX_RAW_STAGES) raw_stages = MAX_RAW_STAGES;
   static const int raw_cap = getenv("CGK_INT4_RAW_STAGES") ? atoi(getenv("CGK_INT4_RAW_STAGES")) : 0;
   if (raw_cap > 0 && raw_cap < raw_stages) raw_stages = raw_cap;
+  if (raw_stages < MIN_RAW_STAGES) raw_stages = MIN_RAW_STAGES;
   CUtensorMap tmX;
   int rc = encode_tmap_bf16_2d(&tmX, x, (uint64_t)M, (uint64_t)K, (uint64_t)ldx, (uint32_t)a_rows, BK);
   if (rc) return rc;

@@ -1,5 +1,9 @@
 """Serving kernels on the GPU against their host restatements (fp32 PyTorch / the C library)."""
 import copy
+import os
+import subprocess
+import sys
+from pathlib import Path
 
 import pytest
 import torch
@@ -14,6 +18,7 @@ from cogito_b200.utils import rng
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
+ROOT = Path(__file__).resolve().parent.parent
 
 
 def test_int4_quantize_dequantize_bit_exact_with_host():
@@ -112,6 +117,18 @@ def test_int4_gemm_by_ways_to_deal_tiles(M, K, N):
     got = lin(x, f32=True)
     assert ((got.double() - ref).norm() / ref.norm()).item() < 2 ** -7 and torch.equal(got.bfloat16(), lin(x))
     _lib.assert_device_ok()
+
+
+# the depth of the weight ring that the environment asks for is raised to the least that the two converting groups can share
+@pytest.mark.parametrize("depth", ["1", "3", "7"])
+def test_int4_gemm_with_a_short_weight_ring(depth):
+    code = ("import torch\nfrom cogito_b200.quant.int4 import Int4Linear\nfrom cogito_b200.ops import _lib\ntorch.manual_seed(0)\n"
+            "lin = Int4Linear(torch.randn(640, 2048) * 0.05, None, 64).to('cuda')\nlin.kernel = 'wb'\nx = torch.randn(48, 2048).bfloat16().to('cuda')\n"
+            "y, ref = lin(x, f32=True).double(), x.double() @ lin.dequantized().double()\n_lib.assert_device_ok()\n"
+            # scale, then weight rounded to bf16 (2^-9 of the terms' norm each), fp32 sums
+            "assert (y - ref).norm() / ref.norm() < 2 ** -7\n")
+    run = subprocess.run([sys.executable, "-c", code], env={**os.environ, "CGK_INT4_RAW_STAGES": depth}, cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
 
 
 @pytest.mark.parametrize("N", [256, 22016])
