@@ -206,7 +206,8 @@ class PagedKVCacheInt4(PagedCache):
             if L.cgk_kv_int4_attention_few(ctypes.byref(a), Tq, Hq):
                 # rows are read where they lie (a slice of a packed projection)
                 if q.stride(3) != 1 or any(s % 8 for s in q.stride()[:3]) or q.data_ptr() % 16:
-                    q = q.contiguous()
+                    # (a contiguous tensor may have any stride along a dimension of length 1 and any address: contiguous() leaves it)
+                    q = q.clone(memory_format=torch.contiguous_format)
                 if splits <= 0:
                     splits = self._sharers(longest, B * self.heads)
                 out = torch.empty(B, Tq, Hq, D, dtype=q.dtype, device=q.device)

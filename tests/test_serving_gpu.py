@@ -435,6 +435,26 @@ def test_kv_attention_shared_by_many_ctas(Hk, Hq, Tq, hist):
     _lib.assert_device_ok()
 
 
+# contiguous queries whose strides or address the kernel cannot use as they are: a dimension of length 1 with the stride of another one, an odd place in a buffer
+@pytest.mark.parametrize("B,Tq", [(2, 1), (1, 3)])
+def test_kv_attention_of_contiguous_queries_with_unusual_strides(B, Tq):
+    torch.manual_seed(B)
+    Hk, Hq, D = 2, 8, 128
+    cache = PagedKVCacheInt4(1, B, 64, Hk, D, 32, page_size=16, device=DEV)
+    cache.append(0, *(torch.randn(B, 30, Hk, D, device=DEV).bfloat16() for _ in range(2)))
+    cache.commit(27)
+    q = torch.randn(B, Tq, Hq, D, device=DEV).bfloat16()
+    want = cache.attention(0, q)
+    if Tq == 1:
+        odd = q[:, 0].unsqueeze(-1).permute(0, 3, 1, 2)         # 'b h d 1 -> b 1 h d'
+        assert odd.is_contiguous() and odd.stride(1) == 1
+    else:
+        odd = torch.empty(q.numel() + 8, device=DEV, dtype=q.dtype)[1:q.numel() + 1].view_as(q).copy_(q)
+        assert odd.is_contiguous() and odd.data_ptr() % 16
+    assert torch.equal(cache.attention(0, odd), want)
+    _lib.assert_device_ok()
+
+
 # pools on smaller boundaries than the few-row kernel's copies: its rule leaves them to the kernels that read single scales, or words
 @pytest.mark.parametrize("group", [32, 64, 128])
 @pytest.mark.parametrize("pages,scales", [(0, 4), (0, 8), (8, 0), (4, 4)])
