@@ -5,6 +5,7 @@ import ctypes
 import numpy as np
 import pytest
 import torch
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from capi_defs import L, T, cg
 from cogito_b200.models.llama import Llama, LlamaConfig, llama_tiny
@@ -13,6 +14,7 @@ from cogito_b200.quant.int4 import Int4Linear, dequantize_int4, quantize_int4
 from cogito_b200.serve.engine import LlamaInt4Engine, SpeculativeDecoder
 from cogito_b200.serve.kv_cache import PagedKVCacheInt4
 from cogito_b200.serve.sampling import filtered_probs, sample, spec_accept, tree_attention_mask
+from cogito_b200.serve.stack import token_rows
 from cogito_b200.utils import rng
 
 
@@ -170,3 +172,22 @@ def test_sharers_of_a_history_in_the_few_row_cache_attention():
     sharers = PagedKVCacheInt4._sharers
     assert [sharers(n, 1) for n in (1, 256, 257, 1024, 2304, 2305, 4608, 4609, 1 << 20)] == [1, 1, 2, 4, 4, 8, 8, 16, 16]
     assert sharers(32768, 8) == 16 and sharers(32768, 16) == 9 and sharers(32768, 128) == 1 and sharers(32768, 1000) == 1
+
+
+# the rows of a step are laid out without work for every entry beyond its list: no tensor operation per entry, whatever their sizes
+@pytest.mark.parametrize("counts", [[1], [4096], [1] * 80, [512] + [1] * 64, [5] * 16, [33, 1, 40, 2]])
+def test_rows_of_a_step_of_the_layer_stack_engine(counts):
+    class Count(TorchDispatchMode):
+        calls = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.calls += 1
+            return func(*args, **(kwargs or {}))
+    rnd = np.random.default_rng(len(counts))
+    parts = [(rnd.integers(0, 1000, n).tolist(), int(rnd.integers(0, 500)), s + 3) for s, n in enumerate(counts)]
+    with Count() as count:
+        rows = token_rows(parts)
+    assert count.calls <= 4
+    want = [[t for p in parts for t in p[0]], [p[1] + i for p in parts for i in range(len(p[0]))], [p[2] for p in parts for _ in p[0]]]
+    assert rows.dtype == torch.int64 and rows.tolist() == want
+    assert torch.equal(token_rows([(torch.tensor(t), b, s) for t, b, s in parts]), rows)
