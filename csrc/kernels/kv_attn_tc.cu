@@ -1,5 +1,5 @@
 // Attention over the paged INT4 KV cache on the tcgen05 tensor cores (head_dim 128): more than 32 query rows per kv head; fewer
-// are faster by warps (kv_attn_mma.cu).
+// are faster by warps (kv_attn_mma.cu), but for pools whose scales lie on too small a boundary for its copies.
 // Reference counterpart: cg_attention_int4_kv (include/cg_quantize.h, declared only).
 //
 // One CTA per (key split, kv head, sequence) handles up to NP query rows (the Tq new tokens of
@@ -283,6 +283,8 @@ cudaError_t launch_np(const KvDev& c, const __nv_bfloat16* q, int Tq, int Hq, fl
 cudaError_t launch_kv_attention_tc(const KvDev& c, const __nv_bfloat16* q, int Tq, int Hq, float scale, int splits,
                                    float* part_acc, float* part_ml, int* status, cudaStream_t stream) {
   const int R = Tq * (Hq / c.heads);
+  if (R <= 16) return launch_np<16>(c, q, Tq, Hq, scale, splits, 1, part_acc, part_ml, status, stream);
+  if (R <= 32) return launch_np<32>(c, q, Tq, Hq, scale, splits, 1, part_acc, part_ml, status, stream);
   return launch_np<64>(c, q, Tq, Hq, scale, splits, (R + 63) / 64, part_acc, part_ml, status, stream);
 }
 }  // namespace cgk

@@ -458,9 +458,10 @@ def test_kv_attention_of_contiguous_queries_with_unusual_strides(B, Tq):
 # pools on smaller boundaries than the few-row kernel's copies: its rule leaves them to the kernels that read single scales, or words
 @pytest.mark.parametrize("group", [32, 64, 128])
 @pytest.mark.parametrize("pages,scales", [(0, 4), (0, 8), (8, 0), (4, 4)])
-def test_kv_attention_of_pools_on_small_boundaries(group, pages, scales):
+@pytest.mark.parametrize("Tq", [3, 5])
+def test_kv_attention_of_pools_on_small_boundaries(group, pages, scales, Tq):
     torch.manual_seed(group + pages)
-    B, hist, Hk, Hq, D, Tq = 2, 150, 2, 8, 128, 3
+    B, hist, Hk, Hq, D = 2, 150, 2, 8, 128
     gpu = PagedKVCacheInt4(1, B, 256, Hk, D, group, page_size=16, device=DEV)
     cpu = PagedKVCacheInt4(1, B, 256, Hk, D, group, page_size=16)
 
