@@ -727,3 +727,49 @@ def test_kv_attention_captured_before_a_larger_call():
         assert torch.equal(got, want)
     assert all((j == 1e30).all() for j in junk)
     _lib.assert_device_ok()
+
+
+# the same with more than 32 rows per kv head, whose kernel is the one with scratch
+def test_kv_attention_of_more_rows_captured_before_a_larger_call():
+    torch.manual_seed(6)
+    B, Hk, Hq, D = 2, 2, 8, 128
+    cache = PagedKVCacheInt4(1, B, 512, Hk, D, 32, page_size=64, device=DEV)
+    cache.append(0, *(torch.randn(B, 420, Hk, D, device=DEV).bfloat16() for _ in range(2)))
+    cache.commit(400)
+    q, more = (torch.randn(B, t, Hq, D, device=DEV).bfloat16() for t in (9, 20))
+    want = cache.attention(0, q)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = cache.attention(0, q)
+    cache.attention(0, more)
+    junk = [torch.full((n,), 1e30, device=DEV) for n in (1 << 8, 1 << 12, 1 << 14, 1 << 16, 1 << 18) for _ in range(4)]
+    for _ in range(2):
+        got.zero_()
+        graph.replay()
+        assert torch.equal(got, want)
+    assert all((j == 1e30).all() for j in junk)
+    _lib.assert_device_ok()
+
+
+# in a captured pass launches overlap their predecessors, in one launched eagerly they do not: the same bits.  4 rows take the
+# warp-level products and one row tile of the cache attention, 20 the tcgen05 products and two
+@pytest.mark.parametrize("tokens", [1, 5])
+@torch.no_grad()
+def test_int4_pass_captured_and_launched_eagerly(tokens):
+    rng.manual_seed(2)
+    cfg = LlamaConfig(vocab_size=1024, n_layer=6, d_model=1024, n_head=8, n_kv_head=2, d_ff=2048, max_seq_len=512)
+    engine = LlamaInt4Engine(Llama(cfg).to(DEV).bfloat16(), 4, 512)
+    engine.forward(torch.randint(0, 1024, (4, 333), device=DEV), commit=True)
+    ids = torch.randint(0, 1024, (4, tokens), device=DEV)
+    want = engine.forward(ids).clone()
+    assert torch.equal(engine.forward(ids), want)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = engine.forward(ids)
+    for _ in range(20):
+        got.zero_()
+        graph.replay()
+        assert torch.equal(got, want)
+    _lib.assert_device_ok()
