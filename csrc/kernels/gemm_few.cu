@@ -24,12 +24,6 @@ struct FewDev {
   const __nv_bfloat16* b; long long ldb, strideB;
 };
 
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t mapped) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(mapped) : "memory");
-  return v;
-}
-
 // epilogue_scalar for four neighbouring columns, all inside the output
 __device__ __forceinline__ void epilogue4(const GemmDev& g, int b, int m, int n, float (&v)[4]) {
 #pragma unroll

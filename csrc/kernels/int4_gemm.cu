@@ -337,11 +337,7 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
       // the CTA that arrives last at the tile's counter turns the parts into the output
       asm volatile("bar.sync 1, 128;" ::: "memory");
       int* counter = g.counters + mt * n_tiles + nt;
-      if (et == 0) {                                        // the barriers hand the others' parts to this thread and its view to them
-        int before;
-        asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
-        *is_last = before == hi - lo && !*dead;
-      }
+      if (et == 0) *is_last = arrive_acq_rel(counter) == hi - lo && !*dead;      // the barriers hand the others' parts to this thread and its view to them
       asm volatile("bar.sync 1, 128;" ::: "memory");
       if (i == ksteps) break;                               // the CTA's last part: all its threads take part in the sum, below
       if (*is_last) {

@@ -86,12 +86,6 @@ __device__ __forceinline__ WaShare wa_share(uint32_t k_units, const Pieces& piec
   return w;
 }
 
-// One thread's arrival for its CTA behind a barrier: what the CTA wrote before is visible to whoever finds it counted.
-__device__ __forceinline__ int arrive_acq_rel(int* counter) {
-  int old;
-  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
-  return old;
-}
 template <int NT>
 __global__ void __launch_bounds__(W_THREADS, 1)
 int4_wa_kernel(const WaDev g) {

@@ -33,15 +33,4 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int LEFT>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
 
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t mapped) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(mapped) : "memory");
-  return v;
-}
-__device__ __forceinline__ float ld_cluster_f1(uint32_t mapped) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(mapped) : "memory");
-  return v;
-}
-
 }  // namespace cgk

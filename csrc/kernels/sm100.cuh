@@ -472,6 +472,23 @@ __device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
   return a;
 }
+// Loads from another CTA's shared memory (`mapped`: cluster_map).
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t mapped) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(mapped) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_cluster_f1(uint32_t mapped) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(mapped) : "memory");
+  return v;
+}
+// One thread's arrival for its CTA behind a barrier: what the CTA wrote before is visible to whoever finds it counted.
+__device__ __forceinline__ int arrive_acq_rel(int* counter) {
+  int before;
+  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+  return before;
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t mapped_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapped_bar) : "memory");
 }
