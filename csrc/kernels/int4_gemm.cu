@@ -31,6 +31,7 @@
 #include <stdlib.h>
 
 #include "host_common.h"
+#include "int4_tile.cuh"
 #include "mma_sync.cuh"
 #include "cogito_kernels.h"
 
@@ -362,30 +363,29 @@ int4_gemm_kernel(const __grid_constant__ CUtensorMap tmX, const Int4Dev g) {
   }
 }
 
-// packed [K][N/2] bytes + scales (flat groups) -> tiles [N/128][K/64][4352]
-__global__ void int4_tile_kernel(const uint8_t* __restrict__ packed, const float* __restrict__ scales, int K, int N, int group,
-                                 uint8_t* __restrict__ tiles) {
-  const int k_tiles = K / BK;
-  const long long blocks = (long long)(N / BN) * k_tiles;
-  for (long long blk = blockIdx.x; blk < blocks; blk += gridDim.x) {
-    const int nt = (int)(blk / k_tiles), ks = (int)(blk % k_tiles);
-    uint8_t* dst = tiles + blk * RAW_BYTES;
-    for (int i = threadIdx.x; i < NIB_BYTES / 4; i += blockDim.x) {       // word i: k half i / 512, feature (i % 512) / 4, word i % 4
-      const int f = nt * BN + ((i & 511) >> 2), k0 = ks * BK + (i >> 9) * 32 + (i & 3) * 8;
-      uint32_t word = 0;
+// packed [K][N/2] bytes + scales (flat groups) -> tiles [N/128][K/64][4352].  A thread has eight columns of half a block's k.
+// 4096 x 32000: 39 us (92 with single nibbles out of eight rows for every word).
+__global__ void __launch_bounds__(256)
+int4_tile_kernel(const uint8_t* __restrict__ packed, const float* __restrict__ scales, int K, int N, int group, uint8_t* __restrict__ tiles) {
+  const int k_tiles = K / BK, groups = N / group;
+  const long long blk = ((long long)blockIdx.x * 256 + threadIdx.x) >> 5;
+  if (blk >= (long long)(N / BN) * k_tiles) return;
+  const int nt = (int)(blk / k_tiles), ks = (int)(blk % k_tiles), t = threadIdx.x & 31, c8 = t & 15, half = t >> 4;
+  uint8_t* const dst = tiles + blk * RAW_BYTES;
+  const uint8_t* const src = packed + ((long long)(ks * BK + half * 32) * N + nt * BN) / 2 + c8 * 4;
+  uint32_t w[4][8];                                                       // [eight k][nibble of the result: k 2 j at j, 2 j + 1 at j + 4]
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {                                       // nibbles j and j + 4: k 2 j and 2 j + 1
-        const uint8_t byte = packed[((long long)(k0 + e) * N + f) >> 1];
-        const uint32_t nib = ((f & 1) ? (byte >> 4) : (byte & 0xF)) ^ 8u;
-        word |= nib << (4 * ((e >> 1) + 4 * (e & 1)));
-      }
-      reinterpret_cast<uint32_t*>(dst)[i] = word;
-    }
-    for (int i = threadIdx.x; i < BK * 2; i += blockDim.x) {
-      const int half = i / BK, k = i % BK;
-      reinterpret_cast<__nv_bfloat16*>(dst + NIB_BYTES)[i] = __float2bfloat16(scales[((long long)(ks * BK + k) * N + nt * BN + half * 64) / group]);
-    }
-  }
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) w[c][e] = load_nibbles(src + (long long)(c * 8 + (e & 3) * 2 + (e >> 2)) * (N / 2), true) ^ 0x88888888u;
+  float s[4];                                                             // scales of four k of a half of the columns
+#pragma unroll
+  for (int j = 0; j < 4; ++j) s[j] = scales[(long long)(ks * BK + c8 * 4 + j) * groups + (nt * BN + half * 64) / group];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) transpose_nibbles(w[c]);
+#pragma unroll
+  for (int g = 0; g < 8; ++g) *reinterpret_cast<uint4*>(dst + half * (NIB_BYTES / 2) + (c8 * 8 + g) * 16) = make_uint4(w[0][g], w[1][g], w[2][g], w[3][g]);
+  *reinterpret_cast<uint2*>(dst + NIB_BYTES + half * (BK * 2) + c8 * 8) = make_uint2(pack_bf16x2(s[0], s[1]), pack_bf16x2(s[2], s[3]));
 }
 }  // namespace
 
@@ -398,7 +398,7 @@ CGK_API int cgk_int4_tile_weights(const void* packed, const float* scales, int K
   CGK_REQUIRE(group >= 64 && group % 64 == 0 && N % group == 0, "cgk_int4_tile_weights: group %d must be a multiple of 64 that divides N", group);
   CGK_REQUIRE(((uintptr_t)packed & 3) == 0 && ((uintptr_t)tiles & 15) == 0, "cgk_int4_tile_weights: misaligned buffer");
   const long long blocks = (long long)(N / BN) * (K / BK);
-  int4_tile_kernel<<<(unsigned)(blocks < 4736 ? blocks : 4736), 256, 0, (cudaStream_t)stream>>>((const uint8_t*)packed, scales, K, N, group, (uint8_t*)tiles);
+  int4_tile_kernel<<<(unsigned)((blocks * 32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const uint8_t*)packed, scales, K, N, group, (uint8_t*)tiles);
   CGK_LAUNCH_CHECK();
   return 0;
 }

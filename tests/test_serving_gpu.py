@@ -119,6 +119,39 @@ def test_int4_gemm_by_ways_to_deal_tiles(M, K, N):
     _lib.assert_device_ok()
 
 
+# the reordered weights hold every nibble (q + 8) and scale where the products read it, also from packed weights off a word's boundary
+@pytest.mark.parametrize("wa,offset", [(True, 0), (True, 1), (True, 2), (False, 0), (False, 4)])
+@pytest.mark.parametrize("K,N", [(64, 128), (192, 384)])
+def test_int4_tiles_hold_the_packed_weights(wa, offset, K, N):
+    torch.manual_seed(K)
+    L, group = _lib.lib(), 128
+    room = torch.randint(0, 256, (K * N // 2 + 16,), dtype=torch.uint8, device=DEV)
+    packed, scales = room[offset:offset + K * N // 2], torch.rand(K * N // group, device=DEV)
+    tiles = torch.zeros((L.cgk_int4_wa_tiles_bytes if wa else L.cgk_int4_tiles_bytes)(K, N), dtype=torch.uint8, device=DEV)
+    _lib.check((L.cgk_int4_wa_tile_weights if wa else L.cgk_int4_tile_weights)(packed.data_ptr(), scales.data_ptr(), K, N, group, tiles.data_ptr(), _lib.stream_ptr()))
+    byte = packed.cpu().view(K, N // 2)
+    u = torch.stack([byte & 0xF, byte >> 4], -1).view(K, N).int() ^ 8                              # q + 8 of [k, n]
+    s = scales.cpu().view(K, N // group).repeat_interleave(group, 1)
+    step = 32 if wa else 64
+    tiles = tiles.cpu().view(N // 128, K // step, -1)
+    words = tiles[:, :, :step * 64].contiguous().view(torch.int32).long() & 0xFFFFFFFF
+    got = torch.stack([(words >> (4 * e)) & 0xF for e in range(8)], -1).int()                    # [tile, step, word, nibble]
+    u = u.view(K // step, step, N // 128, 128).permute(2, 0, 1, 3)                                 # [tile, step, k, column]
+    i, e = torch.arange(got.shape[2])[:, None], torch.arange(8)[None]
+    if wa:
+        lane, r = (i & 127) >> 2, e & 3
+        column, k = (2 * (i >> 7) + ((i & 3) >> 1)) * 16 + (lane >> 2) + (r & 1) * 8, (lane & 3) * 8 + (i & 1) * 4 + (r >> 1) * 2 + (e >> 2)
+    else:
+        column, k = ((i & 511) >> 2) + 0 * e, (i >> 9) * 32 + (i & 3) * 8 + 2 * (e & 3) + (e >> 2)
+    assert torch.equal(got, u[:, :, k, column])
+    s = s.view(K // step, step, N // 128, 128).permute(2, 0, 3, 1)                                 # [tile, step, column, k]
+    if wa:
+        assert torch.equal(tiles[:, :, 2048:].contiguous().view(torch.float32), s[:, :, 0])
+    else:
+        assert torch.equal(tiles[:, :, 4096:].contiguous().view(torch.bfloat16), torch.cat([s[:, :, 0], s[:, :, 64]], -1).bfloat16())
+    _lib.assert_device_ok()
+
+
 # the depth of the weight ring that the environment asks for is raised to the least that the two converting groups can share
 @pytest.mark.parametrize("depth", ["1", "3", "7"])
 def test_int4_gemm_with_a_short_weight_ring(depth):
