@@ -121,11 +121,11 @@ class Int4Linear(torch.nn.Module):
     # "wb" takes the call.  Each of the two kernels has its own tile-major copy of the weights, made on
     # first use; both sum the parts of a shared tile in a fixed order, so a call gives the same bits every time.
     # Times (us, layers one after the other) for 4096 x 6144, 4096 x 4096, 4096 x 22016, 11008 x 4096, 4096 x 32000, 2048 x 11264:
-    #   16 rows   "wa" 8.5 6.5 21.0 11.1 26.3 10.4      "wb" 9.6 8.4 22.5 14.3 30.7 9.3
-    #   17 rows   "wa" 12.6 9.1 31.3 15.8 39.4 15.4     "wb" 9.8 8.6 22.6 14.7 30.8 9.5    (four columns of MMAs instead of two)
-    #   32 rows   "wa" 12.9 9.1 31.8 15.9 40.1 15.6     "wb" 10.1 8.9 23.3 15.0 31.5 9.8
-    #   80 rows                                         "wb" 11.4 10.2 24.8 17.2 34.3 11.3
-    #   200 rows  "wb" 19.5 14.6 44.7 27.2 63.3 18.8    dense 31.4 26.5 104 61.1 131 32.7
+    #   16 rows   "wa" 8.5 6.5 20.6 10.9 25.6 10.4      "wb" 9.5 8.4 21.9 14.2 30.0 9.3
+    #   17 rows   "wa" 12.5 9.0 30.9 15.6 38.6 15.3     "wb" 9.8 8.7 22.3 14.6 30.1 9.4    (four columns of MMAs instead of two)
+    #   32 rows   "wa" 12.8 9.1 31.4 15.6 39.4 15.5     "wb" 10.0 8.9 22.6 15.0 30.5 9.7
+    #   80 rows                                         "wb" 11.4 10.3 25.0 17.5 33.7 11.4
+    #   200 rows  "wb" 19.8 14.7 44.4 27.5 63.1 18.9    dense 31.4 26.5 104 61.1 131 32.7
     # The line to the dense GEMM stays where the weights would be rounded once more than there.
     FEW_ROWS, DENSE_ROWS = 16, 256
     kernel = os.environ.get("COGITO_INT4_KERNEL", "auto")

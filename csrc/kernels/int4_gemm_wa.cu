@@ -5,8 +5,8 @@
 // With few rows in X the product is bound by the weight stream, and what stands between the stream and its bandwidth is the
 // way from nibbles to the tensor core.  A tcgen05 operand has to be written to shared or tensor memory, fenced, handed over by
 // an mbarrier and multiplied by one issuing thread: about 2200 cycles per 128 x 128 weights and SM for 16 rows, of which the
-// conversion is 150.  mma.sync takes the converted words from the registers they were converted in, at an eighth of the
-// tensor core's rate, which 16 rows need half of:
+// conversion is 150.  mma.sync takes the converted words from the registers they were converted in, at a third of
+// the rate, of which 16 rows would need three quarters if the bytes came at copy rate:
 //   * the weights are the A operand: m16 = 16 output features, n8 = 8 rows of X.  A warp owns all 128 features of a tile for 32 k
 //     at a time, so that X costs little beside the weights, and the warps of a CTA take the 32-k steps in turn: no warp waits for
 //     another inside a tile;
@@ -31,10 +31,11 @@
 // adds the bias, writes bf16 and leaves the counter zeroed.  Both orders are fixed, so a call gives the same bits every time.  Few
 // tiles are shared by clusters instead (see launch_wa).
 //
-// What bounds it (16 rows, per 128 x 32 weights, warp and scheduler): 36 MMAs of 8.7 cycles and about 160 two-cycle integer
-// instructions (a shift and a logic operation per pair of weights), which overlap to some 430 cycles, against 380 for the bytes at
-// HBM rate; then the start (1500 cycles to the first data) and the sums at a tile's end (2500).  16 rows, layers one after the
-// other, us: 4096 x 32000 44.6 before, 25.9 now (10.6 for the bytes); 4096 x 22016 34.7, 20.6; 1 row 20.2 and 16.0.
+// What bounds it (counters of one launch, 16 rows, 4096 x 32000): the two warps of a scheduler do their MMAs and their integer work nearly
+// in turn.  Of 43 500 cycles the tensor pipe is busy for 36 % and the integer pipe (a shift and a logic operation per pair of weights) for
+// 39 %; that is 286 and 308 cycles for each of a scheduler's 54 steps of 128 x 32 weights, which at copy rate would arrive every 390.
+// Of the warps' time, barriers (a tile's end) take 13 %, data that has not arrived 9 %.  16 rows, layers one after the other, us:
+// 4096 x 32000 42.9 through tcgen05, 25.6 like this (10.9 for the bytes); 4096 x 22016 34.0, 20.6; 1 row, 4096 x 32000 40.8, 19.8.
 #include <cuda_bf16.h>
 
 #include <atomic>
@@ -350,8 +351,9 @@ int clusters_at_once(int dev, int S, int* fit) {
 
 // Few tiles (at most one for every second SM) are shared by clusters: as many CTAs per tile as run at once, each with a unit per warp at least.
 // The parts meet over distributed shared memory, without the fence, the counter and the round trips of parts in global memory:
-// 16 rows, layers one after the other, 4096 x 4096 6.4 us by clusters of four and 9.9 by pieces, 4096 x 6144 8.3 (two) and 11.1,
-// 11008 x 4096 PLACE.  More tiles would leave SMs idle (4096 x 22016, 172 tiles: whole tiles 33, pieces PLACE).
+// 16 rows, layers one after the other, us by clusters / by pieces / by whole tiles: 4096 x 4096 (four CTAs) 6.5 / 9.9 / 11.9, 11008 x 4096
+// (four) 10.9 / 13.5 / 26.1, 4096 x 6144 (two) 8.5 / 11.1 / 11.8.  More tiles would leave SMs idle, whole ones too: 4096 x 22016 (172 tiles)
+// by pieces 20.6, whole 23.4.
 template <int NT>
 int launch_wa(WaDev g, dim3 grid, int dev, bool choose, cudaStream_t st) {
   CGK_CUDA_CHECK(cudaFuncSetAttribute(int4_wa_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, WaCfg<NT>::SMEM));

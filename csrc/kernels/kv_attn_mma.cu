@@ -15,9 +15,9 @@
 // memory, in the order of the ranks and warps.
 // Values are those of kv_attn_tc.cu: K and V as bf16(q * bf16(scale)), P rounded to bf16 before it is summed.
 //
-// 16 sequences of 641 tokens, 32 query and 8 kv heads, one new token: 11.1 us (24.7 + 2.7 for the kernel that combined the splits before);
-// five: 16.3 (37.4 + 5.2).  10.5 MB of cache are 1.6 us at HBM rate.  The rest is the chain lengths -> page -> keys at the start (3 us),
-// three blocks of some 1.5 us per warp (conversion and MMAs of two warps per scheduler), and the merge (1 us).
+// 16 sequences of 640 tokens, 32 query and 8 kv heads, one new token: 10.4 us (29.2 by tcgen05 with combined splits); five: 15.8 (42.3).
+// 13 MB of cache are 2 us at copy rate.  A round of a CTA's eight blocks takes 2.1 us for one row tile and 3.1 for two (conversion and
+// MMAs of two warps per scheduler); the chain lengths -> page -> keys at the start and the merge are the rest.
 // Long histories of few heads are shared by up to 16 CTAs, if that many clusters run at once.  One sequence of 32 000 tokens, 8 kv heads:
 // 40.8 us (by four CTAs 70.8, tcgen05 with combined splits 66.4), five tokens 64.4 (110; 87.9); one kv head 25.4 (68.5; 35.8), five
 // tokens 38.9 (106; 44.7).

@@ -358,7 +358,7 @@ constexpr int SAMPLE_SHORT_K = 512;
 // wanted values, or a row whose large values lie with few threads (over 1024 reach the bound): 32 counting rounds over the quotients
 // of all logits.  80 rows of 32 000 fp32 logits, top-k 50,
 // top-p 0.9: 55.3 us with 32 counting rounds of three barriers, serial sums and the zeros written last; 26.6 us with bounds by
-// maxima; 15.6 us with 16-byte loads, no divisions, ranks instead of a sort and one chain of sums instead of two.
+// maxima; 16.4 us with 16-byte loads, no divisions, ranks instead of a sort and one chain of sums instead of two.
 // FOURS: fours of neighbours per thread (rows that allow 16-byte loads), else single logits.  QUOTIENTS: every logit is divided as it is read
 // (more wanted values than are bounded by maxima; infinite temperatures, whose quotient of infinities ends on top).
 template <bool FOURS, bool QUOTIENTS>
