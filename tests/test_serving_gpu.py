@@ -739,7 +739,7 @@ def test_speculative_decoding_over_prompts_of_other_lengths():
     _lib.assert_device_ok()
 
 
-# a captured attention call keeps its scratch although a later call needs more
+# a captured attention call gives the same after a later one that needs more (few rows: no scratch to keep)
 def test_kv_attention_captured_before_a_larger_call():
     torch.manual_seed(5)
     B, Hk, Hq, D = 2, 2, 8, 128
@@ -762,7 +762,7 @@ def test_kv_attention_captured_before_a_larger_call():
     _lib.assert_device_ok()
 
 
-# the same with more than 32 rows per kv head, whose kernel is the one with scratch
+# more than 32 rows per kv head: a captured call keeps its scratch although a later call needs more
 def test_kv_attention_of_more_rows_captured_before_a_larger_call():
     torch.manual_seed(6)
     B, Hk, Hq, D = 2, 2, 8, 128
